@@ -205,6 +205,7 @@ Rib200Status rib200_gated_delta(const void *input, const void *conv_weight, cons
     layer.output_norm_weight = output_norm_weight;
     layer.output = output;
     layer.convolution_state = convolution_state;
+    layer.recurrent_state = recurrent_state;
     layer.convolved = floats;
     float *raw = floats + c.convolved_floats;
     layer.raw = raw;
@@ -217,6 +218,10 @@ Rib200Status rib200_gated_delta(const void *input, const void *conv_weight, cons
     layer.epsilon = s.epsilon;
     layer.dtype = dtype;
     layer.weight_dtype = weight_dtype;
+    if (gdn_layer_step_applies(layer)) {
+      launch_gdn_layer_step(layer, cuda_stream);
+      return;
+    }
     launch_gdn_prologue(layer, cuda_stream);
 
     GdnCoreArgs core{};

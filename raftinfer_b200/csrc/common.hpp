@@ -110,19 +110,29 @@ void encode_plain_rows_map(void *map_out, const void *base, bool f32, std::uint6
 // must execute griddepcontrol.wait before it touches anything an earlier kernel of the stream writes or reads.
 #ifdef __CUDACC__
 template <typename... Params, typename... Args>
-inline void launch_programmatic(void (*kernel)(Params...), dim3 grid, dim3 block, std::size_t shared_bytes,
-                                cudaStream_t stream, const char *what, Args &&...args) {
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
+inline void launch_programmatic_cluster(void (*kernel)(Params...), dim3 grid, dim3 block, unsigned int cluster_x,
+                                        std::size_t shared_bytes, cudaStream_t stream, const char *what,
+                                        Args &&...args) {
+  cudaLaunchAttribute attributes[2] = {};
+  attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[0].val.programmaticStreamSerializationAllowed = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = cluster_x;
+  attributes[1].val.clusterDim.y = 1;
+  attributes[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
   config.dynamicSmemBytes = shared_bytes;
   config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
+  config.attrs = attributes;
+  config.numAttrs = cluster_x > 1 ? 2 : 1;
   cuda_ok(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...), what);
+}
+template <typename... Params, typename... Args>
+inline void launch_programmatic(void (*kernel)(Params...), dim3 grid, dim3 block, std::size_t shared_bytes,
+                                cudaStream_t stream, const char *what, Args &&...args) {
+  launch_programmatic_cluster(kernel, grid, block, 1, shared_bytes, stream, what, static_cast<Args &&>(args)...);
 }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_dependents_may_launch() {
@@ -206,6 +216,7 @@ struct GdnLayerArgs {
   const void *conv_weight, *recurrent_a, *dt_bias, *output_norm_weight;
   void *output;      // [tokens][hidden], dtype
   float *convolution_state;
+  float *recurrent_state; // [value_heads][128][128]
   float *convolved;  // [tokens][conv_dim] fp32: q (normalised, scaled), k (normalised), v
   float *beta;       // [tokens][value_heads]
   float *log_decay;  // [tokens][value_heads]
@@ -215,6 +226,9 @@ struct GdnLayerArgs {
   int32_t dtype, weight_dtype;
 };
 void launch_gdn_prologue(const GdnLayerArgs &args, cudaStream_t stream);
+// The whole layer call of one token as one launch, where that form applies (see gdn_layer.cu).
+bool gdn_layer_step_applies(const GdnLayerArgs &args);
+void launch_gdn_layer_step(const GdnLayerArgs &args, cudaStream_t stream);
 void launch_gdn_epilogue(const GdnLayerArgs &args, cudaStream_t stream);
 
 } // namespace rib200

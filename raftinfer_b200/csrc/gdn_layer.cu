@@ -71,6 +71,7 @@ struct LayerParams {
   const void *conv_weight, *recurrent_a, *dt_bias, *output_norm_weight;
   void *output;
   float *convolution_state;
+  float *recurrent_state; // single-token form only
   float *convolved;
   float *beta;
   float *log_decay;
@@ -385,6 +386,251 @@ __global__ void __launch_bounds__(kDim) gdn_epilogue_kernel(const LayerParams p)
   store_any(p.output, index, p.dtype, normalised * silu(z));
 }
 
+// ---- one token in one launch ---------------------------------------------------------------------------
+// A decode step of the layer is latency: 4 MiB of state traffic (0.6 us of HBM) and 25 KB of input.  The four launches
+// of the general path (prologue, history, recurrence, epilogue) cost 12.0 us a layer in a captured chain of 24 layers,
+// most of it hand-over between grids; this form costs 4.8 us (4.2 MB of state in and out: 0.88 TB/s, latency-bound).
+//
+// A cluster serves one key head: four CTAs (32 state columns each) per value head that shares it, one or two value
+// heads.  Everything that has to meet across CTAs meets inside that cluster: the convolution history of the q and k
+// channels is read by all of its CTAs and rewritten by one, and the output norm needs the squares of all four column
+// slices; one cluster barrier covers both (the history is only written behind it).  Three value heads and more to a
+// key head would need more than the portable eight CTAs and take the general path, as other convolution widths do.
+// 128 CTAs of 16 KiB of state each at the model's head counts: a thread's 64 bytes are one round of loads.
+template <int Dtype> struct Scalar;
+template <> struct Scalar<RIB200_DTYPE_F32> {
+  using Type = float;
+  static __device__ __forceinline__ float widen(float x) { return x; }
+  static __device__ __forceinline__ float narrow(float x) { return x; }
+};
+template <> struct Scalar<RIB200_DTYPE_F16> {
+  using Type = __half;
+  static __device__ __forceinline__ float widen(__half x) { return __half2float(x); }
+  static __device__ __forceinline__ __half narrow(float x) { return __float2half_rn(x); }
+};
+template <> struct Scalar<RIB200_DTYPE_BF16> {
+  using Type = __nv_bfloat16;
+  static __device__ __forceinline__ float widen(__nv_bfloat16 x) { return __bfloat162float(x); }
+  static __device__ __forceinline__ __nv_bfloat16 narrow(float x) { return __float2bfloat16_rn(x); }
+};
+
+constexpr int kStepThreads = 256;
+constexpr int kStepSlices = 4;
+constexpr int kStepColumns = kDim / kStepSlices;
+constexpr std::uint32_t kStepMaxRatio = 2; // value heads per key head a portable cluster holds
+
+template <int Dtype, int WeightDtype>
+__global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const LayerParams p) {
+  using Act = Scalar<Dtype>;
+  using Weight = Scalar<WeightDtype>;
+  __shared__ float s_q[kDim];
+  __shared__ float s_k[kDim];
+  __shared__ float s_squares[8];
+  __shared__ float s_gates[2]; // beta, decay
+  __shared__ __align__(16) float s_a[8][kStepColumns];
+  __shared__ __align__(16) float s_b[8][kStepColumns];
+  __shared__ float s_dot[8];
+  __shared__ __align__(16) float s_delta[kStepColumns];
+  __shared__ float s_norm[kStepSlices]; // written by the CTAs of the value head, this one included
+  std::uint32_t rank;
+  std::uint32_t cluster_size;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(cluster_size));
+  const std::uint32_t key_head = blockIdx.x / cluster_size;
+  const std::uint32_t head = key_head + (rank / kStepSlices) * p.key_heads;
+  const std::uint32_t slice = rank % kStepSlices;
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+  float *state = p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns;
+  // The state slice is asked into L2 while the kernel in front of this one still runs; a prefetch is only a hint, the
+  // values are read after the wait.
+  if (tid < kDim) {
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(state + static_cast<std::size_t>(tid) * kDim));
+  }
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
+  grid_dependents_may_launch();
+  grid_dependency_wait();
+
+  // ---- every load of the step in one round ----
+  const int row0 = 16 * warp + (lane >> 3);
+  const int col = 4 * (lane & 7);
+  float4 s[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    s[i] = *reinterpret_cast<const float4 *>(state + static_cast<std::size_t>(row0 + 4 * i) * kDim + col);
+  }
+  const auto *input = static_cast<const typename Act::Type *>(p.input);
+  const auto *conv_weight = static_cast<const typename Weight::Type *>(p.conv_weight);
+  constexpr int kHistory = kFastWidth - 1;
+  struct Channel {
+    typename Act::Type x;
+    typename Weight::Type w[kFastWidth];
+    float history[kHistory];
+  };
+  auto load_channel = [&](std::uint32_t channel, Channel &c) {
+    c.x = input[channel];
+#pragma unroll
+    for (int h = 0; h < kFastWidth; ++h) {
+      c.w[h] = conv_weight[static_cast<std::size_t>(channel) * kFastWidth + h];
+    }
+#pragma unroll
+    for (int h = 0; h < kHistory; ++h) {
+      c.history[h] = p.convolution_state[static_cast<std::size_t>(channel) * kHistory + h];
+    }
+  };
+  auto convolve = [&](const Channel &c) { // the current token's tap first, then the history, oldest first
+    float sum = Act::widen(c.x) * Weight::widen(c.w[kHistory]);
+#pragma unroll
+    for (int h = 0; h < kHistory; ++h) {
+      sum += c.history[h] * Weight::widen(c.w[h]);
+    }
+    return silu(sum);
+  };
+  auto shift_history = [&](std::uint32_t channel, const Channel &c) {
+    float *history = p.convolution_state + static_cast<std::size_t>(channel) * kHistory;
+    history[0] = c.history[1];
+    history[1] = c.history[2];
+    history[2] = Act::widen(c.x);
+  };
+  // threads 0..127: the q channels of the key head, 128..255: its k channels; warp 0 also the slice's v channels
+  const std::uint32_t qk_channel = (tid < kDim ? 0 : p.key_heads * kDim) + key_head * kDim + (tid & (kDim - 1));
+  const std::uint32_t v_channel = 2 * p.key_heads * kDim + head * kDim + slice * kStepColumns + lane;
+  Channel qk;
+  Channel v;
+  typename Act::Type z{};
+  typename Act::Type b{};
+  typename Act::Type a{};
+  typename Weight::Type coefficient{};
+  typename Weight::Type dt{};
+  typename Weight::Type norm_weight{};
+  load_channel(qk_channel, qk);
+  if (warp == 0) {
+    load_channel(v_channel, v);
+    z = input[p.conv_dim + 2 * p.value_heads + head * kDim + slice * kStepColumns + lane];
+    norm_weight = static_cast<const typename Weight::Type *>(p.output_norm_weight)[slice * kStepColumns + lane];
+    b = input[p.conv_dim + head];
+    a = input[p.conv_dim + p.value_heads + head];
+    coefficient = static_cast<const typename Weight::Type *>(p.recurrent_a)[head];
+    dt = static_cast<const typename Weight::Type *>(p.dt_bias)[head];
+  }
+
+  // ---- q, k: convolution, SiLU, sum of squares ----
+  const float qk_value = convolve(qk);
+  float squares = qk_value * qk_value;
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1) {
+    squares += __shfl_xor_sync(0xFFFFFFFFU, squares, offset);
+  }
+  (tid < kDim ? s_q : s_k)[tid & (kDim - 1)] = qk_value;
+  float v_value = 0.0F;
+  float z_gate = 0.0F;
+  if (warp == 0) {
+    v_value = convolve(v);
+    z_gate = Weight::widen(norm_weight) * silu(Act::widen(z));
+    if (lane == 0) {
+      s_gates[0] = 1.0F / (1.0F + expf(-Act::widen(b)));
+      s_gates[1] = expf(Weight::widen(coefficient) * softplus(Act::widen(a) + Weight::widen(dt)));
+    }
+  }
+  if (lane == 0) {
+    s_squares[warp] = squares;
+  }
+  asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+  __syncthreads();
+  const float q_scale = rsqrtf((s_squares[0] + s_squares[1]) + (s_squares[2] + s_squares[3]) + kQkEpsilon) *
+                        rsqrtf(static_cast<float>(kDim));
+  const float k_scale = rsqrtf((s_squares[4] + s_squares[5]) + (s_squares[6] + s_squares[7]) + kQkEpsilon);
+  const float beta = s_gates[0];
+  const float decay = s_gates[1];
+
+  // ---- S^T k and S^T q of the slice, k . q ----
+  float k_row[4];
+  float sums[9] = {};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float k = s_k[row0 + 4 * i] * k_scale;
+    const float q = s_q[row0 + 4 * i] * q_scale;
+    k_row[i] = k;
+    sums[0] += s[i].x * k;
+    sums[1] += s[i].y * k;
+    sums[2] += s[i].z * k;
+    sums[3] += s[i].w * k;
+    sums[4] += s[i].x * q;
+    sums[5] += s[i].y * q;
+    sums[6] += s[i].z * q;
+    sums[7] += s[i].w * q;
+    sums[8] += k * q;
+  }
+#pragma unroll
+  for (int offset = 16; offset >= 8; offset >>= 1) { // the four row groups of the warp
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+      sums[c] += __shfl_xor_sync(0xFFFFFFFFU, sums[c], offset);
+    }
+  }
+  if (lane < 8) {
+    *reinterpret_cast<float4 *>(&s_a[warp][col]) = make_float4(sums[0], sums[1], sums[2], sums[3]);
+    *reinterpret_cast<float4 *>(&s_b[warp][col]) = make_float4(sums[4], sums[5], sums[6], sums[7]);
+    if (lane == 0) {
+      s_dot[warp] = sums[8];
+    }
+  }
+  __syncthreads();
+  float read = 0.0F; // the slice's output vector before the norm: one column per lane of warp 0
+  if (warp == 0) {
+    float a_sum = 0.0F;
+    float b_sum = 0.0F;
+    float dot = 0.0F;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      a_sum += s_a[w][lane];
+      b_sum += s_b[w][lane];
+      dot += s_dot[w];
+    }
+    const float delta = (v_value - decay * a_sum) * beta;
+    s_delta[lane] = delta;
+    read = decay * b_sum + delta * dot;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float norm = read * read;
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+      norm += __shfl_xor_sync(0xFFFFFFFFU, norm, offset);
+    }
+    if (lane < kStepSlices) { // to the four CTAs of this value head
+      std::uint32_t remote;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                   : "=r"(remote)
+                   : "r"(static_cast<std::uint32_t>(__cvta_generic_to_shared(&s_norm[slice]))),
+                     "r"(rank - slice + lane));
+      asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote), "f"(norm) : "memory");
+    }
+    __syncwarp();
+  }
+  // The barrier orders the partial norms and marks the end of everybody's reads of the history.
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  const float4 delta = *reinterpret_cast<const float4 *>(&s_delta[col]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    *reinterpret_cast<float4 *>(state + static_cast<std::size_t>(row0 + 4 * i) * kDim + col) =
+        make_float4(decay * s[i].x + k_row[i] * delta.x, decay * s[i].y + k_row[i] * delta.y,
+                    decay * s[i].z + k_row[i] * delta.z, decay * s[i].w + k_row[i] * delta.w);
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (rank == 0) {
+    shift_history(qk_channel, qk);
+  }
+  if (warp == 0) {
+    shift_history(v_channel, v);
+    const float norm = (s_norm[0] + s_norm[1]) + (s_norm[2] + s_norm[3]);
+    const float scale = rsqrtf(norm / static_cast<float>(kDim) + p.epsilon);
+    static_cast<typename Act::Type *>(p.output)[head * kDim + slice * kStepColumns + lane] =
+        Act::narrow(read * scale * z_gate);
+  }
+}
+
 LayerParams make_params(const GdnLayerArgs &a) {
   LayerParams p{};
   p.input = a.input;
@@ -394,6 +640,7 @@ LayerParams make_params(const GdnLayerArgs &a) {
   p.output_norm_weight = a.output_norm_weight;
   p.output = a.output;
   p.convolution_state = a.convolution_state;
+  p.recurrent_state = a.recurrent_state;
   p.convolved = a.convolved;
   p.beta = a.beta;
   p.log_decay = a.log_decay;
@@ -410,7 +657,43 @@ LayerParams make_params(const GdnLayerArgs &a) {
   return p;
 }
 
+template <int Dtype, int WeightDtype> void launch_step(const LayerParams &p, cudaStream_t stream) {
+  const std::uint32_t cluster = kStepSlices * (p.value_heads / p.key_heads);
+  launch_programmatic_cluster(gdn_layer_step_kernel<Dtype, WeightDtype>, dim3(cluster * p.key_heads),
+                              dim3(kStepThreads), cluster, 0, stream, "gated-delta step launch", p);
+}
+
 } // namespace
+
+bool gdn_layer_step_applies(const GdnLayerArgs &a) {
+  return a.tokens == 1 && a.conv_width == kFastWidth && a.value_heads / a.key_heads <= kStepMaxRatio;
+}
+
+void launch_gdn_layer_step(const GdnLayerArgs &a, cudaStream_t stream) {
+  const LayerParams p = make_params(a);
+  constexpr int kF32 = RIB200_DTYPE_F32;
+  constexpr int kF16 = RIB200_DTYPE_F16;
+  constexpr int kBf16 = RIB200_DTYPE_BF16;
+  if (a.dtype == kF32) {
+    if (a.weight_dtype == kF32) {
+      launch_step<kF32, kF32>(p, stream);
+    } else if (a.weight_dtype == kF16) {
+      launch_step<kF32, kF16>(p, stream);
+    } else {
+      launch_step<kF32, kBf16>(p, stream);
+    }
+  } else if (a.dtype == kF16) {
+    if (a.weight_dtype == kF32) {
+      launch_step<kF16, kF32>(p, stream);
+    } else {
+      launch_step<kF16, kF16>(p, stream);
+    }
+  } else if (a.weight_dtype == kF32) {
+    launch_step<kBf16, kF32>(p, stream);
+  } else {
+    launch_step<kBf16, kBf16>(p, stream);
+  }
+}
 
 void launch_gdn_prologue(const GdnLayerArgs &a, cudaStream_t stream) {
   const LayerParams p = make_params(a);

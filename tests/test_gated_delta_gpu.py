@@ -269,6 +269,19 @@ def test_layer_chunked_prefill_then_decode(dtype):
         run.check(out, want, chunked=True)
 
 
+@pytest.mark.parametrize("hk,hv", [(1, 1), (2, 4), (1, 3), (HK, HV)])
+@pytest.mark.parametrize("dtype,wdtype", [(K.DTYPE_BF16, K.DTYPE_F32), (K.DTYPE_F32, K.DTYPE_F32),
+                                          (K.DTYPE_BF16, K.DTYPE_BF16), (K.DTYPE_F32, K.DTYPE_BF16)])
+def test_layer_single_tokens(hk, hv, dtype, wdtype):
+    """One-token calls back to back on the same states: one launch where a key head has one or two value heads (one
+    cluster each), the general path for three.  FP32 activations are held to the recurrence's FP32 tolerance."""
+    run = LayerRun(0xB2002700 + 8 * hk + hv, hk, hv, 4, dtype, wdtype, 3)
+    for _ in range(3):
+        out, want, _ = run.step(1)
+        run.check(out, want)
+    assert K.device_status(torch.cuda.current_stream()) == 0
+
+
 def test_layer_three_launches_share_device_state_without_a_sync():
     run = LayerRun(0xB2002200, 2, 4, 4, K.DTYPE_F32, K.DTYPE_F32, 6)
     results = [run.step(2, sync=False) for _ in range(3)]
