@@ -196,7 +196,9 @@ Rib200Status rib200_gated_delta(const void *input, const void *conv_weight, cons
     require_aligned(recurrent_state, 16, "gated-delta: recurrent state is not 16-byte aligned");
 
     auto *cuda_stream = static_cast<cudaStream_t>(stream);
-    auto *floats = static_cast<float *>(workspace);
+    // scratch of the chunked kernels first (whole 16-byte pieces), then the FP32 arrays of the general path
+    void *chunk_scratch = workspace;
+    auto *floats = reinterpret_cast<float *>(static_cast<unsigned char *>(workspace) + c.chunk_bytes);
     GdnLayerArgs layer{};
     layer.input = input;
     layer.conv_weight = conv_weight;
@@ -222,6 +224,10 @@ Rib200Status rib200_gated_delta(const void *input, const void *conv_weight, cons
       launch_gdn_layer_step(layer, cuda_stream);
       return;
     }
+    if (layer.tokens >= kChunkThreshold && gdn_layer_chunks_apply(layer)) {
+      launch_gdn_layer_chunks(layer, chunk_scratch, cuda_stream);
+      return;
+    }
     launch_gdn_prologue(layer, cuda_stream);
 
     GdnCoreArgs core{};
@@ -238,7 +244,6 @@ Rib200Status rib200_gated_delta(const void *input, const void *conv_weight, cons
     core.sequences = 1;
     core.key_heads = layer.key_heads;
     core.value_heads = layer.value_heads;
-    void *chunk_scratch = layer.log_decay + c.gate_floats / 2;
     run_core(core, chunk_scratch, cuda_stream);
     launch_gdn_epilogue(layer, cuda_stream);
   });

@@ -89,22 +89,6 @@ struct DecodeArgs {
   bool activations_f32;
   bool early_kv_fetch; // host position only: the cache rows are fetched before the dependent-launch wait
 };
-// 128-byte opaque image of a driver tensor map (TMA descriptor); 64-byte aligned as the driver's type is.
-struct alignas(64) TensorMapBytes {
-  unsigned char bytes[128];
-};
-// Tiled map over a row-major FP32 matrix [rows][row_floats], box [box_rows][box_floats], 128-byte swizzle
-// (box_floats * 4 must be 128).  Defined next to the other tensor-map code in prefill_attention.cu.
-void encode_f32_rows_map(void *map_out, void *base, std::uint64_t row_floats, std::uint64_t rows,
-                         std::uint32_t box_floats, std::uint32_t box_rows);
-
-// Tiled map without swizzle over rows of FP32 or BF16 elements: `rows` rows of `row_elements` elements that lie
-// `row_stride_elements` apart (a head range inside wider token rows); box [box_rows][box_elements]; rows past the
-// last one arrive as zeros.  Base and row stride must be multiples of 16 bytes.
-void encode_plain_rows_map(void *map_out, const void *base, bool f32, std::uint64_t row_elements,
-                           std::uint64_t row_stride_elements, std::uint64_t rows, std::uint32_t box_elements,
-                           std::uint32_t box_rows);
-
 // Launch with programmatic stream serialisation: the grid may become resident while the kernel in front of it on the
 // stream is still running (once that one has executed griddepcontrol.launch_dependents in every CTA, or ended), and
 // must execute griddepcontrol.wait before it touches anything an earlier kernel of the stream writes or reads.
@@ -208,6 +192,7 @@ void launch_gdn_recurrent(const GdnCoreArgs &args, cudaStream_t stream);
 // Chunk-64 WY-form prefill (single sequence); scratch sized by gdn_chunk_workspace_bytes.
 std::size_t gdn_chunk_workspace_bytes(std::size_t tokens, std::size_t key_heads, std::size_t value_heads);
 void launch_gdn_chunked(const GdnCoreArgs &args, void *workspace, cudaStream_t stream);
+void launch_gdn_core_images(const GdnCoreArgs &args, void *workspace, cudaStream_t stream); // its first kernel
 
 // Steps either side of the recurrence inside qwen35_gated_delta (cpp/kernels/qwen35_delta.cu:236-276,
 // 375-411,579-621).
@@ -227,6 +212,11 @@ struct GdnLayerArgs {
 };
 void launch_gdn_prologue(const GdnLayerArgs &args, cudaStream_t stream);
 // The whole layer call of one token as one launch, where that form applies (see gdn_layer.cu).
+// The whole layer call of 64 tokens or more in the chunked kernels (convolution width 4, aligned tensors), and its
+// first kernel; scratch as for launch_gdn_chunked.
+bool gdn_layer_chunks_apply(const GdnLayerArgs &args);
+void launch_gdn_layer_chunks(const GdnLayerArgs &args, void *workspace, cudaStream_t stream);
+void launch_gdn_layer_images(const GdnLayerArgs &args, void *workspace, cudaStream_t stream);
 bool gdn_layer_step_applies(const GdnLayerArgs &args);
 void launch_gdn_layer_step(const GdnLayerArgs &args, cudaStream_t stream);
 void launch_gdn_epilogue(const GdnLayerArgs &args, cudaStream_t stream);
