@@ -784,15 +784,17 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 }
 
 // ---- chain: per (state slice, value head), chunks in order -------------------------------------------------
-// 256 threads.  Warps 0-3 own the 128 lanes of tensor memory and the state (thread = row of every product), warps 4-5
-// make the outputs, warp 6 issues the products, lane 0 of warp 7 streams the operand images of each chunk into a
+// 320 threads.  Warps 0-3 own the 128 lanes of tensor memory and the state (thread = row of every product), warps 4-5
+// make the outputs of the even chunks and warps 8-9 those of the odd ones (a chunk's outputs cost a pair of warps about
+// 3000 cycles, the chain itself 2100 a chunk: with one pair every first product waited for the outputs two chunks back;
+// 4096 tokens 224.2 -> 197.4 us, a chunk 3100 -> 2500 cycles), warp 6 issues the products, lane 0 of warp 7 streams the operand images of each chunk into a
 // three-stage ring, asking for them in L2 some chunks earlier (the records of a long call do not all stay there).  Per chunk:
 //   X  = [Q; W] S0            M 128 (rows 0..63 Q S0, rows 64..127 W S0), N 32, K 128
 //   warps 2-3: Delta = U - X[64..] -> diag(e) Delta and Delta as B operands
 //   SD = K^T (diag(e) Delta)  M 128, N 32, K 64 (K as stored: MN-major A operand)
 //   O2 = P Delta              M 128 (rows 64..127 are don't-care), N 32, K 64
 //   warps 0-3: S = gamma_C S + SD (FP32 registers) -> B operand: the next chunk's first product waits for this
-//   warps 4-5: O = gamma_i (Q S0)_i + O2; in a layer call the four slices of a head are a cluster, exchange the sums of
+//   warps 4-5, 8-9: O = gamma_i (Q S0)_i + O2; in a layer call the four slices of a head are a cluster, exchange the sums of
 //   squares of every token and write norm(O) * weight * SiLU(z)
 // The chain X -> Delta -> SD -> S is latency: nothing but that chain runs in warps 0-3, everything they need from memory
 // is in registers before they wait, and a row of a B operand (32 columns, 64 bytes) is four 16-byte stores because the
@@ -806,7 +808,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 // FP16's normal range differently on either side of a cut).
 // Every mbarrier wait is bounded; when one runs out the CTA records RIB200_DEVICE_WAIT_TIMED_OUT, stops waiting and
 // copying, and runs to its end.
-constexpr int kChainThreads = 256;
+constexpr int kChainThreads = 320;
 constexpr std::uint32_t kStages = 3;
 constexpr std::uint32_t kPrefetchAhead = 3; // chunks between the L2 prefetch and the copy that uses it
 constexpr std::uint32_t kStageQw = 0;                              // [2 blocks][rows 0..63 Q, 64..127 W][128 bytes]
@@ -819,8 +821,11 @@ constexpr std::uint32_t kOperandRow = kSlice * 2;                  // bytes of a
 constexpr std::uint32_t kCsState = kStages * kStageBytes;               // S, 128 rows
 constexpr std::uint32_t kCsEDelta = kCsState + kDim * kOperandRow; // diag(e) Delta, 64 rows
 constexpr std::uint32_t kCsDelta = kCsEDelta + kChunk * kOperandRow;
-constexpr std::uint32_t kCsNorm = kCsDelta + kChunk * kOperandRow; // [2 parities][4 slices][64 tokens]
-constexpr std::uint32_t kCsWeight = kCsNorm + 2 * kGdnSlices * kChunk * 4;
+// [chunk & 3][4 slices][64 tokens]: a peer sends the sums of chunk c + 4 only after this CTA's sums of c + 2, which
+// leave after its threads have read those of c (even and odd chunks have warps of their own, two slots would not do)
+constexpr std::uint32_t kCsNorm = kCsDelta + kChunk * kOperandRow;
+constexpr std::uint32_t kNormSlots = 4;
+constexpr std::uint32_t kCsWeight = kCsNorm + kNormSlots * kGdnSlices * kChunk * 4;
 constexpr std::uint32_t kCsMax = kCsWeight + kSlice * 4;           // [2 parities][4 warps]
 constexpr std::uint32_t kCsScale = kCsMax + 32;                    // [2 parities]{1 / scale of S0, 1 / scale of Delta}
 constexpr std::uint32_t kCsBars = kCsScale + 16;
@@ -832,8 +837,8 @@ enum : std::uint32_t {
   kBarXDone = kBarUsed + kStages,      // [2] by parity of the chunk, as the outputs may lag the chain by more than a chunk
   kBarO2Done = kBarXDone + 2,          // [2]
   kBarOutRead = kBarO2Done + 2,        // [2] X (rows 0..63), O2 and the scales of a chunk have been read (64 threads)
-  kBarNorm = kBarOutRead + 2,          // [2] the four slices' sums of squares
-  kBarEDelta = kBarNorm + 2,           // diag(e) Delta is in shared memory (64 writers)
+  kBarNorm = kBarOutRead + 2,          // [chunk & 3] the four slices' sums of squares
+  kBarEDelta = kBarNorm + kNormSlots,          // diag(e) Delta is in shared memory (64 writers)
   kBarDelta,                           // Delta is in shared memory (64 writers)
   kBarSdDone,
   kBarState,                           // S is in shared memory, X and SD have been read (128 threads)
@@ -1287,7 +1292,8 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
           make_float4(s_reg[c], s_reg[c + 1], s_reg[c + 2], s_reg[c + 3]);
     }
   } else {
-    // ---- warps 4-5: the outputs, thread = token of the chunk ----
+    // ---- warps 4-5 and 8-9: the outputs of the even and of the odd chunks, thread = token of the chunk ----
+    const std::uint32_t parity = warp >> 3;
     const std::uint32_t token = threadIdx.x & 63U;
     const std::uint32_t lane_base = ((warp & 3U) * 32U) << 16;
     const std::size_t column = static_cast<std::size_t>(head) * kDim + slice * kSlice;
@@ -1299,7 +1305,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
         reinterpret_cast<float *>(smem + kCsWeight)[threadIdx.x - 128] =
             load_any(p.norm_weight, slice * kSlice + threadIdx.x - 128, p.weight_dtype);
       }
-      asm volatile("bar.sync 2, 64;\n" ::: "memory");
+      asm volatile("bar.sync 2, 128;\n" ::: "memory");
 #pragma unroll
       for (std::uint32_t r = 0; r < kGdnSlices; ++r) {
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
@@ -1309,9 +1315,13 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
       }
     }
     RingPlace at;
-    for (std::uint32_t chunk = 0; chunk < p.chunks; ++chunk, at.next()) {
+    if (parity != 0) {
+      at.next();
+    }
+    for (std::uint32_t chunk = parity; chunk < p.chunks; chunk += 2, at.next(), at.next()) {
       const std::uint32_t s = chunk & 1U;
       const std::uint32_t stage = base + at.stage * kStageBytes;
+      [[maybe_unused]] const std::uint32_t norm_slot = chunk & (kNormSlots - 1);
       const std::uint32_t tok = chunk * kChunk + token;
       const bool live = tok < p.tokens;
       RowPart<kLayer ? Dtype : RIB200_DTYPE_F32> z{};
@@ -1319,9 +1329,9 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
         if (live) {
           z.load(p.input, static_cast<std::size_t>(tok) * p.token_stride + p.z_column + column);
         }
-        if (threadIdx.x == 128) {
+        if (token == 0) {
           RIB200_GDN_STAMP(chunk, 9);
-          mbarrier_expect_tx(bar(kBarNorm + s), kGdnSlices * kChunk * 4);
+          mbarrier_expect_tx(bar(kBarNorm + norm_slot), kGdnSlices * kChunk * 4);
         }
       }
       wait(bar(kBarRestFull + at.stage), at.phase);
@@ -1329,7 +1339,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
       mbarrier_arrive(bar(kBarRead + at.stage));
       wait(bar(kBarXDone + s), (chunk >> 1) & 1U);
       tcgen05_fence_after();
-      if (threadIdx.x == 128) {
+      if (token == 0) {
         RIB200_GDN_STAMP(chunk, 10);
       }
       float o[kSlice];
@@ -1357,8 +1367,8 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
 #pragma unroll
         for (std::uint32_t r = 0; r < kGdnSlices; ++r) {
           asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(
-                           norm_target[r] + s * (kGdnSlices * kChunk * 4)),
-                       "r"(__float_as_uint(squares)), "r"(norm_bar[r] + s * 8)
+                           norm_target[r] + norm_slot * (kGdnSlices * kChunk * 4)),
+                       "r"(__float_as_uint(squares)), "r"(norm_bar[r] + norm_slot * 8)
                        : "memory");
         }
         const std::uint32_t weights = base + kCsWeight;
@@ -1371,14 +1381,14 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
           o[4 * c + 2] *= w.z * silu_fast(gate.z);
           o[4 * c + 3] *= w.w * silu_fast(gate.w);
         }
-        if (threadIdx.x == 128) {
+        if (token == 0) {
           RIB200_GDN_STAMP(chunk, 11);
         }
-        wait(bar(kBarNorm + s), (chunk >> 1) & 1U);
-        if (threadIdx.x == 128) {
+        wait(bar(kBarNorm + norm_slot), (chunk >> 2) & 1U);
+        if (token == 0) {
           RIB200_GDN_STAMP(chunk, 12);
         }
-        const std::uint32_t norms = base + kCsNorm + s * (kGdnSlices * kChunk * 4) + token * 4;
+        const std::uint32_t norms = base + kCsNorm + norm_slot * (kGdnSlices * kChunk * 4) + token * 4;
         const float sum = (lds32(norms) + lds32(norms + kChunk * 4)) + (lds32(norms + 2 * kChunk * 4) + lds32(norms + 3 * kChunk * 4));
         const float scale = rsqrtf(sum / static_cast<float>(kDim) + p.epsilon);
 #pragma unroll
