@@ -155,6 +155,7 @@ struct PrefillParams {
   std::uint32_t query_heads;
   std::uint32_t group; // query heads per KV head
   std::uint32_t split_min_blocks; // split form: items with fewer key blocks are left to the first CTA (or pair) alone
+  std::uint32_t wait_first;       // no append kernel: the kernel in front made the operands, wait before the first read
   unsigned int *status;
 };
 
@@ -478,7 +479,10 @@ __global__ void __launch_bounds__(256) prefill_append_kernel(const void *key, co
                                                              void *q_parking, std::uint32_t q_tokens,
                                                              std::uint32_t q_heads, std::uint32_t out_heads,
                                                              std::uint32_t out_head_offset) {
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  // The attention kernel is let in only when the kernels in front of this one have ended: it reads queries and gates
+  // that they made before it waits for this kernel.
+  grid_dependency_wait();
+  grid_dependents_may_launch();
   // one thread per 8 elements: [plane][token][kv head][32 pieces of 8]
   const std::size_t pieces = static_cast<std::size_t>(tokens) * kv_heads * 32;
   const std::size_t id = static_cast<std::size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -626,6 +630,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if constexpr (kCluster) {
     cluster_sync_all(); // the partner's barriers exist before anything arrives on them
+  }
+  if (p.wait_first != 0) {
+    grid_dependency_wait();
   }
   // From here the producer warp starts its first loads; the other warps take the SM's tensor memory meanwhile
   // (the allocation takes about as long as those loads) and meet on a barrier of their own before they use it.
@@ -1555,10 +1562,10 @@ template <bool F32, bool Pair, bool Split> void launch(const PrefillArgs &a, cud
   if (append_rows > 0) {
     const std::size_t kv_pieces = static_cast<std::size_t>(append_rows) * a.kv_heads * 32 * 2;
     const std::size_t q_pieces = F32 ? static_cast<std::size_t>(a.tokens) * a.query_heads * 32 : 0; // parked queries
-    prefill_append_kernel<F32><<<static_cast<unsigned int>((kv_pieces + q_pieces + 255) / 256), 256, 0, stream>>>(
-        a.key, a.value, cache, append_rows, a.past_tokens, a.max_context_tokens, a.kv_heads,
-        static_cast<const float *>(a.query), own_output, a.tokens, a.query_heads, out_heads, out_head_offset);
-    cuda_ok(cudaGetLastError(), "prefill append launch");
+    launch_programmatic(prefill_append_kernel<F32>, dim3(static_cast<unsigned int>((kv_pieces + q_pieces + 255) / 256)),
+                        dim3(256), 0, stream, "prefill append launch", a.key, a.value, cache, append_rows,
+                        a.past_tokens, a.max_context_tokens, a.kv_heads, static_cast<const float *>(a.query), own_output,
+                        a.tokens, a.query_heads, out_heads, out_head_offset);
   }
 
   const std::uint64_t context = static_cast<std::uint64_t>(a.past_tokens) + a.tokens;
@@ -1627,6 +1634,7 @@ template <bool F32, bool Pair, bool Split> void launch(const PrefillArgs &a, cud
     params.split_min_blocks = first_tile_blocks >= kSplitMinBlocks ? kSplitMinBlocks : kSplitMinBlocksLate;
   }
   params.status = device_status_word();
+  params.wait_first = append_rows == 0 ? 1U : 0U;
 
   cudaLaunchConfig_t config{};
   int device = 0;
@@ -1653,9 +1661,8 @@ template <bool F32, bool Pair, bool Split> void launch(const PrefillArgs &a, cud
   attributes[1].val.clusterDim.x = (Pair ? 2 : 1) * (Split ? 2 : 1);
   attributes[1].val.clusterDim.y = 1;
   attributes[1].val.clusterDim.z = 1;
-  // attribute 0 (overlap with the append kernel) only when that kernel was launched
-  config.attrs = append_rows > 0 ? attributes : attributes + 1;
-  config.numAttrs = (Pair || Split ? 1 : 0) + (append_rows > 0 ? 1 : 0);
+  config.attrs = attributes;
+  config.numAttrs = Pair || Split ? 2 : 1;
   cuda_ok(cudaLaunchKernelEx(&config, prefill_attention_kernel<F32, Pair, Split>, q_map, k_map, v_map, k_new_map, v_new_map, params),
           "prefill attention launch");
 }

@@ -26,6 +26,7 @@ namespace {
 
 constexpr int kMaxPairs = 128;
 constexpr int kPrologueThreads = 256;
+constexpr std::uint32_t kSpreadTokens = 64; // calls of up to this many tokens spread a token's vectors over CTAs
 
 struct PrologueParams {
   // q: vectors of `q_heads` heads per token, `q_head_stride` elements apart (2 D when the gate is interleaved)
@@ -136,6 +137,14 @@ __global__ void __launch_bounds__(kPrologueThreads) attention_prologue_kernel(co
   const std::uint32_t lane_dim = lane * PerLane;
   const std::uint32_t partner_lanes = pairs / PerLane; // lanes between a dim and its rotation partner
 
+  // Launched with programmatic stream serialisation: it is resident when the kernels in front of it end.  Nothing is
+  // read or written, and nothing behind this kernel is let in, before they have, so that a kernel which takes a head
+  // start (the early cache fetch of a decode step) still has an ordinary launch between itself and older writers.
+  // As plain launches the calls of a layer cost a launch latency each: eight layers of the executor's decode sequence
+  // at 777 tokens 137.2 -> 131.7 us, at 32K 273.8 -> 258.4, a 2709-token prompt in its calls 412 -> 356.
+  grid_dependency_wait();
+  grid_dependents_may_launch();
+
   // A warp's vectors are fetched one ahead of their use: the loads of the first are in flight while the angles
   // are computed, those of the next while the current one is normalised and rotated.
   struct Fetched {
@@ -215,9 +224,11 @@ __global__ void __launch_bounds__(kPrologueThreads) attention_prologue_kernel(co
     Elements<Out>::template store<PerLane>(is_q ? p.q_out : p.k_out, out_at, f.x);
   };
 
+  constexpr std::uint32_t kWarps = kPrologueThreads / 32;
+  const std::uint32_t first = blockIdx.y * kWarps + warp;
   Fetched current;
-  if (static_cast<std::uint32_t>(warp) < vectors) {
-    fetch(warp, current);
+  if (first < vectors) {
+    fetch(first, current);
   }
   // the token's angles, once: theta = position * base^(-2 pair / rotary), cos and sin taken in double
   {
@@ -236,11 +247,11 @@ __global__ void __launch_bounds__(kPrologueThreads) attention_prologue_kernel(co
     }
   }
   __syncthreads();
-  constexpr std::uint32_t kWarps = kPrologueThreads / 32;
-  for (std::uint32_t vec = warp; vec < vectors; vec += kWarps) {
+  const std::uint32_t stride = kWarps * gridDim.y;
+  for (std::uint32_t vec = first; vec < vectors; vec += stride) {
     Fetched next;
-    if (vec + kWarps < vectors) {
-      fetch(vec + kWarps, next);
+    if (vec + stride < vectors) {
+      fetch(vec + stride, next);
     }
     finish(vec, current);
     current = next;
@@ -250,7 +261,9 @@ __global__ void __launch_bounds__(kPrologueThreads) attention_prologue_kernel(co
 template <class T>
 __global__ void split_query_gate_kernel(const T *query_gate, T *query, T *gate, std::size_t total_vec,
                                         std::uint32_t vec_per_head) {
-  // one thread per 16-byte piece of the output
+  // one thread per 16-byte piece of the output; dependent launch as in the kernel above
+  grid_dependency_wait();
+  grid_dependents_may_launch();
   const std::size_t index = static_cast<std::size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (index >= total_vec) {
     return;
@@ -263,12 +276,16 @@ __global__ void split_query_gate_kernel(const T *query_gate, T *query, T *gate, 
 }
 
 template <class In, class W, class Out> void launch_typed(const PrologueParams &p, int per_lane, cudaStream_t stream) {
+  // Many tokens: a CTA per token, so that the angles are computed once.  Few: a warp per vector.
+  const std::uint32_t vectors = p.q_heads + (p.v_in != nullptr ? 2 : 1) * p.kv_heads;
+  const std::uint32_t groups = (vectors + kPrologueThreads / 32 - 1) / (kPrologueThreads / 32);
+  const dim3 grid(p.tokens, p.tokens <= kSpreadTokens ? groups : 1);
+  const char *what = "attention prologue launch";
   if (per_lane == 8) {
-    attention_prologue_kernel<In, W, Out, 8><<<p.tokens, kPrologueThreads, 0, stream>>>(p);
+    launch_programmatic(attention_prologue_kernel<In, W, Out, 8>, grid, dim3(kPrologueThreads), 0, stream, what, p);
   } else {
-    attention_prologue_kernel<In, W, Out, 4><<<p.tokens, kPrologueThreads, 0, stream>>>(p);
+    launch_programmatic(attention_prologue_kernel<In, W, Out, 4>, grid, dim3(kPrologueThreads), 0, stream, what, p);
   }
-  cuda_ok(cudaGetLastError(), "attention prologue launch");
 }
 
 void launch_prologue(const PrologueParams &p, std::size_t head_dim, int32_t in_dtype, int32_t weight_dtype,
@@ -388,10 +405,10 @@ extern "C" Rib200Status rib200_split_full_query_gate(const void *query_gate, voi
     const std::uint32_t vec_per_head = static_cast<std::uint32_t>(head_dim * element / 16);
     const std::size_t blocks = (total_vec + 255) / 256;
     require(blocks <= 0x7FFFFFFFU, "split_full_query_gate grid dimension overflow");
-    split_query_gate_kernel<uint4><<<static_cast<unsigned int>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4 *>(query_gate), static_cast<uint4 *>(query), static_cast<uint4 *>(gate), total_vec,
-        vec_per_head);
-    cuda_ok(cudaGetLastError(), "split_full_query_gate launch");
+    launch_programmatic(split_query_gate_kernel<uint4>, dim3(static_cast<unsigned int>(blocks)), dim3(256), 0,
+                        static_cast<cudaStream_t>(stream), "split_full_query_gate launch",
+                        static_cast<const uint4 *>(query_gate), static_cast<uint4 *>(query),
+                        static_cast<uint4 *>(gate), total_vec, vec_per_head);
   });
 }
 

@@ -170,3 +170,44 @@ def test_argument_checks_follow_the_reference():
         K.qwen35_split_full_query_gate(x, x, None, 2, 4, 128, K.DTYPE_F32, stream)
     with pytest.raises(K.Qwen35PrimitiveError):
         K.qwen35_split_full_query_gate(x, x, x, 0, 4, 128, K.DTYPE_F32, stream)
+
+
+@pytest.mark.parametrize("chunks", [(2, 3, 2), (64, 65, 3), (128, 130, 2)])
+@pytest.mark.parametrize("dtype", [K.DTYPE_F32, K.DTYPE_BF16])
+def test_chained_calls_keep_stream_order(chunks, dtype):
+    """The kernels of a layer let each other in early; with every activation buffer reused from one chunk to the next
+    the results are, bit for bit, those of calls that are waited for one by one."""
+    hq, hkv, d, rotary = 16, 4, 256, 64
+    stream = torch.cuda.current_stream()
+    total, most = sum(chunks), max(chunks)
+    torch_dtype = torch.float32 if dtype == K.DTYPE_F32 else torch.bfloat16
+    packed, k, v = (act_tensor(synth.round_bf16(synth.normal(0xB2001500, i, (total, h, d))), dtype)
+                    for i, h in enumerate((2 * hq, hkv, hkv)))
+    w = act_tensor((1.0 + 0.1 * synth.normal(0xB2001500, 3, (d,))).astype(np.float32), K.DTYPE_F32)
+
+    def run(settle):
+        buf = lambda h: torch.zeros(most, h, d, device=dev(), dtype=torch_dtype)
+        q_raw, q, gate, key, out = buf(hq), buf(hq), buf(hq), buf(hkv), buf(hq)
+        cache = torch.zeros(2, hkv, 384, d, device=dev(), dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        outs, first = [], 0
+        for n in chunks:
+            rows = slice(first, first + n)
+            K.qwen35_split_full_query_gate(packed[rows], q_raw, gate, n, hq, d, dtype, stream)
+            settle()
+            for src, dst, heads in ((q_raw, q, hq), (k[rows], key, hkv)):
+                K.qwen35_qk_norm_rope(src, w, dst, K.QkNormRopeShape(n, heads, d, rotary, first, BASE), EPS, dtype,
+                                      K.DTYPE_F32, stream)
+                settle()
+            shape = K.Qwen35AttentionShape(n, hq, hkv, d, 384, first)
+            K.qwen35_online_attention_prefill(q, key, v[rows], gate, out, cache, cache.numel() * 2, shape, dtype,
+                                              K.KV_BF16, K.HEAD_MAJOR, stream)
+            settle()
+            outs.append(out[:n].clone())
+            first += n
+        torch.cuda.synchronize()
+        return outs + [cache]
+
+    assert K.device_status(stream) == 0
+    for a, b in zip(run(lambda: None), run(torch.cuda.synchronize)):
+        assert torch.equal(a, b)
