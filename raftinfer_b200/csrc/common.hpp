@@ -211,12 +211,12 @@ struct GdnLayerArgs {
   int32_t dtype, weight_dtype;
 };
 void launch_gdn_prologue(const GdnLayerArgs &args, cudaStream_t stream);
-// The whole layer call of one token as one launch, where that form applies (see gdn_layer.cu).
 // The whole layer call of 64 tokens or more in the chunked kernels (convolution width 4, aligned tensors), and its
 // first kernel; scratch as for launch_gdn_chunked.
 bool gdn_layer_chunks_apply(const GdnLayerArgs &args);
 void launch_gdn_layer_chunks(const GdnLayerArgs &args, void *workspace, cudaStream_t stream);
 void launch_gdn_layer_images(const GdnLayerArgs &args, void *workspace, cudaStream_t stream);
+// The whole layer call of fewer than 64 tokens as one launch, where that form applies (see gdn_layer.cu).
 bool gdn_layer_step_applies(const GdnLayerArgs &args);
 void launch_gdn_layer_step(const GdnLayerArgs &args, cudaStream_t stream);
 void launch_gdn_epilogue(const GdnLayerArgs &args, cudaStream_t stream);

@@ -85,6 +85,8 @@ struct LayerParams {
 // grid (2*Hk + Hv head vectors, tokens), 128 threads = the 128 channels of the vector
 __global__ void __launch_bounds__(kDim) gdn_prologue_kernel(const LayerParams p) {
   __shared__ float scratch[4];
+  grid_dependency_wait();
+  grid_dependents_may_launch();
   const std::uint32_t vec = blockIdx.x;
   const std::uint32_t tok = blockIdx.y;
   const std::uint32_t channel = vec * kDim + threadIdx.x;
@@ -179,6 +181,7 @@ constexpr int kFastWidth = 4;
 // current four are convolved, and the last three rows of a step are the history of the next.  The vector after the
 // last one stands for the gates (lane = value head, any head count).
 template <int Dtype> __global__ void __launch_bounds__(256, 3) gdn_prologue_w4_kernel(const LayerParams p) {
+  grid_dependency_wait();
   grid_dependents_may_launch(); // the kernels behind this one set themselves up early and wait for it to end
   const int lane = threadIdx.x & 31;
   const std::uint32_t vec = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -449,8 +452,8 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(state + static_cast<std::size_t>(tid) * kDim));
   }
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
-  grid_dependents_may_launch();
   grid_dependency_wait();
+  grid_dependents_may_launch();
 
   // ---- every load of the step in one round ----
   const int row0 = 16 * warp + (lane >> 3);
@@ -631,6 +634,294 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
   }
 }
 
+// ---- 2 .. 63 tokens in one launch --------------------------------------------------------------------------
+// The calls that end a prompt (the executor cuts a rest into 17, 4 and 2 tokens) are latency as well: the general path
+// took 53 us for 17 tokens and 25 us for 4 (prologue, history, recurrence, epilogue; launch list).  Same split as the
+// one-token form - a cluster per key head, a CTA per 32 state columns - and the same arithmetic in FP32; the tokens go
+// through in tiles of 32: convolution and norms of a tile with a warp per token, then the recurrence with the state in
+// registers, then the output norm, for which the slices of a head exchange their sums once per tile.  In the recurrence
+// a warp owns four columns and a lane four rows of them, so that a token needs no barrier: nine shuffles bring the
+// eight sums (S^T k, S^T q) to eight groups of lanes, four more hand the corrections back.
+constexpr std::uint32_t kShortTile = 32;
+constexpr std::uint32_t kShortMaxTokens = 63; // longer calls run in chunks
+constexpr std::uint32_t kShortRounds = kShortTile / 8; // tokens per warp
+
+template <int Dtype, int WeightDtype>
+__global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const LayerParams p) {
+  using Act = Scalar<Dtype>;
+  using Weight = Scalar<WeightDtype>;
+  using ActType = typename Act::Type;
+  using WeightType = typename Weight::Type;
+  constexpr int kHistory = kFastWidth - 1;
+  __shared__ __align__(16) float s_qk[2][kShortTile][kDim];
+  __shared__ float s_v[kShortTile][kStepColumns];
+  __shared__ float s_out[kShortTile][kStepColumns];
+  __shared__ float s_kq[kShortTile];
+  __shared__ float s_beta[kShortTile];
+  __shared__ float s_decay[kShortTile];
+  __shared__ float s_norm[2][kStepSlices][kShortTile]; // by parity of the tile
+  std::uint32_t rank;
+  std::uint32_t cluster_size;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(cluster_size));
+  const std::uint32_t key_head = blockIdx.x / cluster_size;
+  const std::uint32_t head = key_head + (rank / kStepSlices) * p.key_heads;
+  const std::uint32_t slice = rank % kStepSlices;
+  const std::uint32_t tid = threadIdx.x;
+  const std::uint32_t warp = tid >> 5;
+  const std::uint32_t lane = tid & 31;
+  float *state = p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns;
+  if (tid < kDim) { // a hint; the values are read after the wait
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(state + static_cast<std::size_t>(tid) * kDim));
+  }
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
+  grid_dependency_wait();
+  grid_dependents_may_launch();
+
+  const auto *input = static_cast<const ActType *>(p.input);
+  const auto *conv_weight = static_cast<const WeightType *>(p.conv_weight);
+  // state: lane = rows 4 lane .. + 3, warp = columns 4 warp .. + 3 of the slice
+  float4 s[4];
+#pragma unroll
+  for (std::uint32_t i = 0; i < 4; ++i) {
+    s[i] = *reinterpret_cast<const float4 *>(state + static_cast<std::size_t>(4 * lane + i) * kDim + 4 * warp);
+  }
+  // threads 0..127 convolve the q channels of the key head, 128..255 its k channels; a lane a v channel of the slice
+  const std::uint32_t qk_channel = (tid < kDim ? 0 : p.key_heads * kDim) + key_head * kDim + (tid & (kDim - 1));
+  const std::uint32_t v_channel = 2 * p.key_heads * kDim + head * kDim + slice * kStepColumns + lane;
+  const std::uint32_t z_channel = p.conv_dim + 2 * p.value_heads + head * kDim + slice * kStepColumns + lane;
+  float qk_weight[kFastWidth];
+  float v_weight[kFastWidth];
+  float qk_before[kHistory]; // the three tokens in front of the tile
+  float v_history[kHistory]; // the three in front of the call
+#pragma unroll
+  for (int h = 0; h < kFastWidth; ++h) {
+    qk_weight[h] = Weight::widen(conv_weight[static_cast<std::size_t>(qk_channel) * kFastWidth + h]);
+    v_weight[h] = Weight::widen(conv_weight[static_cast<std::size_t>(v_channel) * kFastWidth + h]);
+  }
+#pragma unroll
+  for (int h = 0; h < kHistory; ++h) {
+    qk_before[h] = p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h];
+    v_history[h] = p.convolution_state[static_cast<std::size_t>(v_channel) * kHistory + h];
+  }
+  const float norm_weight =
+      Weight::widen(static_cast<const WeightType *>(p.output_norm_weight)[slice * kStepColumns + lane]);
+  const float coefficient = Weight::widen(static_cast<const WeightType *>(p.recurrent_a)[head]);
+  const float dt = Weight::widen(static_cast<const WeightType *>(p.dt_bias)[head]);
+  auto v_row = [&](int tok) { // v of a token of this call, or of the history in front of it
+    return tok >= 0 ? Act::widen(input[static_cast<std::size_t>(tok) * p.token_stride + v_channel])
+                    : (tok == -1 ? v_history[2] : (tok == -2 ? v_history[1] : v_history[0]));
+  };
+
+  for (std::uint32_t first = 0, tile = 0; first < p.tokens; first += kShortTile, ++tile) {
+    const std::uint32_t n = min(kShortTile, p.tokens - first);
+    // ---- convolution and SiLU: q and k a channel per thread, v and the gates a token per warp ----
+    {
+      ActType x[kShortTile];
+#pragma unroll
+      for (std::uint32_t t = 0; t < kShortTile; ++t) {
+        if (t < n) {
+          x[t] = input[static_cast<std::size_t>(first + t) * p.token_stride + qk_channel];
+        }
+      }
+      float v_value[kShortRounds];
+#pragma unroll
+      for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+        const std::uint32_t t = warp + 8 * r;
+        if (t < n) {
+          const int tok = static_cast<int>(first + t);
+          float sum = v_row(tok) * v_weight[kHistory]; // the current token's tap first, then the history, oldest first
+#pragma unroll
+          for (int h = 0; h < kHistory; ++h) {
+            sum += v_row(tok - kHistory + h) * v_weight[h];
+          }
+          v_value[r] = silu(sum);
+          if (lane == 0) {
+            const std::size_t gates = static_cast<std::size_t>(tok) * p.token_stride + p.conv_dim + head;
+            s_beta[t] = 1.0F / (1.0F + expf(-Act::widen(input[gates])));
+            s_decay[t] = expf(coefficient * softplus(Act::widen(input[gates + p.value_heads]) + dt));
+          }
+        }
+      }
+#pragma unroll
+      for (std::uint32_t t = 0; t < kShortTile; ++t) {
+        if (t < n) {
+          const float now = Act::widen(x[t]);
+          float sum = now * qk_weight[kHistory];
+#pragma unroll
+          for (int h = 0; h < kHistory; ++h) {
+            sum += qk_before[h] * qk_weight[h];
+          }
+          qk_before[0] = qk_before[1];
+          qk_before[1] = qk_before[2];
+          qk_before[2] = now;
+          s_qk[tid >> 7][t][tid & (kDim - 1)] = silu(sum);
+        }
+      }
+#pragma unroll
+      for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+        if (warp + 8 * r < n) {
+          s_v[warp + 8 * r][lane] = v_value[r];
+        }
+      }
+    }
+    __syncthreads();
+    // ---- norms of q and k, k . q ----
+    for (std::uint32_t t = warp; t < n; t += 8) {
+      float4 q = *reinterpret_cast<const float4 *>(&s_qk[0][t][4 * lane]);
+      float4 k = *reinterpret_cast<const float4 *>(&s_qk[1][t][4 * lane]);
+      float qq = (q.x * q.x + q.y * q.y) + (q.z * q.z + q.w * q.w);
+      float kk = (k.x * k.x + k.y * k.y) + (k.z * k.z + k.w * k.w);
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) {
+        qq += __shfl_xor_sync(0xFFFFFFFFU, qq, offset);
+        kk += __shfl_xor_sync(0xFFFFFFFFU, kk, offset);
+      }
+      const float q_scale = rsqrtf(qq + kQkEpsilon) * rsqrtf(static_cast<float>(kDim));
+      const float k_scale = rsqrtf(kk + kQkEpsilon);
+      q = make_float4(q.x * q_scale, q.y * q_scale, q.z * q_scale, q.w * q_scale);
+      k = make_float4(k.x * k_scale, k.y * k_scale, k.z * k_scale, k.w * k_scale);
+      float kq = (k.x * q.x + k.y * q.y) + (k.z * q.z + k.w * q.w);
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) {
+        kq += __shfl_xor_sync(0xFFFFFFFFU, kq, offset);
+      }
+      *reinterpret_cast<float4 *>(&s_qk[0][t][4 * lane]) = q;
+      *reinterpret_cast<float4 *>(&s_qk[1][t][4 * lane]) = k;
+      if (lane == 0) {
+        s_kq[t] = kq;
+      }
+    }
+    __syncthreads();
+    // ---- the recurrence ----
+    // after the three exchanges lane l holds the sum of column 2 (l / 8 % 2) + (l / 4) % 2, of S^T k below lane 16 and
+    // of S^T q from there on
+    const std::uint32_t my_column = ((lane >> 3) & 1U) * 2 + ((lane >> 2) & 1U);
+    for (std::uint32_t t = 0; t < n; ++t) {
+      const float4 k4 = *reinterpret_cast<const float4 *>(&s_qk[1][t][4 * lane]);
+      const float4 q4 = *reinterpret_cast<const float4 *>(&s_qk[0][t][4 * lane]);
+      const float k[4] = {k4.x, k4.y, k4.z, k4.w};
+      const float q[4] = {q4.x, q4.y, q4.z, q4.w};
+      float a[4] = {};
+      float b[4] = {};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[0] += s[i].x * k[i];
+        a[1] += s[i].y * k[i];
+        a[2] += s[i].z * k[i];
+        a[3] += s[i].w * k[i];
+        b[0] += s[i].x * q[i];
+        b[1] += s[i].y * q[i];
+        b[2] += s[i].z * q[i];
+        b[3] += s[i].w * q[i];
+      }
+      const bool upper = (lane & 16U) != 0;
+      float four[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        four[c] = (upper ? b[c] : a[c]) + __shfl_xor_sync(0xFFFFFFFFU, upper ? a[c] : b[c], 16);
+      }
+      const bool high_pair = (lane & 8U) != 0;
+      float two[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        two[c] = (high_pair ? four[2 + c] : four[c]) +
+                 __shfl_xor_sync(0xFFFFFFFFU, high_pair ? four[c] : four[2 + c], 8);
+      }
+      const bool odd = (lane & 4U) != 0;
+      float sum = (odd ? two[1] : two[0]) + __shfl_xor_sync(0xFFFFFFFFU, odd ? two[0] : two[1], 4);
+      sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 2);
+      sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 1);
+      const float decay = s_decay[t];
+      const float delta = (s_v[t][4 * warp + my_column] - decay * sum) * s_beta[t]; // below lane 16
+      float correction[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        correction[c] = __shfl_sync(0xFFFFFFFFU, delta, 4 * c);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        s[i].x = decay * s[i].x + k[i] * correction[0];
+        s[i].y = decay * s[i].y + k[i] * correction[1];
+        s[i].z = decay * s[i].z + k[i] * correction[2];
+        s[i].w = decay * s[i].w + k[i] * correction[3];
+      }
+      const float low = odd ? correction[1] : correction[0];
+      const float high = odd ? correction[3] : correction[2];
+      if (upper && (lane & 3U) == 0) {
+        s_out[t][4 * warp + my_column] = decay * sum + (high_pair ? high : low) * s_kq[t];
+      }
+    }
+    __syncthreads();
+    // ---- output norm over the four slices, gate ----
+    float z_gate[kShortRounds];
+    float read[kShortRounds];
+#pragma unroll
+    for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+      const std::uint32_t t = warp + 8 * r;
+      if (t < n) {
+        z_gate[r] = norm_weight * silu(Act::widen(input[static_cast<std::size_t>(first + t) * p.token_stride + z_channel]));
+        read[r] = s_out[t][lane];
+      }
+    }
+    if (tile == 0) { // the barrier that says that every CTA of the cluster has started
+      asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+    }
+#pragma unroll
+    for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+      const std::uint32_t t = warp + 8 * r;
+      if (t < n) {
+        float norm = read[r] * read[r];
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) {
+          norm += __shfl_xor_sync(0xFFFFFFFFU, norm, offset);
+        }
+        if (lane < kStepSlices) { // to the four CTAs of this value head
+          std::uint32_t remote;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                       : "=r"(remote)
+                       : "r"(static_cast<std::uint32_t>(__cvta_generic_to_shared(&s_norm[tile & 1U][slice][t]))),
+                         "r"(rank - slice + lane));
+          asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote), "f"(norm) : "memory");
+        }
+      }
+    }
+    __syncwarp();
+    // Orders the partial norms; that of the first tile also marks the end of everybody's reads of the old history.
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+#pragma unroll
+    for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+      const std::uint32_t t = warp + 8 * r;
+      if (t < n) {
+        const float (&norms)[kStepSlices][kShortTile] = s_norm[tile & 1U];
+        const float norm = (norms[0][t] + norms[1][t]) + (norms[2][t] + norms[3][t]);
+        const float scale = rsqrtf(norm / static_cast<float>(kDim) + p.epsilon);
+        static_cast<ActType *>(p.output)[(static_cast<std::size_t>(first + t) * p.value_heads + head) * kDim +
+                                         slice * kStepColumns + lane] = Act::narrow(read[r] * scale * z_gate[r]);
+      }
+    }
+  }
+#pragma unroll
+  for (std::uint32_t i = 0; i < 4; ++i) {
+    *reinterpret_cast<float4 *>(state + static_cast<std::size_t>(4 * lane + i) * kDim + 4 * warp) = s[i];
+  }
+  // the last three tokens of [old history | call] are the next call's history
+  if (rank == 0) {
+#pragma unroll
+    for (int h = 0; h < kHistory; ++h) {
+      p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h] = qk_before[h];
+    }
+  }
+  if (warp == 0) {
+#pragma unroll
+    for (int h = 0; h < kHistory; ++h) {
+      p.convolution_state[static_cast<std::size_t>(v_channel) * kHistory + h] =
+          v_row(static_cast<int>(p.tokens) - kHistory + h);
+    }
+  }
+}
+
 LayerParams make_params(const GdnLayerArgs &a) {
   LayerParams p{};
   p.input = a.input;
@@ -659,14 +950,15 @@ LayerParams make_params(const GdnLayerArgs &a) {
 
 template <int Dtype, int WeightDtype> void launch_step(const LayerParams &p, cudaStream_t stream) {
   const std::uint32_t cluster = kStepSlices * (p.value_heads / p.key_heads);
-  launch_programmatic_cluster(gdn_layer_step_kernel<Dtype, WeightDtype>, dim3(cluster * p.key_heads),
-                              dim3(kStepThreads), cluster, 0, stream, "gated-delta step launch", p);
+  auto *kernel = p.tokens == 1 ? gdn_layer_step_kernel<Dtype, WeightDtype> : gdn_layer_short_kernel<Dtype, WeightDtype>;
+  launch_programmatic_cluster(kernel, dim3(cluster * p.key_heads), dim3(kStepThreads), cluster, 0, stream,
+                              "gated-delta step launch", p);
 }
 
 } // namespace
 
 bool gdn_layer_step_applies(const GdnLayerArgs &a) {
-  return a.tokens == 1 && a.conv_width == kFastWidth && a.value_heads / a.key_heads <= kStepMaxRatio;
+  return a.tokens <= kShortMaxTokens && a.conv_width == kFastWidth && a.value_heads / a.key_heads <= kStepMaxRatio;
 }
 
 void launch_gdn_layer_step(const GdnLayerArgs &a, cudaStream_t stream) {
@@ -697,21 +989,22 @@ void launch_gdn_layer_step(const GdnLayerArgs &a, cudaStream_t stream) {
 
 void launch_gdn_prologue(const GdnLayerArgs &a, cudaStream_t stream) {
   const LayerParams p = make_params(a);
+  const char *what = "gated-delta prologue launch";
   // a call of a few tokens is latency, not bandwidth: the one-CTA-per-vector kernel spreads it wider
   if (a.conv_width == kFastWidth && a.tokens >= 2 * kTokensPerWarp && vector_forms_apply(p)) {
     constexpr std::uint32_t kTokensPerCta = kTokensPerWarp * kStepsPerWarp;
     const dim3 grid((a.tokens + kTokensPerCta - 1) / kTokensPerCta, (2 * a.key_heads + a.value_heads + 1 + 7) / 8);
     if (a.dtype == RIB200_DTYPE_F32) {
-      gdn_prologue_w4_kernel<RIB200_DTYPE_F32><<<grid, 256, 0, stream>>>(p);
+      launch_programmatic(gdn_prologue_w4_kernel<RIB200_DTYPE_F32>, grid, dim3(256), 0, stream, what, p);
     } else if (a.dtype == RIB200_DTYPE_F16) {
-      gdn_prologue_w4_kernel<RIB200_DTYPE_F16><<<grid, 256, 0, stream>>>(p);
+      launch_programmatic(gdn_prologue_w4_kernel<RIB200_DTYPE_F16>, grid, dim3(256), 0, stream, what, p);
     } else {
-      gdn_prologue_w4_kernel<RIB200_DTYPE_BF16><<<grid, 256, 0, stream>>>(p);
+      launch_programmatic(gdn_prologue_w4_kernel<RIB200_DTYPE_BF16>, grid, dim3(256), 0, stream, what, p);
     }
   } else {
-    gdn_prologue_kernel<<<dim3(2 * a.key_heads + a.value_heads, a.tokens), kDim, 0, stream>>>(p);
+    launch_programmatic(gdn_prologue_kernel, dim3(2 * a.key_heads + a.value_heads, a.tokens), dim3(kDim), 0, stream, what,
+                        p);
   }
-  cuda_ok(cudaGetLastError(), "gated-delta prologue launch");
   if (a.conv_width > 1) {
     launch_programmatic(gdn_conv_state_kernel, dim3((p.conv_dim + 255) / 256), dim3(256), 0, stream,
                         "gated-delta convolution-state launch", p);

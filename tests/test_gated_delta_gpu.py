@@ -282,6 +282,19 @@ def test_layer_single_tokens(hk, hv, dtype, wdtype):
     assert K.device_status(torch.cuda.current_stream()) == 0
 
 
+@pytest.mark.parametrize("calls", [(2, 3), (31, 2), (32, 1), (33, 17), (63,)])
+@pytest.mark.parametrize("hk,hv", [(1, 1), (2, 4), (1, 3)])
+@pytest.mark.parametrize("dtype,wdtype", [(K.DTYPE_BF16, K.DTYPE_BF16), (K.DTYPE_F32, K.DTYPE_F32)])
+def test_layer_short_calls(calls, hk, hv, dtype, wdtype):
+    """Calls of 2 to 63 tokens, either side of the 32-token tile, each on the states the one before left: one launch
+    where a key head has one or two value heads, the general path for three."""
+    run = LayerRun(0xB2002900 + 8 * hk + hv, hk, hv, 4, dtype, wdtype, sum(calls))
+    for tokens in calls:
+        out, want, _ = run.step(tokens)
+        run.check(out, want)
+    assert K.device_status(torch.cuda.current_stream()) == 0
+
+
 def test_layer_three_launches_share_device_state_without_a_sync():
     run = LayerRun(0xB2002200, 2, 4, 4, K.DTYPE_F32, K.DTYPE_F32, 6)
     results = [run.step(2, sync=False) for _ in range(3)]
