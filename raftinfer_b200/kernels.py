@@ -11,7 +11,7 @@ from __future__ import annotations
 import ctypes as C
 from dataclasses import dataclass
 
-from . import _lib
+from . import _call, _lib
 from ._lib import lib
 
 # RaftInferDataType, cpp/include/raftinfer/tensor.h:10-15
@@ -39,6 +39,11 @@ class Qwen35DeltaError(RuntimeError):
     def __init__(self, code, message):
         super().__init__(message)
         self.code = code
+
+
+# The launchers go through native functions (csrc/binding.cpp); sizes, plans and the rest through ctypes.
+_call.bind(lambda name: C.cast(getattr(lib, name), C.c_void_p).value, C.ArgumentError, Qwen35PrimitiveError,
+           Qwen35DeltaError)
 
 
 def _check(status, exc=Qwen35PrimitiveError):
@@ -191,18 +196,14 @@ def qwen35_online_attention_workspace_bytes(shape):
 # ---- attention: launchers ----------------------------------------------------------------------
 def qwen35_causal_attention(query, key, value, gate, output, kv_cache, kv_cache_bytes, workspace, workspace_bytes,
                             shape, activation_dtype, policy, stream):
-    s = shape.c()
-    _check(lib.rib200_causal_attention(_ptr(query), _ptr(key), _ptr(value), _ptr(gate), _ptr(output),
-                                       _ptr(kv_cache), kv_cache_bytes, _ptr(workspace), workspace_bytes,
-                                       C.byref(s), activation_dtype, policy.c(), _stream(stream)))
+    _call.rib200_causal_attention(query, key, value, gate, output, kv_cache, kv_cache_bytes, workspace, workspace_bytes,
+                                  shape, activation_dtype, policy, stream)
 
 
 def qwen35_online_attention_prefill(query, key, value, gate, output, kv_cache, kv_cache_bytes, shape,
                                     activation_dtype, cache_dtype, cache_layout, stream):
-    s = shape.c()
-    _check(lib.rib200_online_attention_prefill(_ptr(query), _ptr(key), _ptr(value), _ptr(gate), _ptr(output),
-                                               _ptr(kv_cache), kv_cache_bytes, C.byref(s), activation_dtype,
-                                               cache_dtype, cache_layout, _stream(stream)))
+    _call.rib200_online_attention_prefill(query, key, value, gate, output, kv_cache, kv_cache_bytes, shape,
+                                          activation_dtype, cache_dtype, cache_layout, stream)
 
 
 @dataclass(frozen=True)
@@ -222,26 +223,21 @@ class QkNormRopeShape:
 
 def qwen35_qk_norm_rope(input, weight, output, shape, epsilon, dtype, weight_dtype, stream, device_position=None):
     """cpp/kernels/qwen35_primitives.cuh:61-66"""
-    s = shape.c()
-    _check(lib.rib200_qk_norm_rope(_ptr(input), _ptr(weight), _ptr(output), C.byref(s), epsilon, dtype, weight_dtype,
-                                   _stream(stream), _ptr(device_position)))
+    _call.rib200_qk_norm_rope(input, weight, output, shape, epsilon, dtype, weight_dtype, stream, device_position)
 
 
 def qwen35_split_full_query_gate(query_gate, query, gate, tokens, heads, head_dim, dtype, stream):
     """cpp/kernels/qwen35_primitives.cuh:90-93"""
-    _check(lib.rib200_split_full_query_gate(_ptr(query_gate), _ptr(query), _ptr(gate), tokens, heads, head_dim, dtype,
-                                            _stream(stream)))
+    _call.rib200_split_full_query_gate(query_gate, query, gate, tokens, heads, head_dim, dtype, stream)
 
 
 def attention_prologue(query_gate, key, value, query_norm_weight, key_norm_weight, query, gate, key_out, value_out,
                        shape, rotary_dim, rope_base, epsilon, dtype, weight_dtype, output_dtype, stream,
                        device_position=None):
     """The executor's three pre-attention calls (cpp/execution/qwen35_executor.cu:1989-2015) as one launch."""
-    s = shape.c()
-    _check(lib.rib200_attention_prologue(_ptr(query_gate), _ptr(key), _ptr(value), _ptr(query_norm_weight),
-                                         _ptr(key_norm_weight), _ptr(query), _ptr(gate), _ptr(key_out),
-                                         _ptr(value_out), C.byref(s), rotary_dim, rope_base, epsilon, dtype,
-                                         weight_dtype, output_dtype, _ptr(device_position), _stream(stream)))
+    _call.rib200_attention_prologue(query_gate, key, value, query_norm_weight, key_norm_weight, query, gate, key_out,
+                                    value_out, shape, rotary_dim, rope_base, epsilon, dtype, weight_dtype, output_dtype,
+                                    device_position, stream)
 
 
 def online_attention_decode_from_host(host_token, host_output, device_token, device_output, kv_cache, kv_cache_bytes,
@@ -312,15 +308,12 @@ def qwen35_online_attention_decode(query, key, value, gate, output, kv_cache, kv
                                    device_position, stream):
     """Plan overload (cpp/kernels/qwen35_online_attention.cuh:55-63).  Pass plan=None for the reference's
     plan-less overload (:65-68), which resolves to single-block mode and takes no workspace."""
-    s = shape.c()
     if plan is None:
         plan = qwen35_online_decode_plan(shape, SINGLE_BLOCK, shape.past_tokens + 1)
         workspace, workspace_bytes = None, 0
-    p = plan.c()
-    _check(lib.rib200_online_attention_decode(_ptr(query), _ptr(key), _ptr(value), _ptr(gate), _ptr(output),
-                                              _ptr(kv_cache), kv_cache_bytes, _ptr(workspace), workspace_bytes,
-                                              C.byref(s), activation_dtype, cache_dtype, cache_layout, C.byref(p),
-                                              _ptr(device_position), _stream(stream)))
+    _call.rib200_online_attention_decode(query, key, value, gate, output, kv_cache, kv_cache_bytes, workspace,
+                                         workspace_bytes, shape, activation_dtype, cache_dtype, cache_layout, plan,
+                                         device_position, stream)
 
 
 def online_attention_decode_static_scratch(query, key, value, gate, output, kv_cache, kv_cache_bytes, shape,
@@ -343,10 +336,8 @@ def batched_decode_workspace_bytes(batch, max_context_tokens):
 
 def batched_decode_attention(query, key, value, gate, output, kv_caches, max_context_tokens, positions, batch,
                              largest_max_context_tokens, workspace, workspace_bytes, stream):
-    _check(lib.rib200_batched_decode_attention(_ptr(query), _ptr(key), _ptr(value), _ptr(gate), _ptr(output),
-                                               _ptr(kv_caches), _ptr(max_context_tokens), _ptr(positions), batch,
-                                               largest_max_context_tokens, _ptr(workspace), workspace_bytes,
-                                               _stream(stream)))
+    _call.rib200_batched_decode_attention(query, key, value, gate, output, kv_caches, max_context_tokens, positions,
+                                          batch, largest_max_context_tokens, workspace, workspace_bytes, stream)
 
 
 PAGE_TOKENS = 256
@@ -356,10 +347,8 @@ def paged_decode_attention(query, key, value, gate, output, page_pool, pool_page
                            positions, batch, workspace, workspace_bytes, stream):
     """Batched decode step over a pool of 256-token pages ([2][4][256][256] BF16 each) named by per-sequence block
     tables (uint32, device memory)."""
-    _check(lib.rib200_paged_decode_attention(_ptr(query), _ptr(key), _ptr(value), _ptr(gate), _ptr(output),
-                                             _ptr(page_pool), pool_pages, _ptr(block_tables), max_blocks_per_sequence,
-                                             _ptr(positions), batch, _ptr(workspace), workspace_bytes,
-                                             _stream(stream)))
+    _call.rib200_paged_decode_attention(query, key, value, gate, output, page_pool, pool_pages, block_tables,
+                                        max_blocks_per_sequence, positions, batch, workspace, workspace_bytes, stream)
 
 
 # ---- gated delta ---------------------------------------------------------------------------------
@@ -387,13 +376,10 @@ def qwen35_gated_delta_schedule_diagnostic(shape, bucket_tokens):
 def qwen35_gated_delta(input, conv_weight, recurrent_a, dt_bias, output_norm_weight, output, convolution_state,
                        recurrent_state, workspace, workspace_bytes, shape, dtype, weight_dtype, stream,
                        policy=None):
-    s = shape.c()
     if policy is None:
         policy = qwen35_gated_delta_select_policy(shape, shape.tokens)
-    _check(lib.rib200_gated_delta(_ptr(input), _ptr(conv_weight), _ptr(recurrent_a), _ptr(dt_bias),
-                                  _ptr(output_norm_weight), _ptr(output), _ptr(convolution_state),
-                                  _ptr(recurrent_state), _ptr(workspace), workspace_bytes, C.byref(s), policy.c(),
-                                  dtype, weight_dtype, _stream(stream)), Qwen35DeltaError)
+    _call.rib200_gated_delta(input, conv_weight, recurrent_a, dt_bias, output_norm_weight, output, convolution_state,
+                             recurrent_state, workspace, workspace_bytes, shape, policy, dtype, weight_dtype, stream)
 
 
 def gdn_core_workspace_bytes(tokens, key_heads, value_heads, key_dim, value_dim):
@@ -405,15 +391,12 @@ def gdn_core_workspace_bytes(tokens, key_heads, value_heads, key_dim, value_dim)
 
 def gdn_core(q, k, v, beta, log_decay, state, out, workspace, workspace_bytes, tokens, key_heads, value_heads,
              key_dim, value_dim, qkv_dtype, stream):
-    _check(lib.rib200_gdn_core(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(log_decay), _ptr(state), _ptr(out),
-                               _ptr(workspace), workspace_bytes, tokens, key_heads, value_heads, key_dim,
-                               value_dim, qkv_dtype, _stream(stream)), Qwen35DeltaError)
+    _call.rib200_gdn_core(q, k, v, beta, log_decay, state, out, workspace, workspace_bytes, tokens, key_heads, value_heads,
+                          key_dim, value_dim, qkv_dtype, stream)
 
 
 def batched_gdn_decode(q, k, v, beta, log_decay, states, out, batch, key_heads, value_heads, stream):
-    _check(lib.rib200_batched_gdn_decode(_ptr(q), _ptr(k), _ptr(v), _ptr(beta), _ptr(log_decay), _ptr(states),
-                                         _ptr(out), batch, key_heads, value_heads, _stream(stream)),
-           Qwen35DeltaError)
+    _call.rib200_batched_gdn_decode(q, k, v, beta, log_decay, states, out, batch, key_heads, value_heads, stream)
 
 
 def online_attention_decode_early_kv_fetch(query, key, value, gate, output, kv_cache, kv_cache_bytes, workspace,
@@ -422,12 +405,9 @@ def online_attention_decode_early_kv_fetch(query, key, value, gate, output, kv_c
     """rib200_online_attention_decode_early_kv_fetch: the decode step with a host position whose partition kernel
     fetches cache rows before the kernel in front of it has finished.  The caller promises that no work in flight
     writes the cache rows the step reads (see include/rib200.h)."""
-    s, p = shape.c(), plan.c()
-    _check(lib.rib200_online_attention_decode_early_kv_fetch(_ptr(query), _ptr(key), _ptr(value), _ptr(gate),
-                                                             _ptr(output), _ptr(kv_cache), kv_cache_bytes,
-                                                             _ptr(workspace), workspace_bytes, C.byref(s),
-                                                             activation_dtype, cache_dtype, cache_layout, C.byref(p),
-                                                             _stream(stream)))
+    _call.rib200_online_attention_decode_early_kv_fetch(query, key, value, gate, output, kv_cache, kv_cache_bytes,
+                                                        workspace, workspace_bytes, shape, activation_dtype, cache_dtype,
+                                                        cache_layout, plan, stream)
 
 
 def device_status(stream):
