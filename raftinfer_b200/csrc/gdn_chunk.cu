@@ -427,6 +427,15 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
     bulk_copy_g2s(base + kPsV, p.scratch.v + static_cast<std::size_t>(item) * kGdnVBytes, kGdnVBytes, bar_in);
     bulk_copy_g2s(base + kPsGates, p.scratch.records + static_cast<std::size_t>(item) * kGdnRecBytes + kGdnRecGates,
                   kGdnGateBytes, bar_in);
+    const std::uint32_t next = item + gridDim.x;
+    if (next < items) { // into L2 while this item is worked on (4096 tokens 197.7 -> 193.9 us for the whole layer call)
+      const std::uint32_t next_chunk = next / p.value_heads;
+      const std::uint32_t next_head = next - next_chunk * p.value_heads;
+      prefetch_l2(p.scratch.kq +
+                      (static_cast<std::size_t>(next_chunk) * p.key_heads + next_head % p.key_heads) * kGdnKqBytes,
+                  kGdnKqBytes);
+      prefetch_l2(p.scratch.v + static_cast<std::size_t>(next) * kGdnVBytes, kGdnVBytes);
+    }
   };
   // One lane issues every copy (bulk groups belong to the issuing thread).
   const bool copier = tid == kPrepThreads - 32;
