@@ -9,11 +9,10 @@
 // concern for q and k, which are normalised; V is brought under 2^14 by a power of two per (chunk, head), so that an
 // element keeps its 10 bits down to 2^-27 of the largest one, and the factor is divided out of U in FP32.
 //
-// HBM-bound: 67 MB of BF16 rows read and 67 MB of images written at 4096 tokens (the FP32 q|k|v this replaces were
-// 134 MB).  One CTA per (chunk, head vector), a warp per four tokens, a lane per four channels: the seven rows a warp
-// convolves are fetched at once, whole 256- or 512-byte segments, and every image row leaves as full 128-byte lines.
-// Rows a neighbouring warp fetches too come from L1; eight tokens a warp (256 threads) fetch less but leave 16 warps an
-// SM instead of 32, too few to cover the latency of HBM.
+// 67 MB of BF16 rows read and 67 MB of images written at 4096 tokens (the FP32 q|k|v this replaces were 134 MB), but
+// bound by instruction issue (62 % of the slots, DRAM 20 %, at four dims a lane).  One CTA per (chunk, head vector); the
+// lanes that share a row take four consecutive tokens, whose seven rows are fetched at once, and every image row leaves
+// as full 128-byte lines.  Rows that neighbouring lanes fetch too come from L1.
 
 #include "common.hpp"
 #include "gdn_chunk.hpp"
@@ -25,8 +24,14 @@
 namespace rib200 {
 namespace {
 
-constexpr int kImageThreads = 512;
-constexpr int kTokensPerWarp = kGdnChunk / (kImageThreads / 32);
+constexpr int kTokensPerRun = 4; // consecutive tokens of the lanes that share a row
+constexpr int kRuns = kGdnChunk / kTokensPerRun;
+// a lane has `Count` dims of a row; threads of a CTA and CTAs an SM should hold
+template <int Count> struct Layout {
+  static constexpr int kLanes = kGdnDim / Count;
+  static constexpr int kThreads = kRuns * kLanes;
+  static constexpr int kCtas = Count == 4 ? 2 : 3;
+};
 constexpr int kWidth = 4;
 constexpr int kGateHeads = 32; // value heads per gate CTA
 constexpr float kQkEpsilon = 1.0e-6F;
@@ -43,6 +48,7 @@ struct ImageParams {
   std::size_t q_stride, k_stride, v_stride;
   const float *beta, *log_decay; // [token][value head]
   GdnChunkScratch scratch;
+  std::uint32_t wide; // rows of 16-bit elements start on 16-byte boundaries
   std::uint32_t tokens, chunks, key_heads, value_heads;
 };
 
@@ -56,46 +62,62 @@ __device__ __forceinline__ float load_weight(const void *base, std::size_t index
   return __bfloat162float(static_cast<const __nv_bfloat16 *>(base)[index]);
 }
 
-// Four consecutive elements as they lie in memory, and as FP32.
-template <int Dtype> struct Quad;
-template <> struct Quad<RIB200_DTYPE_F32> {
+// `Count` consecutive elements of a row, four or (16-bit types) eight, as they lie in memory, and as FP32.  `wide`: rows
+// start on 16-byte boundaries (else eight elements come in two pieces).
+template <int Dtype, int Count> struct Piece;
+template <> struct Piece<RIB200_DTYPE_F32, 4> {
   float4 raw;
-  __device__ __forceinline__ void load(const void *base, std::size_t index) {
+  __device__ __forceinline__ void load(const void *base, std::size_t index, bool) {
     raw = *reinterpret_cast<const float4 *>(static_cast<const float *>(base) + index);
   }
   __device__ __forceinline__ void clear() { raw = make_float4(0.0F, 0.0F, 0.0F, 0.0F); }
-  __device__ __forceinline__ float4 value() const { return raw; }
-  static __device__ __forceinline__ float one(const void *base, std::size_t index) {
-    return static_cast<const float *>(base)[index];
+  __device__ __forceinline__ void value(float (&x)[4]) const {
+    x[0] = raw.x;
+    x[1] = raw.y;
+    x[2] = raw.z;
+    x[3] = raw.w;
   }
 };
-template <> struct Quad<RIB200_DTYPE_BF16> {
-  uint2 raw;
-  __device__ __forceinline__ void load(const void *base, std::size_t index) {
-    raw = *reinterpret_cast<const uint2 *>(static_cast<const __nv_bfloat16 *>(base) + index);
+template <int Dtype, int Count> struct Piece {
+  static_assert(Dtype == RIB200_DTYPE_BF16 || Dtype == RIB200_DTYPE_F16, "16-bit elements");
+  std::uint32_t raw[Count / 2];
+  __device__ __forceinline__ void load(const void *base, std::size_t index, bool wide) {
+    const std::uint16_t *src = static_cast<const std::uint16_t *>(base) + index;
+    if constexpr (Count == 8) {
+      if (wide) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(src);
+        raw[0] = v.x;
+        raw[1] = v.y;
+        raw[2] = v.z;
+        raw[3] = v.w;
+        return;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < Count / 4; ++h) {
+      const uint2 v = *reinterpret_cast<const uint2 *>(src + 4 * h);
+      raw[2 * h] = v.x;
+      raw[2 * h + 1] = v.y;
+    }
   }
-  __device__ __forceinline__ void clear() { raw = make_uint2(0U, 0U); }
-  __device__ __forceinline__ float4 value() const {
-    return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xFFFF0000U),
-                       __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xFFFF0000U));
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < Count / 2; ++i) {
+      raw[i] = 0U;
+    }
   }
-  static __device__ __forceinline__ float one(const void *base, std::size_t index) {
-    return __bfloat162float(static_cast<const __nv_bfloat16 *>(base)[index]);
-  }
-};
-template <> struct Quad<RIB200_DTYPE_F16> {
-  uint2 raw;
-  __device__ __forceinline__ void load(const void *base, std::size_t index) {
-    raw = *reinterpret_cast<const uint2 *>(static_cast<const __half *>(base) + index);
-  }
-  __device__ __forceinline__ void clear() { raw = make_uint2(0U, 0U); }
-  __device__ __forceinline__ float4 value() const {
-    const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&raw.x));
-    const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&raw.y));
-    return make_float4(lo.x, lo.y, hi.x, hi.y);
-  }
-  static __device__ __forceinline__ float one(const void *base, std::size_t index) {
-    return __half2float(static_cast<const __half *>(base)[index]);
+  __device__ __forceinline__ void value(float (&x)[Count]) const {
+#pragma unroll
+    for (int i = 0; i < Count / 2; ++i) {
+      if constexpr (Dtype == RIB200_DTYPE_BF16) {
+        x[2 * i] = __uint_as_float(raw[i] << 16);
+        x[2 * i + 1] = __uint_as_float(raw[i] & 0xFFFF0000U);
+      } else {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(&raw[i]));
+        x[2 * i] = v.x;
+        x[2 * i + 1] = v.y;
+      }
+    }
   }
 };
 
@@ -125,10 +147,12 @@ __device__ __forceinline__ unsigned char *record_of(const ImageParams &p, std::u
 }
 
 // Gates of 32 value heads over one chunk: the running sum of the log decays and beta, zero past the last token.
-template <int Dtype, bool Layer>
+template <int Dtype, int Count, bool Layer>
 __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t chunk, std::uint32_t head0) {
   __shared__ float s_decay[kGdnChunk][kGateHeads + 1];
   __shared__ float s_beta[kGdnChunk][kGateHeads + 1];
+  constexpr int kWarps = Layout<Count>::kThreads / 32;
+  constexpr int kTokensPerWarp = kGdnChunk / kWarps;
   const std::uint32_t warp = threadIdx.x >> 5;
   const std::uint32_t lane = threadIdx.x & 31;
   const std::uint32_t head = head0 + lane;
@@ -148,8 +172,8 @@ __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t 
       if (tok < p.tokens) {
         if constexpr (Layer) {
           const std::size_t at = static_cast<std::size_t>(tok) * p.token_stride + p.conv_dim;
-          const float b = Quad<Dtype>::one(p.input, at + head);
-          const float a = Quad<Dtype>::one(p.input, at + p.value_heads + head);
+          const float b = load_weight(p.input, at + head, Dtype);
+          const float a = load_weight(p.input, at + p.value_heads + head, Dtype);
           beta = 1.0F / (1.0F + expf(-b));
           decay = coefficient * softplus(a + dt);
         } else {
@@ -163,7 +187,7 @@ __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t 
     }
   }
   __syncthreads();
-  for (std::uint32_t h = warp; h < kGateHeads && head0 + h < p.value_heads; h += kImageThreads / 32) {
+  for (std::uint32_t h = warp; h < kGateHeads && head0 + h < p.value_heads; h += kWarps) {
     float a = s_decay[lane][h];
     float b = s_decay[lane + 32][h];
 #pragma unroll
@@ -185,7 +209,8 @@ __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t 
 }
 
 // grid (chunks x (2 Hk + Hv head vectors + gate CTAs)), the chunk slowest: the CTAs of a chunk read the same rows
-template <int Dtype, bool Layer> __global__ void __launch_bounds__(kImageThreads, 2) gdn_image_kernel(const ImageParams p) {
+template <int Dtype, int Count, bool Layer>
+__global__ void __launch_bounds__(Layout<Count>::kThreads, Layout<Count>::kCtas) gdn_image_kernel(const ImageParams p) {
   grid_dependents_may_launch(); // the chunk kernels set themselves up early and wait for this grid to end
   grid_dependency_wait();
   const std::uint32_t vectors = 2 * p.key_heads + p.value_heads;
@@ -193,118 +218,161 @@ template <int Dtype, bool Layer> __global__ void __launch_bounds__(kImageThreads
   const std::uint32_t chunk = blockIdx.x / per_chunk;
   const std::uint32_t vec = blockIdx.x - chunk * per_chunk;
   if (vec >= vectors) {
-    gate_arrays<Dtype, Layer>(p, chunk, (vec - vectors) * kGateHeads);
+    gate_arrays<Dtype, Count, Layer>(p, chunk, (vec - vectors) * kGateHeads);
     return;
   }
   const std::uint32_t warp = threadIdx.x >> 5;
   const std::uint32_t lane = threadIdx.x & 31;
-  const std::uint32_t row0 = warp * kTokensPerWarp;
+  constexpr std::uint32_t kLanes = Layout<Count>::kLanes;
+  const std::uint32_t sub = threadIdx.x % kLanes; // a lane has dims Count sub .. Count sub + Count - 1
+  const std::uint32_t row0 = threadIdx.x / kLanes * kTokensPerRun;
   const std::uint32_t tok0 = chunk * kGdnChunk + row0;
   const bool is_q = vec < p.key_heads;
   const bool is_v = vec >= 2 * p.key_heads;
   const std::uint32_t head = is_q ? vec : (is_v ? vec - 2 * p.key_heads : vec - p.key_heads);
+  const bool wide = p.wide != 0;
+  const bool whole = (chunk + 1) * kGdnChunk <= p.tokens; // no row of the chunk is past the last token
 
-  float4 out[kTokensPerWarp];
+  float out[kTokensPerRun][Count];
   if constexpr (Layer) {
-    const std::uint32_t channel = vec * kGdnDim + 4 * lane;
-    // rows tok0 - 3 .. tok0 + 7
-    Quad<Dtype> x[kTokensPerWarp + kWidth - 1];
+    const std::uint32_t channel = vec * kGdnDim + Count * sub;
+    // rows tok0 - 3 .. tok0 + 3
+    Piece<Dtype, Count> x[kTokensPerRun + kWidth - 1];
+    if (whole && chunk > 0) {
+      const std::size_t first = static_cast<std::size_t>(tok0 - (kWidth - 1)) * p.token_stride + channel;
 #pragma unroll
-    for (int r = 0; r < kTokensPerWarp + kWidth - 1; ++r) {
-      const long long tok = static_cast<long long>(tok0) + r - (kWidth - 1);
-      if (tok >= 0 && tok < static_cast<long long>(p.tokens)) {
-        x[r].load(p.input, static_cast<std::size_t>(tok) * p.token_stride + channel);
-      } else {
-        x[r].clear();
-      }
-    }
-    float w[4][kWidth]; // taps of the lane's four channels, oldest first
-    if (p.weight_dtype == RIB200_DTYPE_F32) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float4 taps = *reinterpret_cast<const float4 *>(static_cast<const float *>(p.conv_weight) +
-                                                              static_cast<std::size_t>(channel + c) * kWidth);
-        w[c][0] = taps.x;
-        w[c][1] = taps.y;
-        w[c][2] = taps.z;
-        w[c][3] = taps.w;
+      for (int r = 0; r < kTokensPerRun + kWidth - 1; ++r) {
+        x[r].load(p.input, first + static_cast<std::size_t>(r) * p.token_stride, wide);
       }
     } else {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-#pragma unroll
-        for (int h = 0; h < kWidth; ++h) {
-          w[c][h] = load_weight(p.conv_weight, static_cast<std::size_t>(channel + c) * kWidth + h, p.weight_dtype);
+      for (int r = 0; r < kTokensPerRun + kWidth - 1; ++r) {
+        const int tok = static_cast<int>(tok0) + r - (kWidth - 1);
+        if (tok >= 0 && tok < static_cast<int>(p.tokens)) {
+          x[r].load(p.input, static_cast<std::size_t>(tok) * p.token_stride + channel, wide);
+        } else {
+          x[r].clear();
         }
       }
     }
-    float4 before[kWidth - 1]; // the three rows in front of the warp's own
+    // Taps through shared memory, by tap: a lane's channels are 64 or 128 bytes apart in memory, and fetched from there
+    // the weights took several times the L1 wavefronts of the rows.  Pieces of four channels, even ones first.
+    __shared__ __align__(16) float s_taps[kWidth][kGdnDim];
+    if (threadIdx.x < kGdnDim) {
+      const std::uint32_t c = threadIdx.x;
+      const std::size_t at = (static_cast<std::size_t>(vec) * kGdnDim + c) * kWidth;
+      const std::uint32_t place = Count == 8 ? ((c >> 2) & 1U) * (kGdnDim / 2) + (c >> 3) * 4 + (c & 3U) : c;
+      if (p.weight_dtype == RIB200_DTYPE_F32) {
+        const float4 taps = *reinterpret_cast<const float4 *>(static_cast<const float *>(p.conv_weight) + at);
+        s_taps[0][place] = taps.x;
+        s_taps[1][place] = taps.y;
+        s_taps[2][place] = taps.z;
+        s_taps[3][place] = taps.w;
+      } else {
+#pragma unroll
+        for (int h = 0; h < kWidth; ++h) {
+          s_taps[h][place] = load_weight(p.conv_weight, at + h, p.weight_dtype);
+        }
+      }
+    }
+    __syncthreads();
+    float w[Count][kWidth]; // taps of the lane's channels, oldest first
+#pragma unroll
+    for (int h = 0; h < kWidth; ++h) {
+#pragma unroll
+      for (int q = 0; q < Count / 4; ++q) {
+        const float4 taps = *reinterpret_cast<const float4 *>(&s_taps[h][q * (kGdnDim / 2) + 4 * sub]);
+        w[4 * q][h] = taps.x;
+        w[4 * q + 1][h] = taps.y;
+        w[4 * q + 2][h] = taps.z;
+        w[4 * q + 3][h] = taps.w;
+      }
+    }
+    float before[kWidth - 1][Count]; // the three rows in front of the run
 #pragma unroll
     for (int h = 0; h < kWidth - 1; ++h) {
-      before[h] = x[h].value();
+      x[h].value(before[h]);
     }
     if (tok0 == 0) { // history [channel][3]: element h is the token 3 - h steps before this call's first one
       const float *hist = p.history + static_cast<std::size_t>(channel) * (kWidth - 1);
 #pragma unroll
       for (int h = 0; h < kWidth - 1; ++h) {
-        before[h] = make_float4(hist[h], hist[(kWidth - 1) + h], hist[2 * (kWidth - 1) + h], hist[3 * (kWidth - 1) + h]);
+#pragma unroll
+        for (int c = 0; c < Count; ++c) {
+          before[h][c] = hist[c * (kWidth - 1) + h];
+        }
       }
     }
 #pragma unroll
-    for (int i = 0; i < kTokensPerWarp; ++i) {
-      const float4 now = x[i + kWidth - 1].value();
-      // the reference adds the current token's tap first, then the history taps oldest first
-      float4 sum = make_float4(now.x * w[0][3], now.y * w[1][3], now.z * w[2][3], now.w * w[3][3]);
+    for (int i = 0; i < kTokensPerRun; ++i) {
+      float now[Count];
+      x[i + kWidth - 1].value(now);
 #pragma unroll
-      for (int h = 0; h < kWidth - 1; ++h) {
-        sum.x += before[h].x * w[0][h];
-        sum.y += before[h].y * w[1][h];
-        sum.z += before[h].z * w[2][h];
-        sum.w += before[h].w * w[3][h];
+      for (int c = 0; c < Count; ++c) {
+        // the reference adds the current token's tap first, then the history taps oldest first
+        float sum = now[c] * w[c][3];
+#pragma unroll
+        for (int h = 0; h < kWidth - 1; ++h) {
+          sum += before[h][c] * w[c][h];
+        }
+        before[0][c] = before[1][c];
+        before[1][c] = before[2][c];
+        before[2][c] = now[c];
+        out[i][c] = silu_fast(sum);
       }
-      before[0] = before[1];
-      before[1] = before[2];
-      before[2] = now;
-      out[i] = make_float4(silu_fast(sum.x), silu_fast(sum.y), silu_fast(sum.z), silu_fast(sum.w));
-      if (tok0 + i >= p.tokens) { // rows past the last token are inert
-        out[i] = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+    }
+    if (!whole) { // rows past the last token are inert
+#pragma unroll
+      for (int i = 0; i < kTokensPerRun; ++i) {
+#pragma unroll
+        for (int c = 0; c < Count; ++c) {
+          out[i][c] = tok0 + i < p.tokens ? out[i][c] : 0.0F;
+        }
       }
     }
     if (!is_v) {
       const float q_scale = is_q ? rsqrtf(static_cast<float>(kGdnDim)) : 1.0F;
-      float squares[kTokensPerWarp];
+      float squares[kTokensPerRun];
 #pragma unroll
-      for (int i = 0; i < kTokensPerWarp; ++i) {
-        squares[i] = (out[i].x * out[i].x + out[i].y * out[i].y) + (out[i].z * out[i].z + out[i].w * out[i].w);
+      for (int i = 0; i < kTokensPerRun; ++i) {
+        squares[i] = 0.0F;
+#pragma unroll
+        for (int c = 0; c < Count; c += 4) {
+          squares[i] += (out[i][c] * out[i][c] + out[i][c + 1] * out[i][c + 1]) +
+                        (out[i][c + 2] * out[i][c + 2] + out[i][c + 3] * out[i][c + 3]);
+        }
       }
 #pragma unroll
-      for (int offset = 16; offset > 0; offset >>= 1) {
+      for (int offset = static_cast<int>(kLanes) / 2; offset > 0; offset >>= 1) {
 #pragma unroll
-        for (int i = 0; i < kTokensPerWarp; ++i) {
+        for (int i = 0; i < kTokensPerRun; ++i) {
           squares[i] += __shfl_xor_sync(0xFFFFFFFFU, squares[i], offset);
         }
       }
 #pragma unroll
-      for (int i = 0; i < kTokensPerWarp; ++i) {
+      for (int i = 0; i < kTokensPerRun; ++i) {
         const float scale = rsqrtf(squares[i] + kQkEpsilon) * q_scale;
-        out[i] = make_float4(out[i].x * scale, out[i].y * scale, out[i].z * scale, out[i].w * scale);
+#pragma unroll
+        for (int c = 0; c < Count; ++c) {
+          out[i][c] *= scale;
+        }
       }
     }
   } else {
     const void *source = is_q ? p.q : (is_v ? p.v : p.k);
     const std::size_t stride = is_q ? p.q_stride : (is_v ? p.v_stride : p.k_stride);
-    Quad<Dtype> x[kTokensPerWarp];
+    Piece<Dtype, Count> x[kTokensPerRun];
 #pragma unroll
-    for (int i = 0; i < kTokensPerWarp; ++i) {
+    for (int i = 0; i < kTokensPerRun; ++i) {
       if (tok0 + i < p.tokens) {
-        x[i].load(source, static_cast<std::size_t>(tok0 + i) * stride + head * kGdnDim + 4 * lane);
+        x[i].load(source, static_cast<std::size_t>(tok0 + i) * stride + head * kGdnDim + Count * sub, wide);
       } else {
         x[i].clear();
       }
     }
 #pragma unroll
-    for (int i = 0; i < kTokensPerWarp; ++i) {
-      out[i] = x[i].value();
+    for (int i = 0; i < kTokensPerRun; ++i) {
+      x[i].value(out[i]);
     }
   }
 
@@ -312,22 +380,23 @@ template <int Dtype, bool Layer> __global__ void __launch_bounds__(kImageThreads
   std::uint32_t block;
   float scale = 1.0F;
   if (is_v) {
-    __shared__ float s_max[kImageThreads / 32];
+    constexpr int kWarps = Layout<Count>::kThreads / 32;
+    __shared__ float s_max[kWarps];
     float largest = 0.0F;
 #pragma unroll
-    for (int i = 0; i < kTokensPerWarp; ++i) {
-      largest = fmaxf(largest, fmaxf(fmaxf(fabsf(out[i].x), fabsf(out[i].y)), fmaxf(fabsf(out[i].z), fabsf(out[i].w))));
-    }
+    for (int i = 0; i < kTokensPerRun; ++i) {
 #pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-      largest = fmaxf(largest, __shfl_xor_sync(0xFFFFFFFFU, largest, offset));
+      for (int c = 0; c < Count; ++c) {
+        largest = fmaxf(largest, fabsf(out[i][c]));
+      }
     }
+    largest = __uint_as_float(__reduce_max_sync(0xFFFFFFFFU, __float_as_uint(largest)));
     if (lane == 0) {
       s_max[warp] = largest;
     }
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < kImageThreads / 32; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       largest = fmaxf(largest, s_max[w]);
     }
     // exponent e with largest in [2^e, 2^(e+1)); the scale is 2^(13 - e), kept away from the ends of the FP32 range
@@ -346,23 +415,45 @@ template <int Dtype, bool Layer> __global__ void __launch_bounds__(kImageThreads
             (is_q ? kGdnBlock : 0U); // the Q rows follow the K rows of a block
     block = kGdnKqBlock;
   }
-  // lane: dims 4 lane .. 4 lane + 3, half of the 16-byte piece (lane % 16) / 2 of block lane / 16
-  unsigned char *at = image + (lane >> 4) * block + (lane & 1U) * 8U;
+  // a lane's dims are a 16-byte piece of a row of the image (8 FP16), or half of one
+  const std::uint32_t dim = Count * sub;
+  unsigned char *at = image + (dim >> 6) * block + (dim & 7U) * 2U;
 #pragma unroll
-  for (int i = 0; i < kTokensPerWarp; ++i) {
+  for (int i = 0; i < kTokensPerRun; ++i) {
     const std::uint32_t row = row0 + i;
-    const std::uint32_t piece = ((lane & 15U) >> 1) ^ (row & 7U);
-    *reinterpret_cast<uint2 *>(at + row * kGdnRowBytes + (piece << 4)) =
-        make_uint2(pack_half(out[i].x * scale, out[i].y * scale), pack_half(out[i].z * scale, out[i].w * scale));
+    unsigned char *to = at + row * kGdnRowBytes + ((((dim & 63U) >> 3) ^ (row & 7U)) << 4);
+    std::uint32_t h[Count / 2];
+#pragma unroll
+    for (int c = 0; c < Count / 2; ++c) {
+      h[c] = pack_half(out[i][2 * c] * scale, out[i][2 * c + 1] * scale);
+    }
+    if constexpr (Count == 8) {
+      *reinterpret_cast<uint4 *>(to) = make_uint4(h[0], h[1], h[2], h[3]);
+    } else {
+      *reinterpret_cast<uint2 *>(to) = make_uint2(h[0], h[1]);
+    }
   }
 }
 
+template <int Dtype, int Count, bool Layer> void launch(const ImageParams &p, std::size_t ctas, cudaStream_t stream) {
+  launch_programmatic(gdn_image_kernel<Dtype, Count, Layer>, dim3(static_cast<unsigned int>(ctas)),
+                      dim3(Layout<Count>::kThreads), 0, stream, "gated-delta image launch", p);
+}
+
+// Eight dims a lane is fewer instructions, four is more warps a CTA.  4096 tokens BF16 (4160 CTAs) 193.9 us for the
+// layer call with four and 186.8 with eight; 149 tokens (195 CTAs) 22.1 and 22.9: eight from four waves on.  FP32 has
+// four always (eight would hold 32 bytes a row in registers: 1173 tokens in the executor's calls 127.3 and 134.9 us).
 template <int Dtype, bool Layer> void launch(const ImageParams &p, cudaStream_t stream) {
   const std::uint32_t gate_ctas = (p.value_heads + kGateHeads - 1) / kGateHeads;
   const std::size_t ctas = static_cast<std::size_t>(2 * p.key_heads + p.value_heads + gate_ctas) * p.chunks;
   require(ctas <= 0x7FFFFFFFU, "gated-delta prefill: too many tokens for one launch");
-  launch_programmatic(gdn_image_kernel<Dtype, Layer>, dim3(static_cast<unsigned int>(ctas)), dim3(kImageThreads), 0,
-                      stream, "gated-delta image launch", p);
+  if constexpr (Dtype != RIB200_DTYPE_F32) {
+    if (ctas >= 4 * 3 * 148) {
+      launch<Dtype, 8, Layer>(p, ctas, stream);
+      return;
+    }
+  }
+  launch<Dtype, 4, Layer>(p, ctas, stream);
 }
 
 void fill_sizes(ImageParams &p, void *workspace, std::uint32_t tokens, std::uint32_t key_heads,
@@ -386,6 +477,7 @@ void launch_gdn_layer_images(const GdnLayerArgs &a, void *workspace, cudaStream_
   p.conv_dim = (2 * a.key_heads + a.value_heads) * kGdnDim;
   p.token_stride = p.conv_dim + 2 * a.value_heads + a.value_heads * kGdnDim;
   p.weight_dtype = a.weight_dtype;
+  p.wide = p.token_stride % 8 == 0 && reinterpret_cast<std::uintptr_t>(a.input) % 16 == 0 ? 1U : 0U;
   fill_sizes(p, workspace, a.tokens, a.key_heads, a.value_heads);
   if (a.dtype == RIB200_DTYPE_F32) {
     launch<RIB200_DTYPE_F32, true>(p, stream);
@@ -406,6 +498,7 @@ void launch_gdn_core_images(const GdnCoreArgs &a, void *workspace, cudaStream_t 
   p.v_stride = a.v_stride;
   p.beta = a.beta;
   p.log_decay = a.log_decay;
+  p.wide = 1; // whole heads behind 16-byte aligned pointers
   fill_sizes(p, workspace, a.tokens, a.key_heads, a.value_heads);
   if (a.qkv_f32) {
     launch<RIB200_DTYPE_F32, false>(p, stream);
