@@ -827,6 +827,11 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
 // only decides how the partitions spread over the machine: with many partitions a CTA is a single warp (no
 // cross-warp merge, most CTAs resident); with few, more warps share a partition so that every SM has work and
 // each warp's chain of dependent steps is short.  All shapes are the same kernel template.
+//
+// A batch takes four warps a CTA from 149 CTAs on: its grid spans the longest cache, so many CTAs are empty, and four
+// warps finish a partition in a quarter of the steps.  Against one warp a CTA (864 CTAs, 9 ragged sequences up to 6000
+// tokens) 36.2 and 39.4 us, the same nine at full length 51.7 and 52.1, 24 sequences (1536 CTAs) 69.9 and 83.1, 64 up to
+// 32768 tokens 724.8 and 746.2; two warps a CTA gain on ragged batches (33.1) and lose on full ones (55.0).
 template <bool F32, bool Batched, class T> void configure_once() {
   static std::once_flag flags[64];
   int device = 0;
@@ -871,12 +876,14 @@ void launch_pair(const DecodeParams &params, dim3 partition_grid, dim3 combine_g
   const std::size_t ctas = static_cast<std::size_t>(partition_grid.x) * partition_grid.y * partition_grid.z;
   if (ctas <= 148) {
     launch_pair_tiled<F32, Batched, Tile<8, 3>>(params, partition_grid, combine_grid, combine, stream);
-  } else if (ctas <= 296) {
+  } else if (Batched || ctas <= 296) {
     launch_pair_tiled<F32, Batched, Tile<4, 3>>(params, partition_grid, combine_grid, combine, stream);
-  } else if (ctas <= 592) {
-    launch_pair_tiled<F32, Batched, Tile<2, 3>>(params, partition_grid, combine_grid, combine, stream);
-  } else {
-    launch_pair_tiled<F32, Batched, Tile<1, 3>>(params, partition_grid, combine_grid, combine, stream);
+  } else if constexpr (!Batched) {
+    if (ctas <= 592) {
+      launch_pair_tiled<F32, Batched, Tile<2, 3>>(params, partition_grid, combine_grid, combine, stream);
+    } else {
+      launch_pair_tiled<F32, Batched, Tile<1, 3>>(params, partition_grid, combine_grid, combine, stream);
+    }
   }
 }
 
