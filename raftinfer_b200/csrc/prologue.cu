@@ -26,7 +26,12 @@ namespace {
 
 constexpr int kMaxPairs = 128;
 constexpr int kPrologueThreads = 256;
-constexpr std::uint32_t kSpreadTokens = 64; // calls of up to this many tokens spread a token's vectors over CTAs
+// Calls of up to this many tokens spread a token's vectors over CTAs, a vector per warp (fused prologue 4.3 -> 2.5 us at
+// 1 token, 4.4 -> 2.9 at 96, 4.4 -> 3.8 at 128; at 256 tokens the angles computed again cost more, 5.2 -> 5.4).
+constexpr std::uint32_t kSpreadTokens = 128;
+// Calls of up to this many CTAs, one wave, ask for their operands in L2 before the dependent-launch wait: eight layers at
+// 777 tokens 124.7 -> 118.8 us.  In more waves the hints are traffic without a head start (4096 tokens 168.7 -> 187.1).
+constexpr std::uint32_t kHintCtas = 148;
 
 struct PrologueParams {
   // q: vectors of `q_heads` heads per token, `q_head_stride` elements apart (2 D when the gate is interleaved)
@@ -122,6 +127,31 @@ template <> struct Elements<__nv_bfloat16> {
   }
 };
 
+// L2 hints for what warp `vec` of a token reads first: lane l takes line l of its vector (and of the gate behind it)
+// and, for the first vectors, of the weights.
+__device__ __forceinline__ void hint_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+template <class In, class W, int HeadDim>
+__device__ __forceinline__ void hint_first(const PrologueParams &p, std::uint32_t token, std::uint32_t vec, int lane) {
+  constexpr int kLines = HeadDim * static_cast<int>(sizeof(In)) / 128;
+  constexpr int kWeightLines = HeadDim * static_cast<int>(sizeof(W)) / 128;
+  if (vec >= p.q_heads + 2 * p.kv_heads) {
+    return;
+  }
+  const bool is_q = vec < p.q_heads;
+  const bool is_v = vec >= p.q_heads + p.kv_heads;
+  const std::uint32_t head = is_q ? vec : (is_v ? vec - p.q_heads - p.kv_heads : vec - p.q_heads);
+  const In *base = static_cast<const In *>(is_q ? p.q_in : (is_v ? p.v_in : p.k_in));
+  const std::size_t at = is_q ? (static_cast<std::size_t>(token) * p.q_heads + head) * p.q_head_stride
+                              : (static_cast<std::size_t>(token) * p.kv_heads + head) * HeadDim;
+  const int lines = is_q && p.gate_out != nullptr ? 2 * kLines : kLines;
+  if (base != nullptr && lane < lines) {
+    hint_l2(base + at + lane * (HeadDim / kLines));
+  }
+  if (lane >= 32 - kWeightLines && !is_v) {
+    hint_l2(static_cast<const W *>(is_q ? p.q_weight : p.k_weight) + (lane - (32 - kWeightLines)) * (HeadDim / kWeightLines));
+  }
+}
+
 // In: projection dtype, W: norm-weight dtype, Out: output dtype, PerLane: head_dim / 32
 template <class In, class W, class Out, int PerLane>
 __global__ void __launch_bounds__(kPrologueThreads) attention_prologue_kernel(const PrologueParams p) {
@@ -142,6 +172,10 @@ __global__ void __launch_bounds__(kPrologueThreads) attention_prologue_kernel(co
   // start (the early cache fetch of a decode step) still has an ordinary launch between itself and older writers.
   // As plain launches the calls of a layer cost a launch latency each: eight layers of the executor's decode sequence
   // at 777 tokens 137.2 -> 131.7 us, at 32K 273.8 -> 258.4, a 2709-token prompt in its calls 412 -> 356.
+  // Until then a small call asks for its first vectors and the weights in L2 (hints, no reads).
+  if (gridDim.x * gridDim.y <= kHintCtas) {
+    hint_first<In, W, kHeadDimT>(p, token, blockIdx.y * (kPrologueThreads / 32) + warp, lane);
+  }
   grid_dependency_wait();
   grid_dependents_may_launch();
 
@@ -262,15 +296,19 @@ template <class T>
 __global__ void split_query_gate_kernel(const T *query_gate, T *query, T *gate, std::size_t total_vec,
                                         std::uint32_t vec_per_head) {
   // one thread per 16-byte piece of the output; dependent launch as in the kernel above
-  grid_dependency_wait();
-  grid_dependents_may_launch();
   const std::size_t index = static_cast<std::size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (index >= total_vec) {
-    return;
-  }
   const std::size_t head = index / vec_per_head;
   const std::size_t piece = index - head * vec_per_head;
   const uint4 *src = reinterpret_cast<const uint4 *>(query_gate) + head * 2 * vec_per_head + piece;
+  if (gridDim.x <= kHintCtas && index < total_vec && index % 8 == 0) { // a line each, a hint: nothing is read before the wait
+    hint_l2(src);
+    hint_l2(src + vec_per_head);
+  }
+  grid_dependency_wait();
+  grid_dependents_may_launch();
+  if (index >= total_vec) {
+    return;
+  }
   reinterpret_cast<uint4 *>(query)[index] = src[0];
   reinterpret_cast<uint4 *>(gate)[index] = src[vec_per_head];
 }
