@@ -422,6 +422,39 @@ constexpr int kStepSlices = 4;
 constexpr int kStepColumns = kDim / kStepSlices;
 constexpr std::uint32_t kStepMaxRatio = 2; // value heads per key head a portable cluster holds
 
+// While the kernels in front still run, a single-launch call asks for what it will read: its state rows, and a line per
+// eight channels of taps, history and input.  Hints, no reads: what those kernels write is current in L2 either way.
+__device__ __forceinline__ void hint_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+template <int Dtype, int WeightDtype>
+__device__ __forceinline__ void hint_operands(const LayerParams &p, std::uint32_t key_head, std::uint32_t head,
+                                              std::uint32_t slice) {
+  const auto *input = static_cast<const typename Scalar<Dtype>::Type *>(p.input);
+  const auto *taps = static_cast<const typename Scalar<WeightDtype>::Type *>(p.conv_weight);
+  const std::uint32_t tid = threadIdx.x;
+  auto channel_hints = [&](std::uint32_t channel) {
+    hint_l2(taps + static_cast<std::size_t>(channel) * kFastWidth);
+    hint_l2(p.convolution_state + static_cast<std::size_t>(channel) * (kFastWidth - 1));
+    hint_l2(input + channel);
+  };
+  if (tid < kDim) {
+    hint_l2(p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns +
+            static_cast<std::size_t>(tid) * kDim);
+  } else if (tid < kDim + 32) { // q, then k channels of the key head
+    const std::uint32_t piece = tid - kDim;
+    channel_hints((piece < 16 ? 0 : p.key_heads * kDim) + key_head * kDim + (piece & 15U) * 8);
+  } else if (tid < kDim + 32 + 4) {
+    const std::uint32_t column = head * kDim + slice * kStepColumns + (tid - kDim - 32) * 8;
+    channel_hints(2 * p.key_heads * kDim + column);
+    hint_l2(input + p.conv_dim + 2 * p.value_heads + column);
+  } else if (tid == kDim + 64) {
+    hint_l2(input + p.conv_dim + head);
+    hint_l2(input + p.conv_dim + p.value_heads + head);
+    hint_l2(static_cast<const typename Scalar<WeightDtype>::Type *>(p.recurrent_a) + head);
+    hint_l2(static_cast<const typename Scalar<WeightDtype>::Type *>(p.dt_bias) + head);
+    hint_l2(static_cast<const typename Scalar<WeightDtype>::Type *>(p.output_norm_weight) + slice * kStepColumns);
+  }
+}
+
 template <int Dtype, int WeightDtype>
 __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const LayerParams p) {
   using Act = Scalar<Dtype>;
@@ -446,11 +479,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
   const int warp = tid >> 5;
   const int lane = tid & 31;
   float *state = p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns;
-  // The state slice is asked into L2 while the kernel in front of this one still runs; a prefetch is only a hint, the
-  // values are read after the wait.
-  if (tid < kDim) {
-    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(state + static_cast<std::size_t>(tid) * kDim));
-  }
+  hint_operands<Dtype, WeightDtype>(p, key_head, head, slice);
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
   grid_dependency_wait();
   grid_dependents_may_launch();
@@ -645,6 +674,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
 constexpr std::uint32_t kShortTile = 32;
 constexpr std::uint32_t kShortMaxTokens = 63; // longer calls run in chunks
 constexpr std::uint32_t kShortRounds = kShortTile / 8; // tokens per warp
+constexpr std::uint32_t kShortGroup = 4;               // tokens convolved together
 
 template <int Dtype, int WeightDtype>
 __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const LayerParams p) {
@@ -671,9 +701,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
   const std::uint32_t warp = tid >> 5;
   const std::uint32_t lane = tid & 31;
   float *state = p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns;
-  if (tid < kDim) { // a hint; the values are read after the wait
-    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(state + static_cast<std::size_t>(tid) * kDim));
-  }
+  hint_operands<Dtype, WeightDtype>(p, key_head, head, slice);
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
   grid_dependency_wait();
   grid_dependents_may_launch();
@@ -692,8 +720,8 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
   const std::uint32_t z_channel = p.conv_dim + 2 * p.value_heads + head * kDim + slice * kStepColumns + lane;
   float qk_weight[kFastWidth];
   float v_weight[kFastWidth];
-  float qk_before[kHistory]; // the three tokens in front of the tile
-  float v_history[kHistory]; // the three in front of the call
+  float qk_history[kHistory]; // the three tokens in front of the call
+  float v_history[kHistory];
 #pragma unroll
   for (int h = 0; h < kFastWidth; ++h) {
     qk_weight[h] = Weight::widen(conv_weight[static_cast<std::size_t>(qk_channel) * kFastWidth + h]);
@@ -701,67 +729,82 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
   }
 #pragma unroll
   for (int h = 0; h < kHistory; ++h) {
-    qk_before[h] = p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h];
+    qk_history[h] = p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h];
     v_history[h] = p.convolution_state[static_cast<std::size_t>(v_channel) * kHistory + h];
   }
   const float norm_weight =
       Weight::widen(static_cast<const WeightType *>(p.output_norm_weight)[slice * kStepColumns + lane]);
   const float coefficient = Weight::widen(static_cast<const WeightType *>(p.recurrent_a)[head]);
   const float dt = Weight::widen(static_cast<const WeightType *>(p.dt_bias)[head]);
-  auto v_row = [&](int tok) { // v of a token of this call, or of the history in front of it
-    return tok >= 0 ? Act::widen(input[static_cast<std::size_t>(tok) * p.token_stride + v_channel])
-                    : (tok == -1 ? v_history[2] : (tok == -2 ? v_history[1] : v_history[0]));
+  // a channel's input at a token of this call, or of the history in front of it
+  auto row = [&](std::uint32_t channel, const float (&history)[kHistory], int tok) {
+    return tok >= 0 ? Act::widen(input[static_cast<std::size_t>(tok) * p.token_stride + channel])
+                    : (tok == -1 ? history[2] : (tok == -2 ? history[1] : history[0]));
   };
+  const std::uint32_t last = p.tokens - 1;
 
   for (std::uint32_t first = 0, tile = 0; first < p.tokens; first += kShortTile, ++tile) {
     const std::uint32_t n = min(kShortTile, p.tokens - first);
-    // ---- convolution and SiLU: q and k a channel per thread, v and the gates a token per warp ----
+    // ---- convolution and SiLU: q and k a channel per thread, v and the gates a token per warp.  Whole groups of
+    // tokens without a branch, so that their long dependent chains overlap; rows past the last token are computed from
+    // it and not used. ----
     {
       ActType x[kShortTile];
 #pragma unroll
-      for (std::uint32_t t = 0; t < kShortTile; ++t) {
-        if (t < n) {
-          x[t] = input[static_cast<std::size_t>(first + t) * p.token_stride + qk_channel];
-        }
-      }
-      float v_value[kShortRounds];
+      for (std::uint32_t group = 0; group < kShortTile; group += kShortGroup) {
+        if (group < n) {
 #pragma unroll
-      for (std::uint32_t r = 0; r < kShortRounds; ++r) {
-        const std::uint32_t t = warp + 8 * r;
-        if (t < n) {
-          const int tok = static_cast<int>(first + t);
-          float sum = v_row(tok) * v_weight[kHistory]; // the current token's tap first, then the history, oldest first
-#pragma unroll
-          for (int h = 0; h < kHistory; ++h) {
-            sum += v_row(tok - kHistory + h) * v_weight[h];
-          }
-          v_value[r] = silu(sum);
-          if (lane == 0) {
-            const std::size_t gates = static_cast<std::size_t>(tok) * p.token_stride + p.conv_dim + head;
-            s_beta[t] = 1.0F / (1.0F + expf(-Act::widen(input[gates])));
-            s_decay[t] = expf(coefficient * softplus(Act::widen(input[gates + p.value_heads]) + dt));
+          for (std::uint32_t t = group; t < group + kShortGroup; ++t) {
+            x[t] = input[static_cast<std::size_t>(min(first + t, last)) * p.token_stride + qk_channel];
           }
         }
       }
+      float before[kHistory];
 #pragma unroll
-      for (std::uint32_t t = 0; t < kShortTile; ++t) {
-        if (t < n) {
-          const float now = Act::widen(x[t]);
-          float sum = now * qk_weight[kHistory];
-#pragma unroll
-          for (int h = 0; h < kHistory; ++h) {
-            sum += qk_before[h] * qk_weight[h];
-          }
-          qk_before[0] = qk_before[1];
-          qk_before[1] = qk_before[2];
-          qk_before[2] = now;
-          s_qk[tid >> 7][t][tid & (kDim - 1)] = silu(sum);
-        }
+      for (int h = 0; h < kHistory; ++h) {
+        before[h] = row(qk_channel, qk_history, static_cast<int>(first) - kHistory + h);
       }
 #pragma unroll
       for (std::uint32_t r = 0; r < kShortRounds; ++r) {
-        if (warp + 8 * r < n) {
-          s_v[warp + 8 * r][lane] = v_value[r];
+        if (8 * r < n) {
+          const std::uint32_t t = warp + 8 * r;
+          const int tok = static_cast<int>(min(first + t, last));
+          // the current token's tap first, then the history, oldest first
+          float sum = row(v_channel, v_history, tok) * v_weight[kHistory];
+#pragma unroll
+          for (int h = 0; h < kHistory; ++h) {
+            sum += row(v_channel, v_history, tok - kHistory + h) * v_weight[h];
+          }
+          s_v[t][lane] = silu(sum);
+        }
+      }
+      if (lane < kShortRounds && warp + 8 * lane < n) {
+        const std::uint32_t t = warp + 8 * lane;
+        const std::size_t gates = static_cast<std::size_t>(first + t) * p.token_stride + p.conv_dim + head;
+        s_beta[t] = 1.0F / (1.0F + expf(-Act::widen(input[gates])));
+        s_decay[t] = expf(coefficient * softplus(Act::widen(input[gates + p.value_heads]) + dt));
+      }
+#pragma unroll
+      for (std::uint32_t group = 0; group < kShortTile; group += kShortGroup) {
+        if (group < n) {
+          float value[kShortGroup];
+#pragma unroll
+          for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+            const float now = Act::widen(x[group + t]);
+            float sum = now * qk_weight[kHistory];
+#pragma unroll
+            for (int h = 0; h < kHistory; ++h) {
+              sum += before[h] * qk_weight[h];
+            }
+            before[0] = before[1];
+            before[1] = before[2];
+            before[2] = now;
+            value[t] = silu(sum);
+          }
+#pragma unroll
+          for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+            s_qk[tid >> 7][group + t][tid & (kDim - 1)] = value[t];
+          }
         }
       }
     }
@@ -797,11 +840,18 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
     // after the three exchanges lane l holds the sum of column 2 (l / 8 % 2) + (l / 4) % 2, of S^T k below lane 16 and
     // of S^T q from there on
     const std::uint32_t my_column = ((lane >> 3) & 1U) * 2 + ((lane >> 2) & 1U);
+    float4 next_k = *reinterpret_cast<const float4 *>(&s_qk[1][0][4 * lane]);
+    float4 next_q = *reinterpret_cast<const float4 *>(&s_qk[0][0][4 * lane]);
     for (std::uint32_t t = 0; t < n; ++t) {
-      const float4 k4 = *reinterpret_cast<const float4 *>(&s_qk[1][t][4 * lane]);
-      const float4 q4 = *reinterpret_cast<const float4 *>(&s_qk[0][t][4 * lane]);
-      const float k[4] = {k4.x, k4.y, k4.z, k4.w};
-      const float q[4] = {q4.x, q4.y, q4.z, q4.w};
+      const float k[4] = {next_k.x, next_k.y, next_k.z, next_k.w};
+      const float q[4] = {next_q.x, next_q.y, next_q.z, next_q.w};
+      const float decay = s_decay[t];
+      const float beta = s_beta[t];
+      const float v_value = s_v[t][4 * warp + my_column];
+      const float kq = s_kq[t];
+      const std::uint32_t following = min(t + 1, kShortTile - 1);
+      next_k = *reinterpret_cast<const float4 *>(&s_qk[1][following][4 * lane]);
+      next_q = *reinterpret_cast<const float4 *>(&s_qk[0][following][4 * lane]);
       float a[4] = {};
       float b[4] = {};
 #pragma unroll
@@ -832,8 +882,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
       float sum = (odd ? two[1] : two[0]) + __shfl_xor_sync(0xFFFFFFFFU, odd ? two[0] : two[1], 4);
       sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 2);
       sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 1);
-      const float decay = s_decay[t];
-      const float delta = (s_v[t][4 * warp + my_column] - decay * sum) * s_beta[t]; // below lane 16
+      const float delta = (v_value - decay * sum) * beta; // below lane 16
       float correction[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -849,7 +898,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
       const float low = odd ? correction[1] : correction[0];
       const float high = odd ? correction[3] : correction[2];
       if (upper && (lane & 3U) == 0) {
-        s_out[t][4 * warp + my_column] = decay * sum + (high_pair ? high : low) * s_kq[t];
+        s_out[t][4 * warp + my_column] = decay * sum + (high_pair ? high : low) * kq;
       }
     }
     __syncthreads();
@@ -910,14 +959,15 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const Lay
   if (rank == 0) {
 #pragma unroll
     for (int h = 0; h < kHistory; ++h) {
-      p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h] = qk_before[h];
+      p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h] =
+          row(qk_channel, qk_history, static_cast<int>(p.tokens) - kHistory + h);
     }
   }
   if (warp == 0) {
 #pragma unroll
     for (int h = 0; h < kHistory; ++h) {
       p.convolution_state[static_cast<std::size_t>(v_channel) * kHistory + h] =
-          v_row(static_cast<int>(p.tokens) - kHistory + h);
+          row(v_channel, v_history, static_cast<int>(p.tokens) - kHistory + h);
     }
   }
 }
