@@ -96,7 +96,7 @@ enum : int {
   kBarQFree = 7 + 2 * kSlots,  // the tile's last score product has read Q
   kBarOFree = 8 + 2 * kSlots,  // the tile's epilogue has read O
   kBarDrain = 9 + 2 * kSlots,  // used once, by a CTA that has given up: its MMAs have drained
-  kBarPeerFull = 10 + 2 * kSlots, // split form: the partner's partial result has landed in this CTA's ring
+  kBarPeerFull = 10 + 2 * kSlots, // split form: the partner's half of its partial tile has landed in this CTA's ring
   kBarPeerFree = 11 + 2 * kSlots, // split form: the partner's ring may be written
   kBarStoresDone = 12 + 2 * kSlots, // split form: the producer's write-backs to the cache have read their slots
   kBarCount = 13 + 2 * kSlots
@@ -558,13 +558,18 @@ struct TileWalk {
 //
 // Split == true is for launches with so few (tile, head) items that half of the SMs would idle (a 512-token chunk
 // against a long past): the two CTAs of a cluster take the same item and each runs the ordinary single-CTA loop
-// over half of its key blocks; at the end the second CTA ships its unnormalised O tile and its (maximum, row sum)
-// into the first one's ring through distributed shared memory, and the first merges the two and writes the tile.
-// One item per cluster, so the ring is free when the partial arrives.
-constexpr int kLandingPitch = kHeadDim * 4 + 16;                 // bytes per row of a partial O tile in the ring
-constexpr int kLandingMeta = kTileRows * kLandingPitch;          // then [group][row] maximum, [group][row] row sum
-constexpr int kLandingBytes = kLandingMeta + 4 * kTileRows * 4;
-static_assert(kLandingBytes <= kSlots * kSlotBytes && kLandingBytes % 16 == 0, "partial tile must fit in the ring");
+// over half of its key blocks; at the end each of them ships half of its unnormalised O tile (128 of the 256 columns)
+// and the rows' maxima and sums into the other one's ring through distributed shared memory and finishes the columns
+// that it keeps.  One item per cluster, so the ring is free when the partial arrives.
+// (A copy between two SMs moves about 35 GB/s: the whole tile one way, with one CTA writing all of the output, took
+// twice as long.)
+constexpr int kLandingPitch = 128 * 4 + 16;                      // bytes per row of half a partial O tile
+constexpr int kLandingMeta = kTileRows * kLandingPitch;          // then [row] maximum, [group][row] row sum
+constexpr int kLandingBytes = kLandingMeta + 3 * kTileRows * 4;
+constexpr int kLandingOffset = 80 * 1024;                        // in the ring; what leaves is staged at its start
+static_assert(kLandingBytes <= kLandingOffset && kLandingOffset + kLandingBytes <= kSlots * kSlotBytes &&
+                  kLandingBytes % 16 == 0,
+              "both halves must fit in the ring");
 
 template <bool F32, bool Pair, bool Split>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -656,8 +661,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     tcgen05_fence_after();
   }
   if constexpr (Split) {
-    if (half == 0 && threadIdx.x == 0) {
-      mbar_expect_tx(bar(kBarPeerFull), kLandingBytes); // the partner's partial tile, one bulk copy
+    if (threadIdx.x == 0) {
+      mbar_expect_tx(bar(kBarPeerFull), kLandingBytes); // the partner's half of its partial tile, one bulk copy
     }
   }
   if (threadIdx.x == 0) {
@@ -1216,7 +1221,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const std::size_t dst_base =
           (static_cast<std::size_t>(row0 + row) * p.output_heads + p.output_head_offset + head) * kHeadDim +
           group * 128;
-      const bool live = row < rows;
+      const bool live = row < rows && !(Split && split_here && group != static_cast<int>(half));
       uint4 gate_raw[16]; // BF16 gates of this thread's 128 columns, fetched while the last PV is still running
       if constexpr (!F32) {
         if (live) {
@@ -1253,71 +1258,52 @@ __global__ void __launch_bounds__(kThreads, 1)
         RIB200_STAMP(1, 14); // last PV landed
         RIB200_STAMP_NS(0);
       }
-      if constexpr (Split) {
-        if (half == 1) {
-          // Second half of a split item: the unnormalised O rows, the maximum they are scaled against and the
-          // row-sum shares go to this CTA's own ring (its MMAs have left it), and from there to the first CTA's
-          // ring in one bulk copy through distributed shared memory, once that CTA's MMAs have left theirs.
-          unsigned char *stage = smem + kRingOffset;
-          if (threadIdx.x == 0) {
-            RIB200_STAMP_CTA2(0); // last PV landed
-          }
-          ok = mbar_wait(bar(kBarStoresDone), walk.iteration & 1U, abort_flag); // the cache write-backs are out
-          ok = __all_sync(0xFFFFFFFFU, ok);
-          if (!ok) {
-            break;
-          }
-          if (threadIdx.x == 0) {
-            RIB200_STAMP_CTA2(1); // write-backs out
-          }
+      float inv;
+      float own_weight = 1.0F;  // split form: factors that bring the two halves to a common maximum
+      float peer_weight = 0.0F;
+      const unsigned char *landed = smem + kRingOffset + kLandingOffset;
+      if (Split && split_here) {
+        // The two CTAs of a split item exchange half a tile: group 1 of the first one and group 0 of the second hand
+        // their 128 columns of unnormalised O, with the row's maximum and sums, to the partner, and the other groups
+        // finish the columns that they keep.  The ring is free for it: the MMAs have left it, and the write-backs have
+        // once the producer says so.
+        const std::uint32_t partner = half == 0 ? cta + half_stride : cta - half_stride;
+        ok = mbar_wait(bar(kBarStoresDone), walk.iteration & 1U, abort_flag);
+        ok = __all_sync(0xFFFFFFFFU, ok);
+        if (!ok) {
+          break;
+        }
+        mbar_arrive_cluster_release(map_to_rank(bar(kBarPeerFree), partner));
+        unsigned char *stage = smem + kRingOffset;
+        float *own_meta = reinterpret_cast<float *>(stage + kLandingMeta); // maximum, then the two groups' sums
+        own_meta[(1 + group) * kTileRows + row] = l_sum;
+        const bool ships = group != static_cast<int>(half);
+        if (ships) {
+          own_meta[row] = m_used;
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             std::uint32_t v[32];
             tmem_ld32(tmem_o + lane_base + group * 128 + c * 32, v);
             tmem_wait_ld();
-            uint4 *dst = reinterpret_cast<uint4 *>(stage + row * kLandingPitch + (group * 128 + c * 32) * 4);
+            uint4 *dst = reinterpret_cast<uint4 *>(stage + row * kLandingPitch + c * 128);
 #pragma unroll
             for (int e = 0; e < 32; e += 4) {
               dst[e / 4] = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
             }
           }
-          float *meta = reinterpret_cast<float *>(stage + kLandingMeta);
-          meta[group * kTileRows + row] = m_used;
-          meta[2 * kTileRows + group * kTileRows + row] = l_sum;
-          if (threadIdx.x == 0) {
-            RIB200_STAMP_CTA2(2); // staged
-          }
-          asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-          asm volatile("bar.sync 1, 256;\n" ::: "memory");
-          if (threadIdx.x == 0) {
-            ok = mbar_wait(bar(kBarPeerFree), walk.iteration & 1U, abort_flag);
-            RIB200_STAMP_CTA2(3); // partner's ring free
-            if (ok) {
-              bulk_copy_to_cluster(map_to_rank(ring, cta - half_stride), ring, kLandingBytes,
-                                   map_to_rank(bar(kBarPeerFull), cta - half_stride));
-            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        if (ships) {
+          if ((threadIdx.x & 127U) == 0 && mbar_wait(bar(kBarPeerFree), walk.iteration & 1U, abort_flag)) {
+            bulk_copy_to_cluster(map_to_rank(ring + kLandingOffset, partner), ring, kLandingBytes,
+                                 map_to_rank(bar(kBarPeerFull), partner));
           }
           tcgen05_fence_before();
           arrive_on_leader(kBarOFree);
           continue;
         }
-        // first half: every MMA of this CTA has completed, its ring is free for the partner's partial tile
-        if (split_here) {
-          mbar_arrive_cluster_release(map_to_rank(bar(kBarPeerFree), cta + half_stride));
-        }
-      }
-      // The row sum is the two groups' shares.  They pass through the half of the exchange area that the next
-      // block to run (the first of the next tile) does not use; the first barrier makes sure the partner has
-      // finished reading this tile's last maximum from it.
-      const std::uint32_t sums = ((g0 & 1U) ^ 1U) * 2;
-      asm volatile("bar.sync 1, 256;\n" ::: "memory");
-      exchange[(sums + group) * kTileRows + row] = l_sum;
-      asm volatile("bar.sync 1, 256;\n" ::: "memory");
-      float inv = 1.0F / (l_sum + exchange[(sums + (group ^ 1)) * kTileRows + row]);
-      float own_weight = 1.0F;  // split form: factors that bring the two halves to a common maximum
-      float peer_weight = 0.0F;
-      const unsigned char *landed = smem + kRingOffset;
-      if (Split && split_here) {
+        const float own_sum = own_meta[kTileRows + row] + own_meta[2 * kTileRows + row];
         ok = mbar_wait(bar(kBarPeerFull), walk.iteration & 1U, abort_flag);
         ok = __all_sync(0xFFFFFFFFU, ok);
         if (!ok) {
@@ -1329,12 +1315,21 @@ __global__ void __launch_bounds__(kThreads, 1)
           RIB200_STAMP_NS(1);
         }
         const float *meta = reinterpret_cast<const float *>(landed + kLandingMeta);
-        const float peer_max = meta[group * kTileRows + row];
-        const float peer_sum = meta[2 * kTileRows + row] + meta[3 * kTileRows + row];
+        const float peer_max = meta[row];
+        const float peer_sum = meta[kTileRows + row] + meta[2 * kTileRows + row];
         const float both = fmaxf(m_used, peer_max);
         own_weight = exp2f(m_used - both);
         peer_weight = exp2f(peer_max - both);
-        inv = 1.0F / (own_weight * (l_sum + exchange[(sums + (group ^ 1)) * kTileRows + row]) + peer_weight * peer_sum);
+        inv = 1.0F / (own_weight * own_sum + peer_weight * peer_sum);
+      } else {
+        // The row sum is the two groups' shares.  They pass through the half of the exchange area that the next
+        // block to run (the first of the next tile) does not use; the first barrier makes sure the partner has
+        // finished reading this tile's last maximum from it.
+        const std::uint32_t sums = ((g0 & 1U) ^ 1U) * 2;
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        exchange[(sums + group) * kTileRows + row] = l_sum;
+        asm volatile("bar.sync 1, 256;\n" ::: "memory");
+        inv = 1.0F / (l_sum + exchange[(sums + (group ^ 1)) * kTileRows + row]);
       }
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -1354,7 +1349,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tmem_wait_ld();
         if (Split && split_here) {
-          const float4 *peer = reinterpret_cast<const float4 *>(landed + row * kLandingPitch + (group * 128 + c * 32) * 4);
+          const float4 *peer = reinterpret_cast<const float4 *>(landed + row * kLandingPitch + c * 128);
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const float4 pv = peer[e / 4];
