@@ -392,7 +392,8 @@ __global__ void __launch_bounds__(kDim) gdn_epilogue_kernel(const LayerParams p)
 // ---- one token in one launch ---------------------------------------------------------------------------
 // A decode step of the layer is latency: 4 MiB of state traffic (0.6 us of HBM) and 25 KB of input.  The four launches
 // of the general path (prologue, history, recurrence, epilogue) cost 12.0 us a layer in a captured chain of 24 layers,
-// most of it hand-over between grids; this form costs 4.8 us (4.2 MB of state in and out: 0.88 TB/s, latency-bound).
+// most of it hand-over between grids; this form costs 3.6 us (4.2 MB of state in and out: 1.2 TB/s), 2.2
+// to 2.6 of kernel and the rest hand-over; 4.4 us without the L2 hints in front of the wait.
 //
 // A cluster serves one key head: four CTAs (32 state columns each) per value head that shares it, one or two value
 // heads.  Everything that has to meet across CTAs meets inside that cluster: the convolution history of the q and k
