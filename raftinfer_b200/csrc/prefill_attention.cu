@@ -84,6 +84,9 @@ constexpr float kRescaleThreshold = 8.0F;
 // (a rank's slice of the heads of a long prompt, tiles of 1 .. 32 blocks) the bar is higher.
 constexpr std::uint32_t kSplitMinBlocks = 4;
 constexpr std::uint32_t kSplitMinBlocksLate = 20;
+// ... and between four from here on, where half of the GPU stays free: 17 tokens behind 2688 (FP32, with the steps in
+// front) 33.6 us with two shares and 26.9 with four, 100 behind 4000 37.1 and 29.3; two tiles, 201 behind 1500, 28.8 and 29.0.
+constexpr std::uint32_t kQuarterMinBlocks = 8;
 
 // barrier indices (8 bytes each) inside the barrier block
 enum : int {
@@ -558,20 +561,30 @@ struct TileWalk {
 //
 // Split == true is for launches with so few (tile, head) items that half of the SMs would idle (a 512-token chunk
 // against a long past): the two CTAs of a cluster take the same item and each runs the ordinary single-CTA loop
-// over half of its key blocks; at the end each of them ships half of its unnormalised O tile (128 of the 256 columns)
-// and the rows' maxima and sums into the other one's ring through distributed shared memory and finishes the columns
-// that it keeps.  One item per cluster, so the ring is free when the partial arrives.
+// over half of its key blocks.  At the end every CTA keeps its share of the tile's columns, sends each of the others
+// their share of its unnormalised O tile, with the rows' maxima and sums, through distributed shared memory, and
+// finishes the columns that it keeps.  Parts == 4 does the same over four CTAs (or pairs) and quarters of the keys and
+// columns, for one or two tiles of a prompt's heads.  One item per cluster, so Q's area and the ring are free by then.
 // (A copy between two SMs moves about 35 GB/s: the whole tile one way, with one CTA writing all of the output, took
 // twice as long.)
-constexpr int kLandingPitch = 128 * 4 + 16;                      // bytes per row of half a partial O tile
-constexpr int kLandingMeta = kTileRows * kLandingPitch;          // then [row] maximum, [group][row] row sum
-constexpr int kLandingBytes = kLandingMeta + 3 * kTileRows * 4;
-constexpr int kLandingOffset = 80 * 1024;                        // in the ring; what leaves is staged at its start
-static_assert(kLandingBytes <= kLandingOffset && kLandingOffset + kLandingBytes <= kSlots * kSlotBytes &&
-                  kLandingBytes % 16 == 0,
-              "both halves must fit in the ring");
+constexpr int kStatBytes = 3 * kTileRows * 4; // [row] maximum, then [group][row] sum, in front of a message's rows
+template <int Parts> struct Exchange {
+  static constexpr int kPieces = 8 / Parts;                // pieces of 32 columns that a CTA keeps
+  static constexpr int kPitch = kPieces * 128 + 16;        // bytes per row
+  static constexpr int kBytes = kStatBytes + kTileRows * kPitch; // one message
+  static constexpr int kLanding = kQBytes + 48 * 1024;     // from the start of Q's area, where messages are staged
+  static_assert((Parts - 1) * kBytes <= kLanding && kLanding + (Parts - 1) * kBytes <= kRingOffset + kSlots * kSlotBytes &&
+                    kBytes % 16 == 0,
+                "messages out and in must fit");
+};
+template <> struct Exchange<1> {
+  static constexpr int kPieces = 8;
+  static constexpr int kPitch = 16;
+  static constexpr int kBytes = 16;
+  static constexpr int kLanding = 0;
+};
 
-template <bool F32, bool Pair, bool Split>
+template <bool F32, bool Pair, int Parts>
 __global__ void __launch_bounds__(kThreads, 1)
     prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                              const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap k_new_map,
@@ -593,13 +606,15 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int lane = threadIdx.x & 31;
   // A cluster is a pair of heads, a split of one item, or both: CTAs 0, 1 the pair that takes the first half of
   // the keys, CTAs 2, 3 the pair that takes the second half.
+  constexpr bool Split = Parts > 1;
+  using Message = Exchange<Parts>;
   constexpr bool kCluster = Pair || Split;
-  constexpr std::uint32_t kClusterSize = (Pair ? 2U : 1U) * (Split ? 2U : 1U);
+  constexpr std::uint32_t kClusterSize = (Pair ? 2U : 1U) * Parts;
   const std::uint32_t cta = kCluster ? cluster_rank() : 0U;
   const std::uint32_t rank = Pair ? cta & 1U : 0U;                  // place in the pair: 0 leads it
   const std::uint32_t lead_cta = Pair ? cta & ~1U : cta;            // cluster rank of the pair's leader
-  const std::uint32_t half = Split ? (Pair ? cta >> 1 : cta) : 0U;  // which half of the keys
-  const std::uint32_t half_stride = Pair ? 2U : 1U;                 // cluster ranks between the two halves
+  const std::uint32_t part = Split ? (Pair ? cta >> 1 : cta) : 0U;  // which share of the keys
+  const std::uint32_t part_stride = Pair ? 2U : 1U;                 // cluster ranks between two shares
   const std::uint32_t unit = blockIdx.x / kClusterSize;             // index of this cluster among its peers
   const std::uint32_t units = gridDim.x / kClusterSize;
   constexpr std::uint32_t kRowThreads = Pair ? 2 * kSoftmaxThreads : kSoftmaxThreads; // softmax threads per unit
@@ -617,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(bar(kBarQFree), 1);
     mbar_init(bar(kBarDrain), 1);
     mbar_init(bar(kBarPeerFull), 1);
-    mbar_init(bar(kBarPeerFree), kSoftmaxThreads);
+    mbar_init(bar(kBarPeerFree), Split ? (Parts - 1) * kSoftmaxThreads : 1);
     mbar_init(bar(kBarStoresDone), 1);
     mbar_init(bar(kBarOFree), kRowThreads);
     for (int s = 0; s < kSlots; ++s) {
@@ -660,11 +675,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("bar.sync 3, %0;\n" ::"n"(kThreads - 32) : "memory");
     tcgen05_fence_after();
   }
-  if constexpr (Split) {
-    if (threadIdx.x == 0) {
-      mbar_expect_tx(bar(kBarPeerFull), kLandingBytes); // the partner's half of its partial tile, one bulk copy
-    }
-  }
   if (threadIdx.x == 0) {
     RIB200_STAMP(0, 14); // set-up done
     RIB200_STAMP_NS(3);
@@ -681,23 +691,26 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto tile_blocks = [&](std::uint32_t tile) {
     return (p.past + tile * kTileRows + tile_rows(tile) - 1) / kBlockKeys + 1; // newest visible key / 128 + 1
   };
-  // the key blocks this CTA walks: all of them, or its half in the split form (the hand-over can only start when
-  // both halves are done, so equal halves are best)
+  // bytes of a message: only the tile's live rows travel
+  [[maybe_unused]] auto message_bytes = [&](std::uint32_t tile) {
+    return static_cast<std::uint32_t>(kStatBytes) + tile_rows(tile) * Message::kPitch;
+  };
+  // the key blocks this CTA walks: all of them, or its share in the split form (the exchange can only start when
+  // all shares are done, so equal shares are best)
   // A short item is not worth the hand-over: the first CTA (or pair) of the cluster then walks all of its blocks and
   // the second one sits the item out (it has no other: the split form launches one cluster per item).
   auto split_item = [&](std::uint32_t tile) { return Split && tile_blocks(tile) >= p.split_min_blocks; };
-  auto first_block = [&](std::uint32_t tile) {
-    return split_item(tile) && half == 1 ? (tile_blocks(tile) + 1) / 2 : 0U;
-  };
+  // share i of n blocks is [n i / Parts, n (i + 1) / Parts)
+  auto first_block = [&](std::uint32_t tile) { return split_item(tile) ? tile_blocks(tile) * part / Parts : 0U; };
   auto my_blocks = [&](std::uint32_t tile) {
     const std::uint32_t all = tile_blocks(tile);
     if (!Split) {
       return all;
     }
     if (!split_item(tile)) {
-      return half == 0 ? all : 0U;
+      return part == 0 ? all : 0U;
     }
-    return half == 0 ? (all + 1) / 2 : all - (all + 1) / 2;
+    return all * (part + 1) / Parts - all * part / Parts;
   };
 
   if (warp == kProducerWarp) {
@@ -1221,14 +1234,20 @@ __global__ void __launch_bounds__(kThreads, 1)
       const std::size_t dst_base =
           (static_cast<std::size_t>(row0 + row) * p.output_heads + p.output_head_offset + head) * kHeadDim +
           group * 128;
-      const bool live = row < rows && !(Split && split_here && group != static_cast<int>(half));
+      // the pieces of 32 columns (of the group's four) that this CTA writes
+      const int first_piece = Split && split_here ? max(0, static_cast<int>(part) * Message::kPieces - group * 4) : 0;
+      const int end_piece =
+          Split && split_here ? min(4, (static_cast<int>(part) + 1) * Message::kPieces - group * 4) : 4;
+      const bool live = row < rows && first_piece < end_piece;
       uint4 gate_raw[16]; // BF16 gates of this thread's 128 columns, fetched while the last PV is still running
       if constexpr (!F32) {
         if (live) {
           const uint4 *gp = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(p.gate) + out_base);
 #pragma unroll
           for (int i = 0; i < 16; i += 2) {
-            ld_global_v8(gp + i, gate_raw[i], gate_raw[i + 1]);
+            if (i / 4 >= first_piece && i / 4 < end_piece) {
+              ld_global_v8(gp + i, gate_raw[i], gate_raw[i + 1]);
+            }
           }
         }
       }
@@ -1237,14 +1256,17 @@ __global__ void __launch_bounds__(kThreads, 1)
       float4 gate_now[F32 ? 8 : 1];
       if constexpr (F32) {
         if (live) {
-          const float4 *gsrc = reinterpret_cast<const float4 *>(static_cast<const float *>(p.gate) + out_base);
+          const float4 *gsrc =
+              reinterpret_cast<const float4 *>(static_cast<const float *>(p.gate) + out_base) + first_piece * 8;
 #pragma unroll
           for (int i = 0; i < 8; i += 2) {
             ld_global_v8(gsrc + i, *reinterpret_cast<uint4 *>(&gate_now[i]), *reinterpret_cast<uint4 *>(&gate_now[i + 1]));
           }
 #pragma unroll
           for (int piece = 1; piece < 4; ++piece) {
-            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(gsrc + piece * 8));
+            if (first_piece + piece < end_piece) {
+              asm volatile("prefetch.global.L2 [%0];\n" ::"l"(gsrc + piece * 8));
+            }
           }
         }
       }
@@ -1259,33 +1281,44 @@ __global__ void __launch_bounds__(kThreads, 1)
         RIB200_STAMP_NS(0);
       }
       float inv;
-      float own_weight = 1.0F;  // split form: factors that bring the two halves to a common maximum
-      float peer_weight = 0.0F;
-      const unsigned char *landed = smem + kRingOffset + kLandingOffset;
+      float own_weight = 1.0F; // split form: factors that bring the shares to a common maximum
+      float peer_weights[Split ? Parts - 1 : 1];
       if (Split && split_here) {
-        // The two CTAs of a split item exchange half a tile: group 1 of the first one and group 0 of the second hand
-        // their 128 columns of unnormalised O, with the row's maximum and sums, to the partner, and the other groups
-        // finish the columns that they keep.  The ring is free for it: the MMAs have left it, and the write-backs have
-        // once the producer says so.
-        const std::uint32_t partner = half == 0 ? cta + half_stride : cta - half_stride;
+        // The ring and Q's area are free: the MMAs have left them, and the write-backs to the cache have once the
+        // producer says so.
+        const std::uint32_t in_pair = cta & (part_stride - 1);
+        const std::uint32_t bytes = message_bytes(walk.tile());
+        if (threadIdx.x == 0) {
+          mbar_expect_tx(bar(kBarPeerFull), (Parts - 1) * bytes); // a message from each of the others
+        }
         ok = mbar_wait(bar(kBarStoresDone), walk.iteration & 1U, abort_flag);
         ok = __all_sync(0xFFFFFFFFU, ok);
         if (!ok) {
           break;
         }
-        mbar_arrive_cluster_release(map_to_rank(bar(kBarPeerFree), partner));
-        unsigned char *stage = smem + kRingOffset;
-        float *own_meta = reinterpret_cast<float *>(stage + kLandingMeta); // maximum, then the two groups' sums
-        own_meta[(1 + group) * kTileRows + row] = l_sum;
-        const bool ships = group != static_cast<int>(half);
-        if (ships) {
-          own_meta[row] = m_used;
+        // message slot of CTA (or pair) `from` at `to`: the others in order
+        auto slot_of = [](std::uint32_t from, std::uint32_t to) { return from < to ? from : from - 1; };
+#pragma unroll
+        for (std::uint32_t to = 0; to < static_cast<std::uint32_t>(Parts); ++to) {
+          if (to != part) {
+            mbar_arrive_cluster_release(map_to_rank(bar(kBarPeerFree), to * part_stride + in_pair));
+            float *stat = reinterpret_cast<float *>(smem + slot_of(to, part) * Message::kBytes);
+            if (group == 0) {
+              stat[row] = m_used;
+            }
+            stat[(1 + group) * kTileRows + row] = l_sum;
+          }
+        }
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 4; ++c) {
+          const int piece = group * 4 + c;
+          const std::uint32_t to = static_cast<std::uint32_t>(piece / Message::kPieces);
+          if (to != part) {
             std::uint32_t v[32];
-            tmem_ld32(tmem_o + lane_base + group * 128 + c * 32, v);
+            tmem_ld32(tmem_o + lane_base + piece * 32, v);
             tmem_wait_ld();
-            uint4 *dst = reinterpret_cast<uint4 *>(stage + row * kLandingPitch + c * 128);
+            uint4 *dst = reinterpret_cast<uint4 *>(smem + slot_of(to, part) * Message::kBytes + kStatBytes +
+                                                   row * Message::kPitch + (piece % Message::kPieces) * 128);
 #pragma unroll
             for (int e = 0; e < 32; e += 4) {
               dst[e / 4] = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
@@ -1294,16 +1327,25 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("bar.sync 1, 256;\n" ::: "memory");
-        if (ships) {
-          if ((threadIdx.x & 127U) == 0 && mbar_wait(bar(kBarPeerFree), walk.iteration & 1U, abort_flag)) {
-            bulk_copy_to_cluster(map_to_rank(ring + kLandingOffset, partner), ring, kLandingBytes,
-                                 map_to_rank(bar(kBarPeerFull), partner));
+        // the copies leave from a group that may have nothing to write itself
+        if (threadIdx.x == (part < Parts / 2 ? 128U : 0U) && mbar_wait(bar(kBarPeerFree), walk.iteration & 1U, abort_flag)) {
+#pragma unroll
+          for (std::uint32_t to = 0; to < static_cast<std::uint32_t>(Parts); ++to) {
+            if (to != part) {
+              const std::uint32_t rank_to = to * part_stride + in_pair;
+              bulk_copy_to_cluster(map_to_rank(base + Message::kLanding + slot_of(part, to) * Message::kBytes, rank_to),
+                                   base + slot_of(to, part) * Message::kBytes, bytes,
+                                   map_to_rank(bar(kBarPeerFull), rank_to));
+            }
           }
+        }
+        if (first_piece >= end_piece) {
           tcgen05_fence_before();
           arrive_on_leader(kBarOFree);
           continue;
         }
-        const float own_sum = own_meta[kTileRows + row] + own_meta[2 * kTileRows + row];
+        const float *own_stat = reinterpret_cast<const float *>(smem); // any message's: they carry the same
+        const float own_sum = own_stat[kTileRows + row] + own_stat[2 * kTileRows + row];
         ok = mbar_wait(bar(kBarPeerFull), walk.iteration & 1U, abort_flag);
         ok = __all_sync(0xFFFFFFFFU, ok);
         if (!ok) {
@@ -1311,16 +1353,25 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         fence_cluster();
         if (threadIdx.x == 0 && walk.iteration == 0) {
-          RIB200_STAMP(1, 15); // partner's partial tile landed
+          RIB200_STAMP(1, 15); // the others' shares have landed
           RIB200_STAMP_NS(1);
         }
-        const float *meta = reinterpret_cast<const float *>(landed + kLandingMeta);
-        const float peer_max = meta[row];
-        const float peer_sum = meta[kTileRows + row] + meta[2 * kTileRows + row];
-        const float both = fmaxf(m_used, peer_max);
+        float both = m_used;
+#pragma unroll
+        for (int i = 0; i < Parts - 1; ++i) {
+          const float *stat = reinterpret_cast<const float *>(smem + Message::kLanding + i * Message::kBytes);
+          peer_weights[i] = stat[row];
+          both = fmaxf(both, peer_weights[i]);
+        }
         own_weight = exp2f(m_used - both);
-        peer_weight = exp2f(peer_max - both);
-        inv = 1.0F / (own_weight * own_sum + peer_weight * peer_sum);
+        float sum = own_weight * own_sum;
+#pragma unroll
+        for (int i = 0; i < Parts - 1; ++i) {
+          const float *stat = reinterpret_cast<const float *>(smem + Message::kLanding + i * Message::kBytes);
+          peer_weights[i] = exp2f(peer_weights[i] - both);
+          sum += peer_weights[i] * (stat[kTileRows + row] + stat[2 * kTileRows + row]);
+        }
+        inv = 1.0F / sum;
       } else {
         // The row sum is the two groups' shares.  They pass through the half of the exchange area that the next
         // block to run (the first of the next tile) does not use; the first barrier makes sure the partner has
@@ -1331,13 +1382,17 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("bar.sync 1, 256;\n" ::: "memory");
         inv = 1.0F / (l_sum + exchange[(sums + (group ^ 1)) * kTileRows + row]);
       }
-#pragma unroll
+      constexpr int kUnroll = F32 && Split ? 1 : 4; // BF16 gates sit in registers by piece
+#pragma unroll kUnroll
       for (int c = 0; c < 4; ++c) {
+        if (Split && (c < first_piece || c >= end_piece)) {
+          continue;
+        }
         std::uint32_t v[32];
         tmem_ld32(tmem_o + lane_base + group * 128 + c * 32, v);
         float4 gate_next[F32 ? 8 : 1];
         if constexpr (F32) {
-          if (live && c < 3) {
+          if (live && c + 1 < end_piece) {
             const float4 *gsrc =
                 reinterpret_cast<const float4 *>(static_cast<const float *>(p.gate) + out_base + (c + 1) * 32);
 #pragma unroll
@@ -1349,17 +1404,29 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tmem_wait_ld();
         if (Split && split_here) {
-          const float4 *peer = reinterpret_cast<const float4 *>(landed + row * kLandingPitch + c * 128);
+          const int column = (group * 4 + c) % Message::kPieces * 128;
 #pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            const float4 pv = peer[e / 4];
-            v[e] = __float_as_uint(__uint_as_float(v[e]) * own_weight + pv.x * peer_weight);
-            v[e + 1] = __float_as_uint(__uint_as_float(v[e + 1]) * own_weight + pv.y * peer_weight);
-            v[e + 2] = __float_as_uint(__uint_as_float(v[e + 2]) * own_weight + pv.z * peer_weight);
-            v[e + 3] = __float_as_uint(__uint_as_float(v[e + 3]) * own_weight + pv.w * peer_weight);
+          for (int e = 0; e < 32; ++e) {
+            v[e] = __float_as_uint(__uint_as_float(v[e]) * own_weight);
+          }
+#pragma unroll
+          for (int i = 0; i < Parts - 1; ++i) {
+            const float4 *peer = reinterpret_cast<const float4 *>(smem + Message::kLanding + i * Message::kBytes +
+                                                                  kStatBytes + row * Message::kPitch + column);
+            const float weight = peer_weights[i];
+            if (live) { // rows past the tile's last one have not been sent
+#pragma unroll
+              for (int e = 0; e < 32; e += 4) {
+                const float4 pv = peer[e / 4];
+                v[e] = __float_as_uint(__uint_as_float(v[e]) + pv.x * weight);
+                v[e + 1] = __float_as_uint(__uint_as_float(v[e + 1]) + pv.y * weight);
+                v[e + 2] = __float_as_uint(__uint_as_float(v[e + 2]) + pv.z * weight);
+                v[e + 3] = __float_as_uint(__uint_as_float(v[e + 3]) + pv.w * weight);
+              }
+            }
           }
         }
-        if (c == 3) {
+        if (c + 1 == end_piece) {
           // O has been read: the next tile's first PV may overwrite it
           tcgen05_fence_before();
           arrive_on_leader(kBarOFree);
@@ -1506,17 +1573,35 @@ CUtensorMap make_map(void *base, int rank, const cuuint64_t *dims, const cuuint6
   return map;
 }
 
-template <bool F32, bool Pair, bool Split> void configure_once() {
+// Returns the number of clusters of the split form that fit the device at once (0 for the other forms).
+template <bool F32, bool Pair, int Parts> int configure_once() {
   static std::once_flag flags[64];
+  static int clusters[64] = {};
   int device = 0;
   cuda_ok(cudaGetDevice(&device), "cudaGetDevice");
   require(device >= 0 && device < 64, "device ordinal out of range", RIB200_STATUS_INTERNAL);
-  std::call_once(flags[device], [] {
-    cuda_ok(cudaFuncSetAttribute(prefill_attention_kernel<F32, Pair, Split>,
+  std::call_once(flags[device], [&] {
+    cuda_ok(cudaFuncSetAttribute(prefill_attention_kernel<F32, Pair, Parts>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kSmemBytes),
             "prefill attention shared-memory opt-in");
+    if (Parts > 1) {
+      cudaLaunchAttribute shape{};
+      shape.id = cudaLaunchAttributeClusterDimension;
+      shape.val.clusterDim.x = (Pair ? 2 : 1) * Parts;
+      shape.val.clusterDim.y = 1;
+      shape.val.clusterDim.z = 1;
+      cudaLaunchConfig_t config{};
+      config.gridDim = dim3(shape.val.clusterDim.x, 1, 1);
+      config.blockDim = dim3(kThreads, 1, 1);
+      config.dynamicSmemBytes = kSmemBytes;
+      config.attrs = &shape;
+      config.numAttrs = 1;
+      cuda_ok(cudaOccupancyMaxActiveClusters(&clusters[device], prefill_attention_kernel<F32, Pair, Parts>, &config),
+              "prefill attention cluster count");
+    }
   });
+  return clusters[device];
 }
 
 // Builds made with -DRIB200_TUNING read two switches from the environment, for A/B timing of the kernel forms:
@@ -1542,8 +1627,8 @@ constexpr bool pair_form_enabled() { return true; }
 constexpr bool split_form_enabled() { return true; }
 #endif
 
-template <bool F32, bool Pair, bool Split> void launch(const PrefillArgs &a, cudaStream_t stream) {
-  configure_once<F32, Pair, Split>();
+template <bool F32, bool Pair, int Parts> void launch(const PrefillArgs &a, cudaStream_t stream) {
+  (void)configure_once<F32, Pair, Parts>();
   auto *cache = static_cast<__nv_bfloat16 *>(a.kv_cache);
   // The attention kernel itself writes the key blocks that lie wholly inside this chunk into the cache (BF16
   // inputs).  The append kernel covers the rest: every row for FP32 inputs, else the chunk's rows that share a key
@@ -1637,9 +1722,9 @@ template <bool F32, bool Pair, bool Split> void launch(const PrefillArgs &a, cud
   cuda_ok(cudaGetDevice(&device), "cudaGetDevice");
   cuda_ok(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device), "SM count query");
   const std::uint32_t sms = static_cast<std::uint32_t>(sm_count);
-  if (Split) {
+  if (Parts > 1) {
     // one item (or pair of heads) per cluster
-    config.gridDim = dim3(Pair ? 4 * params.tiles * (a.query_heads / 2) : 2 * params.tiles * a.query_heads, 1, 1);
+    config.gridDim = dim3(Parts * params.tiles * a.query_heads, 1, 1);
   } else if (Pair) {
     const std::uint32_t pair_items = params.tiles * (a.query_heads / 2);
     config.gridDim = dim3(2 * std::min<std::uint32_t>(pair_items, sms / 2), 1, 1);
@@ -1653,12 +1738,12 @@ template <bool F32, bool Pair, bool Split> void launch(const PrefillArgs &a, cud
   attributes[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attributes[0].val.programmaticStreamSerializationAllowed = 1;
   attributes[1].id = cudaLaunchAttributeClusterDimension;
-  attributes[1].val.clusterDim.x = (Pair ? 2 : 1) * (Split ? 2 : 1);
+  attributes[1].val.clusterDim.x = (Pair ? 2 : 1) * Parts;
   attributes[1].val.clusterDim.y = 1;
   attributes[1].val.clusterDim.z = 1;
   config.attrs = attributes;
-  config.numAttrs = Pair || Split ? 2 : 1;
-  cuda_ok(cudaLaunchKernelEx(&config, prefill_attention_kernel<F32, Pair, Split>, q_map, k_map, v_map, k_new_map, v_new_map, params),
+  config.numAttrs = Pair || Parts > 1 ? 2 : 1;
+  cuda_ok(cudaLaunchKernelEx(&config, prefill_attention_kernel<F32, Pair, Parts>, q_map, k_map, v_map, k_new_map, v_new_map, params),
           "prefill attention launch");
 }
 
@@ -1689,17 +1774,33 @@ void launch_prefill_attention(const PrefillArgs &args, cudaStream_t stream) {
   const std::uint32_t last_tile_blocks = (args.past_tokens + args.tokens - 1) / kBlockKeys + 1;
   const bool split = split_form_enabled() && 2 * tiles * args.query_heads <= static_cast<std::uint32_t>(sm_count) &&
                      (first_tile_blocks >= kSplitMinBlocks || last_tile_blocks >= kSplitMinBlocksLate);
+  // ... and between four where that still leaves half of the GPU free (one tile of the model's heads) and gives each two
+  // blocks at least.  (A CTA then writes less than the row segment that the head-sharded form forwards.)
+  const bool quarters = split && args.output_count <= 1 &&
+                        8 * tiles * args.query_heads <= static_cast<std::uint32_t>(sm_count) &&
+                        first_tile_blocks >= kQuarterMinBlocks;
   const bool pair = pair_form_enabled() && (args.query_heads / args.kv_heads) % 2 == 0;
   auto dispatch = [&](auto f32) {
     constexpr bool kF32 = decltype(f32)::value;
-    if (split && pair) {
-      launch<kF32, true, true>(args, stream);
+    // clusters of the quarter form that the device holds at once
+    auto quarters_fit = [&] {
+      const std::uint32_t fit = static_cast<std::uint32_t>(pair ? configure_once<kF32, true, 4>() : configure_once<kF32, false, 4>());
+      return tiles * args.query_heads / (pair ? 2 : 1) <= fit;
+    };
+    if (quarters && quarters_fit()) {
+      if (pair) {
+        launch<kF32, true, 4>(args, stream);
+      } else {
+        launch<kF32, false, 4>(args, stream);
+      }
+    } else if (split && pair) {
+      launch<kF32, true, 2>(args, stream);
     } else if (split) {
-      launch<kF32, false, true>(args, stream);
+      launch<kF32, false, 2>(args, stream);
     } else if (pair) {
-      launch<kF32, true, false>(args, stream);
+      launch<kF32, true, 1>(args, stream);
     } else {
-      launch<kF32, false, false>(args, stream);
+      launch<kF32, false, 1>(args, stream);
     }
   };
   if (args.activations_f32) {
