@@ -382,7 +382,7 @@ Rib200Status rib200_online_attention_decode_from_host(const void *host_token, vo
  * the kernel behind it become resident.  The caller promises in return that whatever wrote rows [0, past_tokens)
  * of that KV cache has completed, or is separated from this step by at least one ordinary kernel launch on the
  * stream (a kernel that does not release its dependents early; the decode kernels of this library do release them
- * early).  True for the reference's executor, where the previous writer of a layer's cache is the previous
+ * early, its other calls only once everything in front of them has ended, which serves as well).  True for the reference's executor, where the previous writer of a layer's cache is the previous
  * token's step, a whole model pass earlier; false for two steps enqueued directly one after the other on the same
  * cache with advancing positions.  The choice is per call: nothing is remembered between calls. */
 Rib200Status rib200_online_attention_decode_early_kv_fetch(const void *query, const void *key, const void *value,
