@@ -260,13 +260,13 @@ def gdn_packed_layer(dev, stream, hbm_peak, tensor_peak, tokens=4096, decode_ste
     res = {"prefill": {"tokens": tokens, "ms": ms, "cv": cv, "flops": flops, "TFLOP/s": flops / ms / 1e9,
                        "frac_of_measured_bf16_peak": flops / ms / 1e9 / tensor_peak, "io_bytes": io_bytes,
                        "io_GB/s": io_bytes / ms / 1e6,
-                       "note": "whole layer call: prologue (conv, SiLU, norms, gates), chunked recurrence, epilogue; "
+                       "note": "whole layer call: operand images (conv, SiLU, norms, gates), chunk products, chain with output norm; "
                                "time includes two state memsets"}}
     ms, cv = _graph_ms(decode, stream, decode_steps, warmup=3, reps=8)
     nbytes = 2 * HV * DK * DK * 4
     res["decode_step"] = {"ms": ms, "cv": cv, "bytes": nbytes, "effective GB/s": nbytes / ms / 1e6,
                           "steps_per_graph": decode_steps,
-                          "note": "single sequence, state L2-resident: latency of the three launches of a layer step"}
+                          "note": "single sequence, state L2-resident: latency of the one launch of a layer step"}
     return res
 
 

@@ -6,8 +6,10 @@
 //   epilogue  per-head RMSNorm(128) * weight * SiLU(z) (cpp/kernels/qwen35_delta.cu:579-621).
 // Unlike the reference's convolution kernel, which walks the tokens serially per channel, every
 // (token, head vector) pair is independent: a tap is read from the token stream or, for the first W-1
-// tokens, from the carried history.  conv_width 4 on aligned tensors takes the warp-per-vector kernels
-// (16-byte accesses); other widths and odd alignments take the one-CTA-per-vector kernels.
+// tokens, from the carried history.  These kernels are the general path: conv_width 4 on aligned tensors takes the
+// warp-per-vector ones (16-byte accesses), other widths and odd alignments the one-CTA-per-vector ones.  Calls of up to
+// 63 tokens with conv_width 4 and at most two value heads per key head are one launch (below), longer ones of that
+// width the chunk kernels (gdn_image.cu, gdn_chunk.cu).
 
 #include "common.hpp"
 
