@@ -342,12 +342,20 @@ __global__ void __launch_bounds__(Layout<Count>::kThreads, Layout<Count>::kCtas)
                         (out[i][c + 2] * out[i][c + 2] + out[i][c + 3] * out[i][c + 3]);
         }
       }
-#pragma unroll
-      for (int offset = static_cast<int>(kLanes) / 2; offset > 0; offset >>= 1) {
+      // the same order of additions for either layout, so that a row's image does not depend on the length of the call:
+      // four dims a lane first join the neighbour that completes eight
+      auto join = [&](int offset) {
 #pragma unroll
         for (int i = 0; i < kTokensPerRun; ++i) {
           squares[i] += __shfl_xor_sync(0xFFFFFFFFU, squares[i], offset);
         }
+      };
+      if constexpr (Count == 4) {
+        join(1);
+      }
+#pragma unroll
+      for (int offset = static_cast<int>(kLanes) / 2; offset > (Count == 4 ? 1 : 0); offset >>= 1) {
+        join(offset);
       }
 #pragma unroll
       for (int i = 0; i < kTokensPerRun; ++i) {
