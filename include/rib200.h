@@ -60,7 +60,8 @@ enum {
   RIB200_DEVICE_POSITION_OUT_OF_RANGE = 1u << 1,    /* *device_position >= max_context_tokens */
   RIB200_DEVICE_WAIT_TIMED_OUT = 1u << 2,           /* a bounded on-device wait gave up */
   RIB200_DEVICE_PAGE_OUT_OF_RANGE = 1u << 3,        /* a block table names a page the pool does not hold */
-  RIB200_DEVICE_POINTER_MISALIGNED = 1u << 4        /* a pointer read on the device is off its required boundary */
+  RIB200_DEVICE_POINTER_MISALIGNED = 1u << 4,       /* a pointer read on the device is off its required boundary */
+  RIB200_DEVICE_DECAY_OUT_OF_RANGE = 1u << 5        /* gated delta, 64 tokens or more: decays grow too much, see there */
 };
 
 /* cpp/kernels/qwen35_attention.cuh:14-21 */
@@ -226,10 +227,15 @@ Rib200Status rib200_gated_delta(const void *input, const void *conv_weight, cons
  * cpp/reference/qwen35.cpp:459-518) on operands that are already convolved and normalised:
  * q, k [tokens][key_heads][key_dim] (q carries 1/sqrt(key_dim)), v [tokens][value_heads][value_dim], all of
  * qkv_dtype (RIB200_DTYPE_BF16 or RIB200_DTYPE_F32); beta and log_decay FP32 [tokens][value_heads]
- * (beta in (0,1), decay = exp(log_decay)); state FP32 [value_heads][key_dim][value_dim] updated in place;
+ * (|k| <= 1, beta in [0,1], decay = exp(log_decay)); state FP32 [value_heads][key_dim][value_dim] updated in place;
  * out FP32 [tokens][value_heads][value_dim] (the vector before the output norm).  The key head of value
  * head h is h % key_heads.  tokens < 64 run the recurrent kernel (one pass over the state per token);
- * longer runs use the chunk-64 WY-form prefill and need rib200_gdn_core_workspace_bytes of scratch.
+ * longer runs use the chunk-64 WY-form prefill and need rib200_gdn_core_workspace_bytes of scratch.  Its products take
+ * operands of eleven significant bits, scaled so that values and states may have any magnitude, in every column (last
+ * index of v and state) for itself; it relies on |k| <= 1 and beta in [0,1].  Log decays are negative as a rule; positive
+ * ones may add up to a factor of 2^20 inside a run of 64 tokens (a chunk), beyond which results lose precision and
+ * RIB200_DEVICE_DECAY_OUT_OF_RANGE is set.  The same holds for rib200_gated_delta, whose log decay is
+ * recurrent_a * softplus(a + dt_bias).
  * key_dim == value_dim == 128 only. */
 Rib200Status rib200_gdn_core_workspace_bytes(size_t tokens, size_t key_heads, size_t value_heads, size_t key_dim,
                                              size_t value_dim, size_t *bytes);

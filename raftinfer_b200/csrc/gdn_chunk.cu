@@ -9,8 +9,9 @@
 //   Delta = U - W S0
 //   O     = diag(exp(G)) Q S0 + P Delta,         P_ij = exp(G_i - G_j) (q_i . k_j) for j <= i
 //   S_C   = exp(G_C) S0 + K^T diag(exp(G_C - G)) Delta
-// Every decay factor is exp of a non-positive number.  A ragged last chunk is padded with inert rows
-// (beta = 0, log decay = 0, k = q = v = 0), which leave the state untouched.
+// |k| <= 1, |q| <= 1 and 0 <= beta <= 1 are assumed.  Decays usually are at most 1; where log decays are positive, the
+// largest product of consecutive ones in a chunk (`growth`) enters the scales below.  A ragged last chunk is padded with
+// inert rows (beta = 0, log decay = 0, k = q = v = 0), which leave the state untouched.
 //
 // Three kernels: gdn_image.cu leaves K, Q and V as FP16 operand images and the gates as arrays; `prepare`, parallel over
 // (chunk, value head), makes W, U and P of them; `chain` walks the chunks of one (value head, 32-column slice of the
@@ -18,9 +19,12 @@
 //
 // Products run on tcgen05 with FP16 operands and FP32 accumulators: the 10-bit mantissa of TF32, half its bytes, and
 // - unlike 32-bit elements - one image serves as K-major and as MN-major operand, so K, Q and V are never transposed
-// and K is never copied with its decays (the decay goes to the rows of Delta).  What could leave FP16's range is scaled
-// by powers of two: V per (chunk, head), Delta and the state per (chunk, slice) from bounds that are known before they
-// are formed; FP32 copies of state and U are kept, and every factor is divided out in FP32.
+// and K is never copied with its decays (the decay goes to the rows of Delta).  TF32 has FP32's range and FP16 has not, so
+// every operand is scaled by powers of two that are divided out in FP32: K, Q, T, W and P, whose elements are at most 1
+// (times growth), by the fixed units of gdn_chunk.hpp; V, Delta and the state, which may have any magnitude, by a factor
+// per (chunk, head, column) from bounds that are known before they are formed.  The columns of V, Delta and the state
+// never meet in a product, so a column loses nothing to the size of another; within a column an element keeps its ten
+// bits down to 2^-27 of the chunk's bound.  FP32 copies of state and U are kept.
 //
 // Dense flops per launch: chunks * value_heads * [2 C^2 (3 dk + 2 dv) + 6 C dk dv].
 
@@ -274,10 +278,11 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const std::uint32_t (&a)[
 //            (a warp reads 32 rows x 32 columns of tensor memory; decay_ij = exp(G_i - G_j) is one exponential per
 //            element in the two squares on the diagonal, in the one below it the product of a row and a column factor
 //            taken against the running sum at the end of the block of 16 columns, both <= 1)
-//   T        = (I + A)^-1 to 22 bits: the four diagonal 16 x 16 blocks by back substitution in FP32 (a row per thread),
-//            then the blocks below them by doubling, -M22^-1 M21 M11^-1, on warp-level tensor tiles with operands split
-//            in two FP16 parts.  The tiles work on the transposed products, (T11^T A21^T) T22^T: the first product's
-//            accumulators are then the second one's A operand, so no intermediate leaves the registers.
+//   T        = (I + A)^-1: the four diagonal 16 x 16 blocks by back substitution in FP32 (a row per thread), then the
+//            blocks below them by doubling, -M22^-1 M21 M11^-1, on warp-level tensor tiles with operands split in two
+//            FP16 parts; A and T are held times 2^14 u there, so that the parts of an element carry 22 bits down to
+//            2^-17 and an absolute 2^-39 below.  The tiles work on the transposed products, (T11^T A21^T) T22^T: the
+//            first product's accumulators are then the second one's A operand, so no intermediate leaves the registers.
 //   [W; *]   = [T diag(beta gamma); T diag(beta)] K      M 128, N 128, K 64   (rows 0..63 are W)
 //   [*; U]   = [T diag(beta gamma); T diag(beta)] V      M 128, N 128, K 64   (rows 64..127 are U)
 //   W (FP16) and U (FP32) leave through bulk copies from shared memory that is idle by then (the Q rows, V, A and T):
@@ -299,8 +304,9 @@ constexpr std::uint32_t kPsA = kPsPstage + kGdnBlock;          //   later: slice
 constexpr std::uint32_t kPsT = kPsA + 2 * kALow;
 constexpr std::uint32_t kPsDiag = kPsT + 2 * kTLow;
 constexpr std::uint32_t kPsGates = kPsDiag + 4 * kDiagBlock * 4;
-constexpr std::uint32_t kPsFactors = kPsGates + kGdnGateBytes; // G log2(e), beta gamma, column factors: 3 x 64 floats
-constexpr std::uint32_t kPsBars = kPsFactors + 3 * kChunk * 4;
+// G log2(e), beta gamma and beta (both over the unit of K), column factors: 4 x 64 floats; what undoes U's scales: 128
+constexpr std::uint32_t kPsFactors = kPsGates + kGdnGateBytes;
+constexpr std::uint32_t kPsBars = kPsFactors + (4 * kChunk + kDim) * 4;
 constexpr std::uint32_t kPsTmemSlot = kPsBars + 24;
 constexpr std::uint32_t kPsAbort = kPsTmemSlot + 4;
 constexpr std::uint32_t kPrepSmemBytes = kPsAbort + 4 + 1024;  // + room to align the base to 1 KiB
@@ -310,6 +316,8 @@ static_assert(kPsGates % 16 == 0 && kPsFactors % 16 == 0 && kPsBars % 8 == 0 && 
 static_assert(2 * (kPrepSmemBytes + 1024) <= 233472, "two CTAs per SM");
 constexpr std::uint32_t kPrepTmemColumns = 256; // W at 0, U at 128; G at 0 before them
 
+// exponent field of u, the power of two that takes a chunk's growth into [1, 2)
+__device__ __forceinline__ std::uint32_t growth_unit(float growth) { return 254U - (__float_as_uint(growth) >> 23); }
 __device__ __forceinline__ std::uint32_t tstack_offset(std::uint32_t row, std::uint32_t col) {
   return row * kGdnRowBytes + (((col >> 3) ^ (row & 7U)) << 4) + ((col & 7U) << 1);
 }
@@ -349,7 +357,14 @@ __device__ __forceinline__ void transposed_fragments(std::uint32_t at, std::uint
   ldmatrix_x4_trans(at, hi);
   ldmatrix_x4_trans(at + kTLow, lo);
 }
-// the accumulators of two neighbouring column tiles as the A fragments of a k block
+// the accumulators of two neighbouring column tiles, times a factor, and as the A fragments of a k block
+__device__ __forceinline__ void rescale(float (&c0)[4], float (&c1)[4], float factor) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    c0[e] *= factor;
+    c1[e] *= factor;
+  }
+}
 __device__ __forceinline__ void accumulator_fragments(const float (&c0)[4], const float (&c1)[4], std::uint32_t (&hi)[4],
                                                       std::uint32_t (&lo)[4]) {
   split_half(c0[0], c0[1], hi[0], lo[0]);
@@ -365,8 +380,10 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
   const float *gates = reinterpret_cast<const float *>(smem + kPsGates);
   const float *s_beta = gates + kGdnGateBeta;
   float *s_g2 = reinterpret_cast<float *>(smem + kPsFactors); // G log2(e)
-  float *s_bg = s_g2 + kChunk;                                // beta exp(G)
-  float *s_cf = s_bg + kChunk;                                // exp(G at the end of the token's block of 16 - G)
+  float *s_bg = s_g2 + kChunk;                                // beta exp(G) / kGdnUnit
+  float *s_bu = s_bg + kChunk;                                // beta / kGdnUnit
+  float *s_cf = s_bu + kChunk;                                // exp(G at the end of the token's block of 16 - G)
+  float *s_undo = s_cf + kChunk;                              // by column: undoes the scales of the product that is U
   const std::uint32_t bar_in = base + kPsBars;
   const std::uint32_t bar_g = bar_in + 8;
   const std::uint32_t bar_wu = bar_in + 16;
@@ -477,8 +494,18 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       const std::uint32_t t = tid - 64;
       const float g = gates[kGdnGateG + t];
       s_g2[t] = g * 1.4426950408889634F;
-      s_bg[t] = s_beta[t] * exp_fast(g);
+      s_bg[t] = s_beta[t] * exp_fast(g) * (1.0F / kGdnUnit);
+      s_bu[t] = s_beta[t] * (1.0F / kGdnUnit);
       s_cf[t] = exp_fast(gates[kGdnGateG + (t | 15U)] - g);
+      const float undo_t = gdn_power(254 - growth_unit(gates[kGdnGateGrowth])) * (1.0F / kGdnUnit);
+      s_undo[t] = gdn_power(254 - gdn_scale_exponent(gates[kGdnGateMax + t])) * undo_t;
+      s_undo[t + kChunk] = gdn_power(254 - gdn_scale_exponent(gates[kGdnGateMax + kChunk + t])) * undo_t;
+    }
+    const std::uint32_t unit = growth_unit(gates[kGdnGateGrowth]); // u; A and T are held times 2^14 u, as G comes times 2^14
+    const float hold = gdn_power(unit + 14);
+    const float release = gdn_power(254 - 14 - unit);
+    if (tid == 0 && gates[kGdnGateGrowth] > kGdnMostGrowth) {
+      atomicOr(p.status, static_cast<unsigned int>(RIB200_DEVICE_DECAY_OUT_OF_RANGE));
     }
     __syncthreads();
 
@@ -495,7 +522,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       if (half <= row_half) {
         tmem_ld32(tmem + lane_base + 32 * half, x);
         const float g2_i = s_g2[i];
-        const float scale_i = is_p ? 1.0F : s_beta[i];
+        const float scale_i = is_p ? gdn_power(unit + kGdnUnitP - 14) : s_beta[i] * gdn_power(unit);
         if (half < row_half) {
 #pragma unroll
           for (std::uint32_t part = 0; part < 2; ++part) {
@@ -542,7 +569,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
           float *diag = reinterpret_cast<float *>(smem + kPsDiag) + (i >> 4) * kDiagBlock + (i & 15U);
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
-            diag[e * kDiagPitch] = lane < 16 ? x[e] : x[16 + e];
+            diag[e * kDiagPitch] = (lane < 16 ? x[e] : x[16 + e]) * release;
           }
         }
 #pragma unroll
@@ -612,11 +639,13 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const std::uint32_t k = 8 * c + 2 * e;
-          split_half(t[k], t[k + 1], hi[e], lo[e]);
+          const float t0 = t[k] * hold;
+          const float t1 = t[k + 1] * hold;
+          split_half(t0, t1, hi[e], lo[e]);
           const float2 bg = *reinterpret_cast<const float2 *>(s_bg + 16 * b + k);
-          const float2 be = *reinterpret_cast<const float2 *>(s_beta + 16 * b + k);
-          with_gamma[e] = pack_half(t[k] * bg.x, t[k + 1] * bg.y);
-          without[e] = pack_half(t[k] * be.x, t[k + 1] * be.y);
+          const float2 bu = *reinterpret_cast<const float2 *>(s_bu + 16 * b + k);
+          with_gamma[e] = pack_half(t0 * bg.x, t1 * bg.y);
+          without[e] = pack_half(t0 * bu.x, t1 * bu.y);
         }
         sts128(t_at(tid, 16 * b + 8 * c), hi[0], hi[1], hi[2], hi[3]);
         sts128(t_at(tid, 16 * b + 8 * c) + kTLow, lo[0], lo[1], lo[2], lo[3]);
@@ -637,8 +666,8 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       const std::uint32_t col = m0 + ((lane >> 3) & 1U) * 8;
       const float bg0 = -s_bg[lo_col];
       const float bg1 = -s_bg[lo_col + 8];
-      const float be0 = -s_beta[lo_col];
-      const float be1 = -s_beta[lo_col + 8];
+      const float be0 = -s_bu[lo_col];
+      const float be1 = -s_bu[lo_col + 8];
       const std::uint32_t with_gamma[4] = {pack_half(z0[0] * bg0, z0[1] * bg0), pack_half(z0[2] * bg1, z0[3] * bg1),
                                            pack_half(z1[0] * bg0, z1[1] * bg0), pack_half(z1[2] * bg1, z1[3] * bg1)};
       const std::uint32_t without[4] = {pack_half(z0[0] * be0, z0[1] * be0), pack_half(z0[2] * be1, z0[3] * be1),
@@ -655,9 +684,11 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       float y[2][4] = {};
       transposed_fragments(t_at(m0, m0), hi, lo);
       tile_step<2>(y, hi, lo, a_matrix + r0 * kAPitch + m0 * 2, kAPitch, kALow);
+      rescale(y[0], y[1], release);
       accumulator_fragments(y[0], y[1], hi, lo);
       float z[2][4] = {};
       tile_step<2>(z, hi, lo, t_at(r0, r0), kTPitch, kTLow);
+      rescale(z[0], z[1], release);
       store_scaled(z[0], z[1], r0, m0);
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
@@ -689,14 +720,18 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       transposed_fragments(t_at(16, m0), hi, lo);
       tile_step<4>(y, hi, lo, a_matrix + 32 * kAPitch + 32, kAPitch, kALow);
       float z[2][4] = {};
+      rescale(y[0], y[1], release);
       accumulator_fragments(y[0], y[1], hi, lo);
       if (warp < 2) { // rows 32..47
         tile_step<2>(z, hi, lo, t_at(32, 32), kTPitch, kTLow);
+        rescale(z[0], z[1], release);
         store_scaled(z[0], z[1], 32, m0);
       } else { // rows 48..63
         tile_step<2>(z, hi, lo, t_at(48, 32), kTPitch, kTLow);
+        rescale(y[2], y[3], release);
         accumulator_fragments(y[2], y[3], hi, lo);
         tile_step<2>(z, hi, lo, t_at(48, 48), kTPitch, kTLow);
+        rescale(z[0], z[1], release);
         store_scaled(z[0], z[1], 48, m0);
       }
     }
@@ -747,17 +782,22 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
         }
       }
     } else {
-      const float inv_scale = gates[kGdnGateInvScale];
       const std::uint32_t stage = base + (half == 0 ? kPsV : kPsA);
+      const std::uint32_t undo_at = smem_address(s_undo);
 #pragma unroll
       for (std::uint32_t part = 0; part < 2; ++part) {
+        float4 undo[8]; // all of them first: a load behind a store of this loop would wait for it
+#pragma unroll
+        for (std::uint32_t c = 0; c < 8; ++c) {
+          undo[c] = lds128(undo_at + (64 * half + 32 * part + 4 * c) * 4);
+        }
         float x[32];
         tmem_ld32(tmem + lane_base + 128 + 64 * half + 32 * part, x);
 #pragma unroll
         for (std::uint32_t c = 0; c < 8; ++c) {
           sts128(stage + part * kGdnSliceU + i * kGdnRowBytes + ((c ^ (i & 7U)) << 4),
-                 __float_as_uint(x[4 * c] * inv_scale), __float_as_uint(x[4 * c + 1] * inv_scale),
-                 __float_as_uint(x[4 * c + 2] * inv_scale), __float_as_uint(x[4 * c + 3] * inv_scale));
+                 __float_as_uint(x[4 * c] * undo[c].x), __float_as_uint(x[4 * c + 1] * undo[c].y),
+                 __float_as_uint(x[4 * c + 2] * undo[c].z), __float_as_uint(x[4 * c + 3] * undo[c].w));
         }
       }
     }
@@ -793,7 +833,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 }
 
 // ---- chain: per (state slice, value head), chunks in order -------------------------------------------------
-// 320 threads.  Warps 0-3 own the 128 lanes of tensor memory and the state (thread = row of every product), warps 4-5
+// 352 threads.  Warps 0-3 own the 128 lanes of tensor memory and the state (thread = row of every product), warps 4-5
 // make the outputs of the even chunks and warps 8-9 those of the odd ones (a chunk's outputs cost a pair of warps about
 // 3000 cycles, the chain itself 2100 a chunk: with one pair every first product waited for the outputs two chunks back;
 // 4096 tokens 224.2 -> 197.4 us, a chunk 3100 -> 2500 cycles), warp 6 issues the products, lane 0 of warp 7 streams the operand images of each chunk into a
@@ -808,16 +848,25 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 // The chain X -> Delta -> SD -> S is latency: nothing but that chain runs in warps 0-3, everything they need from memory
 // is in registers before they wait, and a row of a B operand (32 columns, 64 bytes) is four 16-byte stores because the
 // operand is MN-major (64-byte swizzle).
-// Scales: with M the largest |S0| of the slice (taken while the first product runs) no |Delta| and no new |S| exceeds
-// b = 11.4 M + 66 max|v| (a column of S0 has norm <= sqrt(128) M, each token adds at most max|v|).  Delta is scaled by
-// the power of two that brings b to [2^13, 2^14).  The state is scaled by 2 whenever 2^-4 <= b < 2^14, which leaves it
-// exact to 2^-22 b below its 10 bits, and like Delta otherwise: its image is written before its own maximum is known,
-// from the bound of the chunk before, and a factor that is the same for all ordinary magnitudes keeps a prompt fed in
-// pieces bit-identical to the same prompt in one call (a bound that follows every chunk rounds the few elements below
-// FP16's normal range differently on either side of a cut).
+// Scales, per column: with M the largest |S0| of the column, no |S| after the chunk exceeds
+//   b_S = 11.5 exp(G_C) M + growth sum(beta) max|v|
+// (the column of S0 has norm <= sqrt(128) M, a token adds at most beta |v|; 11.5 and not 11.32 because M is cut to BF16), and
+// no |Delta| exceeds b_D = max(beta) (max|v| + growth (11.5 M + sum(beta) max|v|)).  Delta is scaled by the power of two
+// that brings b_D to [2^13, 2^14).  The new state is scaled by 2 whenever 2^-4 <= b_S < 2^14 and like Delta, from b_S,
+// elsewhere: its image is written before its own maximum is known, and a factor that is the same for all ordinary magnitudes
+// keeps a prompt fed in pieces of whole chunks bit-identical to the same prompt in one call (a bound that follows every
+// chunk rounds the few elements below FP16's normal range differently on either side of a cut).  Inside that window the
+// image of the state is exact to 2^-26.
+// Columns whose bounds lie within 2^10 of each other, as they nearly always do, share the factor of the largest, and
+// everybody works with one number; else every column has its own, which costs some 200 cycles a chunk.  (One factor per
+// (chunk, slice) at all times left a column that is 1e-6 of the slice's largest with errors of 2e-3.  All of the scales
+// together, columns of V, units and growth included, cost 5 % of a layer call: 4096 tokens 186.5 -> 195.8 us, 149 tokens
+// 21.6 -> 23.0.)
+// Warp 10 makes the factors while the first product of the chunk runs, from column maxima that warps 0-3 leave as soon as
+// the state is on its way; the gates it needs it reads from memory two chunks ahead.
 // Every mbarrier wait is bounded; when one runs out the CTA records RIB200_DEVICE_WAIT_TIMED_OUT, stops waiting and
 // copying, and runs to its end.
-constexpr int kChainThreads = 320;
+constexpr int kChainThreads = 352;
 constexpr std::uint32_t kStages = 3;
 constexpr std::uint32_t kPrefetchAhead = 3; // chunks between the L2 prefetch and the copy that uses it
 constexpr std::uint32_t kStageQw = 0;                              // [2 blocks][rows 0..63 Q, 64..127 W][128 bytes]
@@ -825,7 +874,7 @@ constexpr std::uint32_t kStageK = kStageQw + 2 * kGdnKqBlock;      // [2 blocks]
 constexpr std::uint32_t kStageP = kStageK + 2 * kGdnBlock;         // 64 rows; the product's rows 64.. read on into U
 constexpr std::uint32_t kStageU = kStageP + kGdnBlock;
 constexpr std::uint32_t kStageGates = kStageU + kGdnSliceU;
-constexpr std::uint32_t kStageBytes = (kStageGates + kGdnGateBytes + 1023) / 1024 * 1024;
+constexpr std::uint32_t kStageBytes = (kStageGates + kChunk * 4 + 1023) / 1024 * 1024; // of the gates, G
 constexpr std::uint32_t kOperandRow = kSlice * 2;                  // bytes of a B operand row
 constexpr std::uint32_t kCsState = kStages * kStageBytes;               // S, 128 rows
 constexpr std::uint32_t kCsEDelta = kCsState + kDim * kOperandRow; // diag(e) Delta, 64 rows
@@ -835,9 +884,22 @@ constexpr std::uint32_t kCsDelta = kCsEDelta + kChunk * kOperandRow;
 constexpr std::uint32_t kCsNorm = kCsDelta + kChunk * kOperandRow;
 constexpr std::uint32_t kNormSlots = 4;
 constexpr std::uint32_t kCsWeight = kCsNorm + kNormSlots * kGdnSlices * kChunk * 4;
-constexpr std::uint32_t kCsMax = kCsWeight + kSlice * 4;           // [2 parities][4 warps]
-constexpr std::uint32_t kCsScale = kCsMax + 32;                    // [2 parities]{1 / scale of S0, 1 / scale of Delta}
-constexpr std::uint32_t kCsBars = kCsScale + 16;
+constexpr std::uint32_t kCsMax = kCsWeight + kSlice * 4;           // [4 warps][columns] largest |S0|
+// [chunk & 3][factors below][columns].  Warp 10 makes those of a chunk at its head; by then the outputs of the chunk that
+// had the slot before, which may lag, have read theirs: the first product of the chunk before this one waited for them.
+constexpr std::uint32_t kCsScale = kCsMax + 4 * kSlice * 4;
+enum : std::uint32_t {
+  kScaleX = 0,                      // takes X to the scale of Delta
+  kScaleDelta = 1 * kSlice * 4,     // scale of Delta
+  kScaleSd = 2 * kSlice * 4,        // undoes the scale of SD
+  kScaleOutX = 3 * kSlice * 4,      // undoes that of Q S0
+  kScaleOutDelta = 4 * kSlice * 4,  // undoes that of P Delta
+  kScaleState = 5 * kSlice * 4,     // scale of the new S
+  kScaleEqual = 6 * kSlice * 4,     // not 0: the columns have the same factors
+  kScaleBytes = 6 * kSlice * 4 + 16
+};
+constexpr std::uint32_t kScaleSlots = 4;
+constexpr std::uint32_t kCsBars = kCsScale + kScaleSlots * kScaleBytes;
 enum : std::uint32_t {
   kBarQwFull = 0,                      // [stages] bytes of Q and W
   kBarRestFull = kBarQwFull + kStages, // [stages] bytes of K, P, U and the gates
@@ -871,7 +933,7 @@ static_assert(kStageBytes % 1024 == 0 && kStageP % 1024 == 0 && kCsState % 1024 
                   kCsDelta % 512 == 0 && kCsBars % 8 == 0 && kCsWeight % 16 == 0,
               "operand images sit on the boundaries of their swizzle atoms");
 static_assert(kStageP + 2 * kGdnBlock <= kStageBytes, "the don't-care rows of P lie inside the stage");
-static_assert(kChainSmemBytes <= 232448, "fits an SM");
+static_assert(kCsScale % 16 == 0 && kChainSmemBytes <= 232448, "aligned, fits an SM");
 constexpr std::uint32_t kChainTmemColumns = 256; // X at 0 and 32, O2 at 64 and 96 (by parity), SD at 128
 
 // byte offset of the 16-byte piece `piece` of row `row` of a B operand (64-byte rows, 64-byte swizzle)
@@ -884,15 +946,56 @@ __device__ __forceinline__ void store_operand_row(std::uint32_t operand, std::ui
     sts128(operand + operand_piece(row, c), h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]);
   }
 }
-// exponent field of the power of two that brings `bound` into [2^13, 2^14), kept away from the ends of the range
-__device__ __forceinline__ std::uint32_t scale_exponent(float bound) {
-  const int biased = static_cast<int>((__float_as_uint(bound) >> 23) & 255U);
-  return static_cast<std::uint32_t>(min(max(127 + 13 + 127 - biased, 27), 227));
+// exponent field of the scale of a state bounded by `bound`
+__device__ __forceinline__ std::uint32_t state_exponent_of(float bound) {
+  return bound >= 0.0625F && bound < 16384.0F ? 128U : gdn_scale_exponent(bound);
 }
-__device__ __forceinline__ std::uint32_t state_scale_exponent(float bound) {
-  return bound >= 0.0625F && bound < 16384.0F ? 128U : scale_exponent(bound);
+// Lane = column: the bound to scale by, the largest one where the columns' bounds lie within 2^10 of each other (columns of
+// zeros aside), else the column's own.
+__device__ __forceinline__ float level(float bound, bool &equal) {
+  const std::uint32_t bits = __float_as_uint(bound);
+  const float high = __uint_as_float(__reduce_max_sync(0xFFFFFFFFU, bits));
+  const float low = __uint_as_float(__reduce_min_sync(0xFFFFFFFFU, bits == 0U ? 0x7F7FFFFFU : bits));
+  const bool same = low >= high * 0x1p-10F;
+  equal = equal && same;
+  return same ? high : bound;
 }
-__device__ __forceinline__ float power_of(std::uint32_t exponent) { return __uint_as_float(exponent << 23); }
+// factors of the columns in shared memory: one for all, or an array
+struct EqualFactors {
+  float value;
+  __device__ __forceinline__ explicit EqualFactors(std::uint32_t at) : value(lds32(at)) {}
+  __device__ __forceinline__ float4 quad(int) const { return make_float4(value, value, value, value); }
+};
+struct ColumnFactors {
+  std::uint32_t at;
+  __device__ __forceinline__ explicit ColumnFactors(std::uint32_t at) : at(at) {}
+  __device__ __forceinline__ float4 quad(int c) const { return lds128(at + 16 * c); }
+};
+template <class Factors> struct Kind {
+  using Type = Factors;
+};
+// Largest magnitude of every column over the 32 rows of a warp, cut to BF16: lane c gets column c's.  Two columns ride in a
+// word, and each exchange halves the words a lane still holds.
+__device__ __forceinline__ float column_maximum(const float (&s)[kSlice]) {
+  const std::uint32_t lane = threadIdx.x & 31;
+  std::uint32_t held[kSlice / 2];
+#pragma unroll
+  for (int i = 0; i < kSlice / 2; ++i) {
+    held[i] = __byte_perm(__float_as_uint(s[2 * i]), __float_as_uint(s[2 * i + 1]), 0x7632) & 0x7FFF7FFFU;
+  }
+#pragma unroll
+  for (int words = kSlice / 4; words > 0; words >>= 1) { // lanes 2 `words` apart
+    const bool upper = (lane & (2 * words)) != 0;
+#pragma unroll
+    for (int i = 0; i < words; ++i) {
+      const std::uint32_t give = upper ? held[i] : held[i + words];
+      const std::uint32_t keep = upper ? held[i + words] : held[i];
+      held[i] = __vmaxs2(keep, __shfl_xor_sync(0xFFFFFFFFU, give, 2 * words));
+    }
+  }
+  held[0] = __vmaxs2(held[0], __shfl_xor_sync(0xFFFFFFFFU, held[0], 1));
+  return __uint_as_float((lane & 1U) != 0 ? held[0] & 0xFFFF0000U : held[0] << 16);
+}
 
 template <int Dtype> struct RowPart; // 32 elements of a row of activations
 template <> struct RowPart<RIB200_DTYPE_F32> {
@@ -973,7 +1076,6 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
   volatile std::uint32_t *tmem_slot = reinterpret_cast<volatile std::uint32_t *>(smem + kCsTmemSlot);
   volatile std::uint32_t *abort_flag = reinterpret_cast<volatile std::uint32_t *>(smem + kCsAbort);
   volatile float *s_max = reinterpret_cast<volatile float *>(smem + kCsMax);
-  volatile float *s_scale = reinterpret_cast<volatile float *>(smem + kCsScale);
   auto wait = [&](std::uint32_t b, std::uint32_t parity) { bounded_wait(b, parity, abort_flag, p.status); };
 
   grid_dependents_may_launch();
@@ -1008,14 +1110,6 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
   // State slice: row `key` of S in this thread's registers.
   float s_reg[kSlice];
   const std::uint32_t key = threadIdx.x; // warps 0-3
-  auto largest = [&] {
-    float m = 0.0F;
-#pragma unroll
-    for (int c = 0; c < kSlice; ++c) {
-      m = fmaxf(m, fabsf(s_reg[c]));
-    }
-    return __uint_as_float(__reduce_max_sync(0xFFFFFFFFU, __float_as_uint(m)));
-  };
   if (warp < 4) {
 #pragma unroll
     for (int c = 0; c < kSlice; c += 4) {
@@ -1025,10 +1119,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
       s_reg[c + 2] = v.z;
       s_reg[c + 3] = v.w;
     }
-    const float m = largest();
-    if (lane == 0) {
-      s_max[warp] = m;
-    }
+    s_max[warp * kSlice + lane] = column_maximum(s_reg);
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -1041,6 +1132,8 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
   // Launched with programmatic stream serialisation behind the prepare kernel: barriers, tensor memory and the state
   // slice (which that kernel does not touch) are set up while its last CTAs finish; the records are read after this.
   grid_dependency_wait();
+
+  auto scales_of = [&](std::uint32_t chunk) { return base + kCsScale + (chunk & (kScaleSlots - 1)) * kScaleBytes; };
 
   if (warp == 7) {
     // ---- producer ----
@@ -1060,7 +1153,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
         if (chunk + kPrefetchAhead < p.chunks) { // its own U and a quarter of what the four slices share
           const unsigned char *ahead = record(chunk + kPrefetchAhead);
           prefetch_l2(ahead + kGdnRecU + slice * kGdnSliceU, kGdnSliceU);
-          prefetch_l2(ahead + slice * (kGdnRecGates / 4), kGdnRecGates / 4);
+          prefetch_l2(ahead + slice * (kGdnRecU / 4), kGdnRecU / 4);
           prefetch_l2(key_image(chunk + kPrefetchAhead) + slice * (kGdnKqBytes / 4), kGdnKqBytes / 4);
         }
         if (chunk >= kStages) {
@@ -1079,9 +1172,9 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
           bulk_copy_g2s(stage + kStageQw + b * kGdnKqBlock + kGdnBlock, rec + kGdnRecW + b * kGdnBlock, kGdnBlock, full);
         }
         const std::uint32_t rest = bar(kBarRestFull + at.stage);
-        mbarrier_expect_tx(rest, 2 * kGdnBlock + kGdnBlock + kGdnSliceU + kGdnGateBytes);
+        mbarrier_expect_tx(rest, 2 * kGdnBlock + kGdnBlock + kGdnSliceU + kChunk * 4);
         bulk_copy_g2s(stage + kStageU, rec + kGdnRecU + slice * kGdnSliceU, kGdnSliceU, rest);
-        bulk_copy_g2s(stage + kStageGates, rec + kGdnRecGates, kGdnGateBytes, rest);
+        bulk_copy_g2s(stage + kStageGates, rec + kGdnRecGates + kGdnGateG * 4, kChunk * 4, rest);
 #pragma unroll
         for (std::uint32_t b = 0; b < 2; ++b) {
           bulk_copy_g2s(stage + kStageK + b * kGdnBlock, kq + b * kGdnKqBlock, kGdnBlock, rest);
@@ -1168,132 +1261,185 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
         break;
       }
     }
+  } else if (warp == 10) {
+    // ---- the factors of the chunks, lane = column.  It waits for the maxima of the chain's warps (barrier 1), they for its
+    // factors (barrier 3); the five warps walk all chunks whatever happens. ----
+    struct Gates {
+      float largest, growth, beta_sum, beta_max, g_end;
+    };
+    auto gates_of = [&](std::uint32_t chunk) {
+      const float *gates = reinterpret_cast<const float *>(
+          p.scratch.records + (static_cast<std::size_t>(chunk) * p.value_heads + head) * kGdnRecBytes + kGdnRecGates);
+      return Gates{gates[kGdnGateMax + slice * kSlice + lane], gates[kGdnGateGrowth], gates[kGdnGateBetaSum],
+                   gates[kGdnGateBetaMax], gates[kGdnGateG + kChunk - 1]};
+    };
+    auto state_bound = [](const Gates &g, float m) {
+      return 11.5F * exp_fast(g.g_end) * m + g.growth * g.beta_sum * g.largest;
+    };
+    auto column_bound = [&] { // largest |S0| that the four warps have left
+      const volatile float *maxima = s_max + lane;
+      return fmaxf(fmaxf(maxima[0], maxima[kSlice]), fmaxf(maxima[2 * kSlice], maxima[3 * kSlice]));
+    };
+    auto factors_of = [&](std::uint32_t chunk) { return reinterpret_cast<float *>(smem + (scales_of(chunk) - base)) + lane; };
+    Gates now = gates_of(0);                           // of this chunk ...
+    Gates following = gates_of(min(1U, p.chunks - 1)); // ... and of the next
+    std::uint32_t state_exponent;                      // of the scale of S0
+    bool state_equal = true;
+    {
+      const float m = column_bound();
+      state_exponent = state_exponent_of(level(fmaxf(state_bound(now, m), 1.01F * m), state_equal));
+      factors_of(kScaleSlots - 1)[kScaleState / 4] = gdn_power(state_exponent);
+      asm volatile("bar.arrive 3, 160;\n" ::: "memory");
+    }
+    for (std::uint32_t chunk = 0; chunk < p.chunks; ++chunk) {
+      asm volatile("bar.sync 1, 160;\n" ::: "memory");
+      const float m = column_bound();
+      bool equal = state_equal;
+      const std::uint32_t delta_exponent = gdn_scale_exponent(
+          level(now.beta_max * (now.largest + now.growth * (11.5F * m + now.beta_sum * now.largest)), equal));
+      const std::uint32_t unit = growth_unit(now.growth);
+      // X times 2^(unit of W) / (scale of S0) into Delta's scale; out of FP32's range only where X is 0
+      const int x_exponent = static_cast<int>(delta_exponent + 254) - static_cast<int>(state_exponent + unit + kGdnUnitW);
+      float *to = factors_of(chunk);
+      to[kScaleX / 4] = gdn_power(static_cast<std::uint32_t>(min(max(x_exponent, 1), 254)));
+      to[kScaleDelta / 4] = gdn_power(delta_exponent);
+      to[kScaleSd / 4] = gdn_power(254 - delta_exponent) * (1.0F / kGdnUnit);
+      to[kScaleOutX / 4] = gdn_power(254 - state_exponent) * (1.0F / kGdnUnit);
+      to[kScaleOutDelta / 4] = gdn_power(254 - delta_exponent) * gdn_power(254 - kGdnUnitP - unit);
+      state_equal = true;
+      state_exponent = state_exponent_of(level(state_bound(now, m), state_equal));
+      to[kScaleState / 4] = gdn_power(state_exponent);
+      if (lane == 0) {
+        to[kScaleEqual / 4] = equal && state_equal ? 1.0F : 0.0F;
+      }
+      asm volatile("bar.arrive 3, 160;\n" ::: "memory");
+      now = following;
+      following = gates_of(min(chunk + 2, p.chunks - 1));
+    }
   } else if (warp < 4) {
     // ---- the chain: thread = lane of tensor memory ----
     const std::uint32_t lane_base = (warp * 32U) << 16;
     const bool has_w = warp >= 2;                  // rows 64..127 of X: W S0 of token threadIdx.x - 64
     const std::uint32_t token = threadIdx.x & 63U;
     std::uint32_t half_row[16];
-    auto put_state = [&](float scale) {
+    auto put_state = [&](const auto &scale) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        half_row[c] = pack_half(s_reg[2 * c] * scale, s_reg[2 * c + 1] * scale);
+      for (int c = 0; c < kSlice / 4; ++c) {
+        const float4 f = scale.quad(c);
+        half_row[2 * c] = pack_half(s_reg[4 * c] * f.x, s_reg[4 * c + 1] * f.y);
+        half_row[2 * c + 1] = pack_half(s_reg[4 * c + 2] * f.z, s_reg[4 * c + 3] * f.w);
       }
       store_operand_row(base + kCsState, key, half_row);
       fence_proxy_async();
       tcgen05_fence_before();
       mbarrier_arrive(bar(kBarState));
     };
-    float m = fmaxf(fmaxf(s_max[0], s_max[1]), fmaxf(s_max[2], s_max[3]));
-    auto bound_of = [&](std::uint32_t stage) { return 11.4F * m + 66.0F * lds32(stage + kStageGates + kGdnGateMax * 4); };
-    wait(bar(kBarRestFull), 0);
-    std::uint32_t state_exponent = state_scale_exponent(bound_of(base));
-    put_state(power_of(state_exponent));
+    asm volatile("bar.sync 3, 160;\n" ::: "memory"); // the scale of the first S0
+    put_state(ColumnFactors(scales_of(kScaleSlots - 1) + kScaleState));
     RingPlace at;
     for (std::uint32_t chunk = 0; chunk < p.chunks; ++chunk, at.next()) {
       const std::uint32_t s = chunk & 1U;
       const std::uint32_t stage = base + at.stage * kStageBytes;
+      const std::uint32_t scales = scales_of(chunk);
       if (threadIdx.x == 64) {
         RIB200_GDN_STAMP(chunk, 0);
       }
+      s_max[warp * kSlice + lane] = column_maximum(s_reg);
+      asm volatile("bar.arrive 1, 160;\n" ::: "memory");
       wait(bar(kBarRestFull + at.stage), at.phase);
-      const float inv_before = power_of(254 - state_exponent);
-      const float g_end = lds32(stage + kStageGates + (kGdnGateG + kChunk - 1) * 4);
-      const float bound = bound_of(stage);
-      const std::uint32_t exponent = scale_exponent(bound);
-      state_exponent = state_scale_exponent(bound);
-      const float scale = power_of(exponent);
-      const float inv_scale = power_of(254 - exponent);
+      const float g_end = lds32(stage + kStageGates + (kChunk - 1) * 4);
       const float gamma_c = exp_fast(g_end);
+      float4 u[kSlice / 4]; // rows 64..127 alone
+      float decay_to_end = 0.0F;
       if (has_w) {
-        const float e_scale = scale * exp_fast(g_end - lds32(stage + kStageGates + (kGdnGateG + token) * 4));
-        float4 u[kSlice / 4];
+        decay_to_end = exp_fast(g_end - lds32(stage + kStageGates + token * 4));
 #pragma unroll
         for (std::uint32_t c = 0; c < kSlice / 4; ++c) {
           u[c] = lds128(stage + kStageU + token * kGdnRowBytes + ((c ^ (token & 7U)) << 4));
         }
-        mbarrier_arrive(bar(kBarRead + at.stage));
-        wait(bar(kBarXDone + s), (chunk >> 1) & 1U);
+      }
+      mbarrier_arrive(bar(kBarRead + at.stage));
+      asm volatile("bar.sync 3, 160;\n" ::: "memory");
+      auto walk = [&](auto kind) {
+        using Factors = typename decltype(kind)::Type;
+        if (has_w) {
+          const Factors x_scale(scales + kScaleX);
+          {
+            const Factors scale(scales + kScaleDelta);
+#pragma unroll
+            for (int c = 0; c < kSlice / 4; ++c) {
+              const float4 f = scale.quad(c);
+              u[c] = make_float4(u[c].x * f.x, u[c].y * f.y, u[c].z * f.z, u[c].w * f.w);
+            }
+          }
+          wait(bar(kBarXDone + s), (chunk >> 1) & 1U);
+          tcgen05_fence_after();
+          if (threadIdx.x == 64) {
+            RIB200_GDN_STAMP(chunk, 1);
+          }
+          float x[kSlice];
+          tmem_ld32(tmem + lane_base + 32 * s, x);
+#pragma unroll
+          for (int c = 0; c < kSlice / 4; ++c) { // Delta at its scale
+            const float4 f = x_scale.quad(c);
+            x[4 * c] = u[c].x - x[4 * c] * f.x;
+            x[4 * c + 1] = u[c].y - x[4 * c + 1] * f.y;
+            x[4 * c + 2] = u[c].z - x[4 * c + 2] * f.z;
+            x[4 * c + 3] = u[c].w - x[4 * c + 3] * f.w;
+          }
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            half_row[c] = pack_half(x[2 * c] * decay_to_end, x[2 * c + 1] * decay_to_end);
+          }
+          store_operand_row(base + kCsEDelta, token, half_row);
+          fence_proxy_async();
+          tcgen05_fence_before();
+          mbarrier_arrive(bar(kBarEDelta));
+          if (threadIdx.x == 64) {
+            RIB200_GDN_STAMP(chunk, 2);
+          }
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            half_row[c] = pack_half(x[2 * c], x[2 * c + 1]);
+          }
+          if (chunk >= 1) { // P Delta of the chunk before has read its operand
+            wait(bar(kBarO2Done + (s ^ 1U)), ((chunk - 1) >> 1) & 1U);
+          }
+          store_operand_row(base + kCsDelta, token, half_row);
+          fence_proxy_async();
+          mbarrier_arrive(bar(kBarDelta));
+        }
+#pragma unroll
+        for (int c = 0; c < kSlice; ++c) {
+          s_reg[c] *= gamma_c;
+        }
+        const Factors undo(scales + kScaleSd);
+        const Factors scale(scales + kScaleState);
+        wait(bar(kBarSdDone), chunk & 1U);
         tcgen05_fence_after();
-        if (threadIdx.x == 64) { // X was issued after the outputs of two chunks ago had read their scales
-          RIB200_GDN_STAMP(chunk, 1);
-          s_scale[2 * s] = inv_before;
-          s_scale[2 * s + 1] = inv_scale;
-        }
-        float x[kSlice];
-        tmem_ld32(tmem + lane_base + 32 * s, x);
-#pragma unroll
-        for (int c = 0; c < kSlice / 4; ++c) {
-          x[4 * c] = u[c].x - x[4 * c] * inv_before;
-          x[4 * c + 1] = u[c].y - x[4 * c + 1] * inv_before;
-          x[4 * c + 2] = u[c].z - x[4 * c + 2] * inv_before;
-          x[4 * c + 3] = u[c].w - x[4 * c + 3] * inv_before;
-        }
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          half_row[c] = pack_half(x[2 * c] * e_scale, x[2 * c + 1] * e_scale);
-        }
-        store_operand_row(base + kCsEDelta, token, half_row);
-        fence_proxy_async();
-        tcgen05_fence_before();
-        mbarrier_arrive(bar(kBarEDelta));
         if (threadIdx.x == 64) {
-          RIB200_GDN_STAMP(chunk, 2);
+          RIB200_GDN_STAMP(chunk, 3);
         }
-        if (chunk >= 1) { // P Delta of the chunk before has read its operand
-          wait(bar(kBarO2Done + (s ^ 1U)), ((chunk - 1) >> 1) & 1U);
-        }
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          half_row[c] = pack_half(x[2 * c] * scale, x[2 * c + 1] * scale);
-        }
-        store_operand_row(base + kCsDelta, token, half_row);
-        fence_proxy_async();
-        mbarrier_arrive(bar(kBarDelta));
-      } else {
-        mbarrier_arrive(bar(kBarRead + at.stage));
-      }
-#pragma unroll
-      for (int c = 0; c < kSlice; ++c) {
-        s_reg[c] *= gamma_c;
-      }
-      wait(bar(kBarSdDone), chunk & 1U);
-      tcgen05_fence_after();
-      if (threadIdx.x == 64) {
-        RIB200_GDN_STAMP(chunk, 3);
-      }
-      {
         float sd[kSlice];
         tmem_ld32(tmem + lane_base + 128, sd);
 #pragma unroll
-        for (int c = 0; c < kSlice; ++c) {
-          s_reg[c] += sd[c] * inv_scale;
+        for (int c = 0; c < kSlice / 4; ++c) {
+          const float4 f = undo.quad(c);
+          s_reg[4 * c] += sd[4 * c] * f.x;
+          s_reg[4 * c + 1] += sd[4 * c + 1] * f.y;
+          s_reg[4 * c + 2] += sd[4 * c + 2] * f.z;
+          s_reg[4 * c + 3] += sd[4 * c + 3] * f.w;
         }
+        put_state(scale);
+      };
+      if (lds32(scales + kScaleEqual) != 0.0F) {
+        walk(Kind<EqualFactors>{});
+      } else {
+        walk(Kind<ColumnFactors>{});
       }
-      put_state(power_of(state_exponent));
       if (threadIdx.x == 64) {
         RIB200_GDN_STAMP(chunk, 4);
       }
-      // while the next first product runs: the largest |S| (and whether somebody has given up, the same for everybody)
-      m = largest();
-      if (lane == 0) {
-        s_max[4 * (s ^ 1U) + warp] = m;
-      }
-      std::uint32_t stop;
-      asm volatile("{\n"
-                   ".reg .pred in, out;\n"
-                   "setp.ne.u32 in, %1, 0;\n"
-                   "barrier.cta.red.or.pred out, 1, 128, in;\n"
-                   "selp.u32 %0, 1, 0, out;\n"
-                   "}\n"
-                   : "=r"(stop)
-                   : "r"(*abort_flag)
-                   : "memory");
-      if (stop != 0) {
-        break;
-      }
-      const volatile float *maxima = s_max + 4 * (s ^ 1U);
-      m = fmaxf(fmaxf(maxima[0], maxima[1]), fmaxf(maxima[2], maxima[3]));
     }
 #pragma unroll
     for (int c = 0; c < kSlice; c += 4) {
@@ -1344,7 +1490,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
         }
       }
       wait(bar(kBarRestFull + at.stage), at.phase);
-      const float gamma = exp_fast(lds32(stage + kStageGates + (kGdnGateG + token) * 4));
+      const float gamma = exp_fast(lds32(stage + kStageGates + token * 4));
       mbarrier_arrive(bar(kBarRead + at.stage));
       wait(bar(kBarXDone + s), (chunk >> 1) & 1U);
       tcgen05_fence_after();
@@ -1358,14 +1504,27 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
       {
         float o2[kSlice];
         tmem_ld32(tmem + lane_base + 64 + 32 * s, o2);
-        const float scale_x = gamma * s_scale[2 * s];
-        const float scale_o2 = s_scale[2 * s + 1];
+        const std::uint32_t scales = scales_of(chunk);
+        if (lds32(scales + kScaleEqual) != 0.0F) {
+          const float scale_x = gamma * lds32(scales + kScaleOutX);
+          const float scale_o2 = lds32(scales + kScaleOutDelta);
+#pragma unroll
+          for (int c = 0; c < kSlice; ++c) {
+            o[c] = o[c] * scale_x + o2[c] * scale_o2;
+          }
+        } else {
+#pragma unroll
+          for (std::uint32_t c = 0; c < kSlice / 4; ++c) {
+            const float4 undo_x = lds128(scales + kScaleOutX + 16 * c);
+            const float4 undo_delta = lds128(scales + kScaleOutDelta + 16 * c);
+            o[4 * c] = o[4 * c] * (gamma * undo_x.x) + o2[4 * c] * undo_delta.x;
+            o[4 * c + 1] = o[4 * c + 1] * (gamma * undo_x.y) + o2[4 * c + 1] * undo_delta.y;
+            o[4 * c + 2] = o[4 * c + 2] * (gamma * undo_x.z) + o2[4 * c + 2] * undo_delta.z;
+            o[4 * c + 3] = o[4 * c + 3] * (gamma * undo_x.w) + o2[4 * c + 3] * undo_delta.w;
+          }
+        }
         tcgen05_fence_before();
         mbarrier_arrive(bar(kBarOutRead + s));
-#pragma unroll
-        for (int c = 0; c < kSlice; ++c) {
-          o[c] = o[c] * scale_x + o2[c] * scale_o2;
-        }
       }
       if constexpr (kLayer) {
         float squares = 0.0F;
@@ -1420,7 +1579,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 6) {
-    // warps 0-5 waited for the last commits, so nothing is still writing tensor memory
+    // warps 0-5, 8 and 9 waited for the last commits, so nothing is still writing tensor memory
     tcgen05_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kChainTmemColumns) : "memory");
   }

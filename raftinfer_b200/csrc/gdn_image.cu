@@ -5,9 +5,11 @@
 //          (cpp/kernels/qwen35_delta.cu:236-276,375-411,522-529; CPU cpp/reference/qwen35.cpp:417-469);
 //   core   operands that are already convolved and normalised (rib200_gdn_core, and layer calls of other widths).
 //
-// FP16 keeps the 10 mantissa bits that the chunk kernels' products had in TF32, in half the bytes.  The range is no
-// concern for q and k, which are normalised; V is brought under 2^14 by a power of two per (chunk, head), so that an
-// element keeps its 10 bits down to 2^-27 of the largest one, and the factor is divided out of U in FP32.
+// FP16 keeps the 10 mantissa bits of TF32 in half the bytes, but not its range.  q and k are normalised and stored times
+// 2^7, so that an element keeps its 10 bits down to 2^-21.  V is brought under 2^14 by a power of two per (chunk, head,
+// column), divided out of U in FP32: an element keeps its 10 bits down to 2^-27 of the largest one of its column in the
+// chunk, and no column - one of large values, an infinity - takes precision from another.  (With one factor per (chunk,
+// head) a column 2^-27 of the largest was lost, and an infinity wiped out the other 127.)
 //
 // 67 MB of BF16 rows read and 67 MB of images written at 4096 tokens (the FP32 q|k|v this replaces were 134 MB), but
 // bound by instruction issue (62 % of the slots, DRAM 20 %, at four dims a lane).  One CTA per (chunk, head vector); the
@@ -146,7 +148,9 @@ __device__ __forceinline__ unsigned char *record_of(const ImageParams &p, std::u
   return p.scratch.records + (static_cast<std::size_t>(chunk) * p.value_heads + head) * kGdnRecBytes;
 }
 
-// Gates of 32 value heads over one chunk: the running sum of the log decays and beta, zero past the last token.
+// Gates of 32 value heads over one chunk: the running sum of the log decays and beta, zero past the last token; for the
+// chain's bounds the largest product of consecutive decays, which exceeds 1 only where log decays are positive, and sum
+// and maximum of beta.
 template <int Dtype, int Count, bool Layer>
 __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t chunk, std::uint32_t head0) {
   __shared__ float s_decay[kGdnChunk][kGateHeads + 1];
@@ -200,11 +204,34 @@ __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t 
       }
     }
     b += __shfl_sync(0xFFFFFFFFU, a, 31);
+    // largest G_i - G_j over j <= i, the start of the chunk (0) among the j; NaN drops out of minima and maxima
+    float low_a = fminf(a, 0.0F);
+    float low_b = b;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      low_a = fminf(low_a, __shfl_up_sync(0xFFFFFFFFU, low_a, d)); // a lane without a neighbour gets its own value
+      low_b = fminf(low_b, __shfl_up_sync(0xFFFFFFFFU, low_b, d));
+    }
+    low_b = fminf(low_b, __shfl_sync(0xFFFFFFFFU, low_a, 31));
+    float rise = fmaxf(fmaxf(a - low_a, b - low_b), 0.0F);
+    float beta_sum = s_beta[lane][h] + s_beta[lane + 32][h];
+    float beta_max = fmaxf(s_beta[lane][h], s_beta[lane + 32][h]);
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+      rise = fmaxf(rise, __shfl_xor_sync(0xFFFFFFFFU, rise, offset));
+      beta_sum += __shfl_xor_sync(0xFFFFFFFFU, beta_sum, offset);
+      beta_max = fmaxf(beta_max, __shfl_xor_sync(0xFFFFFFFFU, beta_max, offset));
+    }
     float *gates = reinterpret_cast<float *>(record_of(p, chunk, head0 + h) + kGdnRecGates);
     gates[kGdnGateG + lane] = a;
     gates[kGdnGateG + 32 + lane] = b;
     gates[kGdnGateBeta + lane] = s_beta[lane][h];
     gates[kGdnGateBeta + 32 + lane] = s_beta[lane + 32][h];
+    if (lane == 0) {
+      gates[kGdnGateGrowth] = fminf(expf(rise), 0x1p100F);
+      gates[kGdnGateBetaSum] = beta_sum;
+      gates[kGdnGateBetaMax] = beta_max;
+    }
   }
 }
 
@@ -221,8 +248,6 @@ __global__ void __launch_bounds__(Layout<Count>::kThreads, Layout<Count>::kCtas)
     gate_arrays<Dtype, Count, Layer>(p, chunk, (vec - vectors) * kGateHeads);
     return;
   }
-  const std::uint32_t warp = threadIdx.x >> 5;
-  const std::uint32_t lane = threadIdx.x & 31;
   constexpr std::uint32_t kLanes = Layout<Count>::kLanes;
   const std::uint32_t sub = threadIdx.x % kLanes; // a lane has dims Count sub .. Count sub + Count - 1
   const std::uint32_t row0 = threadIdx.x / kLanes * kTokensPerRun;
@@ -232,6 +257,10 @@ __global__ void __launch_bounds__(Layout<Count>::kThreads, Layout<Count>::kCtas)
   const std::uint32_t head = is_q ? vec : (is_v ? vec - 2 * p.key_heads : vec - p.key_heads);
   const bool wide = p.wide != 0;
   const bool whole = (chunk + 1) * kGdnChunk <= p.tokens; // no row of the chunk is past the last token
+  __shared__ std::uint32_t s_largest[Count][kLanes]; // by column: bits of the largest |v| of the chunk
+  if (threadIdx.x < kGdnDim) {
+    s_largest[threadIdx.x / kLanes][threadIdx.x % kLanes] = 0U;
+  }
 
   float out[kTokensPerRun][Count];
   if constexpr (Layer) {
@@ -386,39 +415,40 @@ __global__ void __launch_bounds__(Layout<Count>::kThreads, Layout<Count>::kCtas)
 
   unsigned char *image;
   std::uint32_t block;
-  float scale = 1.0F;
+  float scale[Count];
   if (is_v) {
-    constexpr int kWarps = Layout<Count>::kThreads / 32;
-    __shared__ float s_max[kWarps];
-    float largest = 0.0F;
+    if constexpr (!Layer) {
+      __syncthreads(); // s_largest is set up (a layer call has had its barrier for the taps)
+    }
+    std::uint32_t largest[Count];
 #pragma unroll
-    for (int i = 0; i < kTokensPerRun; ++i) {
+    for (int c = 0; c < Count; ++c) {
+      largest[c] = 0U;
 #pragma unroll
-      for (int c = 0; c < Count; ++c) {
-        largest = fmaxf(largest, fabsf(out[i][c]));
+      for (int i = 0; i < kTokensPerRun; ++i) {
+        largest[c] = max(largest[c], __float_as_uint(fabsf(out[i][c])));
       }
     }
-    largest = __uint_as_float(__reduce_max_sync(0xFFFFFFFFU, __float_as_uint(largest)));
-    if (lane == 0) {
-      s_max[warp] = largest;
+#pragma unroll
+    for (int c = 0; c < Count; ++c) {
+      atomicMax(&s_largest[c][sub], largest[c]);
     }
     __syncthreads();
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) {
-      largest = fmaxf(largest, s_max[w]);
+    for (int c = 0; c < Count; ++c) {
+      scale[c] = gdn_power(gdn_scale_exponent(__uint_as_float(s_largest[c][sub])));
     }
-    // exponent e with largest in [2^e, 2^(e+1)); the scale is 2^(13 - e), kept away from the ends of the FP32 range
-    const int biased = static_cast<int>(__float_as_uint(largest) >> 23);
-    const int exponent = min(max(127 + 13 + 127 - biased, 27), 227);
-    scale = __uint_as_float(static_cast<std::uint32_t>(exponent) << 23);
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < kGdnDim) {
       float *gates = reinterpret_cast<float *>(record_of(p, chunk, head) + kGdnRecGates);
-      gates[kGdnGateInvScale] = __uint_as_float(static_cast<std::uint32_t>(254 - exponent) << 23);
-      gates[kGdnGateMax] = largest;
+      gates[kGdnGateMax + threadIdx.x] = __uint_as_float(s_largest[threadIdx.x % Count][threadIdx.x / Count]);
     }
     image = p.scratch.v + (static_cast<std::size_t>(chunk) * p.value_heads + head) * kGdnVBytes;
     block = kGdnBlock;
   } else {
+#pragma unroll
+    for (int c = 0; c < Count; ++c) {
+      scale[c] = kGdnUnit;
+    }
     image = p.scratch.kq + (static_cast<std::size_t>(chunk) * p.key_heads + head) * kGdnKqBytes +
             (is_q ? kGdnBlock : 0U); // the Q rows follow the K rows of a block
     block = kGdnKqBlock;
@@ -433,7 +463,7 @@ __global__ void __launch_bounds__(Layout<Count>::kThreads, Layout<Count>::kCtas)
     std::uint32_t h[Count / 2];
 #pragma unroll
     for (int c = 0; c < Count / 2; ++c) {
-      h[c] = pack_half(out[i][2 * c] * scale, out[i][2 * c + 1] * scale);
+      h[c] = pack_half(out[i][2 * c] * scale[2 * c], out[i][2 * c + 1] * scale[2 * c + 1]);
     }
     if constexpr (Count == 8) {
       *reinterpret_cast<uint4 *>(to) = make_uint4(h[0], h[1], h[2], h[3]);
