@@ -5,8 +5,10 @@
 // around the library as ctypes does.
 //
 // Nothing of the library is linked in: kernels.py hands over the addresses of the entry points it has loaded and the
-// exception types that carry a failing status.  Accepted and refused are the arguments that ctypes took and refused:
-// integers are Python integers and wrap to their field, floats anything that converts to one.
+// exception types that carry a failing status.  Read here are the plain kinds of arguments: tensors, addresses, streams, the
+// shapes, integers (whatever has __index__; they wrap to their field, as in ctypes) and floats.  A call with any argument
+// that does not read as such goes to `through_ctypes` of kernels.py, so that what ctypes accepts is accepted and what it
+// refuses is refused with its own exceptions.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -20,21 +22,14 @@
 
 namespace {
 
-PyObject *g_argument_error = nullptr; // ctypes.ArgumentError
+PyObject *g_through_ctypes = nullptr; // (name, arguments ...)
 PyObject *g_errors[2] = {nullptr, nullptr}; // attention, gated delta
 PyObject *g_data_ptr = nullptr;
 PyObject *g_cuda_stream = nullptr;
 
-bool refuse(const char *expected, PyObject *got) {
-  PyErr_Format(g_argument_error, "%s expected instead of %s instance", expected, Py_TYPE(got)->tp_name);
-  return false;
-}
-
+// The readers return false for what they do not take, with or without an exception set.
 bool read_integer(PyObject *o, unsigned long long &value) {
-  if (!PyLong_Check(o)) {
-    return refuse("int", o);
-  }
-  value = PyLong_AsUnsignedLongLongMask(o);
+  value = PyLong_AsUnsignedLongLongMask(o); // calls __index__ of what is no int
   return !(value == static_cast<unsigned long long>(-1) && PyErr_Occurred());
 }
 bool read_float(PyObject *o, float &value) {
@@ -87,7 +82,7 @@ bool read_address(PyObject *owned, void *&value) {
     return false;
   }
   unsigned long long v = 0;
-  const bool ok = read_integer(owned, v);
+  const bool ok = PyLong_Check(owned) && read_integer(owned, v);
   Py_DECREF(owned);
   value = reinterpret_cast<void *>(static_cast<std::uintptr_t>(v));
   return ok;
@@ -188,6 +183,7 @@ using P = Pointer;
 // An entry point: its address in the loaded library, the kinds of its arguments and whose errors it raises.
 template <auto Declared, int Errors, class... Kinds> struct Entry {
   static inline decltype(Declared) function = nullptr;
+  static inline PyObject *name = nullptr;
   static PyObject *call(PyObject *, PyObject *const *args, Py_ssize_t count) {
     if (count != static_cast<Py_ssize_t>(sizeof...(Kinds))) {
       PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", static_cast<Py_ssize_t>(sizeof...(Kinds)), count);
@@ -198,7 +194,12 @@ template <auto Declared, int Errors, class... Kinds> struct Entry {
   template <std::size_t... I> static PyObject *run(PyObject *const *args, std::index_sequence<I...>) {
     std::tuple<Kinds...> kinds;
     if (!(std::get<I>(kinds).read(args[I]) && ...)) {
-      return nullptr;
+      PyErr_Clear();
+      if (g_through_ctypes == nullptr) {
+        PyErr_SetString(PyExc_RuntimeError, "entry point is not bound");
+        return nullptr;
+      }
+      return PyObject_CallFunctionObjArgs(g_through_ctypes, name, args[I]..., nullptr);
     }
     if (function == nullptr) {
       PyErr_SetString(PyExc_RuntimeError, "entry point is not bound");
@@ -219,7 +220,10 @@ template <auto Declared, int Errors, class... Kinds> struct Entry {
     }
     Py_RETURN_NONE;
   }
-  static void bind(void *address) { function = reinterpret_cast<decltype(Declared)>(address); }
+  static void bind(void *address, PyObject *bound_name) {
+    function = reinterpret_cast<decltype(Declared)>(address);
+    Py_XSETREF(name, Py_NewRef(bound_name));
+  }
 };
 
 constexpr int kAttention = 0;
@@ -249,7 +253,7 @@ using FastCall = PyObject *(*)(PyObject *, PyObject *const *, Py_ssize_t);
 struct Row {
   const char *name;
   FastCall call;
-  void (*bind)(void *);
+  void (*bind)(void *, PyObject *);
 };
 template <class E> constexpr Row row(const char *name) { return Row{name, &E::call, &E::bind}; }
 const Row kRows[] = {
@@ -268,15 +272,17 @@ const Row kRows[] = {
 };
 constexpr std::size_t kRowCount = sizeof(kRows) / sizeof(kRows[0]);
 
-// bind(address of a name, argument error, attention error, gated-delta error)
+// bind(address of a name, through_ctypes, attention error, gated-delta error)
 PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t count) {
   if (count != 4) {
-    PyErr_SetString(PyExc_TypeError, "bind takes a function and three exception types");
+    PyErr_SetString(PyExc_TypeError, "bind takes two functions and two exception types");
     return nullptr;
   }
   for (const Row &row : kRows) {
-    PyObject *address = PyObject_CallFunction(args[0], "s", row.name);
+    PyObject *name = PyUnicode_FromString(row.name);
+    PyObject *address = name != nullptr ? PyObject_CallOneArg(args[0], name) : nullptr;
     if (address == nullptr) {
+      Py_XDECREF(name);
       return nullptr;
     }
     void *value = PyLong_AsVoidPtr(address);
@@ -285,11 +291,13 @@ PyObject *bind(PyObject *, PyObject *const *args, Py_ssize_t count) {
       if (!PyErr_Occurred()) {
         PyErr_Format(PyExc_ImportError, "%s has no address", row.name);
       }
+      Py_DECREF(name);
       return nullptr;
     }
-    row.bind(value);
+    row.bind(value, name);
+    Py_DECREF(name);
   }
-  Py_XSETREF(g_argument_error, Py_NewRef(args[1]));
+  Py_XSETREF(g_through_ctypes, Py_NewRef(args[1]));
   Py_XSETREF(g_errors[kAttention], Py_NewRef(args[2]));
   Py_XSETREF(g_errors[kDelta], Py_NewRef(args[3]));
   Py_RETURN_NONE;

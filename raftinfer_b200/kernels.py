@@ -42,11 +42,6 @@ class Qwen35DeltaError(RuntimeError):
         self.code = code
 
 
-# The launchers go through native functions (csrc/binding.cpp); sizes, plans and the rest through ctypes.
-_call.bind(lambda name: C.cast(getattr(lib, name), C.c_void_p).value, C.ArgumentError, Qwen35PrimitiveError,
-           Qwen35DeltaError)
-
-
 def _check(status, exc=Qwen35PrimitiveError):
     if status.code != OK:
         raise exc(status.code, (status.message or b"").decode())
@@ -66,6 +61,35 @@ def _stream(stream):
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
+
+
+def _ctypes_arguments(name, arguments):
+    """Arguments of a launcher as ctypes takes them: shapes and plans first, then the rest from left to right."""
+    types = _lib.PROTOTYPES[name]
+    stream_at = len(types) - (2 if name == "rib200_qk_norm_rope" else 1)
+    struct = lambda t: hasattr(t, "_type_") and isinstance(t._type_, type) and issubclass(t._type_, C.Structure)
+    held = {i: arguments[i].c() for i, t in enumerate(types) if struct(t)}
+    out = []
+    for i, (t, x) in enumerate(zip(types, arguments)):
+        if i in held:
+            out.append(C.byref(held[i]))
+        elif t is _lib.vp:
+            out.append(_stream(x) if i == stream_at else _ptr(x))
+        else:
+            out.append(x.c() if issubclass(t, C.Structure) else x)
+    return out
+
+
+def _through_ctypes(name, *arguments):
+    """A launcher call whose arguments are not all of the plain kinds that the native function reads."""
+    _check(getattr(lib, name)(*_ctypes_arguments(name, arguments)),
+           Qwen35DeltaError if name in ("rib200_gated_delta", "rib200_gdn_core", "rib200_batched_gdn_decode")
+           else Qwen35PrimitiveError)
+
+
+# The launchers go through native functions (csrc/binding.cpp); sizes, plans and the rest through ctypes.
+_call.bind(lambda name: C.cast(getattr(lib, name), C.c_void_p).value, _through_ctypes, Qwen35PrimitiveError,
+           Qwen35DeltaError)
 
 
 @dataclass(frozen=True)
