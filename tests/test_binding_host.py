@@ -26,33 +26,49 @@ def test_native_launchers_take_the_declared_arguments_and_refuse_what_ctypes_ref
         call(*floats)
 
 
-def test_native_launchers_pass_every_field_on():
-    """Each refusal of the library names the argument it read; only the one that is off is off."""
+def test_refusals_of_the_library_name_the_argument_that_is_off():
+    """One argument or field off at a time: the refusal's code and text are the library's own for that one."""
     good = dict(tokens=2, query_heads=16, kv_heads=4, head_dim=256, max_context_tokens=256, past_tokens=0)
     call = lambda shape, dtype=K.DTYPE_BF16, policy=K.Qwen35AttentionLaunchPolicy(), cache_bytes=1 << 30, stream=16: \
         K.qwen35_causal_attention(16, 16, 16, 16, 16, 16, cache_bytes, None, 0, K.Qwen35AttentionShape(**shape), dtype,
                                   policy, stream)
-    attempts = [lambda f=f, v=v: call({**good, f: v}) for f, v in
-                [("tokens", 0), ("query_heads", 15), ("kv_heads", 0), ("head_dim", 255), ("max_context_tokens", 1),
-                 ("past_tokens", 255)]]
-    attempts += [lambda: call(good, dtype=9), lambda: call(good, cache_bytes=16), lambda: call(good, stream=None),
-                 lambda: call(good, policy=K.Qwen35AttentionLaunchPolicy(7, 1, 1)),
-                 lambda: call(good, policy=K.Qwen35AttentionLaunchPolicy(1, 1, 9))]
-    for attempt in attempts:
-        with pytest.raises(K.Qwen35PrimitiveError):
+    attempts = [(lambda f=f, v=v: call({**good, f: v}), code, text) for f, v, code, text in
+                [("tokens", 0, K.INVALID_ARGUMENT, "tokens must be positive"),
+                 ("query_heads", 15, K.INVALID_ARGUMENT, "query_heads must be a multiple of kv_heads"),
+                 ("kv_heads", 0, K.INVALID_ARGUMENT, "kv_heads must be positive"),
+                 ("head_dim", 255, K.UNSUPPORTED, "head_dim 256"),
+                 ("max_context_tokens", 1, K.INVALID_ARGUMENT, "context exceeds the cache capacity"),
+                 ("past_tokens", 255, K.INVALID_ARGUMENT, "context exceeds the cache capacity")]]
+    attempts += [(lambda: call(good, dtype=9), K.INVALID_ARGUMENT, "unknown activation dtype"),
+                 (lambda: call(good, cache_bytes=16), K.INVALID_ARGUMENT, "KV cache is too small"),
+                 (lambda: call(good, stream=None), K.INVALID_ARGUMENT, "stream is null"),
+                 (lambda: call(good, policy=K.Qwen35AttentionLaunchPolicy(7, 1, 1)), K.INVALID_ARGUMENT,
+                  "unknown attention implementation"),
+                 (lambda: call(good, policy=K.Qwen35AttentionLaunchPolicy(1, 1, 9)), K.INVALID_ARGUMENT,
+                  "unknown KV cache layout")]
+    for attempt, code, text in attempts:
+        with pytest.raises(K.Qwen35PrimitiveError, match=text) as refusal:
             attempt()
+        assert refusal.value.code == code
     delta = dict(tokens=2, hidden_size=256, key_heads=1, value_heads=2, key_dim=128, value_dim=128, conv_width=4,
                  epsilon=1.0e-6)
-    for field, value in [("tokens", 0), ("hidden_size", 255), ("key_heads", 3), ("value_heads", 3), ("key_dim", 0),
-                         ("value_dim", 64), ("conv_width", 0), ("epsilon", -1.0)]:
-        with pytest.raises(K.Qwen35DeltaError):
-            K.qwen35_gated_delta(16, 16, 16, 16, 16, 16, 16, 16, 16, 1 << 30, K.GatedDeltaShape(**{**delta, field: value}),
-                                 K.DTYPE_F32, K.DTYPE_F32, 16, K.GatedDeltaLaunchPolicy())
-    for policy in (K.GatedDeltaLaunchPolicy(9, 4, False), K.GatedDeltaLaunchPolicy(0, 3, False),
-                   K.GatedDeltaLaunchPolicy(0, 4, True)):
-        with pytest.raises(K.Qwen35DeltaError):
-            K.qwen35_gated_delta(16, 16, 16, 16, 16, 16, 16, 16, 16, 1 << 30, K.GatedDeltaShape(**delta), K.DTYPE_F32,
-                                 K.DTYPE_F32, 16, policy)
+    call = lambda shape, policy=K.GatedDeltaLaunchPolicy(): \
+        K.qwen35_gated_delta(16, 16, 16, 16, 16, 16, 16, 16, 16, 1 << 30, K.GatedDeltaShape(**shape), K.DTYPE_F32,
+                             K.DTYPE_F32, 16, policy)
+    attempts = [(lambda f=f, v=v: call({**delta, f: v}), text) for f, v, text in
+                [("tokens", 0, "tokens must be positive"), ("hidden_size", 255, "must equal hidden_size"),
+                 ("key_heads", 3, "value_heads must be a multiple of key_heads"),
+                 ("value_heads", 3, "must equal hidden_size"), ("key_dim", 0, "key_dim must be positive"),
+                 ("value_dim", 64, "must equal hidden_size"), ("conv_width", 0, "conv_width must be positive"),
+                 ("epsilon", -1.0, "epsilon must be finite and non-negative")]]
+    attempts += [(lambda p=p: call(delta, p), text) for p, text in
+                 [(K.GatedDeltaLaunchPolicy(9, 4, False), "unknown gated-delta schedule"),
+                  (K.GatedDeltaLaunchPolicy(0, 3, False), "four warps per block"),
+                  (K.GatedDeltaLaunchPolicy(0, 4, True), "transposed boundary state")]]
+    for attempt, text in attempts:
+        with pytest.raises(K.Qwen35DeltaError, match=text) as refusal:
+            attempt()
+        assert refusal.value.code == K.INVALID_ARGUMENT
 
 
 # ---- against ctypes, on stand-ins that record what arrives (cpp/recording_stub.cpp) ----

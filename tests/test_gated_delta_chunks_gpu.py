@@ -169,6 +169,24 @@ def in_half(run, dtype):
         run.inp = run.inp.astype(np.float16).astype(np.float32)
 
 
+@pytest.mark.parametrize("hk,hv,tokens", [(HK, HV, 1900), (2, 6, 10400)])
+@pytest.mark.parametrize("dtype", [K.DTYPE_BF16, K.DTYPE_F16])
+def test_long_layer_calls(hk, hv, tokens, dtype):
+    """16-bit calls of 1776 CTAs and more take the image kernel with eight dims a lane, here with a ragged tail and a
+    history; with six value heads the packed rows lie off the 16-byte boundary.  One more token follows on the states."""
+    run = LayerRun(0xB2006500 + hv, hk, hv, 4, dtype, K.DTYPE_F32, tokens + 1)
+    in_half(run, dtype)
+    for count in (tokens, 1):
+        out, want, _ = run.step(count)
+        # the output is rounded to 16 bits: 2^-8 or 2^-11 of the value at most, beside what the products leave
+        got, rounding = to_numpy_f32(out).reshape(want.shape), 2.0 ** (-8 if dtype == K.DTYPE_BF16 else -11)
+        assert np.isfinite(got).all() and (np.abs(got - want) <= rounding * np.abs(want) + 3.0e-2).all()
+        assert compare(got, want)["rel_l2"] <= 1.0e-2
+        assert compare(to_numpy_f32(run.d_cs).reshape(-1), run.cs.reshape(-1))["max_abs"] == 0.0
+        assert compare(to_numpy_f32(run.d_rs).reshape(-1), run.rs.reshape(-1))["rel_l2"] <= 1.0e-3
+    assert K.device_status(torch.cuda.current_stream()) == 0
+
+
 @pytest.mark.parametrize("dtype", [K.DTYPE_BF16, K.DTYPE_F16])
 def test_a_long_layer_call_equals_the_same_tokens_in_pieces(dtype):
     """Pieces of whole chunks take the image kernel with four dims a lane, the whole call the one with eight; outputs,

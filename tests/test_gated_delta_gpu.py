@@ -217,7 +217,7 @@ class LayerRun:
         if self.dtype == K.DTYPE_F32 and not chunked:
             assert m["max_abs"] <= 2.0e-3 and m["rel_l2"] <= 2.0e-4, m  # FP32 recurrent path
         if self.dtype == K.DTYPE_F32 and chunked:
-            assert m["max_abs"] <= 1.5e-2 and m["rel_l2"] <= 2.0e-3, m  # TF32 tensor-core products
+            assert m["max_abs"] <= 1.5e-2 and m["rel_l2"] <= 2.0e-3, m  # products of ten-bit mantissas
         cs = compare(to_numpy_f32(self.d_cs).reshape(-1), self.cs.reshape(-1))
         assert cs["max_abs"] == 0.0, cs
         rs = compare(to_numpy_f32(self.d_rs).reshape(-1), self.rs.reshape(-1))
