@@ -11,8 +11,16 @@ from __future__ import annotations
 import ctypes as C
 from dataclasses import dataclass
 
-from . import _call, _lib
+from . import _lib
 from ._lib import lib
+
+try:
+    from . import _call
+except ImportError as error:
+    raise ImportError(
+        "the package's native functions (raftinfer_b200/_call*.so) are missing or were built for another interpreter: build "
+        "them with `python -c 'import __graft_entry__ as g; g.build()'` (or `make -C raftinfer_b200/csrc "
+        "PYTHON=<interpreter>`, which needs that interpreter's headers).") from error
 
 # RaftInferDataType, cpp/include/raftinfer/tensor.h:10-15
 DTYPE_F32, DTYPE_F16, DTYPE_BF16 = 1, 2, 3

@@ -3,6 +3,8 @@ import ctypes
 import os
 import shutil
 import subprocess
+import sys
+import sysconfig
 
 import numpy as np
 import pytest
@@ -173,3 +175,21 @@ def test_what_ctypes_accepts_is_accepted_and_what_it_refuses_refused_alike(name,
                 assert text(native) == text(reference), (i, candidate)
                 accepted += isinstance(native, bytes)
     assert accepted > 0
+
+
+# ---- the built file ----
+def test_the_native_functions_are_of_this_interpreter_and_say_how_to_be_built(tmp_path):
+    """The file carries the interpreter's ABI tag; where it is missing the import names the way to build it, and a make
+    without Python's headers still gives the library."""
+    assert _call.__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    package = os.path.join(ROOT, "raftinfer_b200")
+    (tmp_path / "raftinfer_b200").mkdir()
+    for name in ("__init__.py", "_lib.py", "kernels.py", "librib200.so"):
+        os.symlink(os.path.join(package, name), tmp_path / "raftinfer_b200" / name)
+    run = subprocess.run([sys.executable, "-c", "import raftinfer_b200.kernels"], cwd=tmp_path, capture_output=True,
+                         text=True, env={**os.environ, "PYTHONPATH": ""})
+    assert run.returncode != 0 and "built for another interpreter" in run.stderr and "g.build()" in run.stderr
+    if shutil.which("make"):
+        plan = subprocess.run(["make", "-n", "-C", os.path.join(package, "csrc"), "PYTHON=/nonexistent/python"],
+                              capture_output=True, text=True)
+        assert plan.returncode == 0 and "binding.cpp" not in plan.stdout
