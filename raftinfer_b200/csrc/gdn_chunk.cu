@@ -858,10 +858,10 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 // chunk rounds the few elements below FP16's normal range differently on either side of a cut).  Inside that window the
 // image of the state is exact to 2^-26.
 // Columns whose bounds lie within 2^10 of each other, as they nearly always do, share the factor of the largest, and
-// everybody works with one number; else every column has its own, which costs some 200 cycles a chunk.  (One factor per
-// (chunk, slice) at all times left a column that is 1e-6 of the slice's largest with errors of 2e-3.  All of the scales
-// together, columns of V, units and growth included, cost 5 % of a layer call: 4096 tokens 186.5 -> 195.8 us, 149 tokens
-// 21.6 -> 23.0.)
+// everybody works with one number; else every column has its own, which costs up to 700 cycles a chunk (4096 tokens 216 us
+// and not 194 if all chunks do so).  One factor per (chunk, slice) at all times left a column that is 1e-6 of the slice's
+// largest with errors of 2e-3.  All of the scales together, columns of V, units and growth included, cost 3 to 5 % of a
+// layer call (replayed calls of 64 tokens 16.8 -> 17.4 us, 512 tokens 30.9 -> 32.5, 4096 tokens 185.5 -> 193.8).
 // Warp 10 makes the factors while the first product of the chunk runs, from column maxima that warps 0-3 leave as soon as
 // the state is on its way; the gates it needs it reads from memory two chunks ahead.
 // Every mbarrier wait is bounded; when one runs out the CTA records RIB200_DEVICE_WAIT_TIMED_OUT, stops waiting and

@@ -194,33 +194,36 @@ __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t 
   for (std::uint32_t h = warp; h < kGateHeads && head0 + h < p.value_heads; h += kWarps) {
     float a = s_decay[lane][h];
     float b = s_decay[lane + 32][h];
+    const bool grows = __any_sync(0xFFFFFFFFU, a > 0.0F || b > 0.0F);
+    // magnitudes, NaN left out: a token that is NaN must not take the scales of the tokens in front of it along
+    const float beta_a = fmaxf(fabsf(s_beta[lane][h]), 0.0F);
+    const float beta_b = fmaxf(fabsf(s_beta[lane + 32][h]), 0.0F);
+    float beta_sum = beta_a + beta_b;
+    const float beta_max = __uint_as_float(__reduce_max_sync(0xFFFFFFFFU, __float_as_uint(fmaxf(beta_a, beta_b))));
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const float ua = __shfl_up_sync(0xFFFFFFFFU, a, d);
       const float ub = __shfl_up_sync(0xFFFFFFFFU, b, d);
+      beta_sum += __shfl_xor_sync(0xFFFFFFFFU, beta_sum, d);
       if (lane >= d) {
         a += ua;
         b += ub;
       }
     }
     b += __shfl_sync(0xFFFFFFFFU, a, 31);
-    // largest G_i - G_j over j <= i, the start of the chunk (0) among the j; NaN drops out of minima and maxima
-    float low_a = fminf(a, 0.0F);
-    float low_b = b;
+    float growth = 1.0F;
+    if (grows) { // largest G_i - G_j over j <= i, the start of the chunk (0) among the j; NaN drops out
+      float low_a = fminf(a, 0.0F);
+      float low_b = b;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      low_a = fminf(low_a, __shfl_up_sync(0xFFFFFFFFU, low_a, d)); // a lane without a neighbour gets its own value
-      low_b = fminf(low_b, __shfl_up_sync(0xFFFFFFFFU, low_b, d));
-    }
-    low_b = fminf(low_b, __shfl_sync(0xFFFFFFFFU, low_a, 31));
-    float rise = fmaxf(fmaxf(a - low_a, b - low_b), 0.0F);
-    float beta_sum = s_beta[lane][h] + s_beta[lane + 32][h];
-    float beta_max = fmaxf(s_beta[lane][h], s_beta[lane + 32][h]);
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) {
-      rise = fmaxf(rise, __shfl_xor_sync(0xFFFFFFFFU, rise, offset));
-      beta_sum += __shfl_xor_sync(0xFFFFFFFFU, beta_sum, offset);
-      beta_max = fmaxf(beta_max, __shfl_xor_sync(0xFFFFFFFFU, beta_max, offset));
+      for (int d = 1; d < 32; d <<= 1) {
+        low_a = fminf(low_a, __shfl_up_sync(0xFFFFFFFFU, low_a, d)); // a lane without a neighbour gets its own value
+        low_b = fminf(low_b, __shfl_up_sync(0xFFFFFFFFU, low_b, d));
+      }
+      low_b = fminf(low_b, __shfl_sync(0xFFFFFFFFU, low_a, 31));
+      const float rise = fmaxf(fmaxf(a - low_a, b - low_b), 0.0F);
+      const float most = __uint_as_float(__reduce_max_sync(0xFFFFFFFFU, __float_as_uint(rise)));
+      growth = fminf(expf(most), 0x1p100F);
     }
     float *gates = reinterpret_cast<float *>(record_of(p, chunk, head0 + h) + kGdnRecGates);
     gates[kGdnGateG + lane] = a;
@@ -228,7 +231,7 @@ __device__ __forceinline__ void gate_arrays(const ImageParams &p, std::uint32_t 
     gates[kGdnGateBeta + lane] = s_beta[lane][h];
     gates[kGdnGateBeta + 32 + lane] = s_beta[lane + 32][h];
     if (lane == 0) {
-      gates[kGdnGateGrowth] = fminf(expf(rise), 0x1p100F);
+      gates[kGdnGateGrowth] = growth;
       gates[kGdnGateBetaSum] = beta_sum;
       gates[kGdnGateBetaMax] = beta_max;
     }
