@@ -95,7 +95,8 @@ template <int Warps, int Slots> struct Tile {
 constexpr float kLog2e = 1.4426950408889634F;
 // Rows of K and of V that a CTA asks for ahead of its turn: 64 MB over the whole grid, half of L2, and at most 128 a
 // CTA.  Eight layers at 32K (512 CTAs): 258 us without, 251 with 64 rows, 242 with 128, 262 with 256 (L2 then loses what
-// it was asked for); two layers at 128K (2048 CTAs): 192 us without, 196 with 128, 234 with 256.
+// it was asked for); two layers at 128K (2048 CTAs): 192 us without, 196 with 128, 234 with 256, and 192 to 194 with the 32
+// that the rule leaves there.
 constexpr std::uint32_t kPrefetchGridRows = 65536U;
 constexpr std::uint32_t kPrefetchMaxRows = 128U;
 constexpr std::uint32_t kPrefetchPiece = 32U; // rows per instruction
@@ -829,9 +830,11 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
 // each warp's chain of dependent steps is short.  All shapes are the same kernel template.
 //
 // A batch takes four warps a CTA from 149 CTAs on: its grid spans the longest cache, so many CTAs are empty, and four
-// warps finish a partition in a quarter of the steps.  Against one warp a CTA (864 CTAs, 9 ragged sequences up to 6000
-// tokens) 36.2 and 39.4 us, the same nine at full length 51.7 and 52.1, 24 sequences (1536 CTAs) 69.9 and 83.1, 64 up to
-// 32768 tokens 724.8 and 746.2; two warps a CTA gain on ragged batches (33.1) and lose on full ones (55.0).
+// warps finish a partition in a quarter of the steps.  The attention call alone behind a flushed L2, against one warp a CTA:
+// 9 ragged sequences up to 6000 tokens (864 CTAs) 35.8 and 37.9 us, the same nine at full length 52.2 and 54.3, 24
+// sequences (1536 CTAs) 68.6 and 78.8, 64 up to 32768 tokens 681 and 705; whole serving steps back to back, the gated-delta
+// half included: nine 38.8 and 41.0, 64 752.8 and 756.9.  Two warps a CTA gain on ragged batches (33.1 a step of nine
+// when this form took 36.2) and lose on full ones (55.0 against 51.7).
 template <bool F32, bool Batched, class T> void configure_once() {
   static std::once_flag flags[64];
   int device = 0;

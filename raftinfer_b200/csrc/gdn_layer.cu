@@ -73,7 +73,7 @@ struct LayerParams {
   const void *conv_weight, *recurrent_a, *dt_bias, *output_norm_weight;
   void *output;
   float *convolution_state;
-  float *recurrent_state; // single-token form only
+  float *recurrent_state; // one-launch forms only (1 to 63 tokens)
   float *convolved;
   float *beta;
   float *log_decay;
@@ -668,14 +668,15 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
 
 // ---- 2 .. 63 tokens in one launch --------------------------------------------------------------------------
 // The calls that end a prompt (the executor cuts a rest into 17, 4 and 2 tokens) are latency as well: the general path
-// took 53 us for 17 tokens and 25 us for 4 (prologue, history, recurrence, epilogue; launch list), this form 19 and 10.5.
+// took 53 us for 17 tokens and 25 us for 4 (prologue, history, recurrence, epilogue; launch list), this form 17.5 and 8.9
+// (replayed calls, as the figures below).
 // Same split as the one-token form - a cluster per key head, a CTA per 32 state columns - and the same arithmetic in
 // FP32; the tokens go through in tiles of 32: convolution and norms of a tile with a warp per token, then the recurrence
 // with the state in registers, then the output norm, for which the slices of a head exchange their sums once per tile.
 // In the recurrence a warp owns four columns and a lane four rows of them, so that a token needs no barrier: nine
 // shuffles bring the eight sums (S^T k, S^T q) to eight groups of lanes, four more hand the corrections back.
 constexpr std::uint32_t kShortTile = 32;
-// Longer calls run in chunks, which is faster (64 tokens 18.6 us, 63 here 47) but has products of ten-bit mantissas;
+// Longer calls run in chunks, which is faster (64 tokens 17.3 us, 63 here 45.6) but has products of ten-bit mantissas;
 // calls of fewer tokens are FP32 throughout, as they always were.
 constexpr std::uint32_t kShortMaxTokens = 63;
 constexpr std::uint32_t kShortRounds = kShortTile / 8; // tokens per warp

@@ -121,12 +121,6 @@ __device__ __forceinline__ long long global_ns() {
       g_trace[(block) * 16 + (slot)] = clock64();                                   \
     }                                                                               \
   } while (0)
-#define RIB200_STAMP_CTA2(slot)                                                     \
-  do {                                                                              \
-    if (blockIdx.x == 2 && blockIdx.y == 0) {                                       \
-      g_trace[120 * 16 + (slot)] = global_ns();                                     \
-    }                                                                               \
-  } while (0)
 #define RIB200_STAMP_NS(slot)                                                       \
   do {                                                                              \
     if (blockIdx.x == 0 && blockIdx.y == 0) {                                       \
@@ -138,9 +132,6 @@ __device__ __forceinline__ long long global_ns() {
   do {                                                                              \
   } while (0)
 #define RIB200_STAMP(block, slot)                                                   \
-  do {                                                                              \
-  } while (0)
-#define RIB200_STAMP_CTA2(slot)                                                     \
   do {                                                                              \
   } while (0)
 #endif
@@ -678,7 +669,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (threadIdx.x == 0) {
     RIB200_STAMP(0, 14); // set-up done
     RIB200_STAMP_NS(3);
-    RIB200_STAMP_CTA2(4);
   }
   const std::uint32_t tmem = *tmem_slot;
   const std::uint32_t tmem_o = tmem;         // columns [0, 256)
