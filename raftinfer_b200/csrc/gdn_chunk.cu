@@ -1312,6 +1312,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
       if (lane == 0) {
         to[kScaleEqual / 4] = equal && state_equal ? 1.0F : 0.0F;
       }
+      __syncwarp();
       asm volatile("bar.arrive 3, 160;\n" ::: "memory");
       now = following;
       following = gates_of(min(chunk + 2, p.chunks - 1));
@@ -1359,6 +1360,7 @@ template <int Dtype> __global__ void __launch_bounds__(kChainThreads, 1) gdn_chu
         }
       }
       mbarrier_arrive(bar(kBarRead + at.stage));
+      __syncwarp(); // lanes may have left the wait above one by one
       asm volatile("bar.sync 3, 160;\n" ::: "memory");
       auto walk = [&](auto kind) {
         using Factors = typename decltype(kind)::Type;
