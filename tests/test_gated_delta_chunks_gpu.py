@@ -88,15 +88,15 @@ def test_columns_of_any_magnitude(name, dtype):
     check_columns(*run_core(q, k, v.astype(np.float32), beta, g, state0.astype(np.float32), dtype), fades=name in FADES)
 
 
-@pytest.mark.parametrize("where", ["value", "state"])
-def test_an_infinity_stays_in_its_column(where):
+@pytest.mark.parametrize("where,what", [("value", np.inf), ("value", np.nan), ("state", np.inf), ("state", np.nan)])
+def test_what_is_not_finite_stays_in_its_column(where, what):
     tokens, hk, hv, seed = 200, 1, 2, 0xB2006100
     q, k, v, beta, g = core_operands(seed, tokens, hk, hv)
     state0 = (0.05 * synth.normal(seed, 5, (hv, DK, DK))).astype(np.float32)
     if where == "value":
-        v[70, 1, 37] = np.inf
+        v[70, 1, 37] = what
     else:
-        state0[1, 3, 37] = np.inf
+        state0[1, 3, 37] = what
     got_out, got_state, want_out, want_state = run_core(q, k, v, beta, g, state0, K.DTYPE_BF16)
     others = [c for c in range(DK) if c != 37]
     check_columns(got_out, got_state, want_out, want_state, others)
@@ -229,6 +229,27 @@ def test_saturated_gates_in_chunks():
     assert m["nonfinite"] == 0 and m["rel_l2"] <= COLUMN_TOLERANCE, m
     m = compare(to_numpy_f32(run.d_rs).reshape(-1), run.rs.reshape(-1))
     assert m["nonfinite"] == 0 and m["rel_l2"] <= COLUMN_TOLERANCE, m
+
+
+@pytest.mark.parametrize("dtype", [K.DTYPE_BF16, K.DTYPE_F16, K.DTYPE_F32])
+def test_layer_with_columns_of_any_magnitude(dtype):
+    """Value channels whose convolution weights are ten decades apart, so that every column has factors of its own, in the
+    form of the chain that norms and gates the outputs; another call follows on the states."""
+    hk, hv, calls = 2, 4, (200, 70)
+    run = LayerRun(0xB2006900, hk, hv, 4, dtype, K.DTYPE_F32, sum(calls))
+    if dtype == K.DTYPE_F16:
+        run.inp = run.inp.astype(np.float16).astype(np.float32)
+    factors = np.resize((10.0 ** -np.arange(10)).astype(np.float32), DK)
+    run.conv_w[2 * hk * DK:] *= np.tile(factors, hv)[:, None]
+    run.rs *= factors
+    run.d_conv_w, run.d_rs = act_tensor(run.conv_w, K.DTYPE_F32), torch.from_numpy(run.rs.copy()).to(dev())
+    for count in calls:
+        out, want, _ = run.step(count)
+        got = to_numpy_f32(out).reshape(want.shape)
+        assert compare(got, want)["nonfinite"] == 0 and compare(got, want)["rel_l2"] <= 1.0e-2
+        errors = column_errors(to_numpy_f32(run.d_rs).reshape(hv, DK, DK), run.rs.reshape(hv, DK, DK), 1)
+        assert errors.max() <= COLUMN_TOLERANCE, errors.max()
+    assert K.device_status(torch.cuda.current_stream()) == 0
 
 
 def test_layer_whose_coefficients_are_positive():
