@@ -17,6 +17,8 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 namespace rib200 {
 namespace {
 
@@ -43,7 +45,18 @@ __device__ __forceinline__ void store_any(void *base, std::size_t index, int32_t
   }
 }
 
-__device__ __forceinline__ float silu(float x) { return x / (1.0F + expf(-x)); }
+// x / d for d >= 1 or infinite: the unit's reciprocal and one step of Newton's iteration on the quotient, q + (x - d q) r, in
+// place of a division, whose slow path keeps the compiler from overlapping the chains of neighbouring tokens.  The
+// remainder is not a number exactly where x or d is infinite or not a number; x r is the quotient then.
+__device__ __forceinline__ float quotient(float x, float d) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+  const float q = x * r;
+  const float remainder = fmaf(-d, q, x);
+  return remainder == remainder ? fmaf(remainder, r, q) : q;
+}
+__device__ __forceinline__ float sigmoid(float x) { return quotient(1.0F, 1.0F + expf(-x)); }
+__device__ __forceinline__ float silu(float x) { return quotient(x, 1.0F + expf(-x)); }
 
 __device__ __forceinline__ float softplus(float x) {
   if (x > 20.0F) {
@@ -82,6 +95,7 @@ struct LayerParams {
   std::uint32_t conv_dim, token_stride;
   float epsilon;
   int32_t dtype, weight_dtype;
+  unsigned int *status; // one-launch forms only
 };
 
 // grid (2*Hk + Hv head vectors, tokens), 128 threads = the 128 channels of the vector
@@ -116,7 +130,7 @@ __global__ void __launch_bounds__(kDim) gdn_prologue_kernel(const LayerParams p)
     const std::size_t gates = static_cast<std::size_t>(tok) * p.token_stride + p.conv_dim;
     const float b = load_any(p.input, gates + head, p.dtype);
     const float a = load_any(p.input, gates + p.value_heads + head, p.dtype);
-    p.beta[static_cast<std::size_t>(tok) * p.value_heads + head] = 1.0F / (1.0F + expf(-b));
+    p.beta[static_cast<std::size_t>(tok) * p.value_heads + head] = sigmoid(b);
     p.log_decay[static_cast<std::size_t>(tok) * p.value_heads + head] =
         load_any(p.recurrent_a, head, p.weight_dtype) * softplus(a + load_any(p.dt_bias, head, p.weight_dtype));
   }
@@ -200,7 +214,7 @@ template <int Dtype> __global__ void __launch_bounds__(256, 3) gdn_prologue_w4_k
         const std::size_t gates = static_cast<std::size_t>(tok) * p.token_stride + p.conv_dim;
         const float b = load_any(p.input, gates + head, p.dtype);
         const float a = load_any(p.input, gates + p.value_heads + head, p.dtype);
-        p.beta[static_cast<std::size_t>(tok) * p.value_heads + head] = 1.0F / (1.0F + expf(-b));
+        p.beta[static_cast<std::size_t>(tok) * p.value_heads + head] = sigmoid(b);
         p.log_decay[static_cast<std::size_t>(tok) * p.value_heads + head] = a_coeff * softplus(a + dt);
       }
     }
@@ -394,13 +408,14 @@ __global__ void __launch_bounds__(kDim) gdn_epilogue_kernel(const LayerParams p)
 // ---- one token in one launch ---------------------------------------------------------------------------
 // A decode step of the layer is latency: 4 MiB of state traffic (0.6 us of HBM) and 25 KB of input.  The four launches
 // of the general path (prologue, history, recurrence, epilogue) cost 12.0 us a layer in a captured chain of 24 layers,
-// most of it hand-over between grids; this form costs 3.6 us (4.2 MB of state in and out: 1.2 TB/s), 2.2
-// to 2.6 of kernel and the rest hand-over; 4.4 us without the L2 hints in front of the wait.
+// most of it hand-over between grids; this form costs 3.2 us (4.2 MB of state in and out: 1.3 TB/s), about
+// 2 of kernel and the rest hand-over; 3.6 us with a cluster barrier in place of the counted exchange of sums, and 4.4 us
+// without the L2 hints in front of the wait.
 //
 // A cluster serves one key head: four CTAs (32 state columns each) per value head that shares it, one or two value
 // heads.  Everything that has to meet across CTAs meets inside that cluster: the convolution history of the q and k
 // channels is read by all of its CTAs and rewritten by one, and the output norm needs the squares of all four column
-// slices; one cluster barrier covers both (the history is only written behind it).  Three value heads and more to a
+// slices; the exchange of those sums covers both (the history is only written behind it).  Three value heads and more to a
 // key head would need more than the portable eight CTAs and take the general path, as other convolution widths do.
 // 128 CTAs of 16 KiB of state each at the model's head counts: a thread's 64 bytes are one round of loads.
 template <int Dtype> struct Scalar;
@@ -458,6 +473,48 @@ __device__ __forceinline__ void hint_operands(const LayerParams &p, std::uint32_
   }
 }
 
+// The slices of a head exchange their sums of squares with stores that count on an mbarrier of the CTA they go to.  A cluster
+// barrier in their place costs a call about 0.5 us more: its release waits for whatever the thread has in flight.  Who has
+// the sums of all slices also knows that their CTAs have read the old history, and that nothing more will come.
+constexpr long long kWaitLimitCycles = 1LL << 28;
+__device__ __forceinline__ std::uint32_t smem_address(const void *p) {
+  return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
+}
+// by one thread, in front of the barrier that says that every CTA of the cluster has started
+__device__ __forceinline__ void expect_sums(std::uint64_t *bar, std::uint32_t bytes) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_address(bar)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_address(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void send_sum(const float *slot, std::uint64_t *bar, std::uint32_t to_rank, float value) {
+  std::uint32_t remote_slot;
+  std::uint32_t remote_bar;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote_slot) : "r"(smem_address(slot)), "r"(to_rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote_bar) : "r"(smem_address(bar)), "r"(to_rank));
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(remote_slot),
+               "r"(__float_as_uint(value)), "r"(remote_bar)
+               : "memory");
+}
+// bounded: when it runs out the status word says so and the call runs to its end
+__device__ __forceinline__ void wait_for_sums(std::uint64_t *bar, unsigned int *status) {
+  const long long started = clock64();
+  std::uint32_t done = 0;
+  while (done == 0) {
+    asm volatile("{\n"
+                 ".reg .pred p;\n"
+                 "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+                 "selp.u32 %0, 1, 0, p;\n"
+                 "}\n"
+                 : "=r"(done)
+                 : "r"(smem_address(bar))
+                 : "memory");
+    if (done == 0 && clock64() - started > kWaitLimitCycles) {
+      atomicOr(status, static_cast<unsigned int>(RIB200_DEVICE_WAIT_TIMED_OUT));
+      return;
+    }
+  }
+}
+
 template <int Dtype, int WeightDtype>
 __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const LayerParams p) {
   using Act = Scalar<Dtype>;
@@ -470,7 +527,10 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
   __shared__ __align__(16) float s_b[8][kStepColumns];
   __shared__ float s_dot[8];
   __shared__ __align__(16) float s_delta[kStepColumns];
-  __shared__ float s_norm[kStepSlices]; // written by the CTAs of the value head, this one included
+  // written by the CTAs of the value head, this one included; in the first CTA also by those of the other value head, to
+  // say that they have read the history of q and k
+  __shared__ float s_norm[kStepMaxRatio * kStepSlices];
+  __shared__ __align__(8) std::uint64_t s_norm_bar;
   std::uint32_t rank;
   std::uint32_t cluster_size;
   asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
@@ -483,6 +543,10 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
   const int lane = tid & 31;
   float *state = p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns;
   hint_operands<Dtype, WeightDtype>(p, key_head, head, slice);
+  if (tid == 0) {
+    expect_sums(&s_norm_bar, (rank == 0 ? cluster_size : kStepSlices) * 4);
+  }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
   grid_dependency_wait();
   grid_dependents_may_launch();
@@ -564,7 +628,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
     v_value = convolve(v);
     z_gate = Weight::widen(norm_weight) * silu(Act::widen(z));
     if (lane == 0) {
-      s_gates[0] = 1.0F / (1.0F + expf(-Act::widen(b)));
+      s_gates[0] = sigmoid(Act::widen(b));
       s_gates[1] = expf(Weight::widen(coefficient) * softplus(Act::widen(a) + Weight::widen(dt)));
     }
   }
@@ -635,17 +699,11 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
       norm += __shfl_xor_sync(0xFFFFFFFFU, norm, offset);
     }
     if (lane < kStepSlices) { // to the four CTAs of this value head
-      std::uint32_t remote;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
-                   : "=r"(remote)
-                   : "r"(static_cast<std::uint32_t>(__cvta_generic_to_shared(&s_norm[slice]))),
-                     "r"(rank - slice + lane));
-      asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote), "f"(norm) : "memory");
+      send_sum(&s_norm[slice], &s_norm_bar, rank - slice + lane, norm);
+    } else if (lane == kStepSlices && rank >= kStepSlices) {
+      send_sum(&s_norm[rank], &s_norm_bar, 0, 0.0F);
     }
-    __syncwarp();
   }
-  // The barrier orders the partial norms and marks the end of everybody's reads of the history.
-  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   const float4 delta = *reinterpret_cast<const float4 *>(&s_delta[col]);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -653,7 +711,9 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
         make_float4(decay * s[i].x + k_row[i] * delta.x, decay * s[i].y + k_row[i] * delta.y,
                     decay * s[i].z + k_row[i] * delta.z, decay * s[i].w + k_row[i] * delta.w);
   }
-  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (rank == 0 || warp == 0) {
+    wait_for_sums(&s_norm_bar, p.status);
+  }
   if (rank == 0) {
     shift_history(qk_channel, qk);
   }
@@ -667,313 +727,519 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
 }
 
 // ---- 2 .. 63 tokens in one launch --------------------------------------------------------------------------
-// The calls that end a prompt (the executor cuts a rest into 17, 4 and 2 tokens) are latency as well: the general path
-// took 53 us for 17 tokens and 25 us for 4 (prologue, history, recurrence, epilogue; launch list), this form 17.5 and 8.9
-// (replayed calls, as the figures below).
-// Same split as the one-token form - a cluster per key head, a CTA per 32 state columns - and the same arithmetic in
-// FP32; the tokens go through in tiles of 32: convolution and norms of a tile with a warp per token, then the recurrence
-// with the state in registers, then the output norm, for which the slices of a head exchange their sums once per tile.
-// In the recurrence a warp owns four columns and a lane four rows of them, so that a token needs no barrier: nine
-// shuffles bring the eight sums (S^T k, S^T q) to eight groups of lanes, four more hand the corrections back.
-constexpr std::uint32_t kShortTile = 32;
-// Longer calls run in chunks, which is faster (64 tokens 17.3 us, 63 here 45.6) but has products of ten-bit mantissas;
-// calls of fewer tokens are FP32 throughout, as they always were.
+// The calls that end a prompt (the executor cuts a rest into 17, 4 and 2 tokens) are latency as well.
+// A cluster of four CTAs per key head, a CTA per 32 state columns of all its value heads, so that the q and k channels are
+// convolved once for both heads and every cluster has SMs of its own: of the one-token form's clusters of eight, 15 fit on
+// the GPU with a CTA per SM, and the CTAs of the sixteenth share.  FP32 throughout.  The whole call goes through in one pass:
+//   loads         rows of 128 q or k channels, or of 32 v channels, a warp at a time into shared memory;
+//   convolution   in place, a channel per thread of warps 0-7 (q, k) and 8-9 (v), while warps 10-11 make the gates;
+//   norms         a warp per group of four tokens: the normalised vectors, and the products k_t . k_j and q_t . k_j of the
+//                 group, of which a lane per value head makes the group's coefficients;
+//   recurrence    a group at a time.  With G_t the product of the group's decays up to t and S0 the state in front of it,
+//                   y_t = beta_t (v_t - G_t S0^T k_t),  delta = (I + L)^-1 y,  L_tj = beta_t (G_t / G_j) (k_t . k_j), j < t
+//                   o_t = G_t S0^T q_t + sum over j <= t of (G_t / G_j) (q_t . k_j) delta_j
+//                   S   = G_3 S0 + sum over t of (G_3 / G_t) k_t delta_t^T
+//                 (the ratios are products of decays, nothing is divided), so that eight reductions over the rows and a
+//                 hand-back of corrections are paid once in four tokens.  A lane owns eight rows of four columns, a warp
+//                 eight columns; 32 sums over 16 lanes are 30 exchanges and leave token t, column c with lane 4 t + c.
+//   output norm   the slices of a head exchange their sums of squares.
+// Replayed calls (BF16), this form and the one before it (a warp per four columns, a token at a time, clusters of eight): 2
+// tokens 8.4 and 10.4 us, 17 14.4 and 18.6, 32 17 and 28.5, 48 22.7 and 39, 63 28 and 47.3.  At 63 tokens 44 k cycles: loads
+// 5 k, convolution 5.5 k, norms 4.4 k, recurrence 26 k - a group takes 1650 cycles of the 1400 that its instructions need
+// with two warps a scheduler - and the output 3 k.
 constexpr std::uint32_t kShortMaxTokens = 63;
-constexpr std::uint32_t kShortRounds = kShortTile / 8; // tokens per warp
-constexpr std::uint32_t kShortGroup = 4;               // tokens convolved together
+constexpr std::uint32_t kShortRows = 64;
+constexpr std::uint32_t kShortGroup = 4;
+constexpr int kShortThreads = 384;
+constexpr std::uint32_t kShortWarps = kShortThreads / 32;
+constexpr std::uint32_t kShortLoads = 6;  // q and k rows a warp has in flight
+constexpr std::uint32_t kShortRounds = (kStepMaxRatio * kShortRows + 4 * kShortWarps - 1) / (4 * kShortWarps);
 
-template <int Dtype, int WeightDtype>
-__global__ void __launch_bounds__(kStepThreads) gdn_layer_short_kernel(const LayerParams p) {
+struct ShortShared {
+  float qk[2][kShortRows][kDim];                  // inputs, then their convolutions, then normalised
+  float v[kStepMaxRatio][kShortRows][kStepColumns]; // inputs, then their convolutions, then the outputs
+  float4 scale[kStepMaxRatio][kShortRows];        // beta_t, G_t, G_3 / G_t, G_3
+  float4 solve[kStepMaxRatio][kShortRows];        // (I + L)^-1 at (t, t ^ 1), (t, t ^ 2), (t, t ^ 3)
+  float4 read[kStepMaxRatio][kShortRows];         // (G_t / G_j) (q_t . k_j) for j = t, t ^ 1, t ^ 2, t ^ 3
+  float dots[kShortRows / kShortGroup][16];
+  float beta[kStepMaxRatio][kShortRows];
+  float decay[kStepMaxRatio][kShortRows];
+  float norm[kStepSlices][kStepMaxRatio * kShortRows];
+  std::uint64_t norm_bar;
+};
+
+// Sums of N values over N neighbouring lanes: lane l of them gets the total of value l.
+template <int N> __device__ __forceinline__ float fold(float (&v)[N]) {
+#pragma unroll
+  for (int half = N / 2; half > 0; half >>= 1) {
+    const bool upper = (threadIdx.x & half) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float give = upper ? v[i] : v[i + half];
+      const float keep = upper ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xFFFFFFFFU, give, half);
+    }
+  }
+  return v[0];
+}
+// four neighbouring elements; Wide: they start on the boundary of one access
+template <int Dtype, bool Wide>
+__device__ __forceinline__ float4 load_quad(const typename Scalar<Dtype>::Type *at) {
+  if constexpr (Wide) {
+    return Io<Dtype>::load4(at, 0);
+  } else {
+    using Act = Scalar<Dtype>;
+    return make_float4(Act::widen(at[0]), Act::widen(at[1]), Act::widen(at[2]), Act::widen(at[3]));
+  }
+}
+
+template <int Dtype, int WeightDtype, bool Wide>
+__global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const LayerParams p) {
   using Act = Scalar<Dtype>;
   using Weight = Scalar<WeightDtype>;
   using ActType = typename Act::Type;
   using WeightType = typename Weight::Type;
-  constexpr int kHistory = kFastWidth - 1;
-  __shared__ __align__(16) float s_qk[2][kShortTile][kDim];
-  __shared__ float s_v[kShortTile][kStepColumns];
-  __shared__ float s_out[kShortTile][kStepColumns];
-  __shared__ float s_kq[kShortTile];
-  __shared__ float s_beta[kShortTile];
-  __shared__ float s_decay[kShortTile];
-  __shared__ float s_norm[2][kStepSlices][kShortTile]; // by parity of the tile
-  std::uint32_t rank;
-  std::uint32_t cluster_size;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
-  asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(cluster_size));
-  const std::uint32_t key_head = blockIdx.x / cluster_size;
-  const std::uint32_t head = key_head + (rank / kStepSlices) * p.key_heads;
-  const std::uint32_t slice = rank % kStepSlices;
+  constexpr std::uint32_t kHistory = kFastWidth - 1;
+  extern __shared__ __align__(16) unsigned char short_smem[];
+  ShortShared &sh = *reinterpret_cast<ShortShared *>(short_smem);
+  std::uint32_t slice;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(slice));
+  const std::uint32_t key_head = blockIdx.x / kStepSlices;
+  const std::uint32_t ratio = p.value_heads / p.key_heads;
+  const std::uint32_t n = p.tokens;
   const std::uint32_t tid = threadIdx.x;
   const std::uint32_t warp = tid >> 5;
   const std::uint32_t lane = tid & 31;
-  float *state = p.recurrent_state + static_cast<std::size_t>(head) * kDim * kDim + slice * kStepColumns;
-  hint_operands<Dtype, WeightDtype>(p, key_head, head, slice);
+  const auto *input = static_cast<const ActType *>(p.input);
+  const auto *conv_weight = static_cast<const WeightType *>(p.conv_weight);
+  auto head_of = [&](std::uint32_t index) { return key_head + (index < ratio ? index : 0U) * p.key_heads; };
+  const std::uint32_t q_channel = key_head * kDim;
+  const std::uint32_t k_channel = (p.key_heads + key_head) * kDim;
+  auto v_channel = [&](std::uint32_t index) { return 2 * p.key_heads * kDim + head_of(index) * kDim + slice * kStepColumns; };
+  auto z_column = [&](std::uint32_t index) {
+    return p.conv_dim + 2 * p.value_heads + head_of(index) * kDim + slice * kStepColumns;
+  };
+  // the channel a thread of warps 0-9 convolves
+  const bool convolves = warp < 8 || (warp < 10 && warp - 8 < ratio);
+  const std::uint32_t channel = warp < 8 ? (warp < 4 ? q_channel : k_channel) + (tid & (kDim - 1)) : v_channel(warp & 1U) + lane;
+  // recurrence: warps 0-3 have the first value head, 4-7 the second one if there is one; a lane's rows are
+  // 4 row_lane + 64 i .. + 3 and its columns `column` .. + 3 of the slice
+  const std::uint32_t h = (warp >> 2) & 1U;
+  const bool recurs = warp < 8 && h < ratio;
+  const std::uint32_t row_lane = lane & 15U;
+  const std::uint32_t column = 8 * (warp & 3U) + 4 * (lane >> 4);
+  float *state = p.recurrent_state + static_cast<std::size_t>(head_of(h)) * kDim * kDim + slice * kStepColumns;
+  auto state_row = [&](std::uint32_t i) {
+    return state + static_cast<std::size_t>(4 * row_lane + 64 * (i >> 2) + (i & 3U)) * kDim + column;
+  };
+
+  // While the kernels in front still run, this one asks for what it will read first (hints, no reads: what those kernels
+  // write is current in L2 either way).
+  if (recurs) {
+    hint_l2(state + static_cast<std::size_t>(tid & (kDim - 1)) * kDim);
+  }
+  if (convolves && lane % 8 == 0) {
+    hint_l2(conv_weight + static_cast<std::size_t>(channel) * kFastWidth);
+    hint_l2(p.convolution_state + static_cast<std::size_t>(channel) * kHistory);
+  }
+  if (warp < n && lane < 16) {
+    const ActType *row = input + static_cast<std::size_t>(warp) * p.token_stride;
+    const std::uint32_t index = (lane >> 2) & 1U;
+    const std::uint32_t what = lane & 3U;
+    hint_l2(row + (lane < 4    ? q_channel + 32 * what
+                   : lane < 8  ? k_channel + 32 * what
+                   : what == 0 ? v_channel(index)
+                   : what == 1 ? p.conv_dim + head_of(index)
+                   : what == 2 ? p.conv_dim + p.value_heads + head_of(index)
+                               : z_column(index)));
+  }
+  const std::uint32_t shift = ratio - 1;
+  const std::uint32_t rows = n << shift; // of v, z and the output: (token, value head)
+  if (tid == 0) {
+    expect_sums(&sh.norm_bar, rows * kStepSlices * 4);
+  }
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // every CTA of the cluster has started
   grid_dependency_wait();
   grid_dependents_may_launch();
 
-  const auto *input = static_cast<const ActType *>(p.input);
-  const auto *conv_weight = static_cast<const WeightType *>(p.conv_weight);
-  // state: lane = rows 4 lane .. + 3, warp = columns 4 warp .. + 3 of the slice
-  float4 s[4];
+  // ---- loads ----
+  float4 raw[kShortLoads];
+  auto load_rows = [&](std::uint32_t from) { // row r of the call's 2 n: q or k (bit 0) of token r / 2
 #pragma unroll
-  for (std::uint32_t i = 0; i < 4; ++i) {
-    s[i] = *reinterpret_cast<const float4 *>(state + static_cast<std::size_t>(4 * lane + i) * kDim + 4 * warp);
-  }
-  // threads 0..127 convolve the q channels of the key head, 128..255 its k channels; a lane a v channel of the slice
-  const std::uint32_t qk_channel = (tid < kDim ? 0 : p.key_heads * kDim) + key_head * kDim + (tid & (kDim - 1));
-  const std::uint32_t v_channel = 2 * p.key_heads * kDim + head * kDim + slice * kStepColumns + lane;
-  const std::uint32_t z_channel = p.conv_dim + 2 * p.value_heads + head * kDim + slice * kStepColumns + lane;
-  float qk_weight[kFastWidth];
-  float v_weight[kFastWidth];
-  float qk_history[kHistory]; // the three tokens in front of the call
-  float v_history[kHistory];
-#pragma unroll
-  for (int h = 0; h < kFastWidth; ++h) {
-    qk_weight[h] = Weight::widen(conv_weight[static_cast<std::size_t>(qk_channel) * kFastWidth + h]);
-    v_weight[h] = Weight::widen(conv_weight[static_cast<std::size_t>(v_channel) * kFastWidth + h]);
-  }
-#pragma unroll
-  for (int h = 0; h < kHistory; ++h) {
-    qk_history[h] = p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h];
-    v_history[h] = p.convolution_state[static_cast<std::size_t>(v_channel) * kHistory + h];
-  }
-  const float norm_weight =
-      Weight::widen(static_cast<const WeightType *>(p.output_norm_weight)[slice * kStepColumns + lane]);
-  const float coefficient = Weight::widen(static_cast<const WeightType *>(p.recurrent_a)[head]);
-  const float dt = Weight::widen(static_cast<const WeightType *>(p.dt_bias)[head]);
-  // a channel's input at a token of this call, or of the history in front of it
-  auto row = [&](std::uint32_t channel, const float (&history)[kHistory], int tok) {
-    return tok >= 0 ? Act::widen(input[static_cast<std::size_t>(tok) * p.token_stride + channel])
-                    : (tok == -1 ? history[2] : (tok == -2 ? history[1] : history[0]));
+    for (std::uint32_t i = 0; i < kShortLoads; ++i) {
+      const std::uint32_t row = from + warp + kShortWarps * i;
+      if (row < 2 * n) {
+        raw[i] = load_quad<Dtype, Wide>(input + static_cast<std::size_t>(row >> 1) * p.token_stride +
+                                        ((row & 1U) == 0 ? q_channel : k_channel) + 4 * lane);
+      }
+    }
   };
-  const std::uint32_t last = p.tokens - 1;
+  auto store_rows = [&](std::uint32_t from) {
+#pragma unroll
+    for (std::uint32_t i = 0; i < kShortLoads; ++i) {
+      const std::uint32_t row = from + warp + kShortWarps * i;
+      if (row < 2 * n) {
+        *reinterpret_cast<float4 *>(&sh.qk[row & 1U][row >> 1][4 * lane]) = raw[i];
+      }
+    }
+  };
+  load_rows(0);
+  // v and z: eight lanes a row
+  const std::uint32_t quad = 4 * (lane & 7U);
+  float4 v_raw[kShortRounds];
+  float4 z[kShortRounds];
+#pragma unroll
+  for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+    const std::uint32_t row = 4 * (warp + kShortWarps * r) + (lane >> 3);
+    if (row < rows) {
+      const ActType *at = input + static_cast<std::size_t>(row >> shift) * p.token_stride + quad;
+      v_raw[r] = load_quad<Dtype, Wide>(at + v_channel(row & shift));
+      z[r] = load_quad<Dtype, Wide>(at + z_column(row & shift));
+    }
+  }
+  float taps[kFastWidth];
+  float window[kHistory + kShortGroup]; // the three tokens in front of the call, then of the group
+  if (convolves) {
+    const float4 four = load_quad<WeightDtype, Wide && WeightDtype == RIB200_DTYPE_F32>(
+        conv_weight + static_cast<std::size_t>(channel) * kFastWidth);
+    taps[0] = four.x;
+    taps[1] = four.y;
+    taps[2] = four.z;
+    taps[3] = four.w;
+#pragma unroll
+    for (std::uint32_t i = 0; i < kHistory; ++i) {
+      window[i] = p.convolution_state[static_cast<std::size_t>(channel) * kHistory + i];
+    }
+  }
+  float4 s[8];
+  if (recurs) {
+#pragma unroll
+    for (std::uint32_t i = 0; i < 8; ++i) {
+      s[i] = *reinterpret_cast<const float4 *>(state_row(i));
+    }
+  }
+  store_rows(0);
+  for (std::uint32_t from = kShortWarps * kShortLoads; from < 2 * n; from += kShortWarps * kShortLoads) {
+    load_rows(from);
+    store_rows(from);
+  }
+#pragma unroll
+  for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+    const std::uint32_t row = 4 * (warp + kShortWarps * r) + (lane >> 3);
+    if (row < rows) {
+      *reinterpret_cast<float4 *>(&sh.v[row & shift][row >> shift][quad]) = v_raw[r];
+    }
+  }
+  __syncthreads();
 
-  for (std::uint32_t first = 0, tile = 0; first < p.tokens; first += kShortTile, ++tile) {
-    const std::uint32_t n = min(kShortTile, p.tokens - first);
-    // ---- convolution and SiLU: q and k a channel per thread, v and the gates a token per warp.  Whole groups of
-    // tokens without a branch, so that their long dependent chains overlap; rows past the last token are computed from
-    // it and not used. ----
-    {
-      ActType x[kShortTile];
+  // ---- convolution and SiLU, whole groups of four tokens, rows past the last one included (they are not used); gates ----
+  float next_history[kHistory] = {}; // the last three tokens of [old history | call]
+  if (convolves) {
+    float *at = warp < 8 ? &sh.qk[warp >> 2][0][tid & (kDim - 1)] : &sh.v[warp & 1U][0][lane];
+    const std::uint32_t pitch = warp < 8 ? kDim : kStepColumns;
 #pragma unroll
-      for (std::uint32_t group = 0; group < kShortTile; group += kShortGroup) {
-        if (group < n) {
+    for (std::uint32_t i = 0; i < kHistory; ++i) {
+      const std::uint32_t source = n + i; // position in [history | call], at least 2
+      next_history[i] = source >= kHistory ? at[(source - kHistory) * pitch] : window[2];
+    }
+#pragma unroll 1
+    for (std::uint32_t group = 0; group < n; group += kShortGroup) {
+      float value[kShortGroup];
 #pragma unroll
-          for (std::uint32_t t = group; t < group + kShortGroup; ++t) {
-            x[t] = input[static_cast<std::size_t>(min(first + t, last)) * p.token_stride + qk_channel];
-          }
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        window[kHistory + t] = at[t * pitch];
+        // the current token's tap first, then the history, oldest first
+        float sum = window[kHistory + t] * taps[kHistory];
+#pragma unroll
+        for (std::uint32_t i = 0; i < kHistory; ++i) {
+          sum += window[t + i] * taps[i];
+        }
+        value[t] = silu(sum);
+      }
+#pragma unroll
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        at[t * pitch] = value[t];
+      }
+#pragma unroll
+      for (std::uint32_t i = 0; i < kHistory; ++i) {
+        window[i] = window[kShortGroup + i];
+      }
+      at += kShortGroup * pitch;
+    }
+  } else if (warp - 10 < ratio) {
+    const std::uint32_t index = warp - 10;
+    const float coefficient = Weight::widen(static_cast<const WeightType *>(p.recurrent_a)[head_of(index)]);
+    const float dt = Weight::widen(static_cast<const WeightType *>(p.dt_bias)[head_of(index)]);
+    for (std::uint32_t t = lane; t < n; t += 32) {
+      const ActType *gates = input + static_cast<std::size_t>(t) * p.token_stride + p.conv_dim + head_of(index);
+      const float b = Act::widen(gates[0]);
+      const float a = Act::widen(gates[p.value_heads]);
+      sh.beta[index][t] = sigmoid(b);
+      sh.decay[index][t] = expf(coefficient * softplus(a + dt));
+    }
+  }
+  __syncthreads();
+
+  // ---- norms and products of a group of tokens per warp; tokens past the last one become zeros ----
+#pragma unroll 1
+  for (std::uint32_t group = warp; kShortGroup * group < n; group += kShortWarps) {
+    const std::uint32_t t0 = kShortGroup * group;
+    float4 q[kShortGroup];
+    float4 k[kShortGroup];
+    auto dot = [](const float4 &x, const float4 &y) { return (x.x * y.x + x.y * y.y) + (x.z * y.z + x.w * y.w); };
+    float squares[2 * kShortGroup];
+#pragma unroll
+    for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+      q[t] = *reinterpret_cast<const float4 *>(&sh.qk[0][t0 + t][4 * lane]);
+      k[t] = *reinterpret_cast<const float4 *>(&sh.qk[1][t0 + t][4 * lane]);
+      squares[t] = dot(q[t], q[t]);
+      squares[kShortGroup + t] = dot(k[t], k[t]);
+    }
+    float sum = fold(squares);
+    sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 8);
+    sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 16);
+    const float scale = rsqrtf(sum + kQkEpsilon) * ((lane & kShortGroup) == 0 ? rsqrtf(static_cast<float>(kDim)) : 1.0F);
+#pragma unroll
+    for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+      const float q_scale = __shfl_sync(0xFFFFFFFFU, scale, t);
+      const float k_scale = __shfl_sync(0xFFFFFFFFU, scale, kShortGroup + t);
+      const bool live = t0 + t < n;
+      q[t] = live ? make_float4(q[t].x * q_scale, q[t].y * q_scale, q[t].z * q_scale, q[t].w * q_scale)
+                  : make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+      k[t] = live ? make_float4(k[t].x * k_scale, k[t].y * k_scale, k[t].z * k_scale, k[t].w * k_scale)
+                  : make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+      *reinterpret_cast<float4 *>(&sh.qk[0][t0 + t][4 * lane]) = q[t];
+      *reinterpret_cast<float4 *>(&sh.qk[1][t0 + t][4 * lane]) = k[t];
+    }
+    // k_t . k_j at 4 t + j for j < t, q_t . k_j at 4 j + t for j <= t: below, and on and above the diagonal of one square
+    float dots[16];
+#pragma unroll
+    for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+#pragma unroll
+      for (std::uint32_t j = 0; j <= t; ++j) {
+        if (j < t) {
+          dots[4 * t + j] = dot(k[t], k[j]);
+        }
+        dots[4 * j + t] = dot(q[t], k[j]);
+      }
+    }
+    float total = fold(dots);
+    total += __shfl_xor_sync(0xFFFFFFFFU, total, 16);
+    if (lane < 16) {
+      sh.dots[group][lane] = total;
+    }
+    __syncwarp();
+    if (lane < ratio) {
+      const float *d = sh.dots[group];
+      float beta[kShortGroup];
+      float decay[kShortGroup];
+      double product[kShortGroup][kShortGroup]; // [t][j]: the decays of the tokens after j up to t, rounded once when used
+#pragma unroll
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        const bool live = t0 + t < n;
+        beta[t] = live ? sh.beta[lane][t0 + t] : 0.0F;
+        decay[t] = live ? sh.decay[lane][t0 + t] : 1.0F;
+      }
+#pragma unroll
+      for (std::uint32_t j = 0; j < kShortGroup; ++j) {
+        product[j][j] = 1.0;
+#pragma unroll
+        for (std::uint32_t t = j + 1; t < kShortGroup; ++t) {
+          product[t][j] = product[t - 1][j] * decay[t];
         }
       }
-      float before[kHistory];
+      float solve[kShortGroup][kShortGroup]; // (I + L)^-1, by rows
 #pragma unroll
-      for (int h = 0; h < kHistory; ++h) {
-        before[h] = row(qk_channel, qk_history, static_cast<int>(first) - kHistory + h);
-      }
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        float row_l[kShortGroup];
 #pragma unroll
-      for (std::uint32_t r = 0; r < kShortRounds; ++r) {
-        if (8 * r < n) {
-          const std::uint32_t t = warp + 8 * r;
-          const int tok = static_cast<int>(min(first + t, last));
-          // the current token's tap first, then the history, oldest first
-          float sum = row(v_channel, v_history, tok) * v_weight[kHistory];
-#pragma unroll
-          for (int h = 0; h < kHistory; ++h) {
-            sum += row(v_channel, v_history, tok - kHistory + h) * v_weight[h];
-          }
-          s_v[t][lane] = silu(sum);
+        for (std::uint32_t j = 0; j < t; ++j) {
+          row_l[j] = static_cast<float>(beta[t] * product[t][j]) * d[4 * t + j];
         }
-      }
-      if (lane < kShortRounds && warp + 8 * lane < n) {
-        const std::uint32_t t = warp + 8 * lane;
-        const std::size_t gates = static_cast<std::size_t>(first + t) * p.token_stride + p.conv_dim + head;
-        s_beta[t] = 1.0F / (1.0F + expf(-Act::widen(input[gates])));
-        s_decay[t] = expf(coefficient * softplus(Act::widen(input[gates + p.value_heads]) + dt));
-      }
 #pragma unroll
-      for (std::uint32_t group = 0; group < kShortTile; group += kShortGroup) {
-        if (group < n) {
-          float value[kShortGroup];
+        for (std::uint32_t j = 0; j < kShortGroup; ++j) {
+          solve[t][j] = j == t ? 1.0F : 0.0F;
+          if (j < t) {
+            float x = -row_l[j];
 #pragma unroll
-          for (std::uint32_t t = 0; t < kShortGroup; ++t) {
-            const float now = Act::widen(x[group + t]);
-            float sum = now * qk_weight[kHistory];
-#pragma unroll
-            for (int h = 0; h < kHistory; ++h) {
-              sum += before[h] * qk_weight[h];
+            for (std::uint32_t i = j + 1; i < t; ++i) {
+              x -= row_l[i] * solve[i][j];
             }
-            before[0] = before[1];
-            before[1] = before[2];
-            before[2] = now;
-            value[t] = silu(sum);
-          }
-#pragma unroll
-          for (std::uint32_t t = 0; t < kShortGroup; ++t) {
-            s_qk[tid >> 7][group + t][tid & (kDim - 1)] = value[t];
+            solve[t][j] = x;
           }
         }
       }
-    }
-    __syncthreads();
-    // ---- norms of q and k, k . q ----
-    for (std::uint32_t t = warp; t < n; t += 8) {
-      float4 q = *reinterpret_cast<const float4 *>(&s_qk[0][t][4 * lane]);
-      float4 k = *reinterpret_cast<const float4 *>(&s_qk[1][t][4 * lane]);
-      float qq = (q.x * q.x + q.y * q.y) + (q.z * q.z + q.w * q.w);
-      float kk = (k.x * k.x + k.y * k.y) + (k.z * k.z + k.w * k.w);
 #pragma unroll
-      for (int offset = 16; offset > 0; offset >>= 1) {
-        qq += __shfl_xor_sync(0xFFFFFFFFU, qq, offset);
-        kk += __shfl_xor_sync(0xFFFFFFFFU, kk, offset);
-      }
-      const float q_scale = rsqrtf(qq + kQkEpsilon) * rsqrtf(static_cast<float>(kDim));
-      const float k_scale = rsqrtf(kk + kQkEpsilon);
-      q = make_float4(q.x * q_scale, q.y * q_scale, q.z * q_scale, q.w * q_scale);
-      k = make_float4(k.x * k_scale, k.y * k_scale, k.z * k_scale, k.w * k_scale);
-      float kq = (k.x * q.x + k.y * q.y) + (k.z * q.z + k.w * q.w);
-#pragma unroll
-      for (int offset = 16; offset > 0; offset >>= 1) {
-        kq += __shfl_xor_sync(0xFFFFFFFFU, kq, offset);
-      }
-      *reinterpret_cast<float4 *>(&s_qk[0][t][4 * lane]) = q;
-      *reinterpret_cast<float4 *>(&s_qk[1][t][4 * lane]) = k;
-      if (lane == 0) {
-        s_kq[t] = kq;
-      }
-    }
-    __syncthreads();
-    // ---- the recurrence ----
-    // after the three exchanges lane l holds the sum of column 2 (l / 8 % 2) + (l / 4) % 2, of S^T k below lane 16 and
-    // of S^T q from there on
-    const std::uint32_t my_column = ((lane >> 3) & 1U) * 2 + ((lane >> 2) & 1U);
-    float4 next_k = *reinterpret_cast<const float4 *>(&s_qk[1][0][4 * lane]);
-    float4 next_q = *reinterpret_cast<const float4 *>(&s_qk[0][0][4 * lane]);
-    for (std::uint32_t t = 0; t < n; ++t) {
-      const float k[4] = {next_k.x, next_k.y, next_k.z, next_k.w};
-      const float q[4] = {next_q.x, next_q.y, next_q.z, next_q.w};
-      const float decay = s_decay[t];
-      const float beta = s_beta[t];
-      const float v_value = s_v[t][4 * warp + my_column];
-      const float kq = s_kq[t];
-      const std::uint32_t following = min(t + 1, kShortTile - 1);
-      next_k = *reinterpret_cast<const float4 *>(&s_qk[1][following][4 * lane]);
-      next_q = *reinterpret_cast<const float4 *>(&s_qk[0][following][4 * lane]);
-      float a[4] = {};
-      float b[4] = {};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        a[0] += s[i].x * k[i];
-        a[1] += s[i].y * k[i];
-        a[2] += s[i].z * k[i];
-        a[3] += s[i].w * k[i];
-        b[0] += s[i].x * q[i];
-        b[1] += s[i].y * q[i];
-        b[2] += s[i].z * q[i];
-        b[3] += s[i].w * q[i];
-      }
-      const bool upper = (lane & 16U) != 0;
-      float four[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        four[c] = (upper ? b[c] : a[c]) + __shfl_xor_sync(0xFFFFFFFFU, upper ? a[c] : b[c], 16);
-      }
-      const bool high_pair = (lane & 8U) != 0;
-      float two[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        two[c] = (high_pair ? four[2 + c] : four[c]) +
-                 __shfl_xor_sync(0xFFFFFFFFU, high_pair ? four[c] : four[2 + c], 8);
-      }
-      const bool odd = (lane & 4U) != 0;
-      float sum = (odd ? two[1] : two[0]) + __shfl_xor_sync(0xFFFFFFFFU, odd ? two[0] : two[1], 4);
-      sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 2);
-      sum += __shfl_xor_sync(0xFFFFFFFFU, sum, 1);
-      const float delta = (v_value - decay * sum) * beta; // below lane 16
-      float correction[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        correction[c] = __shfl_sync(0xFFFFFFFFU, delta, 4 * c);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        s[i].x = decay * s[i].x + k[i] * correction[0];
-        s[i].y = decay * s[i].y + k[i] * correction[1];
-        s[i].z = decay * s[i].z + k[i] * correction[2];
-        s[i].w = decay * s[i].w + k[i] * correction[3];
-      }
-      const float low = odd ? correction[1] : correction[0];
-      const float high = odd ? correction[3] : correction[2];
-      if (upper && (lane & 3U) == 0) {
-        s_out[t][4 * warp + my_column] = decay * sum + (high_pair ? high : low) * kq;
-      }
-    }
-    __syncthreads();
-    // ---- output norm over the four slices, gate ----
-    float z_gate[kShortRounds];
-    float read[kShortRounds];
-#pragma unroll
-    for (std::uint32_t r = 0; r < kShortRounds; ++r) {
-      const std::uint32_t t = warp + 8 * r;
-      if (t < n) {
-        z_gate[r] = norm_weight * silu(Act::widen(input[static_cast<std::size_t>(first + t) * p.token_stride + z_channel]));
-        read[r] = s_out[t][lane];
-      }
-    }
-    if (tile == 0) { // the barrier that says that every CTA of the cluster has started
-      asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
-    }
-#pragma unroll
-    for (std::uint32_t r = 0; r < kShortRounds; ++r) {
-      const std::uint32_t t = warp + 8 * r;
-      if (t < n) {
-        float norm = read[r] * read[r];
-#pragma unroll
-        for (int offset = 16; offset > 0; offset >>= 1) {
-          norm += __shfl_xor_sync(0xFFFFFFFFU, norm, offset);
-        }
-        if (lane < kStepSlices) { // to the four CTAs of this value head
-          std::uint32_t remote;
-          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
-                       : "=r"(remote)
-                       : "r"(static_cast<std::uint32_t>(__cvta_generic_to_shared(&s_norm[tile & 1U][slice][t]))),
-                         "r"(rank - slice + lane));
-          asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(remote), "f"(norm) : "memory");
-        }
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        auto read = [&](std::uint32_t j) { return j <= t ? static_cast<float>(product[t][j]) * d[4 * j + t] : 0.0F; };
+        sh.scale[lane][t0 + t] =
+            make_float4(beta[t], static_cast<float>(decay[0] * product[t][0]), static_cast<float>(product[kShortGroup - 1][t]),
+                        static_cast<float>(decay[0] * product[kShortGroup - 1][0]));
+        sh.solve[lane][t0 + t] = make_float4(solve[t][t ^ 1U], solve[t][t ^ 2U], solve[t][t ^ 3U], 0.0F);
+        sh.read[lane][t0 + t] = make_float4(read(t), read(t ^ 1U), read(t ^ 2U), read(t ^ 3U));
       }
     }
     __syncwarp();
-    // Orders the partial norms; that of the first tile also marks the end of everybody's reads of the old history.
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+  __syncthreads();
+
+  // ---- the recurrence ----
+  if (recurs) {
+    const std::uint32_t t = row_lane >> 2;
+    const bool second = (t & 1U) != 0; // has t ^ 1 in front of it
+    const bool upper = (t & 2U) != 0;  // has t ^ 2 and t ^ 3 in front of it
+#pragma unroll 1
+    for (std::uint32_t group = 0; group < n; group += kShortGroup) {
+      float k[kShortGroup][8];
+      auto fetch = [&](const float *vector, float (&x)[8]) {
+        const float4 low = *reinterpret_cast<const float4 *>(vector + 4 * row_lane);
+        const float4 high = *reinterpret_cast<const float4 *>(vector + 4 * row_lane + 64);
+        x[0] = low.x;
+        x[1] = low.y;
+        x[2] = low.z;
+        x[3] = low.w;
+        x[4] = high.x;
+        x[5] = high.y;
+        x[6] = high.z;
+        x[7] = high.w;
+      };
+      auto products = [&](const float (&x)[8], float *to) { // two chains of four a column
+        float4 low = make_float4(s[0].x * x[0], s[0].y * x[0], s[0].z * x[0], s[0].w * x[0]);
+        float4 high = make_float4(s[4].x * x[4], s[4].y * x[4], s[4].z * x[4], s[4].w * x[4]);
 #pragma unroll
-    for (std::uint32_t r = 0; r < kShortRounds; ++r) {
-      const std::uint32_t t = warp + 8 * r;
-      if (t < n) {
-        const float (&norms)[kStepSlices][kShortTile] = s_norm[tile & 1U];
-        const float norm = (norms[0][t] + norms[1][t]) + (norms[2][t] + norms[3][t]);
-        const float scale = rsqrtf(norm / static_cast<float>(kDim) + p.epsilon);
-        static_cast<ActType *>(p.output)[(static_cast<std::size_t>(first + t) * p.value_heads + head) * kDim +
-                                         slice * kStepColumns + lane] = Act::narrow(read[r] * scale * z_gate[r]);
+        for (int i = 1; i < 4; ++i) {
+          low.x = fmaf(s[i].x, x[i], low.x);
+          low.y = fmaf(s[i].y, x[i], low.y);
+          low.z = fmaf(s[i].z, x[i], low.z);
+          low.w = fmaf(s[i].w, x[i], low.w);
+          high.x = fmaf(s[4 + i].x, x[4 + i], high.x);
+          high.y = fmaf(s[4 + i].y, x[4 + i], high.y);
+          high.z = fmaf(s[4 + i].z, x[4 + i], high.z);
+          high.w = fmaf(s[4 + i].w, x[4 + i], high.w);
+        }
+        to[0] = low.x + high.x;
+        to[1] = low.y + high.y;
+        to[2] = low.z + high.z;
+        to[3] = low.w + high.w;
+      };
+      float a_sums[16];
+      float b_sums[16];
+#pragma unroll
+      for (std::uint32_t i = 0; i < kShortGroup; ++i) {
+        fetch(sh.qk[1][group + i], k[i]);
+        products(k[i], a_sums + 4 * i);
+      }
+#pragma unroll
+      for (std::uint32_t i = 0; i < kShortGroup; ++i) {
+        float q[8];
+        fetch(sh.qk[0][group + i], q);
+        products(q, b_sums + 4 * i);
+      }
+      const float a = fold(a_sums);
+      const float b = fold(b_sums);
+      const float4 scale = sh.scale[h][group + t];
+      const float4 solve = sh.solve[h][group + t];
+      const float4 read = sh.read[h][group + t];
+      float &slot = sh.v[h][group + t][column + (row_lane & 3U)];
+      const float y = group + t < n ? scale.x * (slot - scale.y * a) : 0.0F;
+      const float y1 = __shfl_xor_sync(0xFFFFFFFFU, y, 4);
+      const float y2 = __shfl_xor_sync(0xFFFFFFFFU, y, 8);
+      const float y3 = __shfl_xor_sync(0xFFFFFFFFU, y, 12);
+      float delta = y;
+      delta = second ? fmaf(solve.x, y1, delta) : delta;
+      delta = upper ? fmaf(solve.z, y3, fmaf(solve.y, y2, delta)) : delta;
+      const float corrections = scale.z * delta;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        s[i] = make_float4(s[i].x * scale.w, s[i].y * scale.w, s[i].z * scale.w, s[i].w * scale.w);
+      }
+#pragma unroll
+      for (std::uint32_t i = 0; i < kShortGroup; ++i) {
+        const std::uint32_t from = (lane & 16U) + 4 * i; // the corrections of the lane's four columns
+        const float4 c = make_float4(__shfl_sync(0xFFFFFFFFU, corrections, from), __shfl_sync(0xFFFFFFFFU, corrections, from + 1),
+                                     __shfl_sync(0xFFFFFFFFU, corrections, from + 2),
+                                     __shfl_sync(0xFFFFFFFFU, corrections, from + 3));
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          s[r].x = fmaf(k[i][r], c.x, s[r].x);
+          s[r].y = fmaf(k[i][r], c.y, s[r].y);
+          s[r].z = fmaf(k[i][r], c.z, s[r].z);
+          s[r].w = fmaf(k[i][r], c.w, s[r].w);
+        }
+      }
+      const float d1 = __shfl_xor_sync(0xFFFFFFFFU, delta, 4);
+      const float d2 = __shfl_xor_sync(0xFFFFFFFFU, delta, 8);
+      const float d3 = __shfl_xor_sync(0xFFFFFFFFU, delta, 12);
+      float out = fmaf(read.x, delta, scale.y * b);
+      out = second ? fmaf(read.y, d1, out) : out;
+      out = upper ? fmaf(read.w, d3, fmaf(read.z, d2, out)) : out;
+      slot = out;
+    }
+  }
+  __syncthreads();
+
+  // ---- output norm over the four slices, gate ----
+  asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory"); // every CTA of the cluster has started
+  const float4 norm_weight = load_quad<WeightDtype, false>(static_cast<const WeightType *>(p.output_norm_weight) +
+                                                           slice * kStepColumns + quad);
+  float4 out[kShortRounds];
+#pragma unroll
+  for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+    if (4 * (warp + kShortWarps * r) >= rows) {
+      continue;
+    }
+    const std::uint32_t row = min(4 * (warp + kShortWarps * r) + (lane >> 3), rows - 1);
+    out[r] = *reinterpret_cast<const float4 *>(&sh.v[row & shift][row >> shift][quad]);
+    float squares = (out[r].x * out[r].x + out[r].y * out[r].y) + (out[r].z * out[r].z + out[r].w * out[r].w);
+#pragma unroll
+    for (int offset = 4; offset > 0; offset >>= 1) {
+      squares += __shfl_xor_sync(0xFFFFFFFFU, squares, offset);
+    }
+    if ((lane & 7U) < kStepSlices && 4 * (warp + kShortWarps * r) + (lane >> 3) < rows) { // to the four CTAs
+      send_sum(&sh.norm[slice][row], &sh.norm_bar, lane & 7U, squares);
+    }
+  }
+#pragma unroll
+  for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+    if (4 * (warp + kShortWarps * r) >= rows) {
+      continue;
+    }
+    z[r] = make_float4(norm_weight.x * silu(z[r].x), norm_weight.y * silu(z[r].y), norm_weight.z * silu(z[r].z),
+                       norm_weight.w * silu(z[r].w));
+  }
+  wait_for_sums(&sh.norm_bar, p.status);
+#pragma unroll
+  for (std::uint32_t r = 0; r < kShortRounds; ++r) {
+    const std::uint32_t row = 4 * (warp + kShortWarps * r) + (lane >> 3);
+    if (row < rows) {
+      const float norm = (sh.norm[0][row] + sh.norm[1][row]) + (sh.norm[2][row] + sh.norm[3][row]);
+      const float scale = rsqrtf(norm / static_cast<float>(kDim) + p.epsilon);
+      const float4 x = make_float4(out[r].x * scale * z[r].x, out[r].y * scale * z[r].y, out[r].z * scale * z[r].z,
+                                   out[r].w * scale * z[r].w);
+      auto *to = static_cast<ActType *>(p.output) +
+                 (static_cast<std::size_t>(row >> shift) * p.value_heads + head_of(row & shift)) * kDim +
+                 slice * kStepColumns + quad;
+      if constexpr (Wide) {
+        Io<Dtype>::store4(to, 0, x);
+      } else {
+        to[0] = Act::narrow(x.x);
+        to[1] = Act::narrow(x.y);
+        to[2] = Act::narrow(x.z);
+        to[3] = Act::narrow(x.w);
       }
     }
   }
+  if (recurs) {
 #pragma unroll
-  for (std::uint32_t i = 0; i < 4; ++i) {
-    *reinterpret_cast<float4 *>(state + static_cast<std::size_t>(4 * lane + i) * kDim + 4 * warp) = s[i];
-  }
-  // the last three tokens of [old history | call] are the next call's history
-  if (rank == 0) {
-#pragma unroll
-    for (int h = 0; h < kHistory; ++h) {
-      p.convolution_state[static_cast<std::size_t>(qk_channel) * kHistory + h] =
-          row(qk_channel, qk_history, static_cast<int>(p.tokens) - kHistory + h);
+    for (std::uint32_t i = 0; i < 8; ++i) {
+      *reinterpret_cast<float4 *>(state_row(i)) = s[i];
     }
   }
-  if (warp == 0) {
+  if (convolves && (slice == 0 || warp >= 8)) {
 #pragma unroll
-    for (int h = 0; h < kHistory; ++h) {
-      p.convolution_state[static_cast<std::size_t>(v_channel) * kHistory + h] =
-          row(v_channel, v_history, static_cast<int>(p.tokens) - kHistory + h);
+    for (std::uint32_t i = 0; i < kHistory; ++i) {
+      p.convolution_state[static_cast<std::size_t>(channel) * kHistory + i] = next_history[i];
     }
   }
 }
@@ -1001,14 +1267,34 @@ LayerParams make_params(const GdnLayerArgs &a) {
   p.epsilon = a.epsilon;
   p.dtype = a.dtype;
   p.weight_dtype = a.weight_dtype;
+  p.status = device_status_word();
   return p;
 }
 
+template <int Dtype, int WeightDtype, bool Wide> void launch_short(const LayerParams &p, cudaStream_t stream) {
+  static std::once_flag flags[64];
+  int device = 0;
+  cuda_ok(cudaGetDevice(&device), "cudaGetDevice");
+  require(device >= 0 && device < 64, "device ordinal out of range", RIB200_STATUS_INTERNAL);
+  auto *kernel = gdn_layer_short_kernel<Dtype, WeightDtype, Wide>;
+  std::call_once(flags[device], [&] {
+    cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ShortShared)),
+            "gated-delta short call shared-memory opt-in");
+  });
+  launch_programmatic_cluster(kernel, dim3(kStepSlices * p.key_heads), dim3(kShortThreads), kStepSlices, sizeof(ShortShared),
+                              stream, "gated-delta short call launch", p);
+}
+
 template <int Dtype, int WeightDtype> void launch_step(const LayerParams &p, cudaStream_t stream) {
-  const std::uint32_t cluster = kStepSlices * (p.value_heads / p.key_heads);
-  auto *kernel = p.tokens == 1 ? gdn_layer_step_kernel<Dtype, WeightDtype> : gdn_layer_short_kernel<Dtype, WeightDtype>;
-  launch_programmatic_cluster(kernel, dim3(cluster * p.key_heads), dim3(kStepThreads), cluster, 0, stream,
-                              "gated-delta step launch", p);
+  if (p.tokens == 1) {
+    const std::uint32_t cluster = kStepSlices * (p.value_heads / p.key_heads);
+    launch_programmatic_cluster(gdn_layer_step_kernel<Dtype, WeightDtype>, dim3(cluster * p.key_heads), dim3(kStepThreads),
+                                cluster, 0, stream, "gated-delta step launch", p);
+  } else if (vector_forms_apply(p)) {
+    launch_short<Dtype, WeightDtype, true>(p, stream);
+  } else {
+    launch_short<Dtype, WeightDtype, false>(p, stream);
+  }
 }
 
 } // namespace

@@ -295,6 +295,38 @@ def test_layer_short_calls(calls, hk, hv, dtype, wdtype):
     assert K.device_status(torch.cuda.current_stream()) == 0
 
 
+@pytest.mark.parametrize("tokens", [2, 3, 5, 6, 7, 8, 47, 48, 49, 62])
+@pytest.mark.parametrize("hv", [1, 2])
+@pytest.mark.parametrize("dtype", [K.DTYPE_F32, K.DTYPE_F16])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_layer_short_calls_in_groups(tokens, hv, dtype, aligned):
+    """The one-launch form folds tokens into the state four at a time and loads rows four elements at a time where they are
+    aligned: every remainder of a group, either side of a round of loads and of a round of groups, with one and two value
+    heads, and an input that starts one element off.  FP32 against the bound of the recurrence's FP32 path; FP16 operands
+    are exact on both sides, so that only the output's rounding (2^-11) remains."""
+    half = lambda x: x.astype(np.float16).astype(np.float32)
+    run = LayerRun(0xB2002A00 + tokens, 1, hv, 4, dtype, K.DTYPE_F32, tokens)
+    run.inp = half(run.inp)
+    shape = K.GatedDeltaShape(tokens, hv * DK, 1, hv, DK, DK, 4, 1.0e-6)
+    ws_bytes = K.qwen35_gated_delta_workspace_bytes(shape)
+    ws = torch.zeros(ws_bytes // 4, device=dev())
+    element = act_tensor(run.inp, dtype)
+    buffer = torch.zeros(element.numel() + 1, device=dev(), dtype=element.dtype)
+    d_in = buffer[:-1] if aligned else buffer[1:]
+    d_in.copy_(element.reshape(-1))
+    out = torch.zeros(tokens, hv * DK, device=dev(), dtype=element.dtype)
+    K.qwen35_gated_delta(d_in, run.d_conv_w, run.d_rec_a, run.d_dt, run.d_norm, out, run.d_cs, run.d_rs, ws, ws_bytes, shape,
+                         dtype, K.DTYPE_F32, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    want, run.cs, run.rs = ob.gated_delta_layer(run.inp, run.conv_w, run.rec_a, run.dt_bias, run.norm_w, run.cs, run.rs,
+                                                (tokens, hv * DK, 1, hv, DK, DK, 4, 1.0e-6))
+    m = compare(to_numpy_f32(out), want)
+    assert m["nonfinite"] == 0 and m["rel_l2"] <= (2.0e-6 if dtype == K.DTYPE_F32 else 2.0 ** -11), m
+    assert compare(to_numpy_f32(run.d_cs).reshape(-1), run.cs.reshape(-1))["max_abs"] == 0.0
+    assert compare(to_numpy_f32(run.d_rs).reshape(-1), run.rs.reshape(-1))["rel_l2"] <= 2.0e-6
+    assert K.device_status(torch.cuda.current_stream()) == 0
+
+
 def test_layer_three_launches_share_device_state_without_a_sync():
     run = LayerRun(0xB2002200, 2, 4, 4, K.DTYPE_F32, K.DTYPE_F32, 6)
     results = [run.step(2, sync=False) for _ in range(3)]
