@@ -92,6 +92,10 @@ template <int Warps, int Slots> struct Tile {
   static constexpr int kSmemBytes = kRingBytes + kBarrierBytes;
   static constexpr int kCtasPerSm = (227 * 1024) / (kSmemBytes + 1024) > 0 ? (227 * 1024) / (kSmemBytes + 1024) : 1;
 };
+// Where a cluster shares a partition: what its CTAs send to the owner of a query head, [CTA][owned head][256 values], then
+// [CTA][owned head] maximum and sum, then the mbarrier that counts the bytes.  Behind the ring, which the owner may still read.
+constexpr int kExchangeValues = kGroup * kHeadDim * 4;
+constexpr int kExchangeBytes = kExchangeValues + kGroup * 8 + 16;
 constexpr float kLog2e = 1.4426950408889634F;
 // Rows of K and of V that a CTA asks for ahead of its turn: 64 MB over the whole grid, half of L2, and at most 128 a
 // CTA.  Eight layers at 32K (512 CTAs): 258 us without, 251 with 64 rows, 242 with 128, 262 with 256 (L2 then loses what
@@ -174,6 +178,23 @@ __device__ __forceinline__ void bulk_copy_g2s(std::uint32_t dst, const void *src
           dst),
       "l"(src), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
+}
+
+// stores to a CTA of the cluster, counted on an mbarrier there
+__device__ __forceinline__ std::uint32_t map_to_rank(std::uint32_t addr, std::uint32_t rank) {
+  std::uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(addr), "r"(rank));
+  return remote;
+}
+__device__ __forceinline__ void send4(std::uint32_t dst, float a, float b, float c, float d, std::uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n" ::"r"(dst),
+               "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(__float_as_uint(c)), "r"(__float_as_uint(d)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void send2(std::uint32_t dst, float a, float b, std::uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n" ::"r"(dst),
+               "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(bar)
+               : "memory");
 }
 
 __device__ __forceinline__ void prefetch_l2(const void *src, std::uint32_t bytes, std::uint64_t policy) {
@@ -268,7 +289,7 @@ template <bool F32> __device__ __forceinline__ uint4 load8_as_bf16(const void *b
 // While the kernels in front still run: the first rows of the CTA's share of the cache are asked into L2.  That is a
 // hint and no read - a row that one of those kernels writes is current in L2 either way - and only its extent comes from
 // a position that may still change, clamped to the cache.
-__device__ __forceinline__ void prefetch_rows(const DecodeParams &p) {
+template <int Cluster> __device__ __forceinline__ void prefetch_rows(const DecodeParams &p) {
   if (threadIdx.x >= 2) {
     return;
   }
@@ -277,12 +298,13 @@ __device__ __forceinline__ void prefetch_rows(const DecodeParams &p) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(pos) : "l"(p.pos_array) : "memory");
   }
   const std::uint32_t live = min(pos, p.max_ctx);
-  const std::uint32_t begin = p.partition_tokens == 0 ? 0U : blockIdx.x * p.partition_tokens;
+  const std::uint32_t begin = p.partition_tokens == 0 ? 0U : blockIdx.x * (p.partition_tokens / Cluster);
   if (begin >= live || (p.partition_tokens == 0 && blockIdx.x != 0)) {
     return;
   }
   const std::uint32_t rows =
-      min(live - begin, min(kPrefetchMaxRows, kPrefetchGridRows / (gridDim.x * gridDim.y)));
+      min(live - begin, min(Cluster > 1 ? p.partition_tokens / Cluster : kPrefetchMaxRows,
+                            kPrefetchGridRows / (gridDim.x * gridDim.y)));
   const __nv_bfloat16 *src =
       p.cache + ((static_cast<std::size_t>(threadIdx.x) * kKvHeads + blockIdx.y) * p.max_ctx + begin) * kHeadDim;
   const std::uint64_t policy = evict_first_policy();
@@ -291,9 +313,10 @@ __device__ __forceinline__ void prefetch_rows(const DecodeParams &p) {
   }
 }
 
-// Partition kernel.  grid = (partition capacity, 4 KV heads, sequences), Warps * 32 threads.
-template <bool F32, bool Batched, class T>
+// Partition kernel.  grid = (partition capacity * Cluster, 4 KV heads, sequences), Warps * 32 threads.
+template <bool F32, bool Batched, class T, int Cluster = 1>
 __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partition_kernel(const DecodeParams p) {
+  static_assert(Cluster == 1 || (!Batched && T::kWarps * 32 >= kGroup * 32), "a thread per piece of a head's values");
   constexpr int kWarps = T::kWarps;
   constexpr int kRingSlots = T::kRingSlots;
   constexpr int kRingBytes = T::kRingBytes;
@@ -302,9 +325,21 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
   // made resident early by the kernel before it (the combine kernel of a preceding step does that).  Unless the
   // caller has opted into the early cache fetch, nothing is read or written before that kernel has completed, so
   // the ordering is that of a plain launch, minus the launch latency.
+  [[maybe_unused]] const std::uint32_t exchange = smem_address(smem) + T::kSmemBytes;
+  [[maybe_unused]] const std::uint32_t exchange_stats = exchange + kExchangeValues;
+  [[maybe_unused]] const std::uint32_t exchange_bar = exchange_stats + kGroup * 8;
+  if constexpr (Cluster > 1) {
+    if (threadIdx.x == 0) {
+      mbarrier_init(exchange_bar, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+      mbarrier_expect_tx(exchange_bar, kExchangeValues + kGroup * 8);
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // waited for in front of the exchange
+  }
   if (Batched || p.early_kv == 0) {
     if constexpr (!Batched) {
-      prefetch_rows(p);
+      prefetch_rows<Cluster>(p);
     }
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     // Let the kernel behind this one become resident now; it blocks in its own griddepcontrol.wait until this
@@ -327,18 +362,25 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
   }
   const std::uint32_t ctx = pos + 1;
   const bool direct = p.partition_tokens == 0 || ctx < p.threshold_tokens;
+  const std::uint32_t partition = blockIdx.x / Cluster;
+  [[maybe_unused]] const std::uint32_t rank = blockIdx.x % Cluster;
   std::uint32_t begin = 0;
   std::uint32_t end = ctx;
   if (direct) {
-    if (blockIdx.x != 0) {
+    if (partition != 0) {
       return;
     }
   } else {
-    begin = blockIdx.x * p.partition_tokens;
+    begin = partition * p.partition_tokens;
     if (begin >= ctx) {
       return;
     }
     end = min(ctx, begin + p.partition_tokens);
+  }
+  if constexpr (Cluster > 1) { // this CTA's share, which may be empty
+    const std::uint32_t share = p.partition_tokens / Cluster;
+    begin = min(begin + rank * share, end);
+    end = min(begin + share, end);
   }
 
   const int warp = threadIdx.x >> 5;
@@ -353,7 +395,7 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
   std::uint32_t origin = 0;
   if constexpr (Batched) {
     if (paged) {
-      const std::uint32_t page = p.block_tables[static_cast<std::size_t>(seq) * p.max_blocks + blockIdx.x];
+      const std::uint32_t page = p.block_tables[static_cast<std::size_t>(seq) * p.max_blocks + partition];
       if (page >= p.pool_pages) {
         if (threadIdx.x == 0) {
           atomicOr(p.status, static_cast<unsigned int>(RIB200_DEVICE_PAGE_OUT_OF_RANGE));
@@ -648,6 +690,32 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
   }
   __syncthreads();
 
+  // a piece of eight dims of a head: the output where this partition is the whole context, else the split-k partial
+  auto finish = [&](int head, int dim0, float block_max, float block_sum, const float (&acc)[8]) {
+    if (direct) {
+      const std::size_t out_index = (act_seq * kQueryHeads + head) * kHeadDim + dim0;
+      float gate[8];
+      load8<F32>(p.gate, out_index, gate);
+      float result[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        result[e] = (acc[e] / block_sum) / (1.0F + expf(-gate[e]));
+      }
+      store8<F32>(p.output, out_index, result);
+      return;
+    }
+    const std::size_t partial = static_cast<std::size_t>(head) * p.max_partitions + partition;
+    float *pmax = p.partial_max + act_seq * p.partial_stride;
+    float *psum = p.partial_sum + act_seq * p.partial_stride;
+    float *pval = p.partial_value + act_seq * p.partial_stride * kHeadDim;
+    if (dim0 == 0) {
+      pmax[partial] = block_max;
+      psum[partial] = block_sum;
+    }
+    float *dst = pval + partial * kHeadDim + dim0;
+    *reinterpret_cast<float4 *>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4 *>(dst + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  };
   // 4 heads x 32 eight-dim pieces = 128 work items over the CTA's threads
   for (int item = threadIdx.x; item < kGroup * 32; item += kWarps * 32) {
     const int head_in_group = item >> 5;
@@ -661,7 +729,10 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
     float acc[8] = {0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F};
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
-      const float weight = exp2f((warp_max[w * kGroup + head_in_group] - block_max) * kLog2e);
+      float weight = exp2f((warp_max[w * kGroup + head_in_group] - block_max) * kLog2e);
+      if constexpr (Cluster > 1) { // no warp of an empty share has a maximum
+        weight = block_max == -INFINITY ? 0.0F : weight;
+      }
       block_sum += warp_sum[w * kGroup + head_in_group] * weight;
       const float *src = warp_out + (w * kGroup + head_in_group) * kMergePitch + dim0;
       const float4 a = *reinterpret_cast<const float4 *>(src);
@@ -669,31 +740,58 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
       acc[0] += a.x * weight; acc[1] += a.y * weight; acc[2] += a.z * weight; acc[3] += a.w * weight;
       acc[4] += b.x * weight; acc[5] += b.y * weight; acc[6] += b.z * weight; acc[7] += b.w * weight;
     }
-
-    const int head = kvh * kGroup + head_in_group;
-    if (direct) {
-      const std::size_t out_index = (act_seq * kQueryHeads + head) * kHeadDim + dim0;
-      float gate[8];
-      load8<F32>(p.gate, out_index, gate);
-      float result[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        result[e] = (acc[e] / block_sum) / (1.0F + expf(-gate[e]));
+    if constexpr (Cluster == 1) {
+      finish(kvh * kGroup + head_in_group, dim0, block_max, block_sum, acc);
+    } else {
+      constexpr int kOwned = kGroup / Cluster; // query heads that a CTA puts together
+      if (item == static_cast<int>(threadIdx.x)) {
+        asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory"); // every CTA of the cluster has set its barrier up
       }
-      store8<F32>(p.output, out_index, result);
-      continue;
+      const std::uint32_t owner = static_cast<std::uint32_t>(head_in_group / kOwned);
+      const std::uint32_t row = rank * kOwned + head_in_group % kOwned;
+      const std::uint32_t bar = map_to_rank(exchange_bar, owner);
+      const std::uint32_t values = map_to_rank(exchange + (row * kHeadDim + dim0) * 4, owner);
+      send4(values, acc[0], acc[1], acc[2], acc[3], bar);
+      send4(values + 16, acc[4], acc[5], acc[6], acc[7], bar);
+      if (dim0 == 0) {
+        send2(map_to_rank(exchange_stats + row * 8, owner), block_max, block_sum, bar);
+      }
     }
-    const std::size_t partial = static_cast<std::size_t>(head) * p.max_partitions + blockIdx.x;
-    float *pmax = p.partial_max + act_seq * p.partial_stride;
-    float *psum = p.partial_sum + act_seq * p.partial_stride;
-    float *pval = p.partial_value + act_seq * p.partial_stride * kHeadDim;
-    if ((item & 31) == 0) {
-      pmax[partial] = block_max;
-      psum[partial] = block_sum;
+  }
+  if constexpr (Cluster > 1) {
+    constexpr int kOwned = kGroup / Cluster;
+    // every thread waits: nobody leaves while a peer may still send
+    const long long started = clock64();
+    while (!mbarrier_try_wait(exchange_bar, 0)) {
+      if (clock64() - started > kWaitLimitCycles) {
+        atomicOr(p.status, static_cast<unsigned int>(RIB200_DEVICE_WAIT_TIMED_OUT));
+        break;
+      }
     }
-    float *dst = pval + partial * kHeadDim + dim0;
-    *reinterpret_cast<float4 *>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    *reinterpret_cast<float4 *>(dst + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    if (threadIdx.x < kOwned * 32) {
+      const float *values = reinterpret_cast<const float *>(smem + T::kSmemBytes);
+      const float *stats = values + kGroup * kHeadDim;
+      const int owned = threadIdx.x >> 5;
+      const int dim0 = (threadIdx.x & 31) * 8;
+      float total_max = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < Cluster; ++c) {
+        total_max = fmaxf(total_max, stats[(c * kOwned + owned) * 2]);
+      }
+      float total_sum = 0.0F;
+      float acc[8] = {0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F, 0.0F};
+#pragma unroll
+      for (int c = 0; c < Cluster; ++c) {
+        const float weight = exp2f((stats[(c * kOwned + owned) * 2] - total_max) * kLog2e); // 0 for an empty share
+        total_sum += stats[(c * kOwned + owned) * 2 + 1] * weight;
+        const float *src = values + (c * kOwned + owned) * kHeadDim + dim0;
+        const float4 a = *reinterpret_cast<const float4 *>(src);
+        const float4 b = *reinterpret_cast<const float4 *>(src + 4);
+        acc[0] += a.x * weight; acc[1] += a.y * weight; acc[2] += a.z * weight; acc[3] += a.w * weight;
+        acc[4] += b.x * weight; acc[5] += b.y * weight; acc[6] += b.z * weight; acc[7] += b.w * weight;
+      }
+      finish(kvh * kGroup + static_cast<int>(rank) * kOwned + owned, dim0, total_max, total_sum, acc);
+    }
   }
   RIB200_DECODE_STAMP(g_decode_trace, trace_cta, 3);
 }
@@ -829,55 +927,56 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
 // cross-warp merge, most CTAs resident); with few, more warps share a partition so that every SM has work and
 // each warp's chain of dependent steps is short.  All shapes are the same kernel template.
 //
+// Single sequences whose grid would leave most of the GPU idle share a partition among the CTAs of a cluster: 256 KB of rows
+// through one SM are 3 us.  Four CTAs while they fit beside one another (contexts up to 2304 tokens), two up to 4608; each
+// takes its part of the rows with four warps, and what it has found out about a query head goes to the CTA that owns the
+// head, in stores counted on an mbarrier there, so that the split-k partials are those of whole partitions.  Prologue and
+// step of a layer in a replayed token, with and without: 300 tokens 9.2 and 11.1 us, 777 9.2 and 11.4, 2000 9.5 and 11.8, 4000
+// 11.0 and 11.5; the executor's five launches at 777 12.3 and 14.9.
+//
 // A batch takes four warps a CTA from 149 CTAs on: its grid spans the longest cache, so many CTAs are empty, and four
 // warps finish a partition in a quarter of the steps.  The attention call alone behind a flushed L2, against one warp a CTA:
 // 9 ragged sequences up to 6000 tokens (864 CTAs) 35.8 and 37.9 us, the same nine at full length 52.2 and 54.3, 24
 // sequences (1536 CTAs) 68.6 and 78.8, 64 up to 32768 tokens 681 and 705; whole serving steps back to back, the gated-delta
 // half included: nine 38.8 and 41.0, 64 752.8 and 756.9.  Two warps a CTA gain on ragged batches (33.1 a step of nine
 // when this form took 36.2) and lose on full ones (55.0 against 51.7).
-template <bool F32, bool Batched, class T> void configure_once() {
+template <bool F32, bool Batched, class T, int Cluster> void configure_once() {
   static std::once_flag flags[64];
   int device = 0;
   cuda_ok(cudaGetDevice(&device), "cudaGetDevice");
   require(device >= 0 && device < 64, "device ordinal out of range", RIB200_STATUS_INTERNAL);
   std::call_once(flags[device], [] {
-    cuda_ok(cudaFuncSetAttribute(decode_partition_kernel<F32, Batched, T>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmemBytes),
+    cuda_ok(cudaFuncSetAttribute(decode_partition_kernel<F32, Batched, T, Cluster>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 T::kSmemBytes + (Cluster > 1 ? kExchangeBytes : 0)),
             "decode attention shared-memory opt-in");
   });
 }
 
-template <bool F32, bool Batched, class T>
+template <bool F32, bool Batched, class T, int Cluster = 1>
 void launch_pair_tiled(const DecodeParams &params, dim3 partition_grid, dim3 combine_grid, bool combine,
                        cudaStream_t stream) {
-  configure_once<F32, Batched, T>();
-  cudaLaunchAttribute attribute{};
-  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attribute.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t config{};
-  config.gridDim = partition_grid;
-  config.blockDim = dim3(T::kWarps * 32, 1, 1);
-  config.dynamicSmemBytes = T::kSmemBytes;
-  config.stream = stream;
-  config.attrs = &attribute;
-  config.numAttrs = 1;
-  cuda_ok(cudaLaunchKernelEx(&config, decode_partition_kernel<F32, Batched, T>, params),
-          "decode attention partition launch");
+  configure_once<F32, Batched, T, Cluster>();
+  partition_grid.x *= Cluster;
+  launch_programmatic_cluster(decode_partition_kernel<F32, Batched, T, Cluster>, partition_grid, dim3(T::kWarps * 32), Cluster,
+                              T::kSmemBytes + (Cluster > 1 ? kExchangeBytes : 0), stream,
+                              "decode attention partition launch", params);
   if (!combine) {
     return;
   }
-  config.gridDim = combine_grid;
-  config.blockDim = dim3(256, 1, 1);
-  config.dynamicSmemBytes = 0;
-  cuda_ok(cudaLaunchKernelEx(&config, decode_combine_kernel<F32, Batched>, params),
-          "decode attention combine launch");
+  launch_programmatic(decode_combine_kernel<F32, Batched>, combine_grid, dim3(256), 0, stream,
+                      "decode attention combine launch", params);
 }
 
 template <bool F32, bool Batched>
 void launch_pair(const DecodeParams &params, dim3 partition_grid, dim3 combine_grid, bool combine,
                  cudaStream_t stream) {
   const std::size_t ctas = static_cast<std::size_t>(partition_grid.x) * partition_grid.y * partition_grid.z;
-  if (ctas <= 148) {
+  if (!Batched && params.partition_tokens != 0 && 4 * ctas <= 148) {
+    launch_pair_tiled<F32, false, Tile<4, 3>, 4>(params, partition_grid, combine_grid, combine, stream);
+  } else if (!Batched && params.partition_tokens != 0 && 2 * ctas <= 148) {
+    launch_pair_tiled<F32, false, Tile<4, 3>, 2>(params, partition_grid, combine_grid, combine, stream);
+  } else if (ctas <= 148) {
     launch_pair_tiled<F32, Batched, Tile<8, 3>>(params, partition_grid, combine_grid, combine, stream);
   } else if (Batched || ctas <= 296) {
     launch_pair_tiled<F32, Batched, Tile<4, 3>>(params, partition_grid, combine_grid, combine, stream);

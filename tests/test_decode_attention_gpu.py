@@ -90,6 +90,19 @@ def test_cache_capacity_not_a_partition_multiple():
     run_decode(777, 777, K.SPLIT_K_256, K.DTYPE_F32, seed=0xB2000311)
 
 
+@pytest.mark.parametrize("ctx,max_ctx,mode", [
+    (63, 1024, K.SPLIT_K_256), (64, 1024, K.SPLIT_K_256), (65, 1024, K.SPLIT_K_256), (128, 1024, K.SPLIT_K_256),
+    (193, 1024, K.SPLIT_K_256), (320, 1024, K.SPLIT_K_256), (321, 1024, K.SPLIT_K_256), (448, 1024, K.SPLIT_K_256),
+    (640, 1024, K.SPLIT_K_512), (641, 1024, K.SPLIT_K_512), (2304, 2304, K.SPLIT_K_256), (2305, 2560, K.SPLIT_K_256),
+    (2432, 4608, K.SPLIT_K_256), (2433, 4608, K.SPLIT_K_256), (4608, 4608, K.SPLIT_K_256), (4609, 4864, K.SPLIT_K_256),
+    (9216, 9216, K.SPLIT_K_256)])
+@pytest.mark.parametrize("dtype", [K.DTYPE_BF16, K.DTYPE_F32])
+def test_partitions_shared_by_a_cluster(ctx, max_ctx, mode, dtype):
+    """Grids that leave the GPU idle share a partition among the CTAs of a cluster: contexts either side of a share, whole
+    shares empty, and either side of the lines between four CTAs, two and one a partition; the position on the device."""
+    run_decode(ctx, max_ctx, mode, dtype, seed=0xB2000700 + ctx, device_position=True)
+
+
 @pytest.mark.parametrize("ctx", [4096, 32768, 131072])
 def test_long_contexts(ctx):
     metrics = run_decode(ctx, ctx, K.SPLIT_K_256, K.DTYPE_BF16, seed=0xB2000400 + ctx, device_position=True,
