@@ -285,8 +285,11 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const std::uint32_t (&a)[
 //            first product's accumulators are then the second one's A operand, so no intermediate leaves the registers.
 //   [W; *]   = [T diag(beta gamma); T diag(beta)] K      M 128, N 128, K 64   (rows 0..63 are W)
 //   [*; U]   = [T diag(beta gamma); T diag(beta)] V      M 128, N 128, K 64   (rows 64..127 are U)
-//   W (FP16) and U (FP32) leave through bulk copies from shared memory that is idle by then (the Q rows, V, A and T):
+//   W (FP16) and U (FP32) leave through bulk copies from shared memory that is idle by then (the T image, V, A and T):
 //            straight from the registers every store of a warp would touch 32 lines.
+// A CTA's items are neighbours, so that the second value head of a key head finds the [K; Q] image in place (32 of an item's
+// 50 KB of inputs), and no input waits for all of the item before to leave: the gates come during its inversion, the next
+// image behind its two products, only V behind the stores.
 // Each phase ends in a barrier and most of them occupy few warps, so a CTA alone leaves the SM mostly idle; two share it.
 constexpr int kPrepThreads = 256;
 constexpr std::uint32_t kAPitch = 112;                         // A: rows 16..63, columns 0..47 (what the tiles read)
@@ -296,9 +299,9 @@ constexpr std::uint32_t kTLow = kChunk * kTPitch;
 constexpr std::uint32_t kDiagPitch = 20;                       // floats per column of a diagonal block of A
 constexpr std::uint32_t kDiagBlock = 16 * kDiagPitch + 16;     // floats per block: the two a warp reads miss each other's banks
 constexpr std::uint32_t kPsKq = 0;
-constexpr std::uint32_t kPsWstage = kPsKq + kGdnBlock;         //   later: W, a block in the place of either block of Q rows
 constexpr std::uint32_t kPsV = kPsKq + kGdnKqBytes;            //   later: slices 0 and 1 of U
-constexpr std::uint32_t kPsTstack = kPsV + kGdnVBytes;         // [T diag(beta gamma); T diag(beta)], 128 rows of 128 bytes
+// [T diag(beta gamma); T diag(beta)], 128 rows of 128 bytes; later: W
+constexpr std::uint32_t kPsTstack = kPsV + kGdnVBytes;
 constexpr std::uint32_t kPsPstage = kPsTstack + 128 * kGdnRowBytes;
 constexpr std::uint32_t kPsA = kPsPstage + kGdnBlock;          //   later: slices 2 and 3 of U, over A and T
 constexpr std::uint32_t kPsT = kPsA + 2 * kALow;
@@ -307,11 +310,11 @@ constexpr std::uint32_t kPsGates = kPsDiag + 4 * kDiagBlock * 4;
 // G log2(e), beta gamma and beta (both over the unit of K), column factors: 4 x 64 floats; what undoes U's scales: 128
 constexpr std::uint32_t kPsFactors = kPsGates + kGdnGateBytes;
 constexpr std::uint32_t kPsBars = kPsFactors + (4 * kChunk + kDim) * 4;
-constexpr std::uint32_t kPsTmemSlot = kPsBars + 24;
+constexpr std::uint32_t kPsTmemSlot = kPsBars + 48;
 constexpr std::uint32_t kPsAbort = kPsTmemSlot + 4;
 constexpr std::uint32_t kPrepSmemBytes = kPsAbort + 4 + 1024;  // + room to align the base to 1 KiB
 static_assert(kPsGates % 16 == 0 && kPsFactors % 16 == 0 && kPsBars % 8 == 0 && kPsA % 1024 == 0 && kPsT % 16 == 0 &&
-                  kPsDiag - kPsA >= 2 * kGdnSliceU && kGdnVBytes == 2 * kGdnSliceU,
+                  kPsDiag - kPsA >= 2 * kGdnSliceU && kGdnVBytes == 2 * kGdnSliceU && 2 * kGdnBlock == 128 * kGdnRowBytes,
               "alignment, staging fits");
 static_assert(2 * (kPrepSmemBytes + 1024) <= 233472, "two CTAs per SM");
 constexpr std::uint32_t kPrepTmemColumns = 256; // W at 0, U at 128; G at 0 before them
@@ -384,20 +387,39 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
   float *s_bu = s_bg + kChunk;                                // beta / kGdnUnit
   float *s_cf = s_bu + kChunk;                                // exp(G at the end of the token's block of 16 - G)
   float *s_undo = s_cf + kChunk;                              // by column: undoes the scales of the product that is U
-  const std::uint32_t bar_in = base + kPsBars;
-  const std::uint32_t bar_g = bar_in + 8;
-  const std::uint32_t bar_wu = bar_in + 16;
+  const std::uint32_t bar_kq = base + kPsBars; // the [K; Q] image has landed ...
+  const std::uint32_t bar_gates = bar_kq + 8;  // ... the gates ...
+  const std::uint32_t bar_v = bar_kq + 16;     // ... V
+  const std::uint32_t bar_g = bar_kq + 24;
+  const std::uint32_t bar_wu = bar_kq + 32;
+  const std::uint32_t bar_left = bar_kq + 40; // what the item before has staged has been read
   volatile std::uint32_t *tmem_slot = reinterpret_cast<volatile std::uint32_t *>(smem + kPsTmemSlot);
   volatile std::uint32_t *abort_flag = reinterpret_cast<volatile std::uint32_t *>(smem + kPsAbort);
   const std::uint32_t tid = threadIdx.x;
   const std::uint32_t warp = tid >> 5;
   const std::uint32_t lane = tid & 31;
+  // Items in the order (chunk, key head, value head of the key head), an equal share of them for every CTA: where two value
+  // heads share a key head, the [K; Q] image of every second item is the one in hand.
   const std::uint32_t items = p.chunks * p.value_heads;
+  const std::uint32_t ratio = p.value_heads / p.key_heads;
+  auto share = [&](std::uint32_t cta) {
+    return static_cast<std::uint32_t>(static_cast<std::uint64_t>(items) * cta / gridDim.x);
+  };
+  const std::uint32_t first_item = share(blockIdx.x);
+  const std::uint32_t last_item = share(blockIdx.x + 1);
+  auto record_index = [&](std::uint32_t item) { // of V and the record: (chunk, value head)
+    const std::uint32_t kq = item / ratio;
+    const std::uint32_t chunk = kq / p.key_heads;
+    return static_cast<std::size_t>(chunk) * p.value_heads + (kq - chunk * p.key_heads) + (item - kq * ratio) * p.key_heads;
+  };
 
   if (tid == 0) {
-    mbarrier_init(bar_in, 1);
+    mbarrier_init(bar_kq, 1);
+    mbarrier_init(bar_gates, 1);
+    mbarrier_init(bar_v, 1);
     mbarrier_init(bar_g, 1);
     mbarrier_init(bar_wu, 1);
+    mbarrier_init(bar_left, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -406,10 +428,6 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
                  "r"(kPrepTmemColumns)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
-  // the blocks of the T image above the diagonal stay zero for good
-  for (std::uint32_t at = tid * 16; at < 128 * kGdnRowBytes; at += kPrepThreads * 16) {
-    sts128(base + kPsTstack + at, 0U, 0U, 0U, 0U);
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -434,30 +452,35 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
     }
   }
 
-  auto issue_inputs = [&](std::uint32_t item) {
-    const std::uint32_t chunk = item / p.value_heads;
-    const std::uint32_t head = item - chunk * p.value_heads;
-    const std::size_t kq = static_cast<std::size_t>(chunk) * p.key_heads + head % p.key_heads;
-    fence_proxy_async(); // ordinary stores and loads touched these areas before
-    mbarrier_expect_tx(bar_in, kGdnKqBytes + kGdnVBytes + kGdnGateBytes);
-    bulk_copy_g2s(base + kPsKq, p.scratch.kq + kq * kGdnKqBytes, kGdnKqBytes, bar_in);
-    bulk_copy_g2s(base + kPsV, p.scratch.v + static_cast<std::size_t>(item) * kGdnVBytes, kGdnVBytes, bar_in);
-    bulk_copy_g2s(base + kPsGates, p.scratch.records + static_cast<std::size_t>(item) * kGdnRecBytes + kGdnRecGates,
-                  kGdnGateBytes, bar_in);
-    const std::uint32_t next = item + gridDim.x;
-    if (next < items) { // into L2 while this item is worked on (4096 tokens 197.7 -> 193.9 us for the whole layer call)
-      const std::uint32_t next_chunk = next / p.value_heads;
-      const std::uint32_t next_head = next - next_chunk * p.value_heads;
-      prefetch_l2(p.scratch.kq +
-                      (static_cast<std::size_t>(next_chunk) * p.key_heads + next_head % p.key_heads) * kGdnKqBytes,
-                  kGdnKqBytes);
-      prefetch_l2(p.scratch.v + static_cast<std::size_t>(next) * kGdnVBytes, kGdnVBytes);
+  // One lane issues every copy (bulk groups belong to the issuing thread).  An input is asked for as soon as the item in hand
+  // is done with its area: the gates behind A and P, the image behind the two products, V, whose area U leaves from, last.
+  const bool copier = tid == kPrepThreads - 32;
+  auto issue_kq = [&](std::uint32_t item) {
+    mbarrier_expect_tx(bar_kq, kGdnKqBytes);
+    bulk_copy_g2s(base + kPsKq, p.scratch.kq + static_cast<std::size_t>(item / ratio) * kGdnKqBytes, kGdnKqBytes, bar_kq);
+    const std::uint32_t next = (item / ratio + 1) * ratio; // into L2 while this image is worked on
+    if (next < last_item) {
+      prefetch_l2(p.scratch.kq + static_cast<std::size_t>(next / ratio) * kGdnKqBytes, kGdnKqBytes);
     }
   };
-  // One lane issues every copy (bulk groups belong to the issuing thread).
-  const bool copier = tid == kPrepThreads - 32;
-  if (copier && blockIdx.x < items) {
-    issue_inputs(blockIdx.x);
+  auto issue_gates = [&](std::uint32_t item) {
+    fence_proxy_async(); // those of the item before have been read by ordinary loads
+    mbarrier_expect_tx(bar_gates, kGdnGateBytes);
+    bulk_copy_g2s(base + kPsGates, p.scratch.records + record_index(item) * kGdnRecBytes + kGdnRecGates, kGdnGateBytes,
+                  bar_gates);
+  };
+  auto issue_v = [&](std::uint32_t item) {
+    fence_proxy_async(); // U has been staged here by ordinary stores
+    mbarrier_expect_tx(bar_v, kGdnVBytes);
+    bulk_copy_g2s(base + kPsV, p.scratch.v + record_index(item) * kGdnVBytes, kGdnVBytes, bar_v);
+    if (item + 1 < last_item) {
+      prefetch_l2(p.scratch.v + record_index(item + 1) * kGdnVBytes, kGdnVBytes);
+    }
+  };
+  if (copier && first_item < last_item) {
+    issue_kq(first_item);
+    issue_gates(first_item);
+    issue_v(first_item);
   }
 
   const std::uint32_t quarter = warp & 3; // the 32 tensor-memory lanes this warp may read
@@ -468,17 +491,15 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
   const std::uint32_t t_matrix = base + kPsT;
   auto t_at = [&](std::uint32_t row, std::uint32_t col) { return t_matrix + row * kTPitch + (col & 31U) * 2; };
   std::uint32_t iteration = 0;
-  for (std::uint32_t item = blockIdx.x; item < items; item += gridDim.x, ++iteration) {
+  for (std::uint32_t item = first_item; item < last_item; ++item, ++iteration) {
     const std::uint32_t phase = iteration & 1U;
-    unsigned char *rec = p.scratch.records + static_cast<std::size_t>(item) * kGdnRecBytes; // item = chunk * Hv + head
+    unsigned char *rec = p.scratch.records + record_index(item) * kGdnRecBytes;
+    const bool next_kq = item + 1 < last_item && (item + 1) % ratio == 0; // the next item has another image
     if (tid == 0) {
       RIB200_GDN_STAMP(100 + iteration, 0);
     }
-    wait(bar_in, phase);
-    if (tid == 0) {
-      RIB200_GDN_STAMP(100 + iteration, 1);
-    }
     if (warp == 0) {
+      wait(bar_kq, (item / ratio - first_item / ratio) & 1U);
       tcgen05_fence_after();
       if (elect_one() && *abort_flag == 0) {
         const std::uint64_t kq = smem_desc(base + kPsKq, 16, 1024);
@@ -490,7 +511,12 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
         umma_commit(bar_g);
       }
       __syncwarp();
-    } else if (warp == 2 || warp == 3) {
+    }
+    wait(bar_gates, phase);
+    if (tid == 0) {
+      RIB200_GDN_STAMP(100 + iteration, 1);
+    }
+    if (warp == 2 || warp == 3) {
       const std::uint32_t t = tid - 64;
       const float g = gates[kGdnGateG + t];
       s_g2[t] = g * 1.4426950408889634F;
@@ -510,6 +536,9 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
     __syncthreads();
 
     // ---- rows of G: A (below the diagonal, to shared memory) and P (to its staging area) ----
+    if (iteration > 0) { // until then the staging areas hold P, W and U of the item before
+      wait(bar_left, phase ^ 1U);
+    }
     wait(bar_g, phase);
     tcgen05_fence_after();
     if (tid == 0) {
@@ -599,6 +628,9 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
     if (copier && *abort_flag == 0) {
       bulk_copy_s2g(rec + kGdnRecP, base + kPsPstage, kGdnBlock);
       asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+      if (item + 1 < last_item) {
+        issue_gates(item + 1);
+      }
     }
 
     // ---- T = (I + A)^-1: diagonal blocks, a row per thread: x_c = [c = row] - sum over k > c of x_k A_kc ----
@@ -653,6 +685,15 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
                with_gamma[3]);
         sts128(base + kPsTstack + tstack_offset(kChunk + tid, 16 * b + 8 * c), without[0], without[1], without[2], without[3]);
       }
+    } else { // the other warps: zeros above the diagonal blocks of the T image, where W of the item before was
+      const std::uint32_t at = tid - kChunk; // of 16 rows each of 6, 4 and 2 pieces of eight columns
+      const std::uint32_t b = at < 96 ? 0U : (at < 160 ? 1U : 2U);
+      const std::uint32_t within = at - (b == 0 ? 0U : (b == 1 ? 96U : 160U));
+      const std::uint32_t pieces = 6 - 2 * b;
+      const std::uint32_t row = 16 * b + within / pieces;
+      const std::uint32_t col = 8 * (2 * (b + 1) + within % pieces);
+      sts128(base + kPsTstack + tstack_offset(row, col), 0U, 0U, 0U, 0U);
+      sts128(base + kPsTstack + tstack_offset(kChunk + row, col), 0U, 0U, 0U, 0U);
     }
     __syncthreads();
     if (tid == 0) {
@@ -744,6 +785,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
 
     // ---- the two products with T: B operands are K and V as stored, sixteen tokens = 2 KiB per step ----
     if (warp == 0) {
+      wait(bar_v, phase);
       tcgen05_fence_after();
       if (elect_one() && *abort_flag == 0) {
         const std::uint64_t t_desc = smem_desc(base + kPsTstack, 16, 1024);
@@ -764,6 +806,10 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
     }
     wait(bar_wu, phase);
     tcgen05_fence_after();
+    if (copier && next_kq && *abort_flag == 0) {
+      issue_kq(item + 1);
+    }
+    __syncwarp();
     if (tid == 0) {
       RIB200_GDN_STAMP(100 + iteration, 7);
     }
@@ -776,7 +822,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
         tmem_ld32(tmem + lane_base + 64 * half + 32 * part, x);
 #pragma unroll
         for (std::uint32_t c = 0; c < 4; ++c) {
-          sts128(base + kPsWstage + half * kGdnKqBlock + i * kGdnRowBytes + (((4 * part + c) ^ (i & 7U)) << 4),
+          sts128(base + kPsTstack + half * kGdnBlock + i * kGdnRowBytes + (((4 * part + c) ^ (i & 7U)) << 4),
                  pack_half(x[8 * c], x[8 * c + 1]), pack_half(x[8 * c + 2], x[8 * c + 3]),
                  pack_half(x[8 * c + 4], x[8 * c + 5]), pack_half(x[8 * c + 6], x[8 * c + 7]));
         }
@@ -808,21 +854,24 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       RIB200_GDN_STAMP(100 + iteration, 8);
     }
     if (copier && *abort_flag == 0) {
-      bulk_copy_s2g(rec + kGdnRecW, base + kPsWstage, kGdnBlock);
-      bulk_copy_s2g(rec + kGdnRecW + kGdnBlock, base + kPsWstage + kGdnKqBlock, kGdnBlock);
+      bulk_copy_s2g(rec + kGdnRecW, base + kPsTstack, 2 * kGdnBlock);
       bulk_copy_s2g(rec + kGdnRecU, base + kPsV, 2 * kGdnSliceU);
       bulk_copy_s2g(rec + kGdnRecU + 2 * kGdnSliceU, base + kPsA, 2 * kGdnSliceU);
       asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-      // the staging areas (P's among them) take the next item's inputs and operands once they have been read
       asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
-      if (item + gridDim.x < items) {
-        issue_inputs(item + gridDim.x);
+      mbarrier_arrive(bar_left);
+      if (item + 1 < last_item) {
+        issue_v(item + 1);
       }
     }
     __syncwarp();
   }
   if (copier) {
     asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+    if (*abort_flag != 0) { // inputs may be on their way for an item that nobody waits for
+      for (const long long started = clock64(); clock64() - started < (1LL << 17);) {
+      }
+    }
   }
   tcgen05_fence_before();
   __syncthreads();

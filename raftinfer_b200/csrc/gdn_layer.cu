@@ -474,7 +474,7 @@ __device__ __forceinline__ void hint_operands(const LayerParams &p, std::uint32_
 }
 
 // The slices of a head exchange their sums of squares with stores that count on an mbarrier of the CTA they go to.  A cluster
-// barrier in their place costs a call about 0.5 us more: its release waits for whatever the thread has in flight.  Who has
+// barrier in their place costs a call 0.3 to 0.6 us more: its release waits for whatever the thread has in flight.  Who has
 // the sums of all slices also knows that their CTAs have read the old history, and that nothing more will come.
 constexpr long long kWaitLimitCycles = 1LL << 28;
 __device__ __forceinline__ std::uint32_t smem_address(const void *p) {

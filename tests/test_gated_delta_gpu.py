@@ -136,6 +136,18 @@ def test_chunked_core_other_head_counts(hk, hv, dtype):
     assert m_state["nonfinite"] == 0 and m_state["rel_l2"] <= 1.0e-3, m_state
 
 
+@pytest.mark.parametrize("hk,hv,tokens", [(HK, HV, 600), (11, 33, 640), (31, 31, 650), (9, 18, 1100)])
+@pytest.mark.parametrize("dtype", [K.DTYPE_BF16, K.DTYPE_F32])
+def test_chunked_core_several_items_a_cta(hk, hv, tokens, dtype):
+    """More (chunk, value head) items than the prepare kernel has CTAs: shares of one to three neighbouring items, which
+    begin with the first, the second or the third value head of a key head, so that its image is loaded again, kept, or the
+    only one; a ragged last chunk."""
+    m_out, m_state = run_core(tokens, dtype, seed=0xB2001A00 + 16 * hk + hv, hk=hk, hv=hv)
+    assert m_out["nonfinite"] == 0 and m_out["max_abs"] <= 3.0e-2 and m_out["rel_l2"] <= 2.0e-3, m_out
+    assert m_state["nonfinite"] == 0 and m_state["rel_l2"] <= 1.0e-3, m_state
+    assert K.device_status(torch.cuda.current_stream()) == 0
+
+
 def test_recurrent_core_small_head_counts():
     m_out, m_state = run_core(3, K.DTYPE_F32, seed=0xB2001100, hk=2, hv=4)
     assert m_out["rel_l2"] <= 1.0e-4 and m_state["rel_l2"] <= 1.0e-5
