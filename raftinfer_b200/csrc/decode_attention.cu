@@ -377,8 +377,13 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
     }
     end = min(ctx, begin + p.partition_tokens);
   }
+  [[maybe_unused]] bool alone = Cluster == 1; // nothing to exchange
   if constexpr (Cluster > 1) { // this CTA's share, which may be empty
     const std::uint32_t share = p.partition_tokens / Cluster;
+    alone = direct && ctx <= share;
+    if (alone && rank != 0) {
+      return;
+    }
     begin = min(begin + rank * share, end);
     end = min(begin + share, end);
   }
@@ -740,9 +745,9 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
       acc[0] += a.x * weight; acc[1] += a.y * weight; acc[2] += a.z * weight; acc[3] += a.w * weight;
       acc[4] += b.x * weight; acc[5] += b.y * weight; acc[6] += b.z * weight; acc[7] += b.w * weight;
     }
-    if constexpr (Cluster == 1) {
+    if (alone) {
       finish(kvh * kGroup + head_in_group, dim0, block_max, block_sum, acc);
-    } else {
+    } else if constexpr (Cluster > 1) {
       constexpr int kOwned = kGroup / Cluster; // query heads that a CTA puts together
       if (item == static_cast<int>(threadIdx.x)) {
         asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory"); // every CTA of the cluster has set its barrier up
@@ -759,6 +764,9 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
     }
   }
   if constexpr (Cluster > 1) {
+    if (alone) {
+      return;
+    }
     constexpr int kOwned = kGroup / Cluster;
     // every thread waits: nobody leaves while a peer may still send
     const long long started = clock64();
