@@ -405,13 +405,18 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
   auto share = [&](std::uint32_t cta) {
     return static_cast<std::uint32_t>(static_cast<std::uint64_t>(items) * cta / gridDim.x);
   };
-  const std::uint32_t first_item = share(blockIdx.x);
-  const std::uint32_t last_item = share(blockIdx.x + 1);
+  const bool one_each = items == gridDim.x; // short calls, in which 64-bit divisions would show
+  const std::uint32_t first_item = one_each ? blockIdx.x : share(blockIdx.x);
+  const std::uint32_t last_item = one_each ? blockIdx.x + 1 : share(blockIdx.x + 1);
   auto record_index = [&](std::uint32_t item) { // of V and the record: (chunk, value head)
     const std::uint32_t kq = item / ratio;
     const std::uint32_t chunk = kq / p.key_heads;
-    return static_cast<std::size_t>(chunk) * p.value_heads + (kq - chunk * p.key_heads) + (item - kq * ratio) * p.key_heads;
+    return chunk * p.value_heads + (kq - chunk * p.key_heads) + (item - kq * ratio) * p.key_heads;
   };
+  std::uint32_t record = record_index(first_item); // of the item in hand; the divisions are over before the wait below
+  const std::uint32_t first_kq = first_item / ratio;
+  std::uint32_t kq_index = first_kq;
+  asm volatile("" : "+r"(record), "+r"(kq_index));
 
   if (tid == 0) {
     mbarrier_init(bar_kq, 1);
@@ -455,32 +460,31 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
   // One lane issues every copy (bulk groups belong to the issuing thread).  An input is asked for as soon as the item in hand
   // is done with its area: the gates behind A and P, the image behind the two products, V, whose area U leaves from, last.
   const bool copier = tid == kPrepThreads - 32;
-  auto issue_kq = [&](std::uint32_t item) {
+  auto issue_kq = [&](std::uint32_t index) {
     mbarrier_expect_tx(bar_kq, kGdnKqBytes);
-    bulk_copy_g2s(base + kPsKq, p.scratch.kq + static_cast<std::size_t>(item / ratio) * kGdnKqBytes, kGdnKqBytes, bar_kq);
-    const std::uint32_t next = (item / ratio + 1) * ratio; // into L2 while this image is worked on
-    if (next < last_item) {
-      prefetch_l2(p.scratch.kq + static_cast<std::size_t>(next / ratio) * kGdnKqBytes, kGdnKqBytes);
+    bulk_copy_g2s(base + kPsKq, p.scratch.kq + static_cast<std::size_t>(index) * kGdnKqBytes, kGdnKqBytes, bar_kq);
+    if ((index + 1) * ratio < last_item) { // into L2 while this image is worked on
+      prefetch_l2(p.scratch.kq + static_cast<std::size_t>(index + 1) * kGdnKqBytes, kGdnKqBytes);
     }
   };
-  auto issue_gates = [&](std::uint32_t item) {
+  auto issue_gates = [&](std::uint32_t at) {
     fence_proxy_async(); // those of the item before have been read by ordinary loads
     mbarrier_expect_tx(bar_gates, kGdnGateBytes);
-    bulk_copy_g2s(base + kPsGates, p.scratch.records + record_index(item) * kGdnRecBytes + kGdnRecGates, kGdnGateBytes,
-                  bar_gates);
+    bulk_copy_g2s(base + kPsGates, p.scratch.records + static_cast<std::size_t>(at) * kGdnRecBytes + kGdnRecGates,
+                  kGdnGateBytes, bar_gates);
   };
-  auto issue_v = [&](std::uint32_t item) {
+  auto issue_v = [&](std::uint32_t at) {
     fence_proxy_async(); // U has been staged here by ordinary stores
     mbarrier_expect_tx(bar_v, kGdnVBytes);
-    bulk_copy_g2s(base + kPsV, p.scratch.v + record_index(item) * kGdnVBytes, kGdnVBytes, bar_v);
-    if (item + 1 < last_item) {
-      prefetch_l2(p.scratch.v + record_index(item + 1) * kGdnVBytes, kGdnVBytes);
-    }
+    bulk_copy_g2s(base + kPsV, p.scratch.v + static_cast<std::size_t>(at) * kGdnVBytes, kGdnVBytes, bar_v);
   };
   if (copier && first_item < last_item) {
-    issue_kq(first_item);
-    issue_gates(first_item);
-    issue_v(first_item);
+    issue_kq(kq_index);
+    issue_gates(record);
+    issue_v(record);
+    if (first_item + 1 < last_item) {
+      prefetch_l2(p.scratch.v + static_cast<std::size_t>(record_index(first_item + 1)) * kGdnVBytes, kGdnVBytes);
+    }
   }
 
   const std::uint32_t quarter = warp & 3; // the 32 tensor-memory lanes this warp may read
@@ -493,13 +497,14 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
   std::uint32_t iteration = 0;
   for (std::uint32_t item = first_item; item < last_item; ++item, ++iteration) {
     const std::uint32_t phase = iteration & 1U;
-    unsigned char *rec = p.scratch.records + record_index(item) * kGdnRecBytes;
-    const bool next_kq = item + 1 < last_item && (item + 1) % ratio == 0; // the next item has another image
+    unsigned char *rec = p.scratch.records + static_cast<std::size_t>(record) * kGdnRecBytes;
+    const bool next_kq = item + 1 < last_item && item + 1 == (kq_index + 1) * ratio; // the next item has another image
+    const std::uint32_t next_record = item + 1 < last_item ? record_index(item + 1) : 0U;
     if (tid == 0) {
       RIB200_GDN_STAMP(100 + iteration, 0);
     }
     if (warp == 0) {
-      wait(bar_kq, (item / ratio - first_item / ratio) & 1U);
+      wait(bar_kq, (kq_index - first_kq) & 1U);
       tcgen05_fence_after();
       if (elect_one() && *abort_flag == 0) {
         const std::uint64_t kq = smem_desc(base + kPsKq, 16, 1024);
@@ -629,7 +634,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       bulk_copy_s2g(rec + kGdnRecP, base + kPsPstage, kGdnBlock);
       asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
       if (item + 1 < last_item) {
-        issue_gates(item + 1);
+        issue_gates(next_record);
       }
     }
 
@@ -807,7 +812,7 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
     wait(bar_wu, phase);
     tcgen05_fence_after();
     if (copier && next_kq && *abort_flag == 0) {
-      issue_kq(item + 1);
+      issue_kq(kq_index + 1);
     }
     __syncwarp();
     if (tid == 0) {
@@ -861,10 +866,15 @@ __global__ void __launch_bounds__(kPrepThreads, 2) gdn_chunk_prepare_kernel(cons
       asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
       mbarrier_arrive(bar_left);
       if (item + 1 < last_item) {
-        issue_v(item + 1);
+        issue_v(next_record);
+        if (item + 2 < last_item) {
+          prefetch_l2(p.scratch.v + static_cast<std::size_t>(record_index(item + 2)) * kGdnVBytes, kGdnVBytes);
+        }
       }
     }
     __syncwarp();
+    record = next_record;
+    kq_index += next_kq ? 1U : 0U;
   }
   if (copier) {
     asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
