@@ -742,6 +742,8 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
 //                 (the ratios are products of decays, nothing is divided), so that eight reductions over the rows and a
 //                 hand-back of corrections are paid once in four tokens.  A lane owns eight rows of four columns, a warp
 //                 eight columns; 32 sums over 16 lanes are 30 exchanges and leave token t, column c with lane 4 t + c.
+//                 A group in which a decay is above 1 (a positive coefficient) goes token by token: a product of its decays
+//                 may be infinite where each decay is finite and what it multiplies is zero or small.
 //   output norm   the slices of a head exchange their sums of squares.
 // Replayed calls (BF16), this form and the one before it (a warp per four columns, a token at a time, clusters of eight): 2
 // tokens 8.4 and 10.4 us, 17 14.4 and 18.6, 32 17 and 28.5, 48 22.7 and 39, 63 28 and 47.3.  At 63 tokens 44 k cycles: loads
@@ -759,7 +761,7 @@ struct ShortShared {
   float qk[2][kShortRows][kDim];                  // inputs, then their convolutions, then normalised
   float v[kStepMaxRatio][kShortRows][kStepColumns]; // inputs, then their convolutions, then the outputs
   float4 scale[kStepMaxRatio][kShortRows];        // beta_t, G_t, G_3 / G_t, G_3
-  float4 solve[kStepMaxRatio][kShortRows];        // (I + L)^-1 at (t, t ^ 1), (t, t ^ 2), (t, t ^ 3)
+  float4 solve[kStepMaxRatio][kShortRows];        // (I + L)^-1 at (t, t ^ 1), (t, t ^ 2), (t, t ^ 3); not 0: a decay grows
   float4 read[kStepMaxRatio][kShortRows];         // (G_t / G_j) (q_t . k_j) for j = t, t ^ 1, t ^ 2, t ^ 3
   float dots[kShortRows / kShortGroup][16];
   float beta[kStepMaxRatio][kShortRows];
@@ -1035,11 +1037,13 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
       float beta[kShortGroup];
       float decay[kShortGroup];
       double product[kShortGroup][kShortGroup]; // [t][j]: the decays of the tokens after j up to t, rounded once when used
+      bool grows = false;
 #pragma unroll
       for (std::uint32_t t = 0; t < kShortGroup; ++t) {
         const bool live = t0 + t < n;
         beta[t] = live ? sh.beta[lane][t0 + t] : 0.0F;
         decay[t] = live ? sh.decay[lane][t0 + t] : 1.0F;
+        grows = grows || !(decay[t] <= 1.0F);
       }
 #pragma unroll
       for (std::uint32_t j = 0; j < kShortGroup; ++j) {
@@ -1076,7 +1080,7 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
         sh.scale[lane][t0 + t] =
             make_float4(beta[t], static_cast<float>(decay[0] * product[t][0]), static_cast<float>(product[kShortGroup - 1][t]),
                         static_cast<float>(decay[0] * product[kShortGroup - 1][0]));
-        sh.solve[lane][t0 + t] = make_float4(solve[t][t ^ 1U], solve[t][t ^ 2U], solve[t][t ^ 3U], 0.0F);
+        sh.solve[lane][t0 + t] = make_float4(solve[t][t ^ 1U], solve[t][t ^ 2U], solve[t][t ^ 3U], grows ? 1.0F : 0.0F);
         sh.read[lane][t0 + t] = make_float4(read(t), read(t ^ 1U), read(t ^ 2U), read(t ^ 3U));
       }
     }
@@ -1140,6 +1144,42 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
       const float b = fold(b_sums);
       const float4 scale = sh.scale[h][group + t];
       const float4 solve = sh.solve[h][group + t];
+      if (solve.w != 0.0F) { // of all tokens of the group alike
+#pragma unroll 1
+        for (std::uint32_t token = group; token < min(group + kShortGroup, n); ++token) {
+          float key[8];
+          float query[8];
+          float sums[8]; // S^T k and S^T q of the lane's columns
+          fetch(sh.qk[1][token], key);
+          fetch(sh.qk[0][token], query);
+          products(key, sums);
+          products(query, sums + 4);
+#pragma unroll
+          for (int offset = 8; offset > 0; offset >>= 1) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              sums[i] += __shfl_xor_sync(0xFFFFFFFFU, sums[i], offset);
+            }
+          }
+          const float beta = sh.beta[h][token];
+          const float decay = sh.decay[h][token];
+          const float dot = sh.dots[group / kShortGroup][5 * (token - group)]; // q . k
+          float4 &row = *reinterpret_cast<float4 *>(&sh.v[h][token][column]);
+          const float4 delta = make_float4((row.x - decay * sums[0]) * beta, (row.y - decay * sums[1]) * beta,
+                                           (row.z - decay * sums[2]) * beta, (row.w - decay * sums[3]) * beta);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            s[r] = make_float4(decay * s[r].x + key[r] * delta.x, decay * s[r].y + key[r] * delta.y,
+                               decay * s[r].z + key[r] * delta.z, decay * s[r].w + key[r] * delta.w);
+          }
+          __syncwarp(); // all lanes of the columns have read the values
+          if (row_lane == 0) {
+            row = make_float4(decay * sums[4] + delta.x * dot, decay * sums[5] + delta.y * dot,
+                              decay * sums[6] + delta.z * dot, decay * sums[7] + delta.w * dot);
+          }
+        }
+        continue;
+      }
       const float4 read = sh.read[h][group + t];
       float &slot = sh.v[h][group + t][column + (row_lane & 3U)];
       const float y = group + t < n ? scale.x * (slot - scale.y * a) : 0.0F;

@@ -339,6 +339,43 @@ def test_layer_short_calls_in_groups(tokens, hv, dtype, aligned):
     assert K.device_status(torch.cuda.current_stream()) == 0
 
 
+@pytest.mark.parametrize("tokens,first", [(4, 0), (5, 0), (6, 2), (8, 4), (9, 0), (9, 2), (9, 5)])
+@pytest.mark.parametrize("hv", [1, 2])
+@pytest.mark.parametrize("state", ["zero", "tiny", "mild"])
+def test_layer_short_calls_with_growing_decays(tokens, first, hv, state):
+    """A positive coefficient, for which a decay is above 1.  Four consecutive tokens from `first` on grow by e^22 to e^25
+    each, so that the product of their decays overflows FP32 while every state along the way is finite: it is zero (no values
+    before the growth is over) or starts at 1e-30.  `mild`: decays of up to e^0.5 on an ordinary state.  The second value head
+    decays as usual.  Log decays are exact on both sides, so that 4 e^x of two ulp (1e-6) and the FP32 recurrence (2e-6, as in
+    the ordinary short calls) bound the difference."""
+    run = LayerRun(0xB2002B00 + 16 * tokens + first, 1, hv, 4, K.DTYPE_F32, K.DTYPE_F32, tokens)
+    conv_dim = 2 * DK + hv * DK
+    grown = range(first, first + 4)
+    run.rec_a = np.array([1.0, -1.0][:hv], dtype=np.float32)
+    run.dt_bias = np.zeros(hv, dtype=np.float32)
+    log_decay = synth.normal(0xB2002B01, 0, (tokens,))
+    if state == "mild":  # softplus(a) of -2 to 0.5
+        run.inp[:, conv_dim + hv] = np.clip(log_decay, -2.0, 0.5) - 1.0
+    else:
+        run.inp[:, conv_dim + hv] = -40.0  # a decay of 1 + 4e-18
+        for t in grown:
+            run.inp[t, conv_dim + hv] = 22.0 + (3 * t % 4)
+        run.rs[0] = 0.0 if state == "zero" else 1.0e-30 / 0.05 * run.rs[0]
+        value = slice(2 * DK, 3 * DK)
+        run.inp[:first + 4, value] = 0.0
+        run.cs[value] = 0.0
+    run.d_rec_a, run.d_dt = act_tensor(run.rec_a, K.DTYPE_F32), act_tensor(run.dt_bias, K.DTYPE_F32)
+    run.d_cs, run.d_rs = torch.from_numpy(run.cs.copy()).to(dev()), torch.from_numpy(run.rs.copy()).to(dev())
+    out, want, _ = run.step(tokens)
+    assert np.isfinite(want).all() and np.isfinite(run.rs).all()
+    m = compare(to_numpy_f32(out), want)
+    assert m["nonfinite"] == 0 and m["rel_l2"] <= 3.0e-6, m
+    for head in range(hv):
+        rs = compare(to_numpy_f32(run.d_rs)[head].reshape(-1), run.rs.reshape(hv, -1)[head])
+        assert rs["nonfinite"] == 0 and rs["rel_l2"] <= 3.0e-6, (head, rs)
+    assert K.device_status(torch.cuda.current_stream()) == 0
+
+
 def test_layer_three_launches_share_device_state_without_a_sync():
     run = LayerRun(0xB2002200, 2, 4, 4, K.DTYPE_F32, K.DTYPE_F32, 6)
     results = [run.step(2, sync=False) for _ in range(3)]
