@@ -734,16 +734,19 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
 //   loads         rows of 128 q or k channels, or of 32 v channels, a warp at a time into shared memory;
 //   convolution   in place, a channel per thread of warps 0-7 (q, k) and 8-9 (v), while warps 10-11 make the gates;
 //   norms         a warp per group of four tokens: the normalised vectors, and the products k_t . k_j and q_t . k_j of the
-//                 group, of which a lane per value head makes the group's coefficients;
+//                 group, of which warps 8-11 make the coefficients of all groups;
 //   recurrence    a group at a time.  With G_t the product of the group's decays up to t and S0 the state in front of it,
-//                   y_t = beta_t (v_t - G_t S0^T k_t),  delta = (I + L)^-1 y,  L_tj = beta_t (G_t / G_j) (k_t . k_j), j < t
-//                   o_t = G_t S0^T q_t + sum over j <= t of (G_t / G_j) (q_t . k_j) delta_j
-//                   S   = G_3 S0 + sum over t of (G_3 / G_t) k_t delta_t^T
-//                 (the ratios are products of decays, nothing is divided), so that eight reductions over the rows and a
+//                   u_t = v_t - G_t S0^T k_t
+//                   o_t = G_t S0^T q_t + sum over j <= t of R_tj u_j
+//                   S   = G_3 S0 + sum over t of k_t (sum over j <= t of W_tj u_j)^T
+//                   D = (I + L)^-1 diag(beta),  L_tj = beta_t (G_t / G_j) (k_t . k_j), j < t
+//                   W_tj = (G_3 / G_t) D_tj,  R_tj = sum over i, j <= i <= t, of (G_t / G_i) (q_t . k_i) D_ij
+//                 (the ratios are products of decays, nothing is divided; the coefficients are made in 64 bits and rounded
+//                 once, and G_3 S0 is rounded with its sum and not before), so that eight reductions over the rows and a
 //                 hand-back of corrections are paid once in four tokens.  A lane owns eight rows of four columns, a warp
 //                 eight columns; 32 sums over 16 lanes are 30 exchanges and leave token t, column c with lane 4 t + c.
-//                 A group in which a decay is above 1 (a positive coefficient) goes token by token: a product of its decays
-//                 may be infinite where each decay is finite and what it multiplies is zero or small.
+//                 A head with a decay above 1 (a positive coefficient) goes token by token: a product of its decays may be
+//                 infinite where each decay is finite and what it multiplies is zero or small.
 //   output norm   the slices of a head exchange their sums of squares.
 // Replayed calls (BF16), this form and the one before it (a warp per four columns, a token at a time, clusters of eight): 2
 // tokens 8.4 and 10.4 us, 17 14.4 and 18.6, 32 17 and 28.5, 48 22.7 and 39, 63 28 and 47.3.  At 63 tokens 44 k cycles: loads
@@ -760,12 +763,13 @@ constexpr std::uint32_t kShortRounds = (kStepMaxRatio * kShortRows + 4 * kShortW
 struct ShortShared {
   float qk[2][kShortRows][kDim];                  // inputs, then their convolutions, then normalised
   float v[kStepMaxRatio][kShortRows][kStepColumns]; // inputs, then their convolutions, then the outputs
-  float4 scale[kStepMaxRatio][kShortRows];        // beta_t, G_t, G_3 / G_t, G_3
-  float4 solve[kStepMaxRatio][kShortRows];        // (I + L)^-1 at (t, t ^ 1), (t, t ^ 2), (t, t ^ 3); not 0: a decay grows
-  float4 read[kStepMaxRatio][kShortRows];         // (G_t / G_j) (q_t . k_j) for j = t, t ^ 1, t ^ 2, t ^ 3
+  float2 gain[kStepMaxRatio][kShortRows];         // G_t, G_3
+  float4 write[kStepMaxRatio][kShortRows];        // W_tj for j = t, t ^ 1, t ^ 2, t ^ 3
+  float4 read[kStepMaxRatio][kShortRows];         // R_tj likewise
   float dots[kShortRows / kShortGroup][16];
   float beta[kStepMaxRatio][kShortRows];
   float decay[kStepMaxRatio][kShortRows];
+  bool grows[kStepMaxRatio];                      // a decay is above 1
   float norm[kStepSlices][kStepMaxRatio * kShortRows];
   std::uint64_t norm_bar;
 };
@@ -973,12 +977,19 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
     const std::uint32_t index = warp - 10;
     const float coefficient = Weight::widen(static_cast<const WeightType *>(p.recurrent_a)[head_of(index)]);
     const float dt = Weight::widen(static_cast<const WeightType *>(p.dt_bias)[head_of(index)]);
+    bool grows = false;
     for (std::uint32_t t = lane; t < n; t += 32) {
       const ActType *gates = input + static_cast<std::size_t>(t) * p.token_stride + p.conv_dim + head_of(index);
       const float b = Act::widen(gates[0]);
       const float a = Act::widen(gates[p.value_heads]);
+      const float decay = expf(coefficient * softplus(a + dt));
       sh.beta[index][t] = sigmoid(b);
-      sh.decay[index][t] = expf(coefficient * softplus(a + dt));
+      sh.decay[index][t] = decay;
+      grows = grows || !(decay <= 1.0F);
+    }
+    grows = __any_sync(0xFFFFFFFFU, grows);
+    if (lane == 0) {
+      sh.grows[index] = grows;
     }
   }
   __syncthreads();
@@ -1031,102 +1042,137 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
     if (lane < 16) {
       sh.dots[group][lane] = total;
     }
-    __syncwarp();
-    if (lane < ratio) {
-      const float *d = sh.dots[group];
-      float beta[kShortGroup];
-      float decay[kShortGroup];
-      double product[kShortGroup][kShortGroup]; // [t][j]: the decays of the tokens after j up to t, rounded once when used
-      bool grows = false;
-#pragma unroll
-      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
-        const bool live = t0 + t < n;
-        beta[t] = live ? sh.beta[lane][t0 + t] : 0.0F;
-        decay[t] = live ? sh.decay[lane][t0 + t] : 1.0F;
-        grows = grows || !(decay[t] <= 1.0F);
-      }
-#pragma unroll
-      for (std::uint32_t j = 0; j < kShortGroup; ++j) {
-        product[j][j] = 1.0;
-#pragma unroll
-        for (std::uint32_t t = j + 1; t < kShortGroup; ++t) {
-          product[t][j] = product[t - 1][j] * decay[t];
-        }
-      }
-      float solve[kShortGroup][kShortGroup]; // (I + L)^-1, by rows
-#pragma unroll
-      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
-        float row_l[kShortGroup];
-#pragma unroll
-        for (std::uint32_t j = 0; j < t; ++j) {
-          row_l[j] = static_cast<float>(beta[t] * product[t][j]) * d[4 * t + j];
-        }
-#pragma unroll
-        for (std::uint32_t j = 0; j < kShortGroup; ++j) {
-          solve[t][j] = j == t ? 1.0F : 0.0F;
-          if (j < t) {
-            float x = -row_l[j];
-#pragma unroll
-            for (std::uint32_t i = j + 1; i < t; ++i) {
-              x -= row_l[i] * solve[i][j];
-            }
-            solve[t][j] = x;
-          }
-        }
-      }
-#pragma unroll
-      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
-        auto read = [&](std::uint32_t j) { return j <= t ? static_cast<float>(product[t][j]) * d[4 * j + t] : 0.0F; };
-        sh.scale[lane][t0 + t] =
-            make_float4(beta[t], static_cast<float>(decay[0] * product[t][0]), static_cast<float>(product[kShortGroup - 1][t]),
-                        static_cast<float>(decay[0] * product[kShortGroup - 1][0]));
-        sh.solve[lane][t0 + t] = make_float4(solve[t][t ^ 1U], solve[t][t ^ 2U], solve[t][t ^ 3U], grows ? 1.0F : 0.0F);
-        sh.read[lane][t0 + t] = make_float4(read(t), read(t ^ 1U), read(t ^ 2U), read(t ^ 3U));
-      }
-    }
-    __syncwarp();
   }
   __syncthreads();
 
+  // ---- coefficients, while the warps of the recurrence form the sums of their first group: a thread per group, value head
+  // and token j of the group makes what u_j puts into the tokens from j on ----
+  static_assert(kShortThreads - 256 == kShortRows * kStepMaxRatio, "a thread per value head and token");
+  auto coefficients_made = [] { asm volatile("bar.sync 1, %0;\n" ::"n"(kShortThreads) : "memory"); };
+  if (warp >= 8) {
+    const std::uint32_t group = (tid - 256) / (kStepMaxRatio * kShortGroup);
+    const std::uint32_t head = (tid / kShortGroup) % kStepMaxRatio;
+    const std::uint32_t j = tid % kShortGroup;
+    const std::uint32_t t0 = kShortGroup * group;
+    if (t0 < n && head < ratio) {
+      const float *d = sh.dots[group];
+      double beta[kShortGroup];
+      double decay[kShortGroup];
+      double gain = 1.0; // up to token j
+      double all = 1.0;
+#pragma unroll
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        const bool live = t0 + t < n;
+        beta[t] = live ? sh.beta[head][t0 + t] : 0.0F;
+        decay[t] = live ? sh.decay[head][t0 + t] : 1.0F;
+        all *= decay[t];
+        gain = t == j ? all : gain;
+      }
+      double product[kShortGroup][kShortGroup]; // [t][i]: the decays of the tokens after i up to t
+#pragma unroll
+      for (std::uint32_t i = 0; i < kShortGroup; ++i) {
+        product[i][i] = 1.0;
+#pragma unroll
+        for (std::uint32_t t = i + 1; t < kShortGroup; ++t) {
+          product[t][i] = product[t - 1][i] * decay[t];
+        }
+      }
+      double column[kShortGroup]; // column j of (I + L)^-1 diag(beta)
+#pragma unroll
+      for (std::uint32_t t = 0; t < kShortGroup; ++t) {
+        double sum = 0.0;
+        double out = 0.0;
+#pragma unroll
+        for (std::uint32_t i = 0; i < t; ++i) {
+          sum += product[t][i] * d[4 * t + i] * column[i];
+          out += product[t][i] * d[4 * i + t] * column[i];
+        }
+        column[t] = t == j ? beta[t] : -beta[t] * sum;
+        // the entry of token t at t ^ j; those in front of j are not used
+        reinterpret_cast<float *>(&sh.write[head][t0 + t])[t ^ j] = static_cast<float>(product[kShortGroup - 1][t] * column[t]);
+        reinterpret_cast<float *>(&sh.read[head][t0 + t])[t ^ j] = static_cast<float>(out + d[5 * t] * column[t]);
+      }
+      sh.gain[head][t0 + j] = make_float2(static_cast<float>(gain), static_cast<float>(all));
+    }
+    coefficients_made();
+  } else if (!recurs) {
+    coefficients_made();
+  }
+
   // ---- the recurrence ----
-  if (recurs) {
+  auto fetch = [&](const float *vector, float (&x)[8]) {
+    const float4 low = *reinterpret_cast<const float4 *>(vector + 4 * row_lane);
+    const float4 high = *reinterpret_cast<const float4 *>(vector + 4 * row_lane + 64);
+    x[0] = low.x;
+    x[1] = low.y;
+    x[2] = low.z;
+    x[3] = low.w;
+    x[4] = high.x;
+    x[5] = high.y;
+    x[6] = high.z;
+    x[7] = high.w;
+  };
+  auto products = [&](const float (&x)[8], float *to) { // two chains of four a column
+    float4 low = make_float4(s[0].x * x[0], s[0].y * x[0], s[0].z * x[0], s[0].w * x[0]);
+    float4 high = make_float4(s[4].x * x[4], s[4].y * x[4], s[4].z * x[4], s[4].w * x[4]);
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+      low.x = fmaf(s[i].x, x[i], low.x);
+      low.y = fmaf(s[i].y, x[i], low.y);
+      low.z = fmaf(s[i].z, x[i], low.z);
+      low.w = fmaf(s[i].w, x[i], low.w);
+      high.x = fmaf(s[4 + i].x, x[4 + i], high.x);
+      high.y = fmaf(s[4 + i].y, x[4 + i], high.y);
+      high.z = fmaf(s[4 + i].z, x[4 + i], high.z);
+      high.w = fmaf(s[4 + i].w, x[4 + i], high.w);
+    }
+    to[0] = low.x + high.x;
+    to[1] = low.y + high.y;
+    to[2] = low.z + high.z;
+    to[3] = low.w + high.w;
+  };
+  if (recurs && sh.grows[h]) { // token by token
+    coefficients_made();
+#pragma unroll 1
+    for (std::uint32_t token = 0; token < n; ++token) {
+      float key[8];
+      float query[8];
+      float sums[8]; // S^T k and S^T q of the lane's columns
+      fetch(sh.qk[1][token], key);
+      fetch(sh.qk[0][token], query);
+      products(key, sums);
+      products(query, sums + 4);
+#pragma unroll
+      for (int offset = 8; offset > 0; offset >>= 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          sums[i] += __shfl_xor_sync(0xFFFFFFFFU, sums[i], offset);
+        }
+      }
+      const float beta = sh.beta[h][token];
+      const float decay = sh.decay[h][token];
+      const float dot = sh.dots[token / kShortGroup][5 * (token % kShortGroup)]; // q . k
+      float4 &row = *reinterpret_cast<float4 *>(&sh.v[h][token][column]);
+      const float4 delta = make_float4((row.x - decay * sums[0]) * beta, (row.y - decay * sums[1]) * beta,
+                                       (row.z - decay * sums[2]) * beta, (row.w - decay * sums[3]) * beta);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        s[r] = make_float4(decay * s[r].x + key[r] * delta.x, decay * s[r].y + key[r] * delta.y,
+                           decay * s[r].z + key[r] * delta.z, decay * s[r].w + key[r] * delta.w);
+      }
+      __syncwarp(); // all lanes of the columns have read the values
+      if (row_lane == 0) {
+        row = make_float4(decay * sums[4] + delta.x * dot, decay * sums[5] + delta.y * dot,
+                          decay * sums[6] + delta.z * dot, decay * sums[7] + delta.w * dot);
+      }
+    }
+  } else if (recurs) {
     const std::uint32_t t = row_lane >> 2;
     const bool second = (t & 1U) != 0; // has t ^ 1 in front of it
     const bool upper = (t & 2U) != 0;  // has t ^ 2 and t ^ 3 in front of it
 #pragma unroll 1
     for (std::uint32_t group = 0; group < n; group += kShortGroup) {
       float k[kShortGroup][8];
-      auto fetch = [&](const float *vector, float (&x)[8]) {
-        const float4 low = *reinterpret_cast<const float4 *>(vector + 4 * row_lane);
-        const float4 high = *reinterpret_cast<const float4 *>(vector + 4 * row_lane + 64);
-        x[0] = low.x;
-        x[1] = low.y;
-        x[2] = low.z;
-        x[3] = low.w;
-        x[4] = high.x;
-        x[5] = high.y;
-        x[6] = high.z;
-        x[7] = high.w;
-      };
-      auto products = [&](const float (&x)[8], float *to) { // two chains of four a column
-        float4 low = make_float4(s[0].x * x[0], s[0].y * x[0], s[0].z * x[0], s[0].w * x[0]);
-        float4 high = make_float4(s[4].x * x[4], s[4].y * x[4], s[4].z * x[4], s[4].w * x[4]);
-#pragma unroll
-        for (int i = 1; i < 4; ++i) {
-          low.x = fmaf(s[i].x, x[i], low.x);
-          low.y = fmaf(s[i].y, x[i], low.y);
-          low.z = fmaf(s[i].z, x[i], low.z);
-          low.w = fmaf(s[i].w, x[i], low.w);
-          high.x = fmaf(s[4 + i].x, x[4 + i], high.x);
-          high.y = fmaf(s[4 + i].y, x[4 + i], high.y);
-          high.z = fmaf(s[4 + i].z, x[4 + i], high.z);
-          high.w = fmaf(s[4 + i].w, x[4 + i], high.w);
-        }
-        to[0] = low.x + high.x;
-        to[1] = low.y + high.y;
-        to[2] = low.z + high.z;
-        to[3] = low.w + high.w;
-      };
       float a_sums[16];
       float b_sums[16];
 #pragma unroll
@@ -1142,79 +1188,48 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
       }
       const float a = fold(a_sums);
       const float b = fold(b_sums);
-      const float4 scale = sh.scale[h][group + t];
-      const float4 solve = sh.solve[h][group + t];
-      if (solve.w != 0.0F) { // of all tokens of the group alike
-#pragma unroll 1
-        for (std::uint32_t token = group; token < min(group + kShortGroup, n); ++token) {
-          float key[8];
-          float query[8];
-          float sums[8]; // S^T k and S^T q of the lane's columns
-          fetch(sh.qk[1][token], key);
-          fetch(sh.qk[0][token], query);
-          products(key, sums);
-          products(query, sums + 4);
-#pragma unroll
-          for (int offset = 8; offset > 0; offset >>= 1) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              sums[i] += __shfl_xor_sync(0xFFFFFFFFU, sums[i], offset);
-            }
-          }
-          const float beta = sh.beta[h][token];
-          const float decay = sh.decay[h][token];
-          const float dot = sh.dots[group / kShortGroup][5 * (token - group)]; // q . k
-          float4 &row = *reinterpret_cast<float4 *>(&sh.v[h][token][column]);
-          const float4 delta = make_float4((row.x - decay * sums[0]) * beta, (row.y - decay * sums[1]) * beta,
-                                           (row.z - decay * sums[2]) * beta, (row.w - decay * sums[3]) * beta);
-#pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            s[r] = make_float4(decay * s[r].x + key[r] * delta.x, decay * s[r].y + key[r] * delta.y,
-                               decay * s[r].z + key[r] * delta.z, decay * s[r].w + key[r] * delta.w);
-          }
-          __syncwarp(); // all lanes of the columns have read the values
-          if (row_lane == 0) {
-            row = make_float4(decay * sums[4] + delta.x * dot, decay * sums[5] + delta.y * dot,
-                              decay * sums[6] + delta.z * dot, decay * sums[7] + delta.w * dot);
-          }
-        }
-        continue;
+      if (group == 0) {
+        coefficients_made();
       }
-      const float4 read = sh.read[h][group + t];
+      const float2 gain = sh.gain[h][group + t];
       float &slot = sh.v[h][group + t][column + (row_lane & 3U)];
-      const float y = group + t < n ? scale.x * (slot - scale.y * a) : 0.0F;
-      const float y1 = __shfl_xor_sync(0xFFFFFFFFU, y, 4);
-      const float y2 = __shfl_xor_sync(0xFFFFFFFFU, y, 8);
-      const float y3 = __shfl_xor_sync(0xFFFFFFFFU, y, 12);
-      float delta = y;
-      delta = second ? fmaf(solve.x, y1, delta) : delta;
-      delta = upper ? fmaf(solve.z, y3, fmaf(solve.y, y2, delta)) : delta;
-      const float corrections = scale.z * delta;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        s[i] = make_float4(s[i].x * scale.w, s[i].y * scale.w, s[i].z * scale.w, s[i].w * scale.w);
-      }
-#pragma unroll
-      for (std::uint32_t i = 0; i < kShortGroup; ++i) {
-        const std::uint32_t from = (lane & 16U) + 4 * i; // the corrections of the lane's four columns
-        const float4 c = make_float4(__shfl_sync(0xFFFFFFFFU, corrections, from), __shfl_sync(0xFFFFFFFFU, corrections, from + 1),
-                                     __shfl_sync(0xFFFFFFFFU, corrections, from + 2),
-                                     __shfl_sync(0xFFFFFFFFU, corrections, from + 3));
+      const float u = group + t < n ? fmaf(-gain.x, a, slot) : 0.0F;
+      const float u1 = __shfl_xor_sync(0xFFFFFFFFU, u, 4);
+      const float u2 = __shfl_xor_sync(0xFFFFFFFFU, u, 8);
+      const float u3 = __shfl_xor_sync(0xFFFFFFFFU, u, 12);
+      auto combine = [&](const float4 &entries) {
+        float sum = upper ? fmaf(entries.z, u2, entries.w * u3) : 0.0F;
+        sum = second ? fmaf(entries.y, u1, sum) : sum;
+        return fmaf(entries.x, u, sum);
+      };
+      const float correction = combine(sh.write[h][group + t]);
+      auto corrections = [&](int i) { // of token i for the lane's four columns
+        const int from = static_cast<int>(lane & 16U) + 4 * i;
+        return make_float4(__shfl_sync(0xFFFFFFFFU, correction, from), __shfl_sync(0xFFFFFFFFU, correction, from + 1),
+                           __shfl_sync(0xFFFFFFFFU, correction, from + 2), __shfl_sync(0xFFFFFFFFU, correction, from + 3));
+      };
+      auto two = [](float k0, float c0, float k1, float c1, float sum) { return fmaf(k1, c1, fmaf(k0, c0, sum)); };
+      {
+        const float4 c0 = corrections(0);
+        const float4 c1 = corrections(1);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-          s[r].x = fmaf(k[i][r], c.x, s[r].x);
-          s[r].y = fmaf(k[i][r], c.y, s[r].y);
-          s[r].z = fmaf(k[i][r], c.z, s[r].z);
-          s[r].w = fmaf(k[i][r], c.w, s[r].w);
+          s[r] = make_float4(fmaf(gain.y, s[r].x, two(k[0][r], c0.x, k[1][r], c1.x, 0.0F)),
+                             fmaf(gain.y, s[r].y, two(k[0][r], c0.y, k[1][r], c1.y, 0.0F)),
+                             fmaf(gain.y, s[r].z, two(k[0][r], c0.z, k[1][r], c1.z, 0.0F)),
+                             fmaf(gain.y, s[r].w, two(k[0][r], c0.w, k[1][r], c1.w, 0.0F)));
         }
       }
-      const float d1 = __shfl_xor_sync(0xFFFFFFFFU, delta, 4);
-      const float d2 = __shfl_xor_sync(0xFFFFFFFFU, delta, 8);
-      const float d3 = __shfl_xor_sync(0xFFFFFFFFU, delta, 12);
-      float out = fmaf(read.x, delta, scale.y * b);
-      out = second ? fmaf(read.y, d1, out) : out;
-      out = upper ? fmaf(read.w, d3, fmaf(read.z, d2, out)) : out;
-      slot = out;
+      {
+        const float4 c2 = corrections(2);
+        const float4 c3 = corrections(3);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          s[r] = make_float4(two(k[2][r], c2.x, k[3][r], c3.x, s[r].x), two(k[2][r], c2.y, k[3][r], c3.y, s[r].y),
+                             two(k[2][r], c2.z, k[3][r], c3.z, s[r].z), two(k[2][r], c2.w, k[3][r], c3.w, s[r].w));
+        }
+      }
+      slot = fmaf(gain.x, b, combine(sh.read[h][group + t]));
     }
   }
   __syncthreads();
