@@ -79,6 +79,8 @@ __host__ __device__ constexpr std::uint32_t row_offset(std::uint32_t row) { // b
 }
 constexpr int kMergePitch = kHeadDim + 8;              // floats per (warp, head) row of the merge area
 constexpr long long kWaitLimitCycles = 1LL << 28;      // SM cycles an mbarrier wait may take before giving up
+// ... and the wait for the other CTAs of a cluster, each of which may have waited that long for its rows first
+constexpr long long kExchangeLimitCycles = 4 * kWaitLimitCycles;
 
 // Shape of one CTA: `Warps` warps, each with a private ring of `Slots` slots (K and V slots alternate).
 template <int Warps, int Slots> struct Tile {
@@ -768,13 +770,20 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
       return;
     }
     constexpr int kOwned = kGroup / Cluster;
-    // every thread waits: nobody leaves while a peer may still send
-    const long long started = clock64();
-    while (!mbarrier_try_wait(exchange_bar, 0)) {
-      if (clock64() - started > kWaitLimitCycles) {
-        atomicOr(p.status, static_cast<unsigned int>(RIB200_DEVICE_WAIT_TIMED_OUT));
-        break;
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // all that this warp sends is on its way
+    auto received = [&](long long limit) {
+      const long long started = clock64();
+      while (!mbarrier_try_wait(exchange_bar, 0)) {
+        if (clock64() - started > limit) {
+          return false;
+        }
       }
+      return true;
+    };
+    const bool complete = received(kExchangeLimitCycles);
+    if (!complete) {
+      atomicOr(p.status, static_cast<unsigned int>(RIB200_DEVICE_WAIT_TIMED_OUT));
     }
     if (threadIdx.x < kOwned * 32) {
       const float *values = reinterpret_cast<const float *>(smem + T::kSmemBytes);
@@ -799,6 +808,12 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
         acc[4] += b.x * weight; acc[5] += b.y * weight; acc[6] += b.z * weight; acc[7] += b.w * weight;
       }
       finish(kvh * kGroup + static_cast<int>(rank) * kOwned + owned, dim0, total_max, total_sum, acc);
+    }
+    // Nobody leaves while a peer may still send: a CTA whose wait ran out stays until all have sent, and until that is here.
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory");
+    if (!complete) {
+      received(kWaitLimitCycles);
     }
   }
   RIB200_DECODE_STAMP(g_decode_trace, trace_cta, 3);

@@ -336,6 +336,121 @@ def test_early_kv_fetch_gives_the_same_bits():
     assert not torch.equal(plain[1][0], chain(False, moving_gate=False)[0])
 
 
+@pytest.mark.parametrize("ctx,max_ctx", [(63, 1024), (64, 1024), (65, 1024), (257, 1024), (777, 1024),
+                                         (100, 4096), (129, 4096), (257, 4096), (777, 4096), (4000, 4096)])
+def test_early_kv_fetch_where_a_cluster_shares_a_partition(ctx, max_ctx):
+    """Early cache fetch in the grids whose partitions are shared by four CTAs (1024 rows) and by two (4096): a context that
+    one CTA serves alone, shares that are empty, full and ragged.  Steps back to back on different caches, queries and gates
+    rewritten in front of each, give the bits of the default ordering."""
+    pos, steps = ctx - 1, 4
+    q, gate, k, v = decode_operands(0xB2000B80 + ctx, ctx)
+    shape = K.Qwen35AttentionShape(1, HQ, HKV, D, max_ctx, pos)
+    plan = K.qwen35_online_decode_plan(shape, K.SPLIT_K_256, max_ctx)
+    layout = K.qwen35_online_decode_workspace_layout(shape, plan.resolved_mode)
+    filled = cache_to_device(make_cache(k, v, max_ctx, pos))
+    dk, dv = act_tensor(k[pos], K.DTYPE_BF16), act_tensor(v[pos], K.DTYPE_BF16)
+    stream = torch.cuda.current_stream()
+
+    def run(early):
+        caches = [filled.clone() for _ in range(steps)]
+        ws = torch.zeros(layout.bytes // 4, device=dev())
+        dq, dg = act_tensor(q, K.DTYPE_BF16), act_tensor(gate, K.DTYPE_BF16)
+        outs = [torch.zeros(HQ, D, device=dev(), dtype=torch.bfloat16) for _ in range(steps)]
+        torch.cuda.synchronize()
+        for out, cache in zip(outs, caches):
+            args = (dq, dk, dv, dg, out, cache, cache.numel() * 2, ws, layout.bytes, shape, K.DTYPE_BF16, K.KV_BF16,
+                    K.HEAD_MAJOR, plan)
+            if early:
+                K.online_attention_decode_early_kv_fetch(*args, stream)
+            else:
+                K.qwen35_online_attention_decode(*args, None, stream)
+            dq.copy_((dq.float() * 0.5 + out.float() * 4.0).to(torch.bfloat16))
+            dg.copy_((dg.float() * 0.75 - out.float() * 3.0).to(torch.bfloat16))
+        torch.cuda.synchronize()
+        return torch.stack(outs), torch.stack(caches)
+
+    for want, got in zip(run(False), run(True)):
+        assert torch.equal(got, want)
+    assert K.device_status(stream) == 0
+
+
+def test_replayed_step_moves_across_the_shares_of_a_cluster():
+    """One captured step whose device position moves from a context that one CTA of a cluster serves alone to one that two
+    share, and from one partition to two: the bits of plain calls at those positions."""
+    max_ctx = 1024
+    q, gate, k, v = decode_operands(0xB2000BC0, max_ctx)
+    shape_of = lambda pos: K.Qwen35AttentionShape(1, HQ, HKV, D, max_ctx, pos)
+    plan = K.qwen35_online_decode_plan(shape_of(0), K.SPLIT_K_256, max_ctx)
+    layout = K.qwen35_online_decode_workspace_layout(shape_of(0), plan.resolved_mode)
+    ws = torch.zeros(layout.bytes // 4, device=dev())
+    cache = cache_to_device(make_cache(k, v, max_ctx, max_ctx))
+    dq, dg = act_tensor(q, K.DTYPE_BF16), act_tensor(gate, K.DTYPE_BF16)
+    dk, dv = act_tensor(k[0], K.DTYPE_BF16), act_tensor(v[0], K.DTYPE_BF16)
+    out = torch.zeros(HQ, D, device=dev(), dtype=torch.bfloat16)
+    position = torch.zeros(1, device=dev(), dtype=torch.int32)
+    stream = torch.cuda.current_stream()
+
+    def step(into, where, pos):
+        K.qwen35_online_attention_decode(dq, dk, dv, dg, into, cache, cache.numel() * 2, ws, layout.bytes, shape_of(pos),
+                                         K.DTYPE_BF16, K.KV_BF16, K.HEAD_MAJOR, plan, where, stream)
+
+    step(out, position, 0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        step(out, position, 0)
+        position.add_(1)
+    filled = cache_to_device(make_cache(k, v, max_ctx, max_ctx))
+    for first in (61, 253):
+        position.fill_(first)
+        for pos in range(first, first + 6):
+            cache.copy_(filled)
+            graph.replay()
+            got, want = out.clone(), torch.zeros_like(out)
+            step(want, None, pos)
+            torch.cuda.synchronize()
+            assert torch.equal(got, want), pos
+    assert K.device_status(stream) == 0
+
+
+@pytest.mark.parametrize("ctx,row", [(100, 70), (100, 3), (200, 199), (300, 290)])
+@pytest.mark.parametrize("kind", ["nan", "up", "down"])
+@pytest.mark.parametrize("dtype", [K.DTYPE_BF16, K.DTYPE_F32])
+def test_scores_without_a_number_beside_empty_shares(ctx, row, kind, dtype):
+    """A cached key that is not a number, or whose score with one query head overflows upwards (the head's output is not a
+    number) or downwards (the row has no weight), in a context that leaves shares of a cluster empty: the same heads come
+    out as not a number as in the one-block form, the others agree with it."""
+    max_ctx, pos, head = 1024, ctx - 1, 5
+    q, gate, k, v = decode_operands(0xB2000BE0 + ctx, ctx)
+    if kind == "nan":
+        k[row, head // 4, 7] = np.nan
+    else:
+        k[row, head // 4] = (1.0e38 if kind == "up" else -1.0e38) * np.sign(q[head])
+    k = synth.round_bf16(k)
+    outs = []
+    for mode in (K.SPLIT_K_256, K.SINGLE_BLOCK):
+        shape = K.Qwen35AttentionShape(1, HQ, HKV, D, max_ctx, pos)
+        plan = K.qwen35_online_decode_plan(shape, mode, ctx)
+        layout = K.qwen35_online_decode_workspace_layout(shape, plan.resolved_mode)
+        ws = torch.zeros(max(layout.bytes // 4, 1), device=dev())
+        cache = cache_to_device(make_cache(k, v, max_ctx, pos))
+        out = torch.zeros(HQ, D, device=dev(), dtype=torch.float32 if dtype == K.DTYPE_F32 else torch.bfloat16)
+        stream = torch.cuda.current_stream()
+        K.qwen35_online_attention_decode(act_tensor(q, dtype), act_tensor(k[pos], dtype), act_tensor(v[pos], dtype),
+                                         act_tensor(gate, dtype), out, cache, cache.numel() * 2,
+                                         ws if layout.bytes else None, layout.bytes, shape, dtype, K.KV_BF16, K.HEAD_MAJOR,
+                                         plan, None, stream)
+        torch.cuda.synchronize()
+        assert K.device_status(stream) == 0
+        outs.append(to_numpy_f32(out))
+    got, want = outs
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    spoilt = np.isnan(want).all(axis=1)
+    assert spoilt[head] == (kind != "down") and not spoilt[:4].any() and not spoilt[8:].any()
+    finite = ~np.isnan(want)
+    gate_bf16_outputs(compare(got[finite], want[finite]))
+
+
 def test_decode_from_host_buffers():
     """The host-buffer entry point (copy in, step, copy out, synchronise) gives what the device-buffer call gives."""
     ctx, max_ctx = 1500, 2048
