@@ -164,6 +164,20 @@ __device__ __forceinline__ bool mbarrier_try_wait(std::uint32_t bar, std::uint32
   return done != 0;
 }
 
+// for bytes that other CTAs of the cluster store
+__device__ __forceinline__ bool mbarrier_try_wait_cluster(std::uint32_t bar, std::uint32_t parity) {
+  std::uint32_t done;
+  asm volatile("{\n"
+               ".reg .pred p;\n"
+               "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+               "selp.u32 %0, 1, 0, p;\n"
+               "}\n"
+               : "=r"(done)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return done != 0;
+}
+
 // L2 policy for the cache rows: a step reads each of them once, so they are the first to go.  What the step
 // writes and reads again (the split-k partials) then stays in L2 between the two kernels.
 __device__ __forceinline__ std::uint64_t evict_first_policy() {
@@ -774,7 +788,7 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); // all that this warp sends is on its way
     auto received = [&](long long limit) {
       const long long started = clock64();
-      while (!mbarrier_try_wait(exchange_bar, 0)) {
+      while (!mbarrier_try_wait_cluster(exchange_bar, 0)) {
         if (clock64() - started > limit) {
           return false;
         }
