@@ -475,7 +475,7 @@ __device__ __forceinline__ void hint_operands(const LayerParams &p, std::uint32_
 
 // The slices of a head exchange their sums of squares with stores that count on an mbarrier of the CTA they go to.  A cluster
 // barrier in their place costs a call 0.3 to 0.6 us more: its release waits for whatever the thread has in flight.  Who has
-// the sums of all slices also knows that their CTAs have read the old history, and that nothing more will come.
+// the sums of all slices also knows that their CTAs have read the old history.
 constexpr long long kWaitLimitCycles = 1LL << 28;
 __device__ __forceinline__ std::uint32_t smem_address(const void *p) {
   return static_cast<std::uint32_t>(__cvta_generic_to_shared(p));
@@ -495,8 +495,13 @@ __device__ __forceinline__ void send_sum(const float *slot, std::uint64_t *bar, 
                "r"(__float_as_uint(value)), "r"(remote_bar)
                : "memory");
 }
-// bounded: when it runs out the status word says so and the call runs to its end
-__device__ __forceinline__ void wait_for_sums(std::uint64_t *bar, unsigned int *status) {
+// by every warp behind its last store to a peer; it releases nothing and so waits for nothing
+__device__ __forceinline__ void all_sent() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+}
+// bounded: when it runs out the status word says so, the call runs to its end and the answer is false
+__device__ __forceinline__ bool wait_for_sums(std::uint64_t *bar, unsigned int *status) {
   const long long started = clock64();
   std::uint32_t done = 0;
   while (done == 0) {
@@ -510,8 +515,17 @@ __device__ __forceinline__ void wait_for_sums(std::uint64_t *bar, unsigned int *
                  : "memory");
     if (done == 0 && clock64() - started > kWaitLimitCycles) {
       atomicOr(status, static_cast<unsigned int>(RIB200_DEVICE_WAIT_TIMED_OUT));
-      return;
+      return false;
     }
+  }
+  return true;
+}
+// At the end.  To a CTA that has its sums nobody sends any more, so it may leave (a wait of all for all costs a one-token call
+// 0.06 of its 3.2 us); where the wait ran out, not before all have sent and that is here.
+__device__ __forceinline__ void leave_cluster(std::uint64_t *bar, bool complete, unsigned int *status) {
+  if (!complete) {
+    asm volatile("barrier.cluster.wait;\n" ::: "memory");
+    wait_for_sums(bar, status);
   }
 }
 
@@ -704,6 +718,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
       send_sum(&s_norm[rank], &s_norm_bar, 0, 0.0F);
     }
   }
+  all_sent();
   const float4 delta = *reinterpret_cast<const float4 *>(&s_delta[col]);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -711,9 +726,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
         make_float4(decay * s[i].x + k_row[i] * delta.x, decay * s[i].y + k_row[i] * delta.y,
                     decay * s[i].z + k_row[i] * delta.z, decay * s[i].w + k_row[i] * delta.w);
   }
-  if (rank == 0 || warp == 0) {
-    wait_for_sums(&s_norm_bar, p.status);
-  }
+  const bool complete = (rank != 0 && warp != 0) || wait_for_sums(&s_norm_bar, p.status);
   if (rank == 0) {
     shift_history(qk_channel, qk);
   }
@@ -724,6 +737,7 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
     static_cast<typename Act::Type *>(p.output)[head * kDim + slice * kStepColumns + lane] =
         Act::narrow(read * scale * z_gate);
   }
+  leave_cluster(&s_norm_bar, complete, p.status);
 }
 
 // ---- 2 .. 63 tokens in one launch --------------------------------------------------------------------------
@@ -1255,6 +1269,7 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
       send_sum(&sh.norm[slice][row], &sh.norm_bar, lane & 7U, squares);
     }
   }
+  all_sent();
 #pragma unroll
   for (std::uint32_t r = 0; r < kShortRounds; ++r) {
     if (4 * (warp + kShortWarps * r) >= rows) {
@@ -1263,7 +1278,7 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
     z[r] = make_float4(norm_weight.x * silu(z[r].x), norm_weight.y * silu(z[r].y), norm_weight.z * silu(z[r].z),
                        norm_weight.w * silu(z[r].w));
   }
-  wait_for_sums(&sh.norm_bar, p.status);
+  const bool complete = wait_for_sums(&sh.norm_bar, p.status);
 #pragma unroll
   for (std::uint32_t r = 0; r < kShortRounds; ++r) {
     const std::uint32_t row = 4 * (warp + kShortWarps * r) + (lane >> 3);
@@ -1297,6 +1312,7 @@ __global__ void __launch_bounds__(kShortThreads, 1) gdn_layer_short_kernel(const
       p.convolution_state[static_cast<std::size_t>(channel) * kHistory + i] = next_history[i];
     }
   }
+  leave_cluster(&sh.norm_bar, complete, p.status);
 }
 
 LayerParams make_params(const GdnLayerArgs &a) {
