@@ -47,10 +47,12 @@ __device__ __forceinline__ void store_any(void *base, std::size_t index, int32_t
 
 // x / d for d >= 1 or infinite: the unit's reciprocal and one step of Newton's iteration on the quotient, q + (x - d q) r, in
 // place of a division, whose slow path keeps the compiler from overlapping the chains of neighbouring tokens.  The
-// remainder is not a number exactly where x or d is infinite or not a number; x r is the quotient then.
+// remainder is not a number exactly where x or d is infinite or not a number; x r is the quotient then.  The unit makes the
+// subnormal reciprocals of d above 2^126 zero, so it gets a quarter of d; r keeps 22 bits and more there.
 __device__ __forceinline__ float quotient(float x, float d) {
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(d));
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(0.25F * d));
+  r *= 0.25F;
   const float q = x * r;
   const float remainder = fmaf(-d, q, x);
   return remainder == remainder ? fmaf(remainder, r, q) : q;

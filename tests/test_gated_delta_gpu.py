@@ -376,6 +376,49 @@ def test_layer_short_calls_with_growing_decays(tokens, first, hv, state):
     assert K.device_status(torch.cuda.current_stream()) == 0
 
 
+FAR_GATES = np.concatenate([np.linspace(-88.7, -80.0, 100), [-95.0, -104.0, -200.0, np.inf, np.nan, -30.0, -1.0e-3, 0.0, 1.0e-3],
+                            np.linspace(1.0, 100.0, 19)]).astype(np.float32)
+
+
+@pytest.mark.parametrize("tokens,width", [(1, 4), (5, 4), (3, 3)])
+def test_layer_gates_of_any_size(tokens, width):
+    """SiLU of output gates down to where 1 + e^-z overflows, of an infinite one and of one that is not a number, in the
+    one-launch forms and the general path: the output over that of the same call with gates of 20, whose SiLU is 20.  e^x of
+    two ulp and five roundings bound the difference; below -88.72 the sum is infinite and the result zero."""
+    hidden, conv_dim = DK, 3 * DK
+    outs = []
+    for z in (FAR_GATES, np.full(DK, 20.0, dtype=np.float32)):
+        run = LayerRun(0xB2002D00 + tokens, 1, 1, width, K.DTYPE_F32, K.DTYPE_F32, tokens)
+        run.inp[:, conv_dim + 2:] = z
+        run.d_norm = torch.ones(DK, device=dev())
+        outs.append(to_numpy_f32(run.step(tokens)[0]).astype(np.float64))
+    got = outs[0] / outs[1] * 20.0
+    z = FAR_GATES.astype(np.float64)
+    with np.errstate(over="ignore", invalid="ignore", divide="ignore"):
+        want = np.where(z < -88.72, 0.0, z / (1.0 + np.exp(-z)))
+        got_error = np.abs(got / want - 1.0)
+    finite = np.isfinite(want) & (want != 0.0)
+    assert (got_error[:, finite] <= 7 * 2.0 ** -23).all(), got_error[:, finite].max()
+    assert (got[:, want == 0.0] == 0.0).all()
+    assert np.isinf(got[:, np.isinf(want)]).all() and np.isnan(got[:, np.isnan(want)]).all()
+
+
+@pytest.mark.parametrize("tokens,width", [(1, 4), (5, 4), (3, 3)])
+@pytest.mark.parametrize("b", [-87.0, -87.5, -88.5])
+def test_layer_write_strength_near_the_smallest_float(tokens, width, b):
+    """A sigmoid of 1.6e-38 and below puts subnormal numbers into a zero state; a few units of the last place (2^-149) for
+    e^x of two ulp (4.6 units of a result of 2^-126), the product with the value and the sum over the tokens."""
+    run = LayerRun(0xB2002D80 + tokens, 1, 1, width, K.DTYPE_F32, K.DTYPE_F32, tokens)
+    run.inp[:, 3 * DK] = b
+    run.rs[:] = 0.0
+    run.d_rs = torch.zeros_like(run.d_rs)
+    run.step(tokens)
+    want = run.rs.reshape(-1).astype(np.float64)
+    got = to_numpy_f32(run.d_rs).reshape(-1).astype(np.float64)
+    assert np.abs(want).max() >= 2.0 ** -135
+    assert np.abs(got - want).max() <= 8 * tokens * 2.0 ** -149, np.abs(got - want).max() / 2.0 ** -149
+
+
 def layer_in_64_bits(inp, conv_w, rec_a, dt_bias, norm_w, conv_state, rec_state):
     """A layer call of HK and HV heads in plain torch: (output, state)."""
     inp, conv_w, rec_a, dt_bias, norm_w, conv_state, state = (
