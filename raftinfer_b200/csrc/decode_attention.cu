@@ -100,9 +100,9 @@ constexpr int kExchangeValues = kGroup * kHeadDim * 4;
 constexpr int kExchangeBytes = kExchangeValues + kGroup * 8 + 16;
 constexpr float kLog2e = 1.4426950408889634F;
 // Rows of K and of V that a CTA asks for ahead of its turn: 64 MB over the whole grid, half of L2, and at most 128 a
-// CTA.  Eight layers at 32K (512 CTAs): 258 us without, 251 with 64 rows, 242 with 128, 262 with 256 (L2 then loses what
-// it was asked for); two layers at 128K (2048 CTAs): 192 us without, 196 with 128, 234 with 256, and 192 to 194 with the 32
-// that the rule leaves there.
+// CTA, or its whole share of a partition (64 to 256 rows) where a cluster has one.  Eight layers at 32K (512 CTAs): 258 us
+// without, 251 with 64 rows, 242 with 128, 262 with 256 (L2 then loses what it was asked for); two layers at 128K (2048 CTAs):
+// 192 us without, 196 with 128, 234 with 256, and 192 to 194 with the 32 that the rule leaves there.
 constexpr std::uint32_t kPrefetchGridRows = 65536U;
 constexpr std::uint32_t kPrefetchMaxRows = 128U;
 constexpr std::uint32_t kPrefetchPiece = 32U; // rows per instruction
@@ -965,11 +965,13 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
 // each warp's chain of dependent steps is short.  All shapes are the same kernel template.
 //
 // Single sequences whose grid would leave most of the GPU idle share a partition among the CTAs of a cluster: 256 KB of rows
-// through one SM are 3 us.  Four CTAs while they fit beside one another (contexts up to 2304 tokens), two up to 4608; each
-// takes its part of the rows with four warps, and what it has found out about a query head goes to the CTA that owns the
-// head, in stores counted on an mbarrier there, so that the split-k partials are those of whole partitions.  Prologue and
-// step of a layer in a replayed token, with and without: 300 tokens 9.2 and 11.1 us, 777 9.2 and 11.4, 2000 9.5 and 11.8, 4000
-// 11.0 and 11.5; the executor's five launches at 777 12.3 and 14.9.
+// through one SM are 3 us.  Four CTAs a partition while the grid's four times as many fit beside one another, an SM each (at
+// most 9 partitions), two up to 18.  The grid is what the plan provides for and not the context: planned lengths are powers of
+// two up to the cache's size, so 2100 tokens in a cache of 4096 have two CTAs a partition, and the entry point without a
+// plan goes by its cache alone.  Each CTA takes its part of the rows with four warps, and what it has found out about a query
+// head goes to the CTA that owns the head, in stores counted on an mbarrier there, so that the split-k partials are those of
+// whole partitions.  Prologue and step of a layer in a replayed token, with and without: 300 tokens 9.2 and 11.1 us, 777 9.2
+// and 11.4, 2000 9.5 and 11.8, 4000 11.0 and 11.5; the executor's five launches at 777 12.3 and 14.9.
 //
 // A batch takes four warps a CTA from 149 CTAs on: its grid spans the longest cache, so many CTAs are empty, and four
 // warps finish a partition in a quarter of the steps.  The attention call alone behind a flushed L2, against one warp a CTA:

@@ -764,10 +764,15 @@ __global__ void __launch_bounds__(kStepThreads) gdn_layer_step_kernel(const Laye
 //                 A head with a decay above 1 (a positive coefficient) goes token by token: a product of its decays may be
 //                 infinite where each decay is finite and what it multiplies is zero or small.
 //   output norm   the slices of a head exchange their sums of squares.
-// Replayed calls (BF16), this form and the one before it (a warp per four columns, a token at a time, clusters of eight): 2
-// tokens 8.4 and 10.4 us, 17 14.4 and 18.6, 32 17 and 28.5, 48 22.7 and 39, 63 28 and 47.3.  At 63 tokens 44 k cycles: loads
-// 5 k, convolution 5.5 k, norms 4.4 k, recurrence 26 k - a group takes 1650 cycles of the 1400 that its instructions need
-// with two warps a scheduler - and the output 3 k.
+// 24 layers' calls replayed, a call, BF16 and FP32: 2 tokens 6.2 and 6.4 us, 4 6.4 and 6.5, 17 11.2 and 11.3, 32 15.2 and 15.3,
+// 63 27.1 and 26.4; a token at a time, a warp per four columns in clusters of eight: 7.8, 8.7, 17.2, 25.5 and 26.6, 48.4 and
+// 49.2.  At 63 tokens its 64 SMs issue in 56 % of the cycles; a warp's 5.1 cycles between instructions are 1.2 at barriers,
+// 0.8 for want of an issue slot, 0.7 waiting for memory.  A wait in front of the loop over groups in place of the one inside
+// its first turn gains 0.8 us at 63 tokens and costs 0.25 at 2 to 4, which every prompt ends with.  FP32, distance from 64 bits
+// at 63 tokens: output 1.68e-7, state 2.03e-7; a token at a time 1.72e-7 and 2.10e-7.
+//
+// The line to the chunks is one of accuracy: 64 tokens take 18.3 us (FP32 19.3) in chunks and would take 27.1 (26.5) here, but
+// products of chunks have ten-bit mantissas, which leave the state 4.5e-4 from 64 bits.
 constexpr std::uint32_t kShortMaxTokens = 63;
 constexpr std::uint32_t kShortRows = 64;
 constexpr std::uint32_t kShortGroup = 4;

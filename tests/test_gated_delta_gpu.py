@@ -298,7 +298,7 @@ def test_layer_single_tokens(hk, hv, dtype, wdtype):
 @pytest.mark.parametrize("hk,hv", [(1, 1), (2, 4), (1, 3)])
 @pytest.mark.parametrize("dtype,wdtype", [(K.DTYPE_BF16, K.DTYPE_BF16), (K.DTYPE_F32, K.DTYPE_F32)])
 def test_layer_short_calls(calls, hk, hv, dtype, wdtype):
-    """Calls of 2 to 63 tokens, either side of the 32-token tile, each on the states the one before left: one launch
+    """Calls of 2 to 63 tokens, whole groups of four and ragged ones, each on the states the one before left: one launch
     where a key head has one or two value heads, the general path for three."""
     run = LayerRun(0xB2002900 + 8 * hk + hv, hk, hv, 4, dtype, wdtype, sum(calls))
     for tokens in calls:
