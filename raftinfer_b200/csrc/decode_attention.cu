@@ -79,7 +79,7 @@ __host__ __device__ constexpr std::uint32_t row_offset(std::uint32_t row) { // b
 }
 constexpr int kMergePitch = kHeadDim + 8;              // floats per (warp, head) row of the merge area
 constexpr long long kWaitLimitCycles = 1LL << 28;      // SM cycles an mbarrier wait may take before giving up
-// ... and the wait for the other CTAs of a cluster, each of which may have waited that long for its rows first
+// ... and the wait for the other CTAs of a cluster, each of which may have waited twice that long for its rows first
 constexpr long long kExchangeLimitCycles = 4 * kWaitLimitCycles;
 
 // Shape of one CTA: `Warps` warps, each with a private ring of `Slots` slots (K and V slots alternate).
@@ -474,8 +474,16 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
     }
   };
 
-  // Consumer side of slot n.  Returns false when the wait ran out.
+  // Consumer side of slot n.  Returns false when the wait ran out; what has been issued by then is on its way still.
   bool healthy = true;
+  auto drain = [&](std::uint32_t n) { // from slot n on, as far as the ring reaches
+    const long long started = clock64();
+    for (std::uint32_t m = n; m < min(n + kRingSlots, my_slots); ++m) {
+      while (!mbarrier_try_wait(bars + (m % kRingSlots) * 8, (m / kRingSlots) & 1U) &&
+             clock64() - started <= kWaitLimitCycles) {
+      }
+    }
+  };
   auto wait_slot = [&](std::uint32_t n) {
     const std::uint32_t bar = bars + (n % kRingSlots) * 8;
     const std::uint32_t parity = (n / kRingSlots) & 1U;
@@ -594,6 +602,7 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
       issue(2 * i + kRingSlots - 1);
     }
     if (!wait_slot(2 * i)) {
+      drain(2 * i);
       break;
     }
     fix_rows(2 * i, tok0);
@@ -666,6 +675,7 @@ __global__ void __launch_bounds__(T::kWarps * 32, T::kCtasPerSm) decode_partitio
       issue(2 * i + kRingSlots);
     }
     if (!wait_slot(2 * i + 1)) {
+      drain(2 * i + 1);
       break;
     }
     fix_rows(2 * i + 1, tok0);
